@@ -44,6 +44,18 @@ def attention_workspace(device: torch.device, batch: int, max_blocks: int, block
     return ws
 
 
+def layer_step_workspace(device: torch.device, batch: int, max_blocks: int, block_size: int,
+                         heads: int, head_size: int, hidden: int, dtype: torch.dtype) -> torch.Tensor:
+    """The same per-device scratch tensor, large enough for ``decode_layer_step``."""
+    need = N.lib().aps_decode_layer_step_workspace_bytes(batch, max_blocks, block_size, heads, head_size,
+                                                         hidden, N.DTYPE_ENUM[dtype])
+    ws = _workspaces.get(device)
+    if ws is None or ws.numel() < need:
+        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
+        _workspaces[device] = ws
+    return ws
+
+
 def attention_status(workspace: torch.Tensor) -> int:
     """Status word left by the last attention call that used ``workspace``
     (0 = fine).  Synchronises the current stream."""
@@ -199,7 +211,9 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
     cache writes -- ``hidden_states[r]`` into the hidden cache for hidden-cached requests
     (aptserve_opt.py:108-109), ``new_key[r]`` / ``new_value[r]`` into the K/V planes for
     K/V-cached requests (aptserve_flash_attn.py:338-345, 363-373) -- addressed from the
-    private block tables, then ``hybrid_decode_attention`` over the batch.  ``new_key`` /
+    private block tables, then the attention of ``hybrid_decode_attention`` over the batch: hidden-cached
+    requests are attended directly, with the projections moved to the query and the output, or re-projected
+    when the batch is at most one wave of that kernel (the results agree to rounding).  ``new_key`` /
     ``new_value``: ``[B, H*D]`` (or ``[B, H, D]``) with any row stride; rows of requests of
     the other cache type are ignored.  ``None`` skips that kind of write."""
     dev = N.require_cuda(query, hidden_states, new_key, new_value, kv_cache, hidden_cache, w_k, b_k,
@@ -235,7 +249,7 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
     sl = _i32(seq_lens, "seq_lens")
     ct = _i32(cache_type, "cache_type")
     if workspace is None:
-        workspace = attention_workspace(dev, b, bt.shape[1], bs, h, d)
+        workspace = layer_step_workspace(dev, b, bt.shape[1], bs, h, d, e, query.dtype)
     with torch.cuda.device(dev):
         N.check(N.lib().aps_decode_layer_step(
             N.ptr(out), N.ptr(query), N.ptr(hidden_states), N.ptr(new_key), N.ptr(new_value),

@@ -123,7 +123,14 @@ int launch_kv_attention(const WorkspacePtrs& ws, const void* query, const void* 
                         const void* value_cache, const int32_t* block_tables,
                         const int32_t* seq_lens, const AttnShape& s, cudaStream_t stream);
 
-int launch_combine(const WorkspacePtrs& ws, void* out, const int32_t* seq_lens,
+// Projected outputs of hidden-cached requests for the combine step: part[split][slot][H * D] with
+// slot = hid_slot[request] (-1: K/V-cached), added over the splits and to b_v.
+struct HiddenOutputs {
+  const int* hid_slot; const float* part; const void* b_v; const int32_t* seq_lens;
+  int splits, slots;
+};
+// hidden may be NULL: every request's output is then merged from its softmax partials.
+int launch_combine(const WorkspacePtrs& ws, void* out, const HiddenOutputs* hidden,
                    const AttnShape& s, cudaStream_t stream);
 
 bool kv_attention_supported(int dtype, int head_size);
@@ -169,5 +176,13 @@ int launch_new_token_write(const NewTokenWrite& a, cudaStream_t stream);
 
 int check_hybrid_call(const char* op, const HybridCall& c);
 int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t stream);
+
+// The same attention with the projections of hidden-cached requests moved to the query and the
+// output (hidden_attention.cu).
+constexpr int kGroup = 256;   // hidden requests per pass (bounds the scratch)
+bool folded_supported(int dtype, int heads, int head_size, int hidden);
+size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
+                              int hidden, int dtype);
+int enqueue_folded_attention(const HybridCall& c, cudaStream_t stream);
 
 }  // namespace aps

@@ -14,6 +14,31 @@
 
 using namespace aps;
 
+namespace {
+
+// Which form of the hidden path a step takes, from what the host knows: the hidden rows are attended
+// directly (hidden_attention.cu) unless the whole batch, at the longest its block tables allow, is
+// one wave of tile pairs of the re-projection kernel.  One wave costs E / 64 slabs of 520 cycles: 1 us for a
+// 256-wide layer, 22 us for an OPT-13B layer, 40 us at E = 9216, in one launch against five; both forms
+// read W_k and W_v once (16 us for an OPT-13B layer).  The next size up, two waves, is where they meet: one
+// request of 611 tokens of an OPT-13B layer takes 96 us a call in either form (65 us of it the two waves),
+// and every further wave adds to the re-projection only.
+bool folded_shape(int batch, int max_blocks, int block_size, int heads, int head_size, int hidden, int dtype) {
+  if (!folded_supported(dtype, heads, head_size, hidden)) return false;
+  const int64_t pairs = ((int64_t)batch * max_blocks * block_size + 255) / 256;
+  const int64_t items = pairs * (((int64_t)heads * head_size + 127) / 128);
+  return items > sm_count() / 2 || (heads * head_size) % 128 != 0;
+}
+
+bool use_folded(const HybridCall& c) {
+  const AttnShape& s = c.shape;
+  return folded_shape(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size, s.dtype) &&
+         c.workspace_bytes >= folded_workspace_bytes(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size,
+                                                     c.hidden_size, s.dtype);
+}
+
+}  // namespace
+
 extern "C" int aps_decode_layer_step(void* out, const void* query, const void* hidden_states,
                                      const void* new_key, const void* new_value, void* key_cache,
                                      void* value_cache, void* hidden_cache, const void* w_k,
@@ -50,5 +75,13 @@ extern "C" int aps_decode_layer_step(void* out, const void* query, const void* h
                    num_heads, head_size, hidden_size, hidden_states_stride, new_key_stride,
                    new_value_stride, block_stride, hidden_row_stride, dtype};
   if ((st = launch_new_token_write(nw, cs)) != APS_OK) return st;
+  if (use_folded(c)) return enqueue_folded_attention(c, cs);
   return enqueue_hybrid_attention(c, cs);
+}
+
+extern "C" size_t aps_decode_layer_step_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
+                                                        int num_heads, int head_size, int hidden_size, int dtype) {
+  const size_t base = aps_attention_workspace_bytes(batch, max_blocks_per_seq, block_size, num_heads, head_size);
+  if (base == 0 || !folded_shape(batch, max_blocks_per_seq, block_size, num_heads, head_size, hidden_size, dtype)) return base;
+  return folded_workspace_bytes(batch, max_blocks_per_seq, block_size, num_heads, head_size, hidden_size, dtype);
 }

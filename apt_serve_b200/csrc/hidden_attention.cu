@@ -1,0 +1,1171 @@
+// Hidden-path decode attention with the K / V projections moved to the query and to the output.
+//
+// What it replaces in the reference (paths under additional_designs/):
+//   model_executor/models/aptserve_opt.py:111-124   gather of every cached hidden row and the
+//       kv_only projection of all of them (model_executor/layers/aptserve_linear.py:123-130);
+//   attention/backends/aptserve_flash_attn.py:356-387, :462-473   scatter of the projected K / V and
+//       the paged attention over them.
+//
+// For a hidden-cached request with cached rows x_t and head h,
+//     q . (W_k,h x_t + b_k) = (W_k,h^T q) . x_t + const        (the constant leaves the softmax)
+//     sum_t p_t (W_v,h x_t + b_v) = W_v,h (sum_t p_t x_t) + b_v
+// so the rows are attended as they are, with K = V = X and a head dimension of E.  Re-projecting T
+// rows costs 4 T E H D operations; this form costs 4 E H (D + T): D times less for long contexts.
+// What is left is bound by memory: the rows are read twice (scores, weighted sums) and W_k, W_v once.
+// Measured on one B200: a step of 256 requests of an OPT-13B layer, half of them hidden-cached (94.7k rows),
+// 0.91 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
+// requests, 0.53 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.25 ms against 2.5.
+//
+//   fold_kernel      qt[r][h] = W_k,h^T q[r][h]                       tcgen05, M = 128 columns of E
+//   scores_kernel    s[t][h] = x_t . qt[r][h]                         tcgen05, M = 128 tokens
+//   softmax_kernel   p[t][h] = 2^(scale s - max)                      one warp per (request, head)
+//   sum_kernel       z[r][h] = sum_t p[t][h] x_t / sum_t p[t][h]      tcgen05, M = 128 columns of E
+//   unfold_kernel    y[r][h] = W_v,h z[r][h]                          tcgen05, M = 128 rows of W_v
+// and the combine kernel adds b_v.
+//
+// Precision.  x, W and q are used as they are stored.  The three intermediates that meet a tensor-core
+// operand (qt, p, z) are fp32 values carried as a sum of 16-bit TERMS (value = hi + rest, rest again
+// rounded): two for fp16 (22 bits), three for bf16 (24 bits), each multiplied separately into the same
+// fp32 accumulator.  fp16 has a narrow exponent, so q is normalised by a power of two before it is folded
+// (|q| < 2, undone in the softmax) and p is kept at 2^15 times its value (undone by the
+// normalisation); both then sit well inside the range and the second term keeps its bits.
+//
+// Requests are taken in groups of at most kGroup, so that the scratch (qt, z: kGroup x H x E terms)
+// does not grow with the batch; inside a group they are sorted by length, longest first.
+//
+// Every mbarrier wait is bounded by a clock budget; a wait that runs out records a code in the plan's
+// status word, tells the other warps through shared memory, and the CTA drains and returns.
+
+#include "attention_common.cuh"
+#include "sm100.cuh"
+#include "tensor_maps.cuh"
+
+#include <type_traits>
+
+namespace aps {
+namespace {
+
+constexpr int kTile = 256;                // tokens per scores tile: two M128 accumulators share a qt slab
+constexpr int kSubs = kTile / 16;         // 16-row boxes of the hidden cache per tile
+constexpr int kTileCost = 4;              // fixed cost of a tile in boxes (its qt slab), for the work split
+constexpr int kStepTokens = 32;           // tokens per stage of the sum kernel
+constexpr int kMinPiece = 4 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: four full slabs
+constexpr int kMaxGrid = 256;             // largest grid of the scores kernel the plan keeps bounds for
+constexpr int kMaxSlice = 8;              // 128-column blocks of E per work item of the sum kernel
+constexpr float kProbShift = 15.f;        // p is kept at 2^15 times its value (fp16 range)
+constexpr size_t kRingBytes = 200 * 1024; // shared memory of the operand rings
+
+template <typename T> constexpr int kTerms = std::is_same<T, __nv_bfloat16>::value ? 3 : 2;
+template <typename T> constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+
+// ---- the plan of one group of hidden requests (device memory) --------------------------
+struct GroupPlan {
+  int n;                      // requests of the group
+  int n_tiles;                // scores tiles
+  int weight;                 // total cost of the tiles, in boxes
+  int slice;                  // 128-column blocks per item of the sum kernel
+  int pieces;                 // CTAs the scores work is cut for
+  int req[kGroup];            // batch row of each request, longest first
+  int len[kGroup];            // its length in tokens
+  int tile_off[kGroup + 1];   // first scores tile
+  int blk_off[kGroup + 1];    // first 16-token block of p
+  int w_off[kGroup + 1];      // cost of the tiles before it
+  int bound_tile[kMaxGrid + 1];   // scores work of CTA c: from (bound_tile[c], bound_slab[c]) to the next bound
+  int bound_slab[kMaxGrid + 1];
+};
+
+struct Params {
+  const GroupPlan* plan;
+  const void* query; const void* b_k; const int32_t* block_tables;
+  void* qt;              // [request][term][head][E]
+  float* qscale;         // [request][head] scale * log2(e) / (power of two q was multiplied with)
+  float* scores;         // [tile + CTA][head][kTile] partial scores over a range of E
+  void* probs;           // [16-token block][term][K half][heads padded][8 tokens]
+  float* inv_sum;        // [request][head]
+  void* z;               // [term][head][request capacity][E]
+  float* out_part;       // [split][hidden request][H * D]
+  int* status;
+  int heads, np, head_size, hidden, slabs;   // np: heads padded to a multiple of 16; slabs: E / 64
+  int block_size, max_blocks, n_cap;         // n_cap: requests a group can hold here
+  int group_first;                           // ordinal of the group's first hidden request
+  int n_hidden_cap, splits, stages, grid_scores;
+  int w_box_rows;                            // rows of a W_v box: 128, fewer when W_v has fewer
+  int64_t query_stride;
+  float scale_log2;
+};
+
+template <typename T>
+__device__ __forceinline__ void split_terms(float v, T (&t)[kTerms<T>]) {
+#pragma unroll
+  for (int i = 0; i < kTerms<T>; ++i) {
+    t[i] = Elem<T>::from_float(v);
+    v -= Elem<T>::to_float(t[i]);
+  }
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack_pair(T a, T b) {
+  return (uint32_t)reinterpret_cast<const unsigned short&>(a) | ((uint32_t)reinterpret_cast<const unsigned short&>(b) << 16);
+}
+// Two columns a, b of an accumulator whose rows are the lanes: lane pairs exchange values so that
+// an even lane returns (row, row + 1) of column a and an odd lane (row - 1, row) of column b.
+__device__ __forceinline__ float2 pair_rows(float a, float b, int lane) {
+  const bool odd = (lane & 1) != 0;
+  const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+  return odd ? make_float2(got, b) : make_float2(a, got);
+}
+
+// Copies still in flight get a bounded time to land before the CTA's shared memory is released.
+__device__ __forceinline__ void drain() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 2000000LL) { }
+}
+
+// ---- plan ---------------------------------------------------------------------------
+// One CTA.  K/V-cached requests: the chunk list of the K/V kernel and the partial slots.  Hidden-cached
+// requests: the groups.  Runs of requests per thread, warp-shuffle scans.
+constexpr int kPlanThreads = 1024;
+
+__device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int2& total) {
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) { v.x += x; v.y += y; }
+  }
+  if (lane == 31) warp_sums[warp] = v;
+  __syncthreads();
+  int2 s = warp_sums[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, s.x, o), y = __shfl_up_sync(0xffffffffu, s.y, o);
+    if (lane >= o) { s.x += x; s.y += y; }
+  }
+  total.x = __shfl_sync(0xffffffffu, s.x, 31);
+  total.y = __shfl_sync(0xffffffffu, s.y, 31);
+  const int bx = __shfl_sync(0xffffffffu, s.x, warp > 0 ? warp - 1 : 0);
+  const int by = __shfl_sync(0xffffffffu, s.y, warp > 0 ? warp - 1 : 0);
+  if (warp > 0) { v.x += bx; v.y += by; }
+  return v;   // inclusive
+}
+
+struct PlanArgs {
+  int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
+  const int32_t* seq_lens; const int32_t* cache_type;
+  int batch, max_tokens, kv_present, n_groups, slabs, grid_scores, e_blocks, max_slice, item_target;
+};
+
+__global__ void __launch_bounds__(kPlanThreads)
+step_plan_kernel(const PlanArgs a) {
+  __shared__ int2 warp_sums[32];
+  __shared__ int s_missing;
+  __shared__ int s_req[kGroup], s_len[kGroup], s_toff[kGroup + 1], s_woff[kGroup + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_missing = 0;
+  __syncthreads();
+  const int per = (a.batch + kPlanThreads - 1) / kPlanThreads;
+  const int r0 = min(a.batch, tid * per), r1 = min(a.batch, r0 + per);
+  auto chunks_of = [&](int s) { return a.kv_present ? (s + kChunkTokens - 1) / kChunkTokens : 0; };
+  int2 mine = make_int2(0, 0);
+  for (int r = r0; r < r1; ++r) {
+    const int s = max(0, min(a.seq_lens[r], a.max_tokens));
+    if (a.cache_type[r] != 0) ++mine.y;
+    else { mine.x += chunks_of(s); if (!a.kv_present) s_missing = 1; }
+  }
+  int2 total;
+  const int2 inc = block_scan(mine, warp_sums, tid, total);
+  int o_kv = inc.x - mine.x, o_hid = inc.y - mine.y;
+  for (int r = r0; r < r1; ++r) {
+    const int s = max(0, min(a.seq_lens[r], a.max_tokens));
+    a.part_offset[r] = o_kv;
+    if (a.cache_type[r] != 0) {
+      a.hid_list[o_hid++] = make_int2(r, s);
+    } else {
+      a.hid_slot[r] = -1;
+      const int c = chunks_of(s);
+      for (int j = 0; j < c; ++j) a.kv_chunks[o_kv + j] = make_int2(r, j);
+      o_kv += c;
+    }
+  }
+  if (tid == 0) {
+    a.part_offset[a.batch] = total.x;
+    a.plan[kPlanNumKvChunks] = total.x;
+    a.plan[kPlanKvCounter] = 0;
+    a.plan[kPlanStatus] = s_missing ? kStatusNoKvCache : kStatusOk;
+  }
+  if (tid >= kPlanStatsWord && tid < kPlanStatsWord + 18) a.plan[tid] = 0;
+  for (int g = 0; g < a.n_groups; ++g) {
+    __syncthreads();   // hid_list is complete; the shared arrays are free
+    GroupPlan* gp = a.groups + g;
+    const int n = max(0, min(kGroup, total.y - g * kGroup));
+    if (n == 0) {
+      if (tid == 0) { gp->n = 0; gp->n_tiles = 0; }
+      continue;
+    }
+    // sort by length, longest first: rank = requests that come before (four threads per request)
+    const int i = tid >> 2, part = tid & 3;
+    int2 rec = make_int2(0, -1);
+    if (i < n) rec = a.hid_list[g * kGroup + i];
+    if (part == 0) s_len[i] = rec.y;
+    __syncthreads();
+    int rank = 0;
+    for (int j = part; j < n; j += 4) {
+      const int l = s_len[j];
+      rank += l > rec.y || (l == rec.y && j < i);
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+    __syncthreads();
+    if (i < n && part == 0) {
+      s_req[rank] = rec.x; s_len[rank] = rec.y;
+      gp->req[rank] = rec.x; gp->len[rank] = rec.y;
+      a.hid_slot[rec.x] = g * kGroup + rank;
+    }
+    __syncthreads();
+    if (warp == 0) {   // prefix sums over the sorted requests, eight per lane
+      int t8 = 0, b8 = 0, w8 = 0;
+      for (int k = 0; k < kGroup / 32; ++k) {
+        const int s = lane * (kGroup / 32) + k;
+        if (s >= n) break;
+        const int blocks = (s_len[s] + 15) / 16, tiles = (blocks + kSubs - 1) / kSubs;
+        t8 += tiles; b8 += blocks; w8 += blocks + tiles * kTileCost;
+      }
+      int ti = t8, bi = b8, wi = w8;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, ti, o), y = __shfl_up_sync(0xffffffffu, bi, o),
+                  z = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane >= o) { ti += x; bi += y; wi += z; }
+      }
+      int to = ti - t8, bo = bi - b8, wo = wi - w8;
+      for (int k = 0; k < kGroup / 32; ++k) {
+        const int s = lane * (kGroup / 32) + k;
+        if (s > n) break;
+        s_toff[s] = to; s_woff[s] = wo;
+        gp->tile_off[s] = to; gp->blk_off[s] = bo; gp->w_off[s] = wo;
+        if (s == n) break;
+        const int blocks = (s_len[s] + 15) / 16, tiles = (blocks + kSubs - 1) / kSubs;
+        to += tiles; bo += blocks; wo += blocks + tiles * kTileCost;
+      }
+      if (lane == 31 && n == kGroup) {
+        s_toff[n] = to; s_woff[n] = wo;
+        gp->tile_off[n] = to; gp->blk_off[n] = bo; gp->w_off[n] = wo;
+      }
+    }
+    __syncthreads();
+    const int n_tiles = s_toff[n], weight = s_woff[n];
+    if (tid == 0) {
+      // sum kernel: the widest slice of E that still gives item_target items
+      int slice = a.max_slice;
+      while (slice > 1 && n * ((a.e_blocks + slice - 1) / slice) < a.item_target) --slice;
+      gp->n = n; gp->n_tiles = n_tiles; gp->weight = weight; gp->slice = slice;
+    }
+    // scores kernel: piece c starts at cost c / pieces of the total, rounded down to a slab of a tile.  No
+    // piece is smaller than kMinPiece (more than a full slab), so that none is empty and the partial
+    // sums of a tile stay few.
+    const int pieces = (int)max((int64_t)1, min((int64_t)a.grid_scores, (int64_t)weight * a.slabs / kMinPiece));
+    if (tid == 0) gp->pieces = pieces;
+    if (tid <= a.grid_scores) {
+      int t = n_tiles, slab = 0;
+      if (tid < pieces && weight > 0) {
+        const int64_t pos = (int64_t)tid * weight * a.slabs / pieces;
+        int lo = 0, hi = n;   // last request whose cost offset is <= pos
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((int64_t)s_woff[mid] * a.slabs <= pos) lo = mid; else hi = mid; }
+        const int64_t rem = pos - (int64_t)s_woff[lo] * a.slabs;
+        const int blocks = (s_len[lo] + 15) / 16, tiles = (blocks + kSubs - 1) / kSubs;
+        const int k = min((int)(rem / ((int64_t)(kSubs + kTileCost) * a.slabs)), tiles - 1);
+        const int w = min(kSubs, blocks - k * kSubs) + kTileCost;
+        t = s_toff[lo] + k;
+        slab = (int)((rem - (int64_t)k * (kSubs + kTileCost) * a.slabs) / w);
+      }
+      gp->bound_tile[tid] = t; gp->bound_slab[tid] = slab;
+    }
+  }
+}
+
+// ---- fold ---------------------------------------------------------------------------
+// One CTA per (256 columns of E, head): D[column][request] = sum_d W_k,h[d][column] q[request][d], exact
+// 16-bit operands, fp32 accumulators.  W_k,h arrives as boxes of (64 columns, D rows), i.e. an MN-major A
+// operand; q is gathered by the threads into a K-major B operand, 128 requests at a time.
+constexpr int kFoldThreads = 128;
+constexpr int kFoldCols = 256;
+constexpr int kFoldReqs = 128;
+
+struct FoldAux {
+  uint64_t w_full, mma_done;
+  uint32_t tmem_base;
+  int abort_flag;
+  int req[kFoldReqs];
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kFoldThreads)
+fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
+  constexpr int NT = kTerms<T>;
+  constexpr int kQSlab = kFoldReqs * 128;                 // 64 elements of D for 128 requests
+  constexpr int kQSlabs = (D + 63) / 64;
+  constexpr uint32_t kBox = D * 128;                      // 64 columns of E x D rows
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;
+  const uint32_t w_at = base, q_at = base + 4 * kBox;
+  __shared__ FoldAux aux;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = p.plan->n;
+  if (n == 0) return;
+  const int head = blockIdx.y, col0 = blockIdx.x * kFoldCols;
+  volatile int* abort_flag = &aux.abort_flag;
+  if (threadIdx.x == 0) {
+    mbar_init(&aux.w_full, 1);
+    mbar_init(&aux.mma_done, 1);
+    aux.abort_flag = 0;
+    mbar_init_fence();
+    mbar_expect_tx_addr(smem_u32(&aux.w_full), 4 * kBox);
+    for (int b = 0; b < 4; ++b) tma_load_2d_cta(w_at + b * kBox, &map_w, smem_u32(&aux.w_full), col0 + b * 64, head * D);
+  }
+  if (warp == 1) tmem_alloc(&aux.tmem_base, 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = aux.tmem_base;
+  const T* query = static_cast<const T*>(p.query);
+  T* qt = static_cast<T*>(p.qt);
+  bool ok = true;
+  uint32_t parity = 0;
+  for (int r0 = 0; r0 < n && ok; r0 += kFoldReqs) {
+    const int m = min(kFoldReqs, n - r0), np = (m + 15) & ~15;
+    // ---- stage q: warp w takes requests w, w + 4, ...; lane l elements l * D / 32 ... ----
+    constexpr int EPL = D / 32;   // elements per lane: 4, 2 or 1
+    for (int r = warp; r < np; r += 4 * 8) {
+      T v[8][EPL];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int rr = r + u * 4;
+        const bool in = rr < m;
+        const T* src = query + (in ? (int64_t)p.plan->req[r0 + rr] * p.query_stride + head * D + lane * EPL : 0);
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) v[u][e] = in ? src[e] : Elem<T>::from_float(0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int rr = r + u * 4;
+        if (rr >= np) break;
+        float f[EPL], mx = 0.f;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) { f[e] = Elem<T>::to_float(v[u][e]); mx = fmaxf(mx, fabsf(f[e])); }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        // power of two that brings max |q| into [1, 2); zero, infinite and NaN rows stay as they are
+        int k = 0;
+        if (mx > 0.f && mx < INFINITY) k = max(-100, min(100, (int)((__float_as_uint(mx) >> 23) & 0xff) - 127));
+        const float up = __uint_as_float((uint32_t)(127 - k) << 23), down = __uint_as_float((uint32_t)(127 + k) << 23);
+        unsigned short w[EPL];
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) { const T t = Elem<T>::from_float(f[e] * up); w[e] = reinterpret_cast<const unsigned short&>(t); }
+        const int el = lane * EPL, slab = el / 64, piece = (el % 64) / 8, in_piece = el % 8;
+        const uint32_t dst = q_at + slab * kQSlab + rr * 128 + ((piece ^ (rr & 7)) << 4) + in_piece * 2;
+        if constexpr (EPL == 4) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)), "r"((uint32_t)w[2] | ((uint32_t)w[3] << 16)) : "memory");
+        else if constexpr (EPL == 2) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)) : "memory");
+        else asm volatile("st.shared.b16 [%0], %1;" ::"r"(dst), "h"(w[0]) : "memory");
+        if (blockIdx.x == 0 && lane == 0 && rr < m) p.qscale[(int64_t)(r0 + rr) * p.heads + head] = p.scale_log2 * down;
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+      if (r0 == 0) ok = mbar_wait_warp(smem_u32(&aux.w_full), 0, abort_flag, p.status, 3, lane);
+      tc_fence_after();
+      if (ok && elect_one()) {
+        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
+#pragma unroll
+        for (int mb = 0; mb < 2; ++mb)
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks)
+            tc_mma_cta(tmem + mb * kFoldReqs, desc_lo(w_at + mb * 2 * kBox + ks * 2048, kBox), desc_hi(1024, true),
+                       desc_lo(q_at + (ks / 4) * kQSlab + (ks % 4) * 32, 16), desc_hi(1024, true), idesc, ks != 0);
+        tc_commit_cta(smem_u32(&aux.mma_done));
+      }
+      __syncwarp();
+    }
+    ok = mbar_wait_warp(smem_u32(&aux.mma_done), parity, abort_flag, p.status, 4, lane);
+    parity ^= 1u;
+    if (ok) {
+      tc_fence_after();
+      // lanes are columns of E, accumulator columns are requests
+#pragma unroll 1
+      for (int mb = 0; mb < 2; ++mb) {
+        const int col = col0 + mb * 128 + warp * 32 + lane;
+        if (col0 + mb * 128 >= p.hidden) break;
+#pragma unroll 1
+        for (int c = 0; c < m; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + mb * kFoldReqs + c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
+            const int r = c + j + (lane & 1);
+            if (r < m) {
+              T a[NT], b[NT];
+              split_terms<T>(f.x, a);
+              split_terms<T>(f.y, b);
+#pragma unroll
+              for (int t = 0; t < NT; ++t)
+                *reinterpret_cast<uint32_t*>(qt + (((int64_t)(r0 + r) * NT + t) * p.heads + head) * p.hidden + (col & ~1)) = pack_pair<T>(a[t], b[t]);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+    }
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;   // the accumulators and the q operand are free again
+    tc_fence_after();
+  }
+  if (!ok) drain();
+  __syncthreads();
+  if (warp == 1) tmem_free(tmem, 256);
+}
+
+// ---- scores -------------------------------------------------------------------------
+// D[token][head] = sum_e x[token][e] qt[head][e] for tiles of 256 tokens of one request (two M128
+// accumulators that share the qt slab).  The work is a line of (tile, 64-column slab) steps, cut into one
+// contiguous piece per CTA with equal numbers of boxes: a tile that straddles a cut leaves one partial sum
+// per piece (slot = tile + CTA), added by the softmax kernel, so that one long request uses the whole
+// chip and a large batch has no partly filled last wave.
+// Warps: 0 qt boxes and byte counts, 1 MMA issue, 2-5 epilogue, 6-9 boxes of the hidden cache (four
+// lanes each: one 16-row box per cache block and slab).
+constexpr int kScoresThreads = 320;
+constexpr int kMaxStages = 12;
+
+struct RingAux {
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+struct Ring {
+  uint32_t stage = 0, phase = 0;
+  __device__ __forceinline__ void step(int stages) { if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; } }
+};
+
+__host__ __device__ inline uint32_t scores_stage_bytes(int terms, int np) { return kTile * 128 + terms * np * 128; }
+
+template <typename T>
+__global__ void __launch_bounds__(kScoresThreads, 1)
+scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q, const Params p) {
+  constexpr int NT = kTerms<T>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
+  __shared__ RingAux aux;
+  __shared__ int s_toff[kGroup + 1], s_len[kGroup], s_req[kGroup];
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int n = p.plan->n, cta = blockIdx.x;
+  if (n == 0) return;
+  const int t0 = p.plan->bound_tile[cta], t1 = p.plan->bound_tile[cta + 1];
+  const int b0 = p.plan->bound_slab[cta], b1 = p.plan->bound_slab[cta + 1];
+  if (t0 == t1 && b0 == b1) return;
+  for (int i = threadIdx.x; i <= n; i += kScoresThreads) {
+    s_toff[i] = p.plan->tile_off[i];
+    if (i < n) { s_len[i] = p.plan->len[i]; s_req[i] = p.plan->req[i]; }
+  }
+  const int np = p.np, stages = p.stages;
+  const uint32_t stage_bytes = scores_stage_bytes(NT, np);
+  const int n_buf = 4 * np <= 512 ? 2 : 1;
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < (uint32_t)(n_buf * 2 * np)) tmem_cols <<= 1;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      // one arrival with the byte count (warp 0) and one per slab from each of the warps 6-9, boxes
+      // or not: a stage cannot be filled and freed twice while one of them still waits for it
+      mbar_init(&aux.full[s], 5);
+      mbar_init(&aux.empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
+    aux.abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) tmem_alloc(&aux.tmem_base, tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = aux.tmem_base;
+  volatile int* abort_flag = &aux.abort_flag;
+  const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
+  int slot = 0;   // request of tile t0
+  {
+    int lo = 0, hi = n;
+    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_toff[mid] <= t0) lo = mid; else hi = mid; }
+    slot = lo;
+  }
+  bool ok = true;
+  Ring rg;
+  uint32_t n_local = 0;
+  for (int t = t0; t <= t1 && ok; ++t) {
+    const int sa = t == t0 ? b0 : 0, sb = t == t1 ? b1 : p.slabs;
+    if (sa >= sb) continue;
+    while (t >= s_toff[slot + 1]) ++slot;
+    const int tok0 = (t - s_toff[slot]) * kTile;
+    const int n_sub = min(kSubs, (s_len[slot] - tok0 + 15) >> 4);
+    const uint32_t buf = n_local % n_buf, use = n_local / n_buf;
+    ++n_local;
+    if (warp == 0) {
+      const uint32_t tx = (uint32_t)(n_sub * 2048 + NT * p.heads * 128);
+      for (int s = sa; s < sb; ++s) {
+        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+        const uint32_t bar = full0 + rg.stage * 8;
+        if (lane == 0) mbar_expect_tx_addr(bar, tx);
+        __syncwarp();
+        if (lane < NT)
+          tma_load_2d_cta(ring + rg.stage * stage_bytes + kTile * 128 + lane * np * 128, &map_q, bar, s * 64, (slot * NT + lane) * p.heads);
+        rg.step(stages);
+      }
+    } else if (warp >= 6) {
+      const int sub = (warp - 6) * 4 + lane;
+      int row = 0;
+      const bool has = lane < 4 && sub < n_sub;
+      if (has) {
+        const int tok = tok0 + sub * 16;
+        row = p.block_tables[(int64_t)s_req[slot] * p.max_blocks + tok / p.block_size] * p.block_size + tok % p.block_size;
+      }
+      for (int s = sa; s < sb; ++s) {
+        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+        const uint32_t bar = full0 + rg.stage * 8;
+        if (has) tma_load_2d_cta(ring + rg.stage * stage_bytes + sub * 2048, &map_x, bar, s * 64, row);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_addr(bar);
+        rg.step(stages);
+      }
+    } else if (warp == 1) {
+      if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, false);
+      const int n_m = n_sub > 8 ? 2 : 1;
+      uint32_t acc = 0;
+      for (int s = sa; s < sb; ++s) {
+        if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t a_lo = desc_lo(ring + rg.stage * stage_bytes, 16), b_lo = a_lo + (kTile * 128 >> 4);
+          for (int m = 0; m < n_m; ++m) {
+            const uint32_t d = tmem + (buf * 2 + m) * np;
+            uint32_t first = acc;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+              for (int i = 0; i < NT; ++i) {
+                tc_mma_cta(d, a_lo + m * 1024 + k * 2, desc_hi(1024, true), b_lo + i * (np * 8) + k * 2, desc_hi(1024, true), idesc, first);
+                first = 1u;
+              }
+          }
+          tc_commit_cta(empty0 + rg.stage * 8);
+        }
+        __syncwarp();
+        acc = 1u;
+        rg.step(stages);
+      }
+      if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
+      __syncwarp();
+    } else {
+      const int quarter = warp & 3;
+      if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
+      tc_fence_after();
+      float* dst = p.scores + (int64_t)(t + cta) * p.heads * kTile;
+      const int n_m = n_sub > 8 ? 2 : 1;
+      for (int m = 0; m < n_m; ++m)
+        for (int h0 = 0; h0 < np; h0 += 16) {
+          uint32_t v[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * np + h0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[j]);
+        }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+    }
+  }
+  if (!ok) drain();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_free(tmem, tmem_cols); }
+}
+
+// ---- softmax ------------------------------------------------------------------------
+// One CTA per (request, head) at a time, one warp per tile.  A lane takes eight consecutive tokens of the
+// tile: it adds the tile's partial sums, and after the maximum is known writes the eight weights of each
+// term as one 16-byte piece of the sum kernel's B operand.  The scores of kHold tiles per warp stay in
+// registers (2048 tokens); those of longer requests are added up twice.
+constexpr int kSoftmaxWarps = 4;
+constexpr int kHold = 2;
+
+template <typename T>
+__global__ void __launch_bounds__(kSoftmaxWarps * 32)
+softmax_kernel(const Params p) {
+  constexpr int NT = kTerms<T>;
+  __shared__ float s_max[kSoftmaxWarps], s_sum[kSoftmaxWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const GroupPlan* gp = p.plan;
+  const int n_units = gp->n * p.heads, pieces = gp->pieces;
+  const int64_t work = (int64_t)gp->weight * p.slabs;
+  T* probs = static_cast<T*>(p.probs);
+  for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
+    const int slot = unit / p.heads, h = unit - slot * p.heads;
+    const int len = gp->len[slot];
+    const int tile0 = gp->tile_off[slot], n_tiles = gp->tile_off[slot + 1] - tile0;
+    const float scale = p.qscale[(int64_t)slot * p.heads + h];
+    const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot], w0 = gp->w_off[slot];
+    // scores of this lane's eight tokens of tile k
+    auto load = [&](int k, float (&s)[8]) {
+      // the pieces of the line of (tile, slab) steps that touch this tile: c0 is the last that starts at or
+      // before its first slab, c1 the last that starts at or before its last one
+      const int w = min(kSubs, n_blk - k * kSubs) + kTileCost;
+      const int64_t at = (int64_t)(w0 + k * (kSubs + kTileCost)) * p.slabs;
+      const int c0 = (int)(((at + w) * pieces - 1) / work);
+      const int c1 = min((int)(((at + (int64_t)w * p.slabs) * pieces - 1) / work), pieces - 1);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] = 0.f;
+      const float4* src = reinterpret_cast<const float4*>(p.scores + ((int64_t)(tile0 + k + c0) * p.heads + h) * kTile + lane * 8);
+#pragma unroll 4
+      for (int c = c0; c <= c1; ++c) {
+        const float4 x = src[0], y = src[1];
+        src += p.heads * (kTile / 4);
+        s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
+        s[4] += y.x; s[5] += y.y; s[6] += y.z; s[7] += y.w;
+      }
+      const int tok = k * kTile + lane * 8;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] = tok + e < len ? s[e] * scale : -INFINITY;
+    };
+    float held[kHold][8], mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kHold; ++j) {
+      const int k = warp + j * kSoftmaxWarps;
+      if (k < n_tiles) {
+        load(k, held[j]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mx = fmaxf(mx, held[j][e]);
+      }
+    }
+    for (int k = warp + kHold * kSoftmaxWarps; k < n_tiles; k += kSoftmaxWarps) {
+      float s[8];
+      load(k, s);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, s[e]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) s_max[warp] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kSoftmaxWarps; ++w) mx = fmaxf(mx, s_max[w]);
+    float sum = 0.f;
+    auto store = [&](int k, const float (&s)[8]) {
+      T terms[8][NT];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float w = exp2f(s[e] - mx + kProbShift);
+        sum += w;
+        split_terms<T>(w, terms[e]);
+      }
+      const int blk = k * kSubs + (lane >> 1);
+      if (blk < n_blk) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          uint4 v;
+          v.x = pack_pair<T>(terms[0][t], terms[1][t]); v.y = pack_pair<T>(terms[2][t], terms[3][t]);
+          v.z = pack_pair<T>(terms[4][t], terms[5][t]); v.w = pack_pair<T>(terms[6][t], terms[7][t]);
+          *reinterpret_cast<uint4*>(probs + ((((int64_t)(blk0 + blk) * NT + t) * 2 + (lane & 1)) * p.np + h) * 8) = v;
+        }
+      }
+    };
+#pragma unroll
+    for (int j = 0; j < kHold; ++j) {
+      const int k = warp + j * kSoftmaxWarps;
+      if (k < n_tiles) store(k, held[j]);
+    }
+    for (int k = warp + kHold * kSoftmaxWarps; k < n_tiles; k += kSoftmaxWarps) {
+      float s[8];
+      load(k, s);
+      store(k, s);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float total = 0.f;
+#pragma unroll
+      for (int w = 0; w < kSoftmaxWarps; ++w) total += s_sum[w];
+      p.inv_sum[(int64_t)slot * p.heads + h] = 1.f / total;
+    }
+  }
+}
+
+// ---- weighted sums ------------------------------------------------------------------
+// D[column of E][head] = sum_t x_t[column] p[t][head]: work item = (request, slice of up to kMaxSlice x 128
+// columns), the item's accumulators together in half of the tensor memory, so that the epilogue of one item
+// overlaps the next one's main loop.  Items in order of their length, dealt to the CTAs in snake order.
+// A stage holds 32 tokens: per 16-token cache block and 128 columns one box of (64 columns, 16 rows, 2) =
+// an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
+// K-major B operand).  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
+constexpr int kSumThreads = 192;
+
+__host__ __device__ inline uint32_t probs_block_bytes(int terms, int np) { return (uint32_t)terms * np * 32; }
+__host__ __device__ inline uint32_t sum_stage_bytes(int terms, int np, int slice) {
+  return 2u * slice * 4096 + ((2 * probs_block_bytes(terms, np) + 1023) & ~1023u);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads, 1)
+sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
+  constexpr int NT = kTerms<T>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
+  __shared__ RingAux aux;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const GroupPlan* gp = p.plan;
+  const int n = gp->n;
+  if (n == 0) return;
+  const int np = p.np, e_blocks = p.hidden / 128, slice = gp->slice;
+  const int n_slices = (e_blocks + slice - 1) / slice, n_items = n * n_slices;
+  if ((int)blockIdx.x >= n_items) return;
+  const uint32_t pblk = probs_block_bytes(NT, np), x_bytes = 2u * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
+  const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
+    aux.abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) tmem_alloc(&aux.tmem_base, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = aux.tmem_base;
+  volatile int* abort_flag = &aux.abort_flag;
+  const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
+  bool ok = true;
+  Ring rg;
+  uint32_t n_local = 0;
+  for (int round = 0; ok; ++round) {
+    const int g = gridDim.x;
+    const int item = round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    if (round * g >= n_items) break;
+    if (item >= n_items) continue;
+    const int slot = item / n_slices, first = (item % n_slices) * slice;
+    const int len = gp->len[slot];
+    if (len <= 0) continue;
+    const int n_col = min(slice, e_blocks - first);   // 128-column blocks of this item
+    const int n_blk = (len + 15) >> 4;
+    const uint32_t buf = n_local & 1u, use = n_local >> 1;
+    ++n_local;
+    if (warp == 0) {
+      const int32_t* bt = p.block_tables + (int64_t)gp->req[slot] * p.max_blocks;
+      const char* probs = static_cast<const char*>(p.probs) + (int64_t)gp->blk_off[slot] * pblk;
+      int rows = 0;
+      for (int b = 0; b < n_blk; b += 2) {
+        if ((b & 31) == 0) {   // first cache rows of the next 32 blocks
+          const int tok = (b + lane) * 16;
+          rows = b + lane < n_blk ? bt[tok / p.block_size] * p.block_size + tok % p.block_size : 0;
+        }
+        const int two = min(2, n_blk - b);
+        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+        const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
+        if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)two * (n_col * 4096 + pblk));
+        __syncwarp();
+        const int half = lane >= n_col ? 1 : 0, col = lane - half * n_col;
+        const int row = __shfl_sync(0xffffffffu, rows, (b & 31) + half);
+        if (lane < two * n_col) tma_load_3d_cta(dst + (half * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2);
+        if (lane >= 30 && lane - 30 < two)
+          bulk_load(dst + x_bytes + (lane - 30) * pblk, probs + (int64_t)(b + lane - 30) * pblk, pblk, bar);
+        __syncwarp();
+        rg.step(stages);
+      }
+    } else if (warp == 1) {
+      if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
+      for (int b = 0; b < n_blk; b += 2) {
+        const int two = min(2, n_blk - b);
+        if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+        const uint32_t x_at = ring + rg.stage * stage_bytes, p_at = x_at + x_bytes;
+        const int valid = len - (b + two - 1) * 16;   // tokens of the stage's last block
+        if (valid < 16) {
+          // rows past the sequence length hold whatever the cache block holds; their weights are zero,
+          // but zero times NaN is not
+          const uint32_t at = x_at + (two - 1) * slice * 4096;
+          const int pieces = (16 - valid) * 8;
+          for (int i = lane; i < pieces * 2 * n_col; i += 32) {
+            const int r = valid + (i % pieces) / 8, piece = i % 8, hc = i / pieces;
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + hc * 2048 + r * 128 + piece * 16), "r"(0u) : "memory");
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          for (int k = 0; k < two; ++k) {
+            const uint32_t acc = (b + k) != 0;
+            const uint32_t a_lo = desc_lo(x_at + k * slice * 4096, 2048), b_lo = desc_lo(p_at + k * pblk, (uint32_t)np * 16);
+            for (int col = 0; col < n_col; ++col)
+#pragma unroll
+              for (int i = 0; i < NT; ++i)
+                tc_mma_cta(tmem + buf * 256 + col * np, a_lo + col * 256, desc_hi(1024, true), b_lo + i * (np * 2),
+                           desc_hi(128, false), idesc, i == 0 ? acc : 1u);
+          }
+          tc_commit_cta(empty0 + rg.stage * 8);
+        }
+        __syncwarp();
+        rg.step(stages);
+      }
+      if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
+      __syncwarp();
+    } else {
+      const int quarter = warp & 3;
+      const float* inv = p.inv_sum + (int64_t)slot * p.heads;
+      T* z = static_cast<T*>(p.z);
+      if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
+      tc_fence_after();
+      for (int col = 0; col < n_col; ++col) {
+        const int e = (first + col) * 128 + quarter * 32 + lane;
+        for (int h0 = 0; h0 < np; h0 += 16) {
+          uint32_t v[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
+            const int h = h0 + j + (lane & 1);
+            if (h < p.heads) {
+              const float w = inv[h];
+              T a[NT], b[NT];
+              split_terms<T>(f.x * w, a);
+              split_terms<T>(f.y * w, b);
+#pragma unroll
+              for (int t = 0; t < NT; ++t)
+                *reinterpret_cast<uint32_t*>(z + (((int64_t)t * p.heads + h) * p.n_cap + slot) * p.hidden + (e & ~1)) = pack_pair<T>(a[t], b[t]);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+    }
+  }
+  if (!ok) drain();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_free(tmem, 512); }
+}
+
+// ---- unfold -------------------------------------------------------------------------
+// D[row of W_v][request] = sum_e W_v[row][e] z[request][head of the row][e]: one CTA per (128 rows of W_v,
+// range of E, 128 / HT requests), HT = 128 / D heads per 128 rows.  Rows of every head are multiplied with
+// every one of the HT heads' z and the epilogue keeps the matching quarter (half): for D = 128 nothing
+// is wasted.  Partial sums over the ranges of E are added by the combine kernel.
+constexpr int kUnfoldThreads = 192;
+
+__host__ __device__ inline uint32_t unfold_stage_bytes(int terms) { return 16384u + (uint32_t)terms * 16384u; }
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kUnfoldThreads, 1)
+unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_z, const Params p) {
+  constexpr int NT = kTerms<T>, HT = 128 / D, NC = 128 / HT;   // NC: requests per CTA
+  constexpr uint32_t kZHead = NC * 128;                        // bytes of one (term, head) slab
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
+  __shared__ RingAux aux;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int n = p.plan->n, r0 = blockIdx.z * NC;
+  if (r0 >= n) return;
+  const int m = min(NC, n - r0), boxes = (m + 15) / 16;
+  const int head0 = blockIdx.x * HT, n_heads = min(HT, p.heads - head0);
+  const int sa = (int)((int64_t)p.slabs * blockIdx.y / gridDim.y), sb = (int)((int64_t)p.slabs * (blockIdx.y + 1) / gridDim.y);
+  const uint32_t stage_bytes = unfold_stage_bytes(NT);
+  constexpr int stages = kRingBytes / (16384 + NT * 16384);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
+    mbar_init(&aux.acc_full[0], 1);
+    aux.abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) tmem_alloc(&aux.tmem_base, 128);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = aux.tmem_base;
+  volatile int* abort_flag = &aux.abort_flag;
+  const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
+  bool ok = true;
+  Ring rg;
+  if (warp == 0) {
+    const int n_boxes = NT * n_heads * boxes;
+    for (int s = sa; s < sb; ++s) {
+      if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+      const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
+      if (lane == 0) {
+        mbar_expect_tx_addr(bar, (uint32_t)p.w_box_rows * 128 + (uint32_t)n_boxes * 2048);
+        tma_load_2d_cta(dst, &map_w, bar, s * 64, head0 * D);
+      }
+      __syncwarp();
+      for (int i = lane; i < n_boxes; i += 32) {   // i = (term, head, box of 16 requests)
+        const int b = i % boxes, hh = (i / boxes) % n_heads, t = i / (boxes * n_heads);
+        tma_load_2d_cta(dst + 16384 + (t * HT + hh) * kZHead + b * 2048, &map_z, bar, s * 64,
+                        (t * p.heads + head0 + hh) * p.n_cap + r0 + b * 16);
+      }
+      __syncwarp();
+      rg.step(stages);
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)(boxes * 16), false);
+    uint32_t acc = 0;
+    for (int s = sa; s < sb; ++s) {
+      if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t a_lo = desc_lo(ring + rg.stage * stage_bytes, 16), b_lo = a_lo + (16384 >> 4);
+        for (int hh = 0; hh < n_heads; ++hh) {
+          uint32_t first = acc;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+              tc_mma_cta(tmem + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (kZHead >> 4) + k * 2,
+                         desc_hi(1024, true), idesc, first);
+              first = 1u;
+            }
+        }
+        tc_commit_cta(empty0 + rg.stage * 8);
+      }
+      __syncwarp();
+      acc = 1u;
+      rg.step(stages);
+    }
+    if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[0]));
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3;
+    ok = mbar_wait_warp(smem_u32(&aux.acc_full[0]), 0, abort_flag, p.status, 4, lane);
+    if (ok) {
+      tc_fence_after();
+      const int row = quarter * 32 + lane, hh = row / D;
+      if (hh < n_heads) {   // uniform in a warp: D is 32, 64 or 128
+        const int width = p.heads * D;
+        float* dst = p.out_part + ((int64_t)blockIdx.y * p.n_hidden_cap + p.group_first + r0) * width + head0 * D + row;
+        for (int c = 0; c < m; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + hh * NC + c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < m) dst[(int64_t)(c + j) * width] = __uint_as_float(v[j]);
+        }
+      }
+    }
+  }
+  if (!ok) drain();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_free(tmem, 128); }
+}
+
+// ---- scratch and host side --------------------------------------------------------------
+int terms_of(int dtype) { return dtype == APS_BF16 ? 3 : 2; }
+
+struct Layout {
+  int np, n_cap, n_groups, splits, max_slice;
+  size_t off_groups, off_slot, off_list, off_qscale, off_inv, off_scores, off_probs, off_qz, off_part, total;
+};
+
+Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_size, int hidden, int dtype) {
+  Layout l;
+  const int nt = terms_of(dtype);
+  l.np = (heads + 15) / 16 * 16;
+  l.n_cap = ((batch < kGroup ? batch : kGroup) + 15) / 16 * 16;
+  l.n_groups = (batch + kGroup - 1) / kGroup;
+  // one wave of unfold CTAs; at least four slabs each
+  const int w_tiles = (heads * head_size + 127) / 128, slabs = hidden / 64;
+  int splits = 148 / w_tiles;
+  if (splits > slabs / 4) splits = slabs / 4;
+  l.splits = splits < 1 ? 1 : splits;
+  int ms = 256 / l.np;
+  if (ms > kMaxSlice) ms = kMaxSlice;
+  while (ms > 1 && 3 * sum_stage_bytes(nt, l.np, ms) > kRingBytes) --ms;   // at least three stages
+  l.max_slice = ms;
+  const int64_t max_tokens = (int64_t)max_blocks * block_size;
+  const int64_t tiles = (int64_t)l.n_cap * ((max_tokens + kTile - 1) / kTile) + kMaxGrid;
+  const int64_t blks = (int64_t)l.n_cap * ((max_tokens + 15) / 16);
+  size_t o = 0;
+  auto take = [&](size_t bytes) { const size_t at = o; o = align_up(o + bytes, 256); return at; };
+  l.off_groups = take((size_t)l.n_groups * sizeof(GroupPlan));
+  l.off_slot = take((size_t)batch * sizeof(int));
+  l.off_list = take((size_t)batch * sizeof(int2));
+  l.off_qscale = take((size_t)l.n_cap * heads * sizeof(float));
+  l.off_inv = take((size_t)l.n_cap * heads * sizeof(float));
+  l.off_scores = take((size_t)tiles * heads * kTile * sizeof(float));
+  l.off_probs = take((size_t)blks * probs_block_bytes(nt, l.np));
+  // qt is dead once the scores are there, z is written after them: one buffer
+  l.off_qz = take((size_t)l.n_cap * nt * heads * hidden * 2);
+  l.off_part = take((size_t)l.splits * l.n_groups * kGroup * heads * head_size * sizeof(float));
+  l.total = o;
+  return l;
+}
+
+int map_2d(CUtensorMap* map, const void* base, int dtype, uint64_t cols, uint64_t rows, uint64_t row_stride,
+           uint32_t box_rows, const char* what) {
+  TensorMapSpec spec{};
+  spec.base = base; spec.dtype = dtype; spec.rank = 2;
+  spec.dims[0] = cols; spec.dims[1] = rows;
+  spec.strides_bytes[0] = row_stride * 2;
+  spec.box[0] = 64; spec.box[1] = box_rows;
+  return cached_tensor_map(map, spec, what);
+}
+
+// Dynamic shared memory above 48 KB has to be allowed once per kernel and device.
+template <typename K>
+int allow_smem(K kernel, size_t bytes, bool* done) {
+  int dev = 0;
+  APS_CUDA(cudaGetDevice(&dev));
+  APS_REQUIRE(dev >= 0 && dev < 64, APS_ERR_CUDA, "device index %d out of range", dev);
+  if (!done[dev]) {
+    APS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    done[dev] = true;
+  }
+  return APS_OK;
+}
+
+struct Maps { CUtensorMap x_scores, x_sum, q, wk, wv, z; };
+
+template <typename T, int D>
+int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, cudaStream_t stream) {
+  constexpr int NT = kTerms<T>;
+  const size_t ring = 1024 + kRingBytes;
+  int st;
+  {
+    static bool done[64] = {false};
+    constexpr size_t smem = 1024 + 4 * D * 128 + ((D + 63) / 64) * kFoldReqs * 128;
+    auto k = fold_kernel<T, D>;
+    if ((st = allow_smem(k, smem, done)) != APS_OK) return st;
+    k<<<dim3((p.hidden + kFoldCols - 1) / kFoldCols, p.heads), kFoldThreads, smem, stream>>>(m.wk, p);
+    if ((st = launch_status("fold_kernel")) != APS_OK) return st;
+  }
+  {
+    static bool done[64] = {false};
+    auto k = scores_kernel<T>;
+    if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
+    const int fit = (int)(kRingBytes / scores_stage_bytes(NT, p.np));
+    p.stages = fit < kMaxStages ? fit : kMaxStages;
+    k<<<p.grid_scores, kScoresThreads, ring, stream>>>(m.x_scores, m.q, p);
+    if ((st = launch_status("scores_kernel")) != APS_OK) return st;
+  }
+  const int units = n_cap * p.heads, resident = sm_count() * 12;
+  softmax_kernel<T><<<units < resident ? units : resident, kSoftmaxWarps * 32, 0, stream>>>(p);
+  if ((st = launch_status("softmax_kernel")) != APS_OK) return st;
+  {
+    static bool done[64] = {false};
+    auto k = sum_kernel<T>;
+    if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
+    k<<<sm_count(), kSumThreads, ring, stream>>>(m.x_sum, p);
+    if ((st = launch_status("sum_kernel")) != APS_OK) return st;
+  }
+  {
+    static bool done[64] = {false};
+    auto k = unfold_kernel<T, D>;
+    if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
+    constexpr int kReqs = 128 / (128 / D);
+    k<<<dim3(w_tiles, p.splits, (n_cap + kReqs - 1) / kReqs), kUnfoldThreads, ring, stream>>>(m.wv, m.z, p);
+    if ((st = launch_status("unfold_kernel")) != APS_OK) return st;
+  }
+  return APS_OK;
+}
+
+}  // namespace
+
+bool folded_supported(int dtype, int heads, int head_size, int hidden) {
+  return (dtype == APS_F16 || dtype == APS_BF16) && (head_size == 128 || head_size == 64 || head_size == 32) &&
+         heads > 0 && heads <= 256 && hidden > 0 && hidden % 128 == 0;
+}
+
+size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
+                              int hidden, int dtype) {
+  return align_up(workspace_layout(batch, max_blocks_per_seq, block_size, heads, head_size).total, 256) +
+         layout_of(batch, max_blocks_per_seq, block_size, heads, head_size, hidden, dtype).total;
+}
+
+int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
+  const AttnShape& s = c.shape;
+  APS_REQUIRE(c.hidden_cache && c.w_k && c.w_v, APS_ERR_NULL_POINTER, "decode_layer_step: null pointer");
+  APS_REQUIRE(c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size && c.w_stride >= c.hidden_size,
+              APS_ERR_SHAPE, "decode_layer_step: bad hidden sizes / strides");
+  APS_REQUIRE(c.hidden_row_stride % 8 == 0 && c.w_stride % 8 == 0 && aligned_to(c.hidden_cache, 16) &&
+                  aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16),
+              APS_ERR_MISALIGNED, "decode_layer_step: hidden cache and weights must be 16-byte aligned with 16-byte row strides");
+  const WorkspaceLayout w = workspace_layout(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size);
+  const WorkspacePtrs ws = workspace_ptrs(c.workspace, w);
+  const Layout l = layout_of(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size, s.dtype);
+  char* b = static_cast<char*>(c.workspace) + align_up(w.total, 256);
+  GroupPlan* groups = reinterpret_cast<GroupPlan*>(b + l.off_groups);
+  const bool have_kv = c.key_cache != nullptr && c.value_cache != nullptr;
+  const int nt = terms_of(s.dtype), e_blocks = c.hidden_size / 128;
+  int st;
+  APS_REQUIRE(sm_count() <= kMaxGrid, APS_ERR_UNSUPPORTED, "decode_layer_step: more SMs than the plan keeps bounds for");
+
+  PlanArgs pa{};
+  pa.plan = ws.plan; pa.part_offset = ws.part_offset; pa.kv_chunks = ws.kv_chunks;
+  pa.hid_slot = reinterpret_cast<int*>(b + l.off_slot); pa.hid_list = reinterpret_cast<int2*>(b + l.off_list);
+  pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
+  pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
+  pa.slabs = c.hidden_size / 64; pa.grid_scores = sm_count(); pa.e_blocks = e_blocks;
+  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 3 * sm_count();
+  step_plan_kernel<<<1, kPlanThreads, 0, cs>>>(pa);
+  if ((st = launch_status("step_plan_kernel")) != APS_OK) return st;
+  if (have_kv &&
+      (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
+
+  Maps m;
+  const uint64_t hd = (uint64_t)s.heads * s.head_size;
+  void* qz = b + l.off_qz;
+  if ((st = map_2d(&m.x_scores, c.hidden_cache, s.dtype, c.hidden_size, c.num_hidden_rows, c.hidden_row_stride, 16, "hidden cache")) != APS_OK) return st;
+  {
+    TensorMapSpec spec{};
+    spec.base = c.hidden_cache; spec.dtype = s.dtype; spec.rank = 3;
+    spec.dims[0] = 64; spec.dims[1] = c.num_hidden_rows; spec.dims[2] = c.hidden_size / 64;
+    spec.strides_bytes[0] = c.hidden_row_stride * 2; spec.strides_bytes[1] = 128;
+    spec.box[0] = 64; spec.box[1] = 16; spec.box[2] = 2;
+    if ((st = cached_tensor_map(&m.x_sum, spec, "hidden cache")) != APS_OK) return st;
+  }
+  if ((st = map_2d(&m.q, qz, s.dtype, c.hidden_size, (uint64_t)l.n_cap * nt * s.heads, c.hidden_size, s.heads, "folded queries")) != APS_OK) return st;
+  if ((st = map_2d(&m.wk, c.w_k, s.dtype, c.hidden_size, hd, c.w_stride, s.head_size, "W_k")) != APS_OK) return st;
+  if ((st = map_2d(&m.wv, c.w_v, s.dtype, c.hidden_size, hd, c.w_stride, hd < 128 ? (uint32_t)hd : 128, "W_v")) != APS_OK) return st;
+  if ((st = map_2d(&m.z, qz, s.dtype, c.hidden_size, (uint64_t)nt * s.heads * l.n_cap, c.hidden_size, 16, "weighted sums")) != APS_OK) return st;
+
+  Params p{};
+  p.query = c.query; p.block_tables = c.block_tables;
+  p.qt = qz; p.z = qz;
+  p.qscale = reinterpret_cast<float*>(b + l.off_qscale); p.inv_sum = reinterpret_cast<float*>(b + l.off_inv);
+  p.scores = reinterpret_cast<float*>(b + l.off_scores); p.probs = b + l.off_probs;
+  p.out_part = reinterpret_cast<float*>(b + l.off_part);
+  p.status = ws.plan + kPlanStatus;
+  p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
+  p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
+  p.n_hidden_cap = l.n_groups * kGroup; p.splits = l.splits; p.grid_scores = pa.grid_scores;
+  p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
+  p.w_box_rows = hd < 128 ? (int)hd : 128;
+  const int w_tiles = (int)((hd + 127) / 128);
+  ScopedProfile prof(1, cs);
+  for (int g = 0; g < l.n_groups; ++g) {
+    p.plan = groups + g;
+    p.group_first = g * kGroup;
+    const bool bf16 = s.dtype == APS_BF16;
+    switch (s.head_size) {
+      case 128: st = bf16 ? launch_group<__nv_bfloat16, 128>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 128>(m, p, l.n_cap, w_tiles, cs); break;
+      case 64: st = bf16 ? launch_group<__nv_bfloat16, 64>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 64>(m, p, l.n_cap, w_tiles, cs); break;
+      default: st = bf16 ? launch_group<__nv_bfloat16, 32>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 32>(m, p, l.n_cap, w_tiles, cs); break;
+    }
+    if (st != APS_OK) return st;
+  }
+  const HiddenOutputs ho{pa.hid_slot, p.out_part, c.b_v, c.seq_lens, l.splits, p.n_hidden_cap};
+  return launch_combine(ws, c.out, &ho, s, cs);
+}
+
+}  // namespace aps

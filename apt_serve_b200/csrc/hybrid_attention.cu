@@ -47,6 +47,7 @@
 // and the CTA drains, frees its tensor memory and returns.
 
 #include "attention_common.cuh"
+#include "sm100.cuh"
 #include "tensor_maps.cuh"
 
 #include <cuda.h>
@@ -70,7 +71,6 @@ constexpr int kThreads = 320;          // warps 0 and 6-9 TMA producers, 1 MMA i
 constexpr int kStages = 6;
 constexpr int kBBytes = kBN / 2 * kBKBytes;      // 16 KB: this CTA's half of the W rows
 constexpr int kStageBytes = kABytes + kBBytes;   // 32 KB
-constexpr long long kWaitBudget = 4000000000LL;  // clock cycles (~2 s) before a wait gives up
 
 struct SmemAux {
   uint64_t full[kStages];
@@ -97,68 +97,10 @@ constexpr size_t smem_bytes() {
   return 1024 /*alignment slack*/ + (size_t)kStages * kStageBytes + sizeof(SmemAux);
 }
 
-// ---- PTX wrappers --------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx_addr(uint32_t bar_addr, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_addr(uint32_t bar_addr) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
-}
+// ---- PTX wrappers of the CTA pair --------------------------------------------------------------
 // Arrive on a barrier given by its shared::cluster address (own CTA or the peer).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar_addr, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
-  return ok != 0;
-}
-// Bounded wait.  Returns false when it gave up (or another warp already did): the code goes
-// to the CTA's abort flag and, first come first served, to the status word in global memory.
-__device__ __forceinline__ bool mbar_wait_addr(uint32_t bar_addr, uint32_t parity, volatile int* abort_flag,
-                                               int* status, int code, long long budget = kWaitBudget) {
-  if (mbar_try_wait_addr(bar_addr, parity)) return true;
-  const long long t0 = clock64();
-  int spins = 0;
-  while (!mbar_try_wait_addr(bar_addr, parity)) {
-    if ((++spins & 255) == 0) {
-      if (*abort_flag != 0) return false;
-      if (clock64() - t0 > budget) {
-        *abort_flag = code;
-        if (status != nullptr) atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-  return true;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status, int code) {
-  return mbar_wait_addr(smem_u32(bar), parity, abort_flag, status, code);
-}
-// The same for a whole converged warp: every lane tests the barrier once; if that fails
-// lane 0 does the bounded wait and the others take its verdict.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar_addr, uint32_t parity, volatile int* abort_flag,
-                                               int* status, int code, int lane) {
-  if (__all_sync(0xffffffffu, mbar_try_wait_addr(bar_addr, parity))) return true;
-  const bool got = lane != 0 || mbar_wait_addr(bar_addr, parity, abort_flag, status, code);
-  return __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
-}
-// True in exactly one lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -183,23 +125,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
       ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y), "l"(l2_policy) : "memory");
 }
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_normal() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // The barrier is named by a shared::cluster address (own CTA or peer).
 __device__ __forceinline__ void tc_commit(uint32_t bar_cluster_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
@@ -216,18 +141,6 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint32_t a_lo, uint3
       "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 // Barrier over the 128 epilogue threads that also ANDs a per-thread flag, so that
 // all of them take the same decision after a bounded wait.
@@ -950,7 +863,7 @@ int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t cs) {
                       s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size,
                       s.query_stride, c.hidden_row_stride, c.w_stride, s.scale, s.dtype};
     if ((st = launch_hidden_simt(ws, sa, cs)) != APS_OK) return st;
-    return launch_combine(ws, c.out, c.seq_lens, s, cs);
+    return launch_combine(ws, c.out, nullptr, s, cs);
   }
   HiddenParams p{};
   p.plan = ws.plan; p.part_offset = ws.part_offset; p.hid_subs = ws.hid_subs; p.first_tile = ws.first_tile; p.hid_rows = ws.hid_rows;
@@ -971,7 +884,7 @@ int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t cs) {
                        : launch_hidden<__half, kModeAttend, 4>(mx, mk, mv, p, cs); break;
   }
   if (st != APS_OK) return st;
-  return launch_combine(ws, c.out, c.seq_lens, s, cs);
+  return launch_combine(ws, c.out, nullptr, s, cs);
 }
 
 int check_hybrid_call(const char* op, const HybridCall& c) {

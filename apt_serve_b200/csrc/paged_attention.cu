@@ -623,7 +623,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 combine_kernel(const int* __restrict__ plan, const int* __restrict__ part_offset, const float* __restrict__ part_ml,
                const float* __restrict__ part_acc, T* __restrict__ out, int batch, int heads,
-               int head_size, int64_t out_stride) {
+               int head_size, int64_t out_stride, const HiddenOutputs hid) {
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (unit >= batch * heads) return;
@@ -633,6 +633,26 @@ combine_kernel(const int* __restrict__ plan, const int* __restrict__ part_offset
   const int status = plan[kPlanStatus];
   if (status >= kStatusWaitFirst && status <= kStatusWaitLast) {
     for (int d = lane; d < head_size; d += 32) dst[d] = Elem<T>::from_float(__int_as_float(0x7fc00000));
+    return;
+  }
+  const int hid_slot = hid.hid_slot != nullptr ? hid.hid_slot[req] : -1;
+  if (hid_slot >= 0) {
+    const T* b_v = static_cast<const T*>(hid.b_v);
+    const bool empty = hid.seq_lens[req] <= 0;
+    const int64_t width = (int64_t)heads * head_size;
+    for (int d = lane * 4; d < head_size; d += 128) {
+      const float* src = hid.part + hid_slot * width + (int64_t)h * head_size + d;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int k = 0; k < hid.splits; ++k) {
+        const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)k * hid.slots * width);
+        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+      }
+      const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        dst[d + e] = Elem<T>::from_float(empty ? 0.f : v[e] + (b_v != nullptr ? Elem<T>::to_float(b_v[(int64_t)h * head_size + d + e]) : 0.f));
+    }
     return;
   }
   // the lanes share the request's partials for the maximum and the denominator (butterfly
@@ -774,23 +794,23 @@ int launch_kv_attention(const WorkspacePtrs& ws, const void* query, const void* 
   }
 }
 
-int launch_combine(const WorkspacePtrs& ws, void* out, const int32_t* seq_lens, const AttnShape& s,
+int launch_combine(const WorkspacePtrs& ws, void* out, const HiddenOutputs* hidden, const AttnShape& s,
                    cudaStream_t stream) {
-  (void)seq_lens;
+  const HiddenOutputs hid = hidden != nullptr ? *hidden : HiddenOutputs{};
   const int units = s.batch * s.heads;
   const int grid = (units + 7) / 8;
   switch (s.dtype) {
     case APS_F32:
       combine_kernel<float><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                     (float*)out, s.batch, s.heads, s.head_size, s.out_stride);
+                                                     (float*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
       break;
     case APS_F16:
       combine_kernel<__half><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                      (__half*)out, s.batch, s.heads, s.head_size, s.out_stride);
+                                                      (__half*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
       break;
     case APS_BF16:
       combine_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                             (__nv_bfloat16*)out, s.batch, s.heads, s.head_size, s.out_stride);
+                                                             (__nv_bfloat16*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
       break;
     default: return fail(APS_ERR_DTYPE, "decode attention: unsupported dtype %d", s.dtype);
   }
@@ -857,7 +877,7 @@ extern "C" int aps_paged_decode_attention(void* out, const void* query, const vo
   cudaStream_t cs = (cudaStream_t)stream;
   if ((st = launch_plan(ws, seq_lens, nullptr, block_tables, batch, max_blocks_per_seq, block_size, false, true, cs)) != APS_OK) return st;
   if ((st = launch_kv_attention(ws, query, key_cache, value_cache, block_tables, seq_lens, s, cs)) != APS_OK) return st;
-  return launch_combine(ws, out, seq_lens, s, cs);
+  return launch_combine(ws, out, nullptr, s, cs);
 }
 
 extern "C" int aps_attention_status(const void* workspace, int* host_status, void* stream) {
@@ -938,5 +958,5 @@ extern "C" int aps_paged_decode_attention_static(void* out, const void* query, c
   // nothing left over from the previous call is ever read
   if ((st = launch_plan(ws, seq_lens, nullptr, block_tables, batch, max_blocks_per_seq, block_size, false, true, cs)) != APS_OK) return st;
   if ((st = launch_kv_attention(ws, query, key_cache, value_cache, block_tables, seq_lens, s, cs)) != APS_OK) return st;
-  return launch_combine(ws, out, seq_lens, s, cs);
+  return launch_combine(ws, out, nullptr, s, cs);
 }

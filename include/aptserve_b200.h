@@ -292,7 +292,12 @@ int aps_kv_reprojection(void* kv, const void* x, const int32_t* block_ids, int64
  *      hidden-cached requests (hidden_to_cache, opt.py:108-109), new_key[r] /
  *      new_value[r] -> K/V planes for K/V-cached requests (the private-cache half of
  *      mixed_kv_to_cache, fa.py:363-373, or reshape_and_cache_flash, fa.py:338-345);
- *   2. aps_hybrid_decode_attention over the batch.
+ *   2. the attention of aps_hybrid_decode_attention over the batch.  With a workspace of
+ *      aps_decode_layer_step_workspace_bytes the hidden-cached requests of fp16 / bf16 layers
+ *      (head size 128, 64 or 32, hidden_size a multiple of 128) are attended directly:
+ *      scores X (W_k^T q), outputs W_v (P X) + b_v, which is the same result without
+ *      re-projecting the rows; a batch of at most one wave of the re-projection kernel, any
+ *      other shape and a smaller workspace are re-projected.
  * hidden_states [B, hidden_size], new_key / new_value [B, H*D] (rows of the other
  * cache type are ignored; a NULL pointer skips that kind of write), every pointer
  * and row 16-byte aligned.  All other arguments as in aps_hybrid_decode_attention.
@@ -309,6 +314,14 @@ int aps_decode_layer_step(void* out, const void* query, const void* hidden_state
                           int64_t hidden_row_stride, int64_t num_hidden_rows, int64_t w_stride,
                           float scale, void* workspace, size_t workspace_bytes, int dtype,
                           void* stream);
+
+/*
+ * Bytes of scratch aps_decode_layer_step works best with (256-byte aligned).  A step whose
+ * workspace is smaller, but holds aps_attention_workspace_bytes, re-projects the cached hidden
+ * rows; with this much it can attend them directly (see aps_decode_layer_step).
+ */
+size_t aps_decode_layer_step_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
+                                             int num_heads, int head_size, int hidden_size, int dtype);
 
 /*
  * Reads the status word the attention kernels keep in `workspace` for the last call

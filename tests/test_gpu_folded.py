@@ -1,0 +1,107 @@
+"""The layer-step's hidden path with the projections moved to the query and the output
+(csrc/hidden_attention.cu) at the sizes where its tiles, stages, groups and splits end.
+
+Tolerance of the hidden-cached requests' rows: the intermediates carry at least 22 bits, so what is left
+is the rounding of the output, half a unit of its last place (u = 2^-11 of the value in fp16, 2^-8 in bf16),
+and an eighth of that, relative to the rows' root mean square, for the sums and the oracle's own fp32.
+K/V-cached requests: the 2e-2 of the other attention tests (their weights are rounded to the cache type)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import hybrid_cache_oracle as O
+from apt_serve_b200 import _native as N
+from apt_serve_b200 import attention as A
+from apt_serve_b200.workloads import LayerShape, make_decode_workload
+
+from helpers import assert_close
+
+pytestmark = pytest.mark.gpu
+
+HALF_ULP = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def run_step(w):
+    m = w.meta
+    d = w.shape
+    args = (len(w.seq_lens), m.private_block_tables.shape[1], d.block_size, w.heads, d.head_dim)
+    assert (N.lib().aps_decode_layer_step_workspace_bytes(*args, d.hidden, N.DTYPE_ENUM[d.dtype])
+            > N.lib().aps_attention_workspace_bytes(*args)), "this size does not take the path under test"
+    wk, bk, wv, bv = w.kv_weights()
+    out = A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache,
+                              wk, bk, wv, bv, m.private_block_tables, m.seq_lens_tensor, m.cache_type, w.scale)
+    A.raise_on_device_status()
+    return out
+
+
+def check(w_cpu, what):
+    w = w_cpu.to("cuda")
+    out = run_step(w)
+    again = run_step(w)
+    assert torch.equal(out, again), f"{what}: two runs on the same inputs differ"
+    ref = O.decode_layer_step(w_cpu.hidden_states, w_cpu.query, w_cpu.new_key, w_cpu.new_value, w_cpu.kv_cache,
+                              w_cpu.hidden_cache, *w_cpu.kv_weights(), w_cpu.meta, w_cpu.scale)
+    hid = [r for r, u in enumerate(w_cpu.use_hidden) if u]
+    kv = [r for r, u in enumerate(w_cpu.use_hidden) if not u]
+    if hid:
+        x, y = out[hid].float().cpu(), ref[hid].float()
+        u = HALF_ULP[w_cpu.shape.dtype]
+        rms = y.pow(2).mean(dim=1, keepdim=True).sqrt()
+        bad = ~((x - y).abs() <= u * y.abs() + u / 8 * rms)
+        assert not bad.any(), (what, int(bad.sum()), float(((x - y).abs() / rms).max()))
+    if kv:
+        assert_close(out[kv], ref[kv], what)
+
+
+F, B = torch.float16, torch.bfloat16
+# (heads, head size, hidden, dtype, lengths, every how many requests one is K/V-cached)
+CASES = {
+    "edges of tiles and stages": (8, 128, 1024, F, (1, 15, 16, 17, 31, 32, 33, 255, 256, 257, 511, 512, 513, 529), 0),
+    "the same in bf16, mixed": (8, 128, 1024, B, (1, 15, 16, 17, 31, 32, 33, 255, 256, 257, 511, 512, 513, 529), 4),
+    "one long request": (40, 128, 512, F, (2048,), 0),
+    "one token": (72, 128, 256, B, (1, 257), 0),
+    "heads not a multiple of 16, wide rows": (9, 128, 9216, B, (300, 17, 640, 1, 256, 120, 900), 3),
+    "two heads per row tile": (5, 64, 384, F, (300, 17, 640, 1, 256, 120, 900), 3),
+    "four heads per row tile": (33, 32, 256, B, (300, 17, 640, 1, 256, 120, 900), 0),
+    "a narrow hidden size": (12, 64, 128, F, (700, 5, 90, 1, 64), 0),
+    "fewer projection rows than a tile": (1, 64, 128, F, (700, 5, 90), 0),
+    "wide accumulators": (160, 32, 128, F, (70, 260, 5, 90), 0),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_step_against_the_oracle(name):
+    heads, d, e, dtype, lens, every = CASES[name]
+    hidden = [not (every and i % every == 1) for i in range(len(lens))]
+    w = make_decode_workload(LayerShape("t", heads, d, e, dtype), list(lens), hidden, seed=len(lens), device="cpu")
+    check(w, name)
+
+
+@pytest.mark.parametrize("n_hidden", [256, 257, 600])
+def test_groups_of_hidden_requests(n_hidden):
+    rng = np.random.default_rng(n_hidden)
+    lens = [int(x) for x in rng.integers(1, 60, size=n_hidden + 20)]
+    hidden = [True] * n_hidden + [False] * 20
+    order = rng.permutation(len(lens))
+    w = make_decode_workload(LayerShape("t", 4, 64, 256, F), [lens[i] for i in order], [hidden[i] for i in order],
+                             seed=2, device="cpu")
+    check(w, f"{n_hidden} hidden requests")
+
+
+def test_larger_cache_blocks_and_garbage_behind_the_sequences():
+    lens = [21, 150, 40, 511, 256, 33, 1030]
+    w = make_decode_workload(LayerShape("t", 8, 128, 1024, F, block_size=32), lens, [True] * len(lens), seed=6, device="cpu")
+    rows = O.flat_rows(w.hidden_cache)
+    for r, s in enumerate(lens):
+        if s % 32:
+            last = w.block_tables[r][-1]
+            rows[last * 32 + s % 32: last * 32 + 32] = float("nan")
+    check(w, "garbage tail")
+
+
+def test_small_and_large_queries_keep_their_bits():
+    """The folded query is normalised per request and head: queries and hidden rows of very different sizes."""
+    w = make_decode_workload(LayerShape("t", 8, 128, 1024, F), [300] * 12, [True] * 12, seed=8, device="cpu")
+    for r, s in enumerate((1e-6, 1e-4, 1e-2, 1.0, 8.0, 30.0, 1e-6, 1e-4, 1e-2, 1.0, 8.0, 0.0)):
+        w.query[r] *= s
+    check(w, "query sizes")
