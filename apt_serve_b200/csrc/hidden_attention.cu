@@ -49,8 +49,10 @@ constexpr int kTile = 256;                // tokens per scores tile: two M128 ac
 constexpr int kSubs = kTile / 16;         // 16-row boxes of the hidden cache per tile
 constexpr int kTileCost = 4;              // fixed cost of a tile in boxes (its qt slab), for the work split
 constexpr int kStepTokens = 32;           // tokens per stage of the sum kernel
-constexpr int kMinPiece = 4 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: four full slabs
-constexpr int kMaxGrid = 256;             // largest grid of the scores kernel the plan keeps bounds for
+constexpr int kMinPiece = 2 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: two full steps
+constexpr int kMaxGrid = 192;             // most SMs the plan keeps bounds of pieces for
+constexpr int kMaxLevels = 5;             // sizes of pieces the scores work is cut into
+constexpr int kMaxPieces = kMaxGrid * kMaxLevels;
 constexpr int kMaxSlice = 8;              // 128-column blocks of E per work item of the sum kernel
 constexpr float kProbShift = 15.f;        // p is kept at 2^15 times its value (fp16 range)
 constexpr size_t kRingBytes = 200 * 1024; // shared memory of the operand rings
@@ -64,22 +66,44 @@ struct GroupPlan {
   int n_tiles;                // scores tiles
   int weight;                 // total cost of the tiles, in boxes
   int slice;                  // 128-column blocks per item of the sum kernel
-  int pieces;                 // CTAs the scores work is cut for
+  int levels, per_level;      // pieces of the scores work: levels x per_level
+  int next_piece, next_item;  // work counters of the scores and the sum kernel
   int req[kGroup];            // batch row of each request, longest first
   int len[kGroup];            // its length in tokens
   int tile_off[kGroup + 1];   // first scores tile
   int blk_off[kGroup + 1];    // first 16-token block of p
   int w_off[kGroup + 1];      // cost of the tiles before it
-  int bound_tile[kMaxGrid + 1];   // scores work of CTA c: from (bound_tile[c], bound_slab[c]) to the next bound
-  int bound_slab[kMaxGrid + 1];
+  int bound_tile[kMaxPieces + 1];   // piece c: from (bound_tile[c], bound_step[c]) to the next bound
+  int bound_step[kMaxPieces + 1];
 };
 
+// The scores work is a line of X box-steps, cut into pieces that are handed out in order: `levels` sizes, each
+// half of the one before (the last two alike), `per_level` pieces of each.  Large pieces first keep the
+// number of cut tiles down, small ones last let the CTAs end together: one equal piece per CTA left the SMs
+// idle for a fifth of the kernel (they do not get equal shares of the memory bandwidth).  In units of the
+// smallest size there are per_level << (levels - 1) of them; piece c starts at unit_of_piece(c), position
+// X * unit / units.
+__host__ __device__ inline int unit_of_piece(int c, int levels, int per_level) {
+  const int l = c / per_level, k = c - l * per_level;
+  const int size = l >= levels - 2 ? 1 : 1 << (levels - 2 - l);
+  return l >= levels ? per_level << (levels - 1) : per_level * ((1 << (levels - 1)) - (1 << (levels - 1 - l))) + k * size;
+}
+// The last piece that starts at or before `unit`.
+__host__ __device__ inline int piece_of_unit(int unit, int levels, int per_level) {
+  int l = 0;
+  for (; l < levels - 1; ++l)
+    if (unit < per_level * ((1 << (levels - 1)) - (1 << (levels - 2 - l)))) break;
+  const int size = l >= levels - 2 ? 1 : 1 << (levels - 2 - l);
+  const int k = (unit - per_level * ((1 << (levels - 1)) - (1 << (levels - 1 - l)))) / size;
+  return l * per_level + (k < per_level ? k : per_level - 1);
+}
+
 struct Params {
-  const GroupPlan* plan;
+  GroupPlan* plan;
   const void* query; const void* b_k; const int32_t* block_tables;
   void* qt;              // [request][term][head][E]
   float* qscale;         // [request][head] scale * log2(e) / (power of two q was multiplied with)
-  float* scores;         // [tile + CTA][head][kTile] partial scores over a range of E
+  float* scores;         // [tile + piece][head][kTile] partial scores over a range of E
   void* probs;           // [16-token block][term][K half][heads padded][8 tokens]
   float* inv_sum;        // [request][head]
   void* z;               // [term][head][request capacity][E]
@@ -88,7 +112,7 @@ struct Params {
   int heads, np, head_size, hidden, slabs;   // np: heads padded to a multiple of 16; slabs: E / 64
   int block_size, max_blocks, n_cap;         // n_cap: requests a group can hold here
   int group_first;                           // ordinal of the group's first hidden request
-  int n_hidden_cap, splits, stages, grid_scores;
+  int n_hidden_cap, splits, grid_scores;
   int w_box_rows;                            // rows of a W_v box: 128, fewer when W_v has fewer
   int64_t query_stride;
   float scale_log2;
@@ -151,7 +175,7 @@ __device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int
 struct PlanArgs {
   int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
   const int32_t* seq_lens; const int32_t* cache_type;
-  int batch, max_tokens, kv_present, n_groups, slabs, grid_scores, e_blocks, max_slice, item_target;
+  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target;
 };
 
 __global__ void __launch_bounds__(kPlanThreads)
@@ -256,229 +280,268 @@ step_plan_kernel(const PlanArgs a) {
     if (tid == 0) {
       // sum kernel: the widest slice of E that still gives item_target items
       int slice = a.max_slice;
-      while (slice > 1 && n * ((a.e_blocks + slice - 1) / slice) < a.item_target) --slice;
+      while (slice > 1 && n * ((a.steps + slice - 1) / slice) < a.item_target) --slice;
       gp->n = n; gp->n_tiles = n_tiles; gp->weight = weight; gp->slice = slice;
     }
-    // scores kernel: piece c starts at cost c / pieces of the total, rounded down to a slab of a tile.  No
-    // piece is smaller than kMinPiece (more than a full slab), so that none is empty and the partial
-    // sums of a tile stay few.
-    const int pieces = (int)max((int64_t)1, min((int64_t)a.grid_scores, (int64_t)weight * a.slabs / kMinPiece));
-    if (tid == 0) gp->pieces = pieces;
-    if (tid <= a.grid_scores) {
-      int t = n_tiles, slab = 0;
-      if (tid < pieces && weight > 0) {
-        const int64_t pos = (int64_t)tid * weight * a.slabs / pieces;
+    // cut the scores work.  No piece is smaller than kMinPiece (more than a full step), so that none is empty
+    // and the partial sums of a tile stay few.
+    const int64_t work = (int64_t)weight * a.steps;
+    const int per_level = (int)max((int64_t)1, min((int64_t)a.grid_scores, work / kMinPiece));
+    int levels = 1;
+    while (levels < kMaxLevels && work / ((int64_t)per_level << levels) >= kMinPiece) ++levels;
+    if (tid == 0) { gp->levels = levels; gp->per_level = per_level; gp->next_piece = 0; gp->next_item = 0; }
+    for (int c = tid; c <= levels * per_level; c += kPlanThreads) {
+      int t = n_tiles, step = 0;
+      if (c < levels * per_level && weight > 0) {
+        const int64_t pos = work * unit_of_piece(c, levels, per_level) / ((int64_t)per_level << (levels - 1));
         int lo = 0, hi = n;   // last request whose cost offset is <= pos
-        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((int64_t)s_woff[mid] * a.slabs <= pos) lo = mid; else hi = mid; }
-        const int64_t rem = pos - (int64_t)s_woff[lo] * a.slabs;
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((int64_t)s_woff[mid] * a.steps <= pos) lo = mid; else hi = mid; }
+        const int64_t rem = pos - (int64_t)s_woff[lo] * a.steps;
         const int blocks = (s_len[lo] + 15) / 16, tiles = (blocks + kSubs - 1) / kSubs;
-        const int k = min((int)(rem / ((int64_t)(kSubs + kTileCost) * a.slabs)), tiles - 1);
+        const int k = min((int)(rem / ((int64_t)(kSubs + kTileCost) * a.steps)), tiles - 1);
         const int w = min(kSubs, blocks - k * kSubs) + kTileCost;
         t = s_toff[lo] + k;
-        slab = (int)((rem - (int64_t)k * (kSubs + kTileCost) * a.slabs) / w);
+        step = (int)((rem - (int64_t)k * (kSubs + kTileCost) * a.steps) / w);
       }
-      gp->bound_tile[tid] = t; gp->bound_slab[tid] = slab;
+      gp->bound_tile[c] = t; gp->bound_step[c] = step;
     }
   }
 }
 
 // ---- fold ---------------------------------------------------------------------------
-// One CTA per (256 columns of E, head): D[column][request] = sum_d W_k,h[d][column] q[request][d], exact
-// 16-bit operands, fp32 accumulators.  W_k,h arrives as boxes of (64 columns, D rows), i.e. an MN-major A
-// operand; q is gathered by the threads into a K-major B operand, 128 requests at a time.
-constexpr int kFoldThreads = 128;
-constexpr int kFoldCols = 256;
+// D[column of E][request] = sum_d W_k,h[d][column] q[request][d], exact 16-bit operands, fp32 accumulators.
+// One CTA per (range of E, head, 128 requests): q is gathered once by all threads into a K-major B operand
+// and stays; W_k,h streams past it in tiles of 128 columns (two boxes of 64 columns x D rows, an MN-major
+// A operand) through a two-stage ring, the accumulators are double-buffered.  Two CTAs per SM.
+// Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
+constexpr int kFoldThreads = 192;
 constexpr int kFoldReqs = 128;
+constexpr int kFoldStages = 2;
 
 struct FoldAux {
-  uint64_t w_full, mma_done;
+  uint64_t full[kFoldStages], empty[kFoldStages], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int req[kFoldReqs];
 };
 
+template <int D> constexpr size_t fold_smem() {
+  return 1024 + (size_t)kFoldStages * 2 * D * 128 + (size_t)((D + 63) / 64) * kFoldReqs * 128;
+}
+
+// Gathers q[request][head] of m requests from ordinal r0 on (zero rows up to np) into shared memory: slabs of
+// 64 elements, rows of 128 bytes, 128-byte swizzle.  All warps of the CTA.
 template <typename T, int D>
-__global__ void __launch_bounds__(kFoldThreads)
+__device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, int r0, int m, int np, int head, bool keep_scale) {
+  constexpr int kWarps = kFoldThreads / 32, U = 4, EPL = D / 32;   // U requests at a time, EPL elements per lane
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* query = static_cast<const T*>(p.query);
+  for (int r = warp; r < np; r += kWarps * U) {
+    T v[U][EPL];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int rr = r + u * kWarps;
+      const bool in = rr < m;
+      const T* src = query + (in ? (int64_t)p.plan->req[r0 + rr] * p.query_stride + head * D + lane * EPL : 0);
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) v[u][e] = in ? src[e] : Elem<T>::from_float(0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int rr = r + u * kWarps;
+      if (rr >= np) break;
+      float f[EPL], mx = 0.f;
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) { f[e] = Elem<T>::to_float(v[u][e]); mx = fmaxf(mx, fabsf(f[e])); }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      // power of two that brings max |q| into [1, 2); zero, infinite and NaN rows stay as they are
+      int k = 0;
+      if (mx > 0.f && mx < INFINITY) k = max(-100, min(100, (int)((__float_as_uint(mx) >> 23) & 0xff) - 127));
+      const float up = __uint_as_float((uint32_t)(127 - k) << 23), down = __uint_as_float((uint32_t)(127 + k) << 23);
+      unsigned short w[EPL];
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) { const T t = Elem<T>::from_float(f[e] * up); w[e] = reinterpret_cast<const unsigned short&>(t); }
+      const int el = lane * EPL, slab = el / 64, piece = (el % 64) / 8, in_piece = el % 8;
+      const uint32_t dst = q_at + slab * (kFoldReqs * 128) + rr * 128 + ((piece ^ (rr & 7)) << 4) + in_piece * 2;
+      if constexpr (EPL == 4) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)), "r"((uint32_t)w[2] | ((uint32_t)w[3] << 16)) : "memory");
+      else if constexpr (EPL == 2) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)) : "memory");
+      else asm volatile("st.shared.b16 [%0], %1;" ::"r"(dst), "h"(w[0]) : "memory");
+      if (keep_scale && lane == 0 && rr < m) p.qscale[(int64_t)(r0 + rr) * p.heads + head] = p.scale_log2 * down;
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // read by the tensor cores next
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kFoldThreads, 2)
 fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
   constexpr int NT = kTerms<T>;
-  constexpr int kQSlab = kFoldReqs * 128;                 // 64 elements of D for 128 requests
-  constexpr int kQSlabs = (D + 63) / 64;
-  constexpr uint32_t kBox = D * 128;                      // 64 columns of E x D rows
+  constexpr uint32_t kBox = D * 128, kStage = 2 * kBox;   // 64 columns of E x D rows; two of them
   extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;
-  const uint32_t w_at = base, q_at = base + 4 * kBox;
+  const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u, q_at = ring + kFoldStages * kStage;
   __shared__ FoldAux aux;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = p.plan->n;
-  if (n == 0) return;
-  const int head = blockIdx.y, col0 = blockIdx.x * kFoldCols;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int n = p.plan->n, r0 = blockIdx.z * kFoldReqs, head = blockIdx.y;
+  if (r0 >= n) return;
+  const int m = min(kFoldReqs, n - r0), np = (m + 15) & ~15;
+  const int blocks = p.hidden / 128;
+  const int ta = blocks * blockIdx.x / gridDim.x, tb = blocks * (blockIdx.x + 1) / gridDim.x;
   volatile int* abort_flag = &aux.abort_flag;
   if (threadIdx.x == 0) {
-    mbar_init(&aux.w_full, 1);
-    mbar_init(&aux.mma_done, 1);
+    for (int s = 0; s < kFoldStages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
     aux.abort_flag = 0;
     mbar_init_fence();
-    mbar_expect_tx_addr(smem_u32(&aux.w_full), 4 * kBox);
-    for (int b = 0; b < 4; ++b) tma_load_2d_cta(w_at + b * kBox, &map_w, smem_u32(&aux.w_full), col0 + b * 64, head * D);
+    for (int i = 0; i < kFoldStages && ta + i < tb; ++i) {   // the first tiles are on their way while q is staged
+      const uint32_t bar = smem_u32(&aux.full[i]), dst = ring + i * kStage;
+      mbar_expect_tx_addr(bar, kStage);
+      tma_load_2d_cta(dst, &map_w, bar, (ta + i) * 128, head * D);
+      tma_load_2d_cta(dst + kBox, &map_w, bar, (ta + i) * 128 + 64, head * D);
+    }
   }
-  if (warp == 1) tmem_alloc(&aux.tmem_base, 256);
+  if (warp == 1) tmem_alloc(&aux.tmem_base, 2 * kFoldReqs);
+  stage_queries<T, D>(p, q_at, r0, m, np, head, blockIdx.x == 0);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = aux.tmem_base;
-  const T* query = static_cast<const T*>(p.query);
-  T* qt = static_cast<T*>(p.qt);
   bool ok = true;
-  uint32_t parity = 0;
-  for (int r0 = 0; r0 < n && ok; r0 += kFoldReqs) {
-    const int m = min(kFoldReqs, n - r0), np = (m + 15) & ~15;
-    // ---- stage q: warp w takes requests w, w + 4, ...; lane l elements l * D / 32 ... ----
-    constexpr int EPL = D / 32;   // elements per lane: 4, 2 or 1
-    for (int r = warp; r < np; r += 4 * 8) {
-      T v[8][EPL];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int rr = r + u * 4;
-        const bool in = rr < m;
-        const T* src = query + (in ? (int64_t)p.plan->req[r0 + rr] * p.query_stride + head * D + lane * EPL : 0);
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) v[u][e] = in ? src[e] : Elem<T>::from_float(0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int rr = r + u * 4;
-        if (rr >= np) break;
-        float f[EPL], mx = 0.f;
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) { f[e] = Elem<T>::to_float(v[u][e]); mx = fmaxf(mx, fabsf(f[e])); }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        // power of two that brings max |q| into [1, 2); zero, infinite and NaN rows stay as they are
-        int k = 0;
-        if (mx > 0.f && mx < INFINITY) k = max(-100, min(100, (int)((__float_as_uint(mx) >> 23) & 0xff) - 127));
-        const float up = __uint_as_float((uint32_t)(127 - k) << 23), down = __uint_as_float((uint32_t)(127 + k) << 23);
-        unsigned short w[EPL];
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) { const T t = Elem<T>::from_float(f[e] * up); w[e] = reinterpret_cast<const unsigned short&>(t); }
-        const int el = lane * EPL, slab = el / 64, piece = (el % 64) / 8, in_piece = el % 8;
-        const uint32_t dst = q_at + slab * kQSlab + rr * 128 + ((piece ^ (rr & 7)) << 4) + in_piece * 2;
-        if constexpr (EPL == 4) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)), "r"((uint32_t)w[2] | ((uint32_t)w[3] << 16)) : "memory");
-        else if constexpr (EPL == 2) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)) : "memory");
-        else asm volatile("st.shared.b16 [%0], %1;" ::"r"(dst), "h"(w[0]) : "memory");
-        if (blockIdx.x == 0 && lane == 0 && rr < m) p.qscale[(int64_t)(r0 + rr) * p.heads + head] = p.scale_log2 * down;
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-      if (r0 == 0) ok = mbar_wait_warp(smem_u32(&aux.w_full), 0, abort_flag, p.status, 3, lane);
-      tc_fence_after();
-      if (ok && elect_one()) {
-        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
-#pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
-#pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks)
-            tc_mma_cta(tmem + mb * kFoldReqs, desc_lo(w_at + mb * 2 * kBox + ks * 2048, kBox), desc_hi(1024, true),
-                       desc_lo(q_at + (ks / 4) * kQSlab + (ks % 4) * 32, 16), desc_hi(1024, true), idesc, ks != 0);
-        tc_commit_cta(smem_u32(&aux.mma_done));
+  if (warp == 0) {
+    for (int t = ta + kFoldStages; t < tb; ++t) {
+      const int i = t - ta, s = i % kFoldStages;
+      if (!mbar_wait_warp(smem_u32(&aux.empty[s]), (uint32_t)(i / kFoldStages - 1) & 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+      if (lane == 0) {
+        const uint32_t bar = smem_u32(&aux.full[s]), dst = ring + s * kStage;
+        mbar_expect_tx_addr(bar, kStage);
+        tma_load_2d_cta(dst, &map_w, bar, t * 128, head * D);
+        tma_load_2d_cta(dst + kBox, &map_w, bar, t * 128 + 64, head * D);
       }
       __syncwarp();
     }
-    ok = mbar_wait_warp(smem_u32(&aux.mma_done), parity, abort_flag, p.status, 4, lane);
-    parity ^= 1u;
-    if (ok) {
+  } else if (warp == 1) {
+    const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
+    for (int t = ta; t < tb; ++t) {
+      const int i = t - ta, s = i % kFoldStages, buf = i & 1;
+      if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
+      if (!mbar_wait_warp(smem_u32(&aux.full[s]), (uint32_t)(i / kFoldStages) & 1u, abort_flag, p.status, 3, lane)) { ok = false; break; }
       tc_fence_after();
-      // lanes are columns of E, accumulator columns are requests
-#pragma unroll 1
-      for (int mb = 0; mb < 2; ++mb) {
-        const int col = col0 + mb * 128 + warp * 32 + lane;
-        if (col0 + mb * 128 >= p.hidden) break;
-#pragma unroll 1
-        for (int c = 0; c < m; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + mb * kFoldReqs + c, v);
-          tmem_ld_wait();
+      if (elect_one()) {
+        const uint32_t a_lo = desc_lo(ring + s * kStage, kBox);
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
-            const int r = c + j + (lane & 1);
-            if (r < m) {
-              T a[NT], b[NT];
-              split_terms<T>(f.x, a);
-              split_terms<T>(f.y, b);
+        for (int ks = 0; ks < D / 16; ++ks)
+          tc_mma_cta(tmem + buf * kFoldReqs, a_lo + ks * 128, desc_hi(1024, true),
+                     desc_lo(q_at + (ks / 4) * (kFoldReqs * 128) + (ks % 4) * 32, 16), desc_hi(1024, true), idesc, ks != 0);
+        tc_commit_cta(smem_u32(&aux.empty[s]));
+        tc_commit_cta(smem_u32(&aux.acc_full[buf]));
+      }
+      __syncwarp();
+    }
+  } else {
+    // lanes are columns of E, accumulator columns are requests
+    const int quarter = warp & 3;
+    const int64_t req_stride = (int64_t)NT * p.heads * p.hidden, term_stride = (int64_t)p.heads * p.hidden;
+    T* qt = static_cast<T*>(p.qt) + (r0 + (lane & 1)) * req_stride + (int64_t)head * p.hidden + quarter * 32 + (lane & ~1);
+    for (int t = ta; t < tb; ++t) {
+      const int i = t - ta, buf = i & 1;
+      if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
+      tc_fence_after();
+      T* dst = qt + t * 128;
+      for (int c = 0; c < np; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + buf * kFoldReqs + c, v);
+        tmem_ld_wait();
 #pragma unroll
-              for (int t = 0; t < NT; ++t)
-                *reinterpret_cast<uint32_t*>(qt + (((int64_t)(r0 + r) * NT + t) * p.heads + head) * p.hidden + (col & ~1)) = pack_pair<T>(a[t], b[t]);
-            }
+        for (int j = 0; j < 16; j += 2) {
+          const float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
+          if (c + j + (lane & 1) < m) {
+            T x[NT], y[NT];
+            split_terms<T>(f.x, x);
+            split_terms<T>(f.y, y);
+#pragma unroll
+            for (int k = 0; k < NT; ++k) *reinterpret_cast<uint32_t*>(dst + k * term_stride) = pack_pair<T>(x[k], y[k]);
           }
+          dst += 2 * req_stride;
         }
       }
       tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
     }
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;   // the accumulators and the q operand are free again
-    tc_fence_after();
   }
   if (!ok) drain();
+  tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_free(tmem, 256);
+  if (warp == 1) { tc_fence_after(); tmem_free(tmem, 2 * kFoldReqs); }
 }
 
 // ---- scores -------------------------------------------------------------------------
 // D[token][head] = sum_e x[token][e] qt[head][e] for tiles of 256 tokens of one request (two M128
-// accumulators that share the qt slab).  The work is a line of (tile, 64-column slab) steps, cut into one
-// contiguous piece per CTA with equal numbers of boxes: a tile that straddles a cut leaves one partial sum
-// per piece (slot = tile + CTA), added by the softmax kernel, so that one long request uses the whole
-// chip and a large batch has no partly filled last wave.
-// Warps: 0 qt boxes and byte counts, 1 MMA issue, 2-5 epilogue, 6-9 boxes of the hidden cache (four
-// lanes each: one 16-row box per cache block and slab).
-constexpr int kScoresThreads = 320;
+// accumulators that share a qt step).  The work is a line of (tile, 128 columns of E) steps, cut into
+// contiguous pieces (see unit_of_piece): a tile that straddles a cut leaves one partial sum per piece (slot =
+// tile + piece), added by the softmax kernel, so that one long request uses the whole chip and a large
+// batch has no partly filled last wave.  94.7k rows of an OPT-13B layer (0.97 GB): 221 us, 247 us with one
+// equal piece per CTA.
+// A box is (64 columns, 8 rows, 2): 256 contiguous bytes of a cached row, so that a DRAM page is left after
+// 256 bytes and not 128, and 8-row groups that lie 2 KB apart, as the K-major operand needs them.  X and qt
+// have a ring each: a unit of X is 128 tokens x 128 columns (32 KB), a unit of qt serves both halves of a
+// tile.  Warps: 0 qt boxes, 1 MMA issue, 2-5 epilogue, 6-7 boxes of X (eight lanes each).
+constexpr int kScoresThreads = 256;
 constexpr int kMaxStages = 12;
+constexpr uint32_t kUnitBytes = 128 * 256;
+constexpr size_t kScoresRing = 216 * 1024;
 
 struct RingAux {
-  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], q_full[2], q_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
+
+constexpr int kItemSlots = 4;
+// Work items passed from the copying warp that takes them to the other warps of the CTA.
+struct ItemRing { uint64_t full[kItemSlots], empty[kItemSlots]; int item[kItemSlots]; };
 
 struct Ring {
   uint32_t stage = 0, phase = 0;
   __device__ __forceinline__ void step(int stages) { if (++stage == (uint32_t)stages) { stage = 0; phase ^= 1u; } }
 };
 
-__host__ __device__ inline uint32_t scores_stage_bytes(int terms, int np) { return kTile * 128 + terms * np * 128; }
+__host__ __device__ inline uint32_t scores_q_bytes(int terms, int np) { return (uint32_t)terms * np * 256; }
+// qt units in the ring: two unless they leave less than two units of X
+__host__ __device__ inline int scores_q_units(int terms, int np) {
+  return 2 * scores_q_bytes(terms, np) + 2 * kUnitBytes <= kScoresRing ? 2 : 1;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kScoresThreads, 1)
 scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q, const Params p) {
   constexpr int NT = kTerms<T>;
   extern __shared__ uint8_t smem_raw[];
-  const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
+  const uint32_t x_ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
   __shared__ int s_toff[kGroup + 1], s_len[kGroup], s_req[kGroup];
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n = p.plan->n, cta = blockIdx.x;
-  if (n == 0) return;
-  const int t0 = p.plan->bound_tile[cta], t1 = p.plan->bound_tile[cta + 1];
-  const int b0 = p.plan->bound_slab[cta], b1 = p.plan->bound_slab[cta + 1];
-  if (t0 == t1 && b0 == b1) return;
+  __shared__ ItemRing items;
+  GroupPlan* gp = p.plan;
+  const int n = gp->n, n_pieces = gp->levels * gp->per_level;
+  if (n == 0 || (int)blockIdx.x >= n_pieces) return;
   for (int i = threadIdx.x; i <= n; i += kScoresThreads) {
-    s_toff[i] = p.plan->tile_off[i];
-    if (i < n) { s_len[i] = p.plan->len[i]; s_req[i] = p.plan->req[i]; }
+    s_toff[i] = gp->tile_off[i];
+    if (i < n) { s_len[i] = gp->len[i]; s_req[i] = gp->req[i]; }
   }
-  const int np = p.np, stages = p.stages;
-  const uint32_t stage_bytes = scores_stage_bytes(NT, np);
+  const int np = p.np, steps = p.hidden / 128;
+  const uint32_t q_bytes = scores_q_bytes(NT, np);
+  const int nq = scores_q_units(NT, np), nx = min(kMaxStages, (int)((kScoresRing - nq * q_bytes) / kUnitBytes));
+  const uint32_t q_ring = x_ring + nx * kUnitBytes;
   const int n_buf = 4 * np <= 512 ? 2 : 1;
   uint32_t tmem_cols = 32;
   while (tmem_cols < (uint32_t)(n_buf * 2 * np)) tmem_cols <<= 1;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
-      // one arrival with the byte count (warp 0) and one per slab from each of the warps 6-9, boxes
-      // or not: a stage cannot be filled and freed twice while one of them still waits for it
-      mbar_init(&aux.full[s], 5);
-      mbar_init(&aux.empty[s], 1);
+    for (int s = 0; s < nx; ++s) { mbar_init(&aux.full[s], 2); mbar_init(&aux.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&aux.q_full[b], 1); mbar_init(&aux.q_empty[b], 1);
+      mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4);
     }
-    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
+    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], kScoresThreads / 32 - 1); }
     aux.abort_flag = 0;
     mbar_init_fence();
   }
@@ -489,98 +552,139 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   const uint32_t tmem = aux.tmem_base;
   volatile int* abort_flag = &aux.abort_flag;
   const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
-  int slot = 0;   // request of tile t0
-  {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_toff[mid] <= t0) lo = mid; else hi = mid; }
-    slot = lo;
-  }
+  const uint32_t q_full0 = smem_u32(&aux.q_full[0]), q_empty0 = smem_u32(&aux.q_empty[0]);
   bool ok = true;
-  Ring rg;
+  Ring xr, qr, ir;
   uint32_t n_local = 0;
-  for (int t = t0; t <= t1 && ok; ++t) {
-    const int sa = t == t0 ? b0 : 0, sb = t == t1 ? b1 : p.slabs;
-    if (sa >= sb) continue;
-    while (t >= s_toff[slot + 1]) ++slot;
-    const int tok0 = (t - s_toff[slot]) * kTile;
-    const int n_sub = min(kSubs, (s_len[slot] - tok0 + 15) >> 4);
-    const uint32_t buf = n_local % n_buf, use = n_local / n_buf;
-    ++n_local;
+  int next = blockIdx.x;   // the first piece needs no counter
+  while (ok) {
+    int piece;
     if (warp == 0) {
-      const uint32_t tx = (uint32_t)(n_sub * 2048 + NT * p.heads * 128);
-      for (int s = sa; s < sb; ++s) {
-        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-        const uint32_t bar = full0 + rg.stage * 8;
-        if (lane == 0) mbar_expect_tx_addr(bar, tx);
-        __syncwarp();
-        if (lane < NT)
-          tma_load_2d_cta(ring + rg.stage * stage_bytes + kTile * 128 + lane * np * 128, &map_q, bar, s * 64, (slot * NT + lane) * p.heads);
-        rg.step(stages);
+      piece = next;
+      if (!mbar_wait_warp(smem_u32(&items.empty[ir.stage]), ir.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+      if (lane == 0) {
+        items.item[ir.stage] = piece;
+        mbar_arrive_addr(smem_u32(&items.full[ir.stage]));
       }
-    } else if (warp >= 6) {
-      const int sub = (warp - 6) * 4 + lane;
-      int row = 0;
-      const bool has = lane < 4 && sub < n_sub;
-      if (has) {
-        const int tok = tok0 + sub * 16;
-        row = p.block_tables[(int64_t)s_req[slot] * p.max_blocks + tok / p.block_size] * p.block_size + tok % p.block_size;
-      }
-      for (int s = sa; s < sb; ++s) {
-        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-        const uint32_t bar = full0 + rg.stage * 8;
-        if (has) tma_load_2d_cta(ring + rg.stage * stage_bytes + sub * 2048, &map_x, bar, s * 64, row);
-        __syncwarp();
-        if (lane == 0) mbar_arrive_addr(bar);
-        rg.step(stages);
-      }
-    } else if (warp == 1) {
-      if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, false);
-      const int n_m = n_sub > 8 ? 2 : 1;
-      uint32_t acc = 0;
-      for (int s = sa; s < sb; ++s) {
-        if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t a_lo = desc_lo(ring + rg.stage * stage_bytes, 16), b_lo = a_lo + (kTile * 128 >> 4);
-          for (int m = 0; m < n_m; ++m) {
-            const uint32_t d = tmem + (buf * 2 + m) * np;
-            uint32_t first = acc;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-#pragma unroll
-              for (int i = 0; i < NT; ++i) {
-                tc_mma_cta(d, a_lo + m * 1024 + k * 2, desc_hi(1024, true), b_lo + i * (np * 8) + k * 2, desc_hi(1024, true), idesc, first);
-                first = 1u;
-              }
-          }
-          tc_commit_cta(empty0 + rg.stage * 8);
-        }
-        __syncwarp();
-        acc = 1u;
-        rg.step(stages);
-      }
-      if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
-      __syncwarp();
     } else {
-      const int quarter = warp & 3;
-      if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
-      tc_fence_after();
-      float* dst = p.scores + (int64_t)(t + cta) * p.heads * kTile;
-      const int n_m = n_sub > 8 ? 2 : 1;
-      for (int m = 0; m < n_m; ++m)
-        for (int h0 = 0; h0 < np; h0 += 16) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * np + h0, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[j]);
-        }
-      tc_fence_before();
+      if (!mbar_wait_warp(smem_u32(&items.full[ir.stage]), ir.phase, abort_flag, p.status, 6, lane)) { ok = false; break; }
+      piece = items.item[ir.stage];
       __syncwarp();
-      if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+      if (lane == 0) mbar_arrive_addr(smem_u32(&items.empty[ir.stage]));
+    }
+    ir.step(kItemSlots);
+    if (piece >= n_pieces) break;
+    if (warp == 0) {
+      if (lane == 0) next = (int)gridDim.x + atomicAdd(&gp->next_piece, 1);
+      next = __shfl_sync(0xffffffffu, next, 0);
+    }
+    const int t0 = gp->bound_tile[piece], t1 = gp->bound_tile[piece + 1];
+    const int b0 = gp->bound_step[piece], b1 = gp->bound_step[piece + 1];
+    int slot = 0;   // request of tile t0
+    {
+      int lo = 0, hi = n;
+      while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_toff[mid] <= t0) lo = mid; else hi = mid; }
+      slot = lo;
+    }
+    for (int t = t0; t <= t1 && ok; ++t) {
+      const int sa = t == t0 ? b0 : 0, sb = t == t1 ? b1 : steps;
+      if (sa >= sb) continue;
+      while (t >= s_toff[slot + 1]) ++slot;
+      const int tok0 = (t - s_toff[slot]) * kTile;
+      const int n_sub = min(kSubs, (s_len[slot] - tok0 + 15) >> 4);
+      const int n_m = n_sub > 8 ? 2 : 1;
+      const uint32_t buf = n_local % n_buf, use = n_local / n_buf;
+      ++n_local;
+      if (warp == 0) {
+        for (int s = sa; s < sb; ++s) {
+          if (!mbar_wait_warp(q_empty0 + qr.stage * 8, qr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+          const uint32_t bar = q_full0 + qr.stage * 8;
+          if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
+          __syncwarp();
+          if (lane < 2 * NT)   // lane = (term, half of the columns)
+            tma_load_2d_cta(q_ring + qr.stage * q_bytes + lane * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
+          __syncwarp();
+          qr.step(nq);
+        }
+      } else if (warp >= 6) {
+        // box g of a unit: rows 8 g ... of its 128 tokens; warp 6 the first eight, warp 7 the others
+        const int g = (warp - 6) * 8 + lane;
+        int row[2] = {0, 0};
+        bool has[2] = {false, false};
+        int boxes[2];
+  #pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const int sub = m * 8 + (g >> 1);
+          has[m] = lane < 8 && sub < n_sub;
+          boxes[m] = max(0, min(8, 2 * (n_sub - m * 8) - (warp - 6) * 8));
+          if (has[m]) {
+            const int tok = tok0 + sub * 16;
+            row[m] = p.block_tables[(int64_t)s_req[slot] * p.max_blocks + tok / p.block_size] * p.block_size + tok % p.block_size + (g & 1) * 8;
+          }
+        }
+        for (int s = sa; s < sb && ok; ++s) {
+  #pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            if (m >= n_m) break;
+            if (!mbar_wait_warp(empty0 + xr.stage * 8, xr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+            const uint32_t bar = full0 + xr.stage * 8;
+            if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)boxes[m] * 2048);
+            __syncwarp();
+            if (has[m]) tma_load_3d_cta(x_ring + xr.stage * kUnitBytes + g * 2048, &map_x, bar, 0, row[m], s * 2);
+            __syncwarp();
+            xr.step(nx);
+          }
+        }
+      } else if (warp == 1) {
+        if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, false);
+        for (int s = sa; s < sb && ok; ++s) {
+          if (!mbar_wait_warp(q_full0 + qr.stage * 8, qr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+          for (int m = 0; m < n_m; ++m) {
+            if (!mbar_wait_warp(full0 + xr.stage * 8, xr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t a_lo = desc_lo(x_ring + xr.stage * kUnitBytes, 16), b_lo = desc_lo(q_ring + qr.stage * q_bytes, 16);
+              const uint32_t d = tmem + (buf * 2 + m) * np;
+              uint32_t acc = s != sa;
+  #pragma unroll
+              for (int j = 0; j < 2; ++j)
+  #pragma unroll
+                for (int k = 0; k < 4; ++k)
+  #pragma unroll
+                  for (int i = 0; i < NT; ++i) {
+                    tc_mma_cta(d, a_lo + j * 64 + k * 2, desc_hi(2048, true), b_lo + (i * 2 + j) * (np * 8) + k * 2, desc_hi(1024, true), idesc, acc);
+                    acc = 1u;
+                  }
+              tc_commit_cta(empty0 + xr.stage * 8);
+              if (m == n_m - 1) tc_commit_cta(q_empty0 + qr.stage * 8);
+            }
+            __syncwarp();
+            xr.step(nx);
+          }
+          qr.step(nq);
+        }
+        if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
+        __syncwarp();
+      } else {
+        const int quarter = warp & 3;
+        if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
+        tc_fence_after();
+        float* dst = p.scores + (int64_t)(t + piece) * p.heads * kTile;
+        for (int m = 0; m < n_m; ++m)
+          for (int h0 = 0; h0 < np; h0 += 16) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * np + h0, v);
+            tmem_ld_wait();
+  #pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[j]);
+          }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+      }
     }
   }
   if (!ok) drain();
@@ -604,8 +708,9 @@ softmax_kernel(const Params p) {
   __shared__ float s_max[kSoftmaxWarps], s_sum[kSoftmaxWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const GroupPlan* gp = p.plan;
-  const int n_units = gp->n * p.heads, pieces = gp->pieces;
-  const int64_t work = (int64_t)gp->weight * p.slabs;
+  const int n_units = gp->n * p.heads, levels = gp->levels, per_level = gp->per_level, steps = p.hidden / 128;
+  const int64_t units = (int64_t)per_level << (levels - 1);
+  const int64_t work = (int64_t)gp->weight * steps;
   T* probs = static_cast<T*>(p.probs);
   for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
     const int slot = unit / p.heads, h = unit - slot * p.heads;
@@ -615,12 +720,12 @@ softmax_kernel(const Params p) {
     const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot], w0 = gp->w_off[slot];
     // scores of this lane's eight tokens of tile k
     auto load = [&](int k, float (&s)[8]) {
-      // the pieces of the line of (tile, slab) steps that touch this tile: c0 is the last that starts at or
-      // before its first slab, c1 the last that starts at or before its last one
+      // the pieces of the line of (tile, step) that touch this tile: c0 is the last that starts at or
+      // before its first step, c1 the last that starts at or before its last one
       const int w = min(kSubs, n_blk - k * kSubs) + kTileCost;
-      const int64_t at = (int64_t)(w0 + k * (kSubs + kTileCost)) * p.slabs;
-      const int c0 = (int)(((at + w) * pieces - 1) / work);
-      const int c1 = min((int)(((at + (int64_t)w * p.slabs) * pieces - 1) / work), pieces - 1);
+      const int64_t at = (int64_t)(w0 + k * (kSubs + kTileCost)) * steps;
+      const int c0 = piece_of_unit((int)(((at + w) * units - 1) / work), levels, per_level);
+      const int c1 = piece_of_unit((int)(((at + (int64_t)w * steps) * units - 1) / work), levels, per_level);
 #pragma unroll
       for (int e = 0; e < 8; ++e) s[e] = 0.f;
       const float4* src = reinterpret_cast<const float4*>(p.scores + ((int64_t)(tile0 + k + c0) * p.heads + h) * kTile + lane * 8);
@@ -703,7 +808,8 @@ softmax_kernel(const Params p) {
 // ---- weighted sums ------------------------------------------------------------------
 // D[column of E][head] = sum_t x_t[column] p[t][head]: work item = (request, slice of up to kMaxSlice x 128
 // columns), the item's accumulators together in half of the tensor memory, so that the epilogue of one item
-// overlaps the next one's main loop.  Items in order of their length, dealt to the CTAs in snake order.
+// overlaps the next one's main loop.  Items in order of their length, longest first, handed out by a counter:
+// the copying warp takes the next one when it has requested all of its item and passes it to the other warps.
 // A stage holds 32 tokens: per 16-token cache block and 128 columns one box of (64 columns, 16 rows, 2) =
 // an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
 // K-major B operand).  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
@@ -722,7 +828,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const GroupPlan* gp = p.plan;
+  __shared__ ItemRing items;
+  GroupPlan* gp = p.plan;
   const int n = gp->n;
   if (n == 0) return;
   const int np = p.np, e_blocks = p.hidden / 128, slice = gp->slice;
@@ -733,6 +840,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
+    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 5); }
     aux.abort_flag = 0;
     mbar_init_fence();
   }
@@ -746,11 +854,29 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   bool ok = true;
   Ring rg;
   uint32_t n_local = 0;
-  for (int round = 0; ok; ++round) {
-    const int g = gridDim.x;
-    const int item = round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
-    if (round * g >= n_items) break;
-    if (item >= n_items) continue;
+  Ring ir;
+  int next = blockIdx.x;   // the first item needs no counter
+  while (ok) {
+    int item;
+    if (warp == 0) {
+      item = next;
+      if (!mbar_wait_warp(smem_u32(&items.empty[ir.stage]), ir.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+      if (lane == 0) {
+        items.item[ir.stage] = item;
+        mbar_arrive_addr(smem_u32(&items.full[ir.stage]));
+      }
+    } else {
+      if (!mbar_wait_warp(smem_u32(&items.full[ir.stage]), ir.phase, abort_flag, p.status, 6, lane)) { ok = false; break; }
+      item = items.item[ir.stage];
+      __syncwarp();
+      if (lane == 0) mbar_arrive_addr(smem_u32(&items.empty[ir.stage]));
+    }
+    ir.step(kItemSlots);
+    if (item >= n_items) break;
+    if (warp == 0) {
+      if (lane == 0) next = (int)gridDim.x + atomicAdd(&gp->next_item, 1);
+      next = __shfl_sync(0xffffffffu, next, 0);
+    }
     const int slot = item / n_slices, first = (item % n_slices) * slice;
     const int len = gp->len[slot];
     if (len <= 0) continue;
@@ -993,7 +1119,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   while (ms > 1 && 3 * sum_stage_bytes(nt, l.np, ms) > kRingBytes) --ms;   // at least three stages
   l.max_slice = ms;
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
-  const int64_t tiles = (int64_t)l.n_cap * ((max_tokens + kTile - 1) / kTile) + kMaxGrid;
+  const int64_t tiles = (int64_t)l.n_cap * ((max_tokens + kTile - 1) / kTile) + kMaxPieces;
   const int64_t blks = (int64_t)l.n_cap * ((max_tokens + 15) / 16);
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o = align_up(o + bytes, 256); return at; };
@@ -1038,24 +1164,24 @@ struct Maps { CUtensorMap x_scores, x_sum, q, wk, wv, z; };
 
 template <typename T, int D>
 int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, cudaStream_t stream) {
-  constexpr int NT = kTerms<T>;
   const size_t ring = 1024 + kRingBytes;
   int st;
   {
     static bool done[64] = {false};
-    constexpr size_t smem = 1024 + 4 * D * 128 + ((D + 63) / 64) * kFoldReqs * 128;
+    constexpr size_t smem = fold_smem<D>();
     auto k = fold_kernel<T, D>;
     if ((st = allow_smem(k, smem, done)) != APS_OK) return st;
-    k<<<dim3((p.hidden + kFoldCols - 1) / kFoldCols, p.heads), kFoldThreads, smem, stream>>>(m.wk, p);
+    const int blocks = p.hidden / 128, chunks = (n_cap + kFoldReqs - 1) / kFoldReqs;
+    int splits = 2 * sm_count() / p.heads;   // one wave at two CTAs per SM when one chunk of requests is in use
+    splits = splits < 1 ? 1 : splits > blocks ? blocks : splits;
+    k<<<dim3(splits, p.heads, chunks), kFoldThreads, smem, stream>>>(m.wk, p);
     if ((st = launch_status("fold_kernel")) != APS_OK) return st;
   }
   {
     static bool done[64] = {false};
     auto k = scores_kernel<T>;
-    if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
-    const int fit = (int)(kRingBytes / scores_stage_bytes(NT, p.np));
-    p.stages = fit < kMaxStages ? fit : kMaxStages;
-    k<<<p.grid_scores, kScoresThreads, ring, stream>>>(m.x_scores, m.q, p);
+    if ((st = allow_smem(k, 1024 + kScoresRing, done)) != APS_OK) return st;
+    k<<<p.grid_scores, kScoresThreads, 1024 + kScoresRing, stream>>>(m.x_scores, m.q, p);
     if ((st = launch_status("scores_kernel")) != APS_OK) return st;
   }
   const int units = n_cap * p.heads, resident = sm_count() * 12;
@@ -1083,7 +1209,8 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, cudaStream_t s
 
 bool folded_supported(int dtype, int heads, int head_size, int hidden) {
   return (dtype == APS_F16 || dtype == APS_BF16) && (head_size == 128 || head_size == 64 || head_size == 32) &&
-         heads > 0 && heads <= 256 && hidden > 0 && hidden % 128 == 0;
+         heads > 0 && heads <= 256 && hidden > 0 && hidden % 128 == 0 &&
+         scores_q_bytes(terms_of(dtype), (heads + 15) / 16 * 16) + 2 * kUnitBytes <= kScoresRing;
 }
 
 size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
@@ -1115,8 +1242,8 @@ int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
   pa.hid_slot = reinterpret_cast<int*>(b + l.off_slot); pa.hid_list = reinterpret_cast<int2*>(b + l.off_list);
   pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
-  pa.slabs = c.hidden_size / 64; pa.grid_scores = sm_count(); pa.e_blocks = e_blocks;
-  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 3 * sm_count();
+  pa.steps = e_blocks; pa.grid_scores = sm_count(); pa.steps = e_blocks;
+  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 8 * sm_count();
   step_plan_kernel<<<1, kPlanThreads, 0, cs>>>(pa);
   if ((st = launch_status("step_plan_kernel")) != APS_OK) return st;
   if (have_kv &&
@@ -1125,14 +1252,16 @@ int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
   Maps m;
   const uint64_t hd = (uint64_t)s.heads * s.head_size;
   void* qz = b + l.off_qz;
-  if ((st = map_2d(&m.x_scores, c.hidden_cache, s.dtype, c.hidden_size, c.num_hidden_rows, c.hidden_row_stride, 16, "hidden cache")) != APS_OK) return st;
   {
+    // cached rows as [64 columns][rows][E / 64], boxes of (64, 8 or 16 rows, 2)
     TensorMapSpec spec{};
     spec.base = c.hidden_cache; spec.dtype = s.dtype; spec.rank = 3;
     spec.dims[0] = 64; spec.dims[1] = c.num_hidden_rows; spec.dims[2] = c.hidden_size / 64;
     spec.strides_bytes[0] = c.hidden_row_stride * 2; spec.strides_bytes[1] = 128;
     spec.box[0] = 64; spec.box[1] = 16; spec.box[2] = 2;
     if ((st = cached_tensor_map(&m.x_sum, spec, "hidden cache")) != APS_OK) return st;
+    spec.box[1] = 8;
+    if ((st = cached_tensor_map(&m.x_scores, spec, "hidden cache")) != APS_OK) return st;
   }
   if ((st = map_2d(&m.q, qz, s.dtype, c.hidden_size, (uint64_t)l.n_cap * nt * s.heads, c.hidden_size, s.heads, "folded queries")) != APS_OK) return st;
   if ((st = map_2d(&m.wk, c.w_k, s.dtype, c.hidden_size, hd, c.w_stride, s.head_size, "W_k")) != APS_OK) return st;

@@ -67,7 +67,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar_addr, uint32_t parit
                                                int* status, int code, int lane) {
   if (__all_sync(0xffffffffu, mbar_try_wait_addr(bar_addr, parity))) return true;
   const bool got = lane != 0 || mbar_wait_addr(bar_addr, parity, abort_flag, status, code);
-  return __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
+  const bool all = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
+  __syncwarp();   // what lane 0 acquired is visible to the other lanes
+  return all;
 }
 // True in exactly one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
