@@ -173,6 +173,7 @@ struct NewTokenWrite {
   int dtype;
 };
 int launch_new_token_write(const NewTokenWrite& a, cudaStream_t stream);
+int read_metadata_status(int* host_status, cudaStream_t stream);   // metadata_ops.cu
 
 int check_hybrid_call(const char* op, const HybridCall& c);
 int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t stream);

@@ -612,7 +612,7 @@ extern "C" int aps_cache_ops_status(int* host_status, void* stream) {
   APS_CUDA(cudaGetSymbolAddress(&addr, g_copy_status));
   APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   APS_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-  return APS_OK;
+  return *host_status != 0 ? APS_OK : read_metadata_status(host_status, (cudaStream_t)stream);
 }
 
 // Block moves between one plane of a GPU cache and one plane of the pinned CPU cache (or

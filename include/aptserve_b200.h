@@ -343,8 +343,9 @@ int aps_attention_status(const void* workspace, int* host_status, void* stream);
 int aps_reprojection_cycles(const void* workspace, unsigned long long* host_cycles, void* stream);
 
 /*
- * Status of the bulk-copy cache writes on the current device: 0, or 1 once a bounded
- * wait on a bulk load ran out (the launch then stopped copying).  Synchronises `stream`.
+ * Status of the cache operations on the current device: 0, 1 once a bounded wait on a bulk load
+ * ran out (the launch then stopped copying), or 2 once aps_derive_private_tables met an index
+ * outside its tensor.  Synchronises `stream`.
  */
 int aps_cache_ops_status(int* host_status, void* stream);
 
@@ -400,6 +401,22 @@ int aps_expand_decode_metadata(const int32_t* block_tables, const int32_t* block
                                int64_t* hidden_cache_use_input, int64_t num_tot_tokens,
                                int64_t num_hidden_tokens, int64_t* counts, void* scratch,
                                size_t scratch_bytes, void* stream);
+
+/*
+ * The private block tables and the cache-type mask of a decode batch, from the reference's own metadata
+ * (model_runner.py:515-564: a hidden-cached request's block_tables row is its SHARED table, its
+ * private slots are its run of slot_mapping).  tables: int32 [B, max_blocks_per_seq], contiguous;
+ * cache_type: int32 [B]; block_tables: int32 rows of block_tables_stride elements; slot_mapping [num_slots],
+ * hidden_holder_upd [B], hidden_cache_use_input [num_hidden]: the reference's int64 tensors;
+ * seq_lens: int32 [B].  A hidden-cached request's entries past its length are 0.  Negative indices
+ * count from the end; an index outside its tensor gives a 0 entry and sets the status word that
+ * aps_cache_ops_status reads.
+ */
+int aps_derive_private_tables(int32_t* tables, int32_t* cache_type, const int32_t* block_tables,
+                              const int64_t* slot_mapping, int64_t num_slots, const int64_t* hidden_holder_upd,
+                              const int64_t* hidden_cache_use_input, int64_t num_hidden, const int32_t* seq_lens,
+                              int batch, int max_blocks_per_seq, int64_t block_tables_stride, int block_size,
+                              void* stream);
 
 /*
  * Timing hook for benchmarks (no counterpart in the reference, whose kernels are

@@ -104,3 +104,46 @@ def test_counts_that_disagree_with_the_device_side_batch_write_nothing():
 def test_zero_length_is_refused_on_the_host():
     with pytest.raises(ValueError, match=">= 1"):
         expand_decode_metadata([5, 0], [True, False], [[0], [1]], [[2], []], 16, "cuda")
+
+
+@pytest.mark.parametrize("bs", [16, 32])
+@pytest.mark.parametrize("lens,hid", [
+    ([1], [True]),
+    ([16, 17, 2048, 5], [True, True, True, True]),
+    ([129, 1, 64, 300, 16, 15], [False, True, False, True, True, False]),
+    ([int(x) for x in np.random.default_rng(3).integers(1, 2100, size=300)], [i % 3 == 0 for i in range(300)]),
+])
+def test_derived_tables_equal_the_tensor_form(lens, hid, bs):
+    """The one-launch derivation against the same thing as tensor operations, in every form it accepts."""
+    from dataclasses import replace
+    from apt_serve_b200.metadata import _derive_with_tensor_ops, derive_private_block_tables
+    tables, shared = batch(lens, hid, 1, bs)
+    m = build_decode_metadata(lens, hid, tables, shared, bs).to("cuda")
+    wide = torch.full((len(lens), m.block_tables.shape[1] + 3), 7, dtype=torch.int32, device="cuda")
+    wide[:, :-3] = m.block_tables
+    forms = [m,
+             replace(m, block_tables=wide[:, :-3]),                                   # rows with a stride of their own
+             replace(m, hidden_cache_use_input=m.hidden_cache_use_input.flip(0) - len(lens)),   # any order, from the end
+             replace(m, seq_lens_tensor=m.seq_lens_tensor.long())]                    # a type the kernel does not take
+    for f in forms:
+        got, want = derive_private_block_tables(f, bs), _derive_with_tensor_ops(f, bs)
+        for a, b in zip(got, want):
+            assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+def test_derived_tables_bound_their_indices():
+    """A claim that points outside slot_mapping: nothing is read there, the entries are 0, the status says so."""
+    import ctypes
+    from apt_serve_b200 import _native as N
+    lib, host = N.lib(), ctypes.c_int(0)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    i64 = dict(dtype=torch.int64, device="cuda")
+    tables, ctype = torch.full((2, 4), -5, **i32), torch.full((2,), -5, **i32)
+    bt, lens = torch.arange(8, **i32).view(2, 4), torch.tensor([40, 7], **i32)
+    slots, upd, rows = torch.arange(32, 64, **i64), torch.tensor([39, 40], **i64), torch.tensor([0], **i64)
+    stream = N.current_stream(tables.device)
+    N.check(lib.aps_derive_private_tables(N.ptr(tables), N.ptr(ctype), N.ptr(bt), N.ptr(slots), 32, N.ptr(upd),
+                                          N.ptr(rows), 1, N.ptr(lens), 2, 4, 4, 16, stream))
+    N.check(lib.aps_cache_ops_status(ctypes.addressof(host), stream))
+    assert tables.tolist() == [[2, 3, 0, 0], [4, 5, 6, 7]] and ctype.tolist() == [1, 0]
+    assert host.value == 2
