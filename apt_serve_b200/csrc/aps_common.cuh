@@ -8,6 +8,8 @@
 #include <stdio.h>
 #include <stdarg.h>
 
+#include <utility>
+
 #include "../../include/aptserve_b200.h"
 
 namespace aps {
@@ -41,6 +43,38 @@ inline int launch_status(const char* what) {
     return fail(APS_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
   return APS_OK;
 }
+
+// ---- chained launches ----------------------------------------------------------------
+// The kernels of one call run one after the other on the caller's stream, most of them for 5 - 30 us; a plain
+// launch leaves 2 us between two of them and starts every one with cold CTAs.  They are therefore launched as
+// programmatic dependents: the next kernel's CTAs become resident and set themselves up while the last one
+// drains.  What makes this equal to stream order:
+//   - every kernel launched here calls chain_wait() (all earlier kernels are complete, their writes visible)
+//     in every CTA, before it touches anything that another kernel touches - or, where its comment says
+//     which earlier kernels it needs and why they are complete, before it exits, so that its own completion
+//     still implies that of everything before it;
+//   - chain_next() comes after the CTA's tensor memory is allocated: a CTA of the next kernel cannot take
+//     columns that this kernel still has to get.
+// chain_wait() returns at once in a kernel launched the plain way, and work enqueued the plain way behind a
+// chained kernel waits for it as always.
+// Measured on one B200, plain -> chained: a step of one OPT-13B request 89 -> 67 us, of 48 OPT-1.3B requests 149 -> 127,
+// of 256 OPT-13B requests 890 -> 875.
+template <typename... P, typename... A>
+inline int launch_chained(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                          cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  APS_REQUIRE(e == cudaSuccess, APS_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
+  return APS_OK;
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline int dtype_size(int dtype) {
   switch (dtype) {

@@ -184,6 +184,7 @@ constexpr int kGroup = 256;   // hidden requests per pass (bounds the scratch)
 bool folded_supported(int dtype, int heads, int head_size, int hidden);
 size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
                               int hidden, int dtype);
-int enqueue_folded_attention(const HybridCall& c, cudaStream_t stream);
+// behind_write: the kernel enqueued last on the stream is launch_new_token_write's.
+int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
 
 }  // namespace aps

@@ -75,7 +75,7 @@ extern "C" int aps_decode_layer_step(void* out, const void* query, const void* h
                    num_heads, head_size, hidden_size, hidden_states_stride, new_key_stride,
                    new_value_stride, block_stride, hidden_row_stride, dtype};
   if ((st = launch_new_token_write(nw, cs)) != APS_OK) return st;
-  if (use_folded(c)) return enqueue_folded_attention(c, cs);
+  if (use_folded(c)) return enqueue_folded_attention(c, hidden_states != nullptr || new_key != nullptr, cs);
   return enqueue_hybrid_attention(c, cs);
 }
 

@@ -175,8 +175,12 @@ __device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int
 struct PlanArgs {
   int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
   const int32_t* seq_lens; const int32_t* cache_type;
-  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target;
+  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target, wait_last;
 };
+
+// Behind the write of the new tokens' cache rows (wait_last) it runs beside it: it reads only the call's
+// arguments, and what it writes (the scratch) was last used by kernels before that write, which were complete when
+// the write let this kernel start.  It waits for the write before it exits.  As a call's first kernel it waits first.
 
 __global__ void __launch_bounds__(kPlanThreads)
 step_plan_kernel(const PlanArgs a) {
@@ -185,6 +189,8 @@ step_plan_kernel(const PlanArgs a) {
   __shared__ int s_req[kGroup], s_len[kGroup], s_toff[kGroup + 1], s_woff[kGroup + 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_missing = 0;
+  if (!a.wait_last) chain_wait();
+  chain_next();
   __syncthreads();
   const int per = (a.batch + kPlanThreads - 1) / kPlanThreads;
   const int r0 = min(a.batch, tid * per), r1 = min(a.batch, r0 + per);
@@ -306,6 +312,7 @@ step_plan_kernel(const PlanArgs a) {
       gp->bound_tile[c] = t; gp->bound_step[c] = step;
     }
   }
+  chain_wait();
 }
 
 // ---- fold ---------------------------------------------------------------------------
@@ -313,6 +320,9 @@ step_plan_kernel(const PlanArgs a) {
 // One CTA per (range of E, head, 128 requests): q is gathered once by all threads into a K-major B operand
 // and stays; W_k,h streams past it in tiles of 128 columns (two boxes of 64 columns x D rows, an MN-major
 // A operand) through a two-stage ring, the accumulators are double-buffered.  Two CTAs per SM.
+// Behind the K/V kernel it does not wait for that kernel (wait_last): it needs the plan, which was complete when the
+// K/V kernel let it start, and writes qt, which no kernel since the plan touches; its CTAs fill the SMs that the
+// K/V kernel leaves.  It waits before it exits.
 // Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
 constexpr int kFoldThreads = 192;
 constexpr int kFoldReqs = 128;
@@ -374,15 +384,16 @@ __device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, in
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kFoldThreads, 2)
-fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
+fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int wait_last) {
   constexpr int NT = kTerms<T>;
   constexpr uint32_t kBox = D * 128, kStage = 2 * kBox;   // 64 columns of E x D rows; two of them
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u, q_at = ring + kFoldStages * kStage;
   __shared__ FoldAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  if (!wait_last) chain_wait();
   const int n = p.plan->n, r0 = blockIdx.z * kFoldReqs, head = blockIdx.y;
-  if (r0 >= n) return;
+  if (r0 >= n) { chain_wait(); return; }
   const int m = min(kFoldReqs, n - r0), np = (m + 15) & ~15;
   const int blocks = p.hidden / 128;
   const int ta = blocks * blockIdx.x / gridDim.x, tb = blocks * (blockIdx.x + 1) / gridDim.x;
@@ -404,6 +415,7 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_next();
   const uint32_t tmem = aux.tmem_base;
   bool ok = true;
   if (warp == 0) {
@@ -472,6 +484,7 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p) {
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_free(tmem, 2 * kFoldReqs); }
+  chain_wait();
 }
 
 // ---- scores -------------------------------------------------------------------------
@@ -521,6 +534,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   __shared__ int s_toff[kGroup + 1], s_len[kGroup], s_req[kGroup];
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   __shared__ ItemRing items;
+  chain_wait();
   GroupPlan* gp = p.plan;
   const int n = gp->n, n_pieces = gp->levels * gp->per_level;
   if (n == 0 || (int)blockIdx.x >= n_pieces) return;
@@ -549,6 +563,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_next();
   const uint32_t tmem = aux.tmem_base;
   volatile int* abort_flag = &aux.abort_flag;
   const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
@@ -707,6 +722,8 @@ softmax_kernel(const Params p) {
   constexpr int NT = kTerms<T>;
   __shared__ float s_max[kSoftmaxWarps], s_sum[kSoftmaxWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  chain_wait();
+  chain_next();
   const GroupPlan* gp = p.plan;
   const int n_units = gp->n * p.heads, levels = gp->levels, per_level = gp->per_level, steps = p.hidden / 128;
   const int64_t units = (int64_t)per_level << (levels - 1);
@@ -829,6 +846,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   __shared__ RingAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   __shared__ ItemRing items;
+  chain_wait();
   GroupPlan* gp = p.plan;
   const int n = gp->n;
   if (n == 0) return;
@@ -848,6 +866,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_next();
   const uint32_t tmem = aux.tmem_base;
   volatile int* abort_flag = &aux.abort_flag;
   const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
@@ -1002,6 +1021,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  chain_wait();
   const int n = p.plan->n, r0 = blockIdx.z * NC;
   if (r0 >= n) return;
   const int m = min(NC, n - r0), boxes = (m + 15) / 16;
@@ -1019,6 +1039,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_next();
   const uint32_t tmem = aux.tmem_base;
   volatile int* abort_flag = &aux.abort_flag;
   const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
@@ -1163,7 +1184,7 @@ int allow_smem(K kernel, size_t bytes, bool* done) {
 struct Maps { CUtensorMap x_scores, x_sum, q, wk, wv, z; };
 
 template <typename T, int D>
-int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, cudaStream_t stream) {
+int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv, cudaStream_t stream) {
   const size_t ring = 1024 + kRingBytes;
   int st;
   {
@@ -1174,33 +1195,32 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, cudaStream_t s
     const int blocks = p.hidden / 128, chunks = (n_cap + kFoldReqs - 1) / kFoldReqs;
     int splits = 2 * sm_count() / p.heads;   // one wave at two CTAs per SM when one chunk of requests is in use
     splits = splits < 1 ? 1 : splits > blocks ? blocks : splits;
-    k<<<dim3(splits, p.heads, chunks), kFoldThreads, smem, stream>>>(m.wk, p);
-    if ((st = launch_status("fold_kernel")) != APS_OK) return st;
+    if ((st = launch_chained("fold_kernel", k, dim3(splits, p.heads, chunks), kFoldThreads, smem, stream, m.wk, p,
+                             behind_kv ? 1 : 0)) != APS_OK) return st;
   }
   {
     static bool done[64] = {false};
     auto k = scores_kernel<T>;
     if ((st = allow_smem(k, 1024 + kScoresRing, done)) != APS_OK) return st;
-    k<<<p.grid_scores, kScoresThreads, 1024 + kScoresRing, stream>>>(m.x_scores, m.q, p);
-    if ((st = launch_status("scores_kernel")) != APS_OK) return st;
+    if ((st = launch_chained("scores_kernel", k, p.grid_scores, kScoresThreads, 1024 + kScoresRing, stream, m.x_scores,
+                             m.q, p)) != APS_OK) return st;
   }
   const int units = n_cap * p.heads, resident = sm_count() * 12;
-  softmax_kernel<T><<<units < resident ? units : resident, kSoftmaxWarps * 32, 0, stream>>>(p);
-  if ((st = launch_status("softmax_kernel")) != APS_OK) return st;
+  if ((st = launch_chained("softmax_kernel", softmax_kernel<T>, units < resident ? units : resident, kSoftmaxWarps * 32, 0,
+                           stream, p)) != APS_OK) return st;
   {
     static bool done[64] = {false};
     auto k = sum_kernel<T>;
     if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
-    k<<<sm_count(), kSumThreads, ring, stream>>>(m.x_sum, p);
-    if ((st = launch_status("sum_kernel")) != APS_OK) return st;
+    if ((st = launch_chained("sum_kernel", k, sm_count(), kSumThreads, ring, stream, m.x_sum, p)) != APS_OK) return st;
   }
   {
     static bool done[64] = {false};
     auto k = unfold_kernel<T, D>;
     if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
     constexpr int kReqs = 128 / (128 / D);
-    k<<<dim3(w_tiles, p.splits, (n_cap + kReqs - 1) / kReqs), kUnfoldThreads, ring, stream>>>(m.wv, m.z, p);
-    if ((st = launch_status("unfold_kernel")) != APS_OK) return st;
+    if ((st = launch_chained("unfold_kernel", k, dim3(w_tiles, p.splits, (n_cap + kReqs - 1) / kReqs), kUnfoldThreads, ring,
+                             stream, m.wv, m.z, p)) != APS_OK) return st;
   }
   return APS_OK;
 }
@@ -1219,7 +1239,7 @@ size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
          layout_of(batch, max_blocks_per_seq, block_size, heads, head_size, hidden, dtype).total;
 }
 
-int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
+int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t cs) {
   const AttnShape& s = c.shape;
   APS_REQUIRE(c.hidden_cache && c.w_k && c.w_v, APS_ERR_NULL_POINTER, "decode_layer_step: null pointer");
   APS_REQUIRE(c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size && c.w_stride >= c.hidden_size,
@@ -1242,10 +1262,9 @@ int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
   pa.hid_slot = reinterpret_cast<int*>(b + l.off_slot); pa.hid_list = reinterpret_cast<int2*>(b + l.off_list);
   pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
-  pa.steps = e_blocks; pa.grid_scores = sm_count(); pa.steps = e_blocks;
-  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 8 * sm_count();
-  step_plan_kernel<<<1, kPlanThreads, 0, cs>>>(pa);
-  if ((st = launch_status("step_plan_kernel")) != APS_OK) return st;
+  pa.steps = e_blocks; pa.grid_scores = sm_count();
+  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 8 * sm_count(); pa.wait_last = behind_write ? 1 : 0;
+  if ((st = launch_chained("step_plan_kernel", step_plan_kernel, 1, kPlanThreads, 0, cs, pa)) != APS_OK) return st;
   if (have_kv &&
       (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
 
@@ -1287,9 +1306,9 @@ int enqueue_folded_attention(const HybridCall& c, cudaStream_t cs) {
     p.group_first = g * kGroup;
     const bool bf16 = s.dtype == APS_BF16;
     switch (s.head_size) {
-      case 128: st = bf16 ? launch_group<__nv_bfloat16, 128>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 128>(m, p, l.n_cap, w_tiles, cs); break;
-      case 64: st = bf16 ? launch_group<__nv_bfloat16, 64>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 64>(m, p, l.n_cap, w_tiles, cs); break;
-      default: st = bf16 ? launch_group<__nv_bfloat16, 32>(m, p, l.n_cap, w_tiles, cs) : launch_group<__half, 32>(m, p, l.n_cap, w_tiles, cs); break;
+      case 128: st = bf16 ? launch_group<__nv_bfloat16, 128>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 128>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
+      case 64: st = bf16 ? launch_group<__nv_bfloat16, 64>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 64>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
+      default: st = bf16 ? launch_group<__nv_bfloat16, 32>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 32>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
     }
     if (st != APS_OK) return st;
   }

@@ -60,6 +60,8 @@ plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restr
   __shared__ int s_kv_missing;
   const int tid = threadIdx.x;
   if (tid == 0) s_kv_missing = 0;
+  chain_wait();
+  chain_next();
   __syncthreads();
   const int per = (batch + kPlanThreads - 1) / kPlanThreads;
   const int r0 = min(batch, tid * per), r1 = min(batch, r0 + per);
@@ -205,6 +207,8 @@ kv_attention_kernel(int* __restrict__ plan, const int* __restrict__ part_offset,
   __shared__ int s_base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % C::LPR, tsel = lane / C::LPR;
+  chain_wait();
+  chain_next();
   const int total = plan[kPlanNumKvChunks] * heads;
   const int64_t row_stride = (int64_t)heads * D;
 
@@ -409,7 +413,6 @@ kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   __shared__ uint64_t bars[kTmaWarps][S];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, j = lane & 3;
-  const int total = plan[kPlanNumKvChunks] * heads;
   const uint32_t ring = (((uint32_t)__cvta_generic_to_shared(ring_raw) + 1023u) & ~1023u) + warp * (S * kStageBytes);
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(&bars[warp][0]);
   if (lane == 0) {
@@ -419,6 +422,9 @@ kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
+  chain_wait();
+  chain_next();
+  const int total = plan[kPlanNumKvChunks] * heads;
 
   auto next_index = [&]() {
     int idx = 0;
@@ -626,6 +632,8 @@ combine_kernel(const int* __restrict__ plan, const int* __restrict__ part_offset
                int head_size, int64_t out_stride, const HiddenOutputs hid) {
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  chain_wait();
+  chain_next();
   if (unit >= batch * heads) return;
   const int req = unit / heads, h = unit % heads;
   const int p0 = part_offset[req], p1 = part_offset[req + 1];
@@ -732,21 +740,19 @@ int launch_kv_typed(const WorkspacePtrs& ws, const void* query, const void* key_
       int per_sm = 0;
       APS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTmaWarps * 32, kSmem));
       APS_REQUIRE(per_sm > 0, APS_ERR_CUDA, "the K/V streaming kernel does not fit on this device");
-      kernel<<<sm_count() * per_sm, kTmaWarps * 32, kSmem, stream>>>(
-          mk, mv, ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query, block_tables,
-          seq_lens, s.max_blocks_per_seq, s.heads, s.block_size, s.query_stride, scale_log2);
-      return launch_status("kv_attention_tma_kernel");
+      return launch_chained("kv_attention_tma_kernel", kernel, sm_count() * per_sm, kTmaWarps * 32, kSmem, stream,
+                            mk, mv, ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query,
+                            block_tables, seq_lens, s.max_blocks_per_seq, s.heads, s.block_size, s.query_stride, scale_log2);
     }
   }
   ScopedProfile prof(0, stream);
   // CUDA-core arithmetic: 2 persistent CTAs of 8 warps per SM
   const int grid = sm_count() * 2;
   const int threads = kKvWarps * 32;
-  kv_attention_kernel<T, D><<<grid, threads, 0, stream>>>(
+  return launch_chained("kv_attention_kernel", kv_attention_kernel<T, D>, grid, threads, 0, stream,
       ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query,
       (const T*)key_cache, (const T*)value_cache, block_tables, seq_lens, s.max_blocks_per_seq,
       s.heads, s.block_size, s.query_stride, s.block_stride, scale_log2);
-  return launch_status("kv_attention_kernel");
 }
 
 template <typename T>
@@ -775,12 +781,10 @@ bool kv_attention_supported(int dtype, int head_size) {
 int launch_plan(const WorkspacePtrs& ws, const int32_t* seq_lens, const int32_t* cache_type,
                 const int32_t* block_tables, int batch, int max_blocks_per_seq, int block_size,
                 bool pack_tiles, bool kv_present, cudaStream_t stream) {
-  plan_kernel<<<1, kPlanThreads, 0, stream>>>(ws.plan, ws.part_offset, ws.kv_chunks, ws.hid_tiles,
-                                              ws.first_tile, ws.hid_subs, ws.hid_rows, seq_lens,
-                                              cache_type, block_tables, batch,
-                                              max_blocks_per_seq * block_size, max_blocks_per_seq,
-                                              block_size, pack_tiles ? 1 : 0, kv_present ? 1 : 0);
-  return launch_status("plan_kernel");
+  return launch_chained("plan_kernel", plan_kernel, 1, kPlanThreads, 0, stream, ws.plan, ws.part_offset, ws.kv_chunks,
+                        ws.hid_tiles, ws.first_tile, ws.hid_subs, ws.hid_rows, seq_lens, cache_type, block_tables,
+                        batch, max_blocks_per_seq * block_size, max_blocks_per_seq, block_size, pack_tiles ? 1 : 0,
+                        kv_present ? 1 : 0);
 }
 
 int launch_kv_attention(const WorkspacePtrs& ws, const void* query, const void* key_cache,
@@ -801,20 +805,16 @@ int launch_combine(const WorkspacePtrs& ws, void* out, const HiddenOutputs* hidd
   const int grid = (units + 7) / 8;
   switch (s.dtype) {
     case APS_F32:
-      combine_kernel<float><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                     (float*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
-      break;
+      return launch_chained("combine_kernel", combine_kernel<float>, grid, 256, 0, stream, ws.plan, ws.part_offset,
+                            ws.part_ml, ws.part_acc, (float*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
     case APS_F16:
-      combine_kernel<__half><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                      (__half*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
-      break;
+      return launch_chained("combine_kernel", combine_kernel<__half>, grid, 256, 0, stream, ws.plan, ws.part_offset,
+                            ws.part_ml, ws.part_acc, (__half*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
     case APS_BF16:
-      combine_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(ws.plan, ws.part_offset, ws.part_ml, ws.part_acc,
-                                                             (__nv_bfloat16*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
-      break;
+      return launch_chained("combine_kernel", combine_kernel<__nv_bfloat16>, grid, 256, 0, stream, ws.plan, ws.part_offset,
+                            ws.part_ml, ws.part_acc, (__nv_bfloat16*)out, s.batch, s.heads, s.head_size, s.out_stride, hid);
     default: return fail(APS_ERR_DTYPE, "decode attention: unsupported dtype %d", s.dtype);
   }
-  return launch_status("combine_kernel");
 }
 
 // Argument checks shared by the two attention entry points.

@@ -105,3 +105,59 @@ def test_small_and_large_queries_keep_their_bits():
     for r, s in enumerate((1e-6, 1e-4, 1e-2, 1.0, 8.0, 30.0, 1e-6, 1e-4, 1e-2, 1.0, 8.0, 0.0)):
         w.query[r] *= s
     check(w, "query sizes")
+
+
+def _step_into(w, out, ws):
+    m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
+    return A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache, wk, bk, wv,
+                               bv, m.private_block_tables, m.seq_lens_tensor, m.cache_type, w.scale, out=out, workspace=ws)
+
+
+def _chain_workloads():
+    lens = [300, 17, 640, 1, 256, 120, 900, 33]
+    return [make_decode_workload(LayerShape("t", 8, d, 1024, t), [x + 3 * i for x in lens], h, seed=30 + i, device="cuda")
+            for i, (d, t, h) in enumerate([(128, F, [True, False] * 4), (64, B, [True] * 8), (128, B, [False, True] * 4),
+                                           (64, F, [True, True, False, False] * 2)])]
+
+
+def test_steps_that_follow_each_other_on_one_scratch():
+    """The launches of a step overlap; steps of different shapes, enqueued without a wait between them on one
+    scratch, with the step's inputs written just before it, give what each gives alone."""
+    ws = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    ws_kv = A.attention_workspace(ws.device, 8, 64, 16, 8, 128)
+    cases = _chain_workloads()
+    want = []
+    for w in cases:
+        want.append((_step_into(w, torch.empty_like(w.query), ws), A.paged_decode_attention(
+            w.query, w.kv_cache[0], w.kv_cache[1], w.meta.private_block_tables % w.kv_cache.shape[1], w.meta.seq_lens_tensor,
+            w.scale, workspace=ws_kv)))
+        torch.cuda.synchronize()
+    live = [w.query.clone() for w in cases]
+    for _ in range(20):
+        got = []
+        for w, q in zip(cases, live):
+            w.query.zero_()
+            out = torch.full_like(w.query, float("nan"))
+            w.query.copy_(q)
+            got.append((_step_into(w, out, ws), A.paged_decode_attention(
+                w.query, w.kv_cache[0], w.kv_cache[1], w.meta.private_block_tables % w.kv_cache.shape[1],
+                w.meta.seq_lens_tensor, w.scale, workspace=ws)))
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+def test_chained_step_replays_from_a_cuda_graph():
+    ws = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    for w in _chain_workloads()[:2]:
+        want = _step_into(w, torch.empty_like(w.query), ws).clone()
+        torch.cuda.synchronize()
+        out, g = torch.empty_like(w.query), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            _step_into(w, out, ws)
+            _step_into(w, out, ws)
+        for _ in range(3):
+            out.zero_()
+            g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
