@@ -187,7 +187,9 @@ def hybrid_decode_attention(query: torch.Tensor, kv_cache: Optional[torch.Tensor
     sl = _i32(seq_lens, "seq_lens")
     ct = _i32(cache_type, "cache_type")
     if workspace is None:
-        workspace = attention_workspace(dev, b, bt.shape[1], bs, h, d)
+        # fp32: the layer-step's scratch lets the call attend the hidden rows directly, as the layer-step does
+        workspace = (layer_step_workspace(dev, b, bt.shape[1], bs, h, d, e, query.dtype)
+                     if query.dtype == torch.float32 else attention_workspace(dev, b, bt.shape[1], bs, h, d))
     with torch.cuda.device(dev):
         N.check(N.lib().aps_hybrid_decode_attention(
             N.ptr(out), N.ptr(query), N.ptr(kc), N.ptr(vc), N.ptr(hidden_cache), N.ptr(w_k),

@@ -187,4 +187,10 @@ size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
 // behind_write: the kernel enqueued last on the stream is launch_new_token_write's.
 int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
 
+// Its fp32 counterpart on the CUDA cores (hidden_fp32.cu).
+bool folded32_shape(int dtype, int heads, int head_size, int hidden);
+bool folded32_supported(const HybridCall& c);
+size_t folded32_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size, int hidden);
+int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
+
 }  // namespace aps

@@ -75,13 +75,17 @@ extern "C" int aps_decode_layer_step(void* out, const void* query, const void* h
                    num_heads, head_size, hidden_size, hidden_states_stride, new_key_stride,
                    new_value_stride, block_stride, hidden_row_stride, dtype};
   if ((st = launch_new_token_write(nw, cs)) != APS_OK) return st;
-  if (use_folded(c)) return enqueue_folded_attention(c, hidden_states != nullptr || new_key != nullptr, cs);
+  const bool behind_write = hidden_states != nullptr || new_key != nullptr;
+  if (use_folded(c)) return enqueue_folded_attention(c, behind_write, cs);
+  if (folded32_supported(c)) return enqueue_folded32_attention(c, behind_write, cs);
   return enqueue_hybrid_attention(c, cs);
 }
 
 extern "C" size_t aps_decode_layer_step_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
                                                         int num_heads, int head_size, int hidden_size, int dtype) {
   const size_t base = aps_attention_workspace_bytes(batch, max_blocks_per_seq, block_size, num_heads, head_size);
+  if (base != 0 && folded32_shape(dtype, num_heads, head_size, hidden_size))
+    return folded32_workspace_bytes(batch, max_blocks_per_seq, block_size, num_heads, head_size, hidden_size);
   if (base == 0 || !folded_shape(batch, max_blocks_per_seq, block_size, num_heads, head_size, hidden_size, dtype)) return base;
   return folded_workspace_bytes(batch, max_blocks_per_seq, block_size, num_heads, head_size, hidden_size, dtype);
 }

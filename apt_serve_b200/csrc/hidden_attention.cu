@@ -38,6 +38,7 @@
 
 #include "attention_common.cuh"
 #include "sm100.cuh"
+#include "step_plan.cuh"
 #include "tensor_maps.cuh"
 
 #include <type_traits>
@@ -50,32 +51,12 @@ constexpr int kSubs = kTile / 16;         // 16-row boxes of the hidden cache pe
 constexpr int kTileCost = 4;              // fixed cost of a tile in boxes (its qt slab), for the work split
 constexpr int kStepTokens = 32;           // tokens per stage of the sum kernel
 constexpr int kMinPiece = 2 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: two full steps
-constexpr int kMaxGrid = 192;             // most SMs the plan keeps bounds of pieces for
-constexpr int kMaxLevels = 5;             // sizes of pieces the scores work is cut into
-constexpr int kMaxPieces = kMaxGrid * kMaxLevels;
 constexpr int kMaxSlice = 8;              // 128-column blocks of E per work item of the sum kernel
 constexpr float kProbShift = 15.f;        // p is kept at 2^15 times its value (fp16 range)
 constexpr size_t kRingBytes = 200 * 1024; // shared memory of the operand rings
 
 template <typename T> constexpr int kTerms = std::is_same<T, __nv_bfloat16>::value ? 3 : 2;
 template <typename T> constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-
-// ---- the plan of one group of hidden requests (device memory) --------------------------
-struct GroupPlan {
-  int n;                      // requests of the group
-  int n_tiles;                // scores tiles
-  int weight;                 // total cost of the tiles, in boxes
-  int slice;                  // 128-column blocks per item of the sum kernel
-  int levels, per_level;      // pieces of the scores work: levels x per_level
-  int next_piece, next_item;  // work counters of the scores and the sum kernel
-  int req[kGroup];            // batch row of each request, longest first
-  int len[kGroup];            // its length in tokens
-  int tile_off[kGroup + 1];   // first scores tile
-  int blk_off[kGroup + 1];    // first 16-token block of p
-  int w_off[kGroup + 1];      // cost of the tiles before it
-  int bound_tile[kMaxPieces + 1];   // piece c: from (bound_tile[c], bound_step[c]) to the next bound
-  int bound_step[kMaxPieces + 1];
-};
 
 // The scores work is a line of X box-steps, cut into pieces that are handed out in order: `levels` sizes, each
 // half of the one before (the last two alike), `per_level` pieces of each.  Large pieces first keep the
@@ -171,12 +152,6 @@ __device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int
   if (warp > 0) { v.x += bx; v.y += by; }
   return v;   // inclusive
 }
-
-struct PlanArgs {
-  int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
-  const int32_t* seq_lens; const int32_t* cache_type;
-  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target, wait_last;
-};
 
 // Behind the write of the new tokens' cache rows (wait_last) it runs beside it: it reads only the call's
 // arguments, and what it writes (the scratch) was last used by kernels before that write, which were complete when
@@ -1227,6 +1202,10 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv
 
 }  // namespace
 
+int launch_step_plan(const PlanArgs& a, cudaStream_t stream) {
+  return launch_chained("step_plan_kernel", step_plan_kernel, 1, kPlanThreads, 0, stream, a);
+}
+
 bool folded_supported(int dtype, int heads, int head_size, int hidden) {
   return (dtype == APS_F16 || dtype == APS_BF16) && (head_size == 128 || head_size == 64 || head_size == 32) &&
          heads > 0 && heads <= 256 && hidden > 0 && hidden % 128 == 0 &&
@@ -1264,7 +1243,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
   pa.steps = e_blocks; pa.grid_scores = sm_count();
   pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 8 * sm_count(); pa.wait_last = behind_write ? 1 : 0;
-  if ((st = launch_chained("step_plan_kernel", step_plan_kernel, 1, kPlanThreads, 0, cs, pa)) != APS_OK) return st;
+  if ((st = launch_step_plan(pa, cs)) != APS_OK) return st;
   if (have_kv &&
       (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
 

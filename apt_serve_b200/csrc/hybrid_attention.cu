@@ -924,6 +924,9 @@ extern "C" int aps_hybrid_decode_attention(void* out, const void* query, const v
   c.workspace = workspace; c.workspace_bytes = workspace_bytes;
   int st = check_hybrid_call("hybrid_decode_attention", c);
   if (st != APS_OK || batch == 0) return st;
+  // fp32 has no tensor-core form of the re-projection to prefer: with the layer-step's scratch the hidden rows
+  // are attended directly here too
+  if (folded32_supported(c)) return enqueue_folded32_attention(c, false, (cudaStream_t)stream);
   return enqueue_hybrid_attention(c, (cudaStream_t)stream);
 }
 

@@ -1,0 +1,37 @@
+// The device-side plan of a layer-step whose hidden-cached requests are attended directly: the K/V kernel's chunk list
+// and the groups of hidden-cached requests.  Written by step_plan_kernel (hidden_attention.cu).
+#pragma once
+
+#include "attention_common.cuh"
+
+namespace aps {
+
+constexpr int kMaxGrid = 192;             // most SMs the plan keeps bounds of pieces for
+constexpr int kMaxLevels = 5;             // sizes of pieces the scores work is cut into
+constexpr int kMaxPieces = kMaxGrid * kMaxLevels;
+
+// ---- the plan of one group of hidden requests (device memory) --------------------------
+struct GroupPlan {
+  int n;                      // requests of the group
+  int n_tiles;                // scores tiles
+  int weight;                 // total cost of the tiles, in boxes
+  int slice;                  // 128-column blocks per item of the sum kernel
+  int levels, per_level;      // pieces of the scores work: levels x per_level
+  int next_piece, next_item;  // work counters of the scores and the sum kernel
+  int req[kGroup];            // batch row of each request, longest first
+  int len[kGroup];            // its length in tokens
+  int tile_off[kGroup + 1];   // first scores tile
+  int blk_off[kGroup + 1];    // first 16-token block of p
+  int w_off[kGroup + 1];      // cost of the tiles before it
+  int bound_tile[kMaxPieces + 1];   // piece c: from (bound_tile[c], bound_step[c]) to the next bound
+  int bound_step[kMaxPieces + 1];
+};
+
+struct PlanArgs {
+  int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
+  const int32_t* seq_lens; const int32_t* cache_type;
+  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target, wait_last;
+};
+int launch_step_plan(const PlanArgs& a, cudaStream_t stream);
+
+}  // namespace aps

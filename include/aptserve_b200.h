@@ -247,7 +247,9 @@ int aps_paged_decode_attention_static(void* out, const void* query, const void* 
  * (2*NB*BS for the reference layout).  fp16 / bf16 with head_size 128, 64 or 32 and
  * num_heads * head_size a multiple of 128 use the tcgen05 path (two heads of 64 or four
  * of 32 share one accumulator tile); other supported combinations (fp32, other head
- * counts) use a CUDA-core re-projection.
+ * counts) use a CUDA-core re-projection, or, in fp32 with hidden_size and strides in multiples of
+ * four and a workspace of aps_decode_layer_step_workspace_bytes, attend the rows directly (see
+ * aps_decode_layer_step).
  * key_cache / value_cache may both be NULL for a batch without K/V-cached requests;
  * if such a batch does hold K/V-cached requests their output rows are zero and the
  * status word (aps_attention_status) reads 8.
@@ -294,9 +296,10 @@ int aps_kv_reprojection(void* kv, const void* x, const int32_t* block_ids, int64
  *      mixed_kv_to_cache, fa.py:363-373, or reshape_and_cache_flash, fa.py:338-345);
  *   2. the attention of aps_hybrid_decode_attention over the batch.  With a workspace of
  *      aps_decode_layer_step_workspace_bytes the hidden-cached requests of fp16 / bf16 layers
- *      (head size 128, 64 or 32, hidden_size a multiple of 128) are attended directly:
+ *      (head size 128, 64 or 32, hidden_size a multiple of 128; fp32: a multiple of 4) are
+ *      attended directly:
  *      scores X (W_k^T q), outputs W_v (P X) + b_v, which is the same result without
- *      re-projecting the rows; a batch of at most one wave of the re-projection kernel, any
+ *      re-projecting the rows; a 16-bit batch of at most one wave of the re-projection kernel, any
  *      other shape and a smaller workspace are re-projected.
  * hidden_states [B, hidden_size], new_key / new_value [B, H*D] (rows of the other
  * cache type are ignored; a NULL pointer skips that kind of write), every pointer
