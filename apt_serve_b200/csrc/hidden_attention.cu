@@ -494,6 +494,11 @@ struct Ring {
 };
 
 __host__ __device__ inline uint32_t scores_q_bytes(int terms, int np) { return (uint32_t)terms * np * 256; }
+// The terms of qt as further columns of the B operand (N = terms x np, an accumulator per term, added in the epilogue)
+// where N and the accumulators allow: the tensor cores read every X row from shared memory once per instruction, 4 KB
+// or 32 cycles of its bandwidth against 12 - 24 of arithmetic, so an instruction per term costs two or three
+// times that.
+__host__ __device__ inline bool stacked_terms(int terms, int np) { return terms * np <= 256; }
 // qt units in the ring: two unless they leave less than two units of X
 __host__ __device__ inline int scores_q_units(int terms, int np) {
   return 2 * scores_q_bytes(terms, np) + 2 * kUnitBytes <= kScoresRing ? 2 : 1;
@@ -521,9 +526,10 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   const uint32_t q_bytes = scores_q_bytes(NT, np);
   const int nq = scores_q_units(NT, np), nx = min(kMaxStages, (int)((kScoresRing - nq * q_bytes) / kUnitBytes));
   const uint32_t q_ring = x_ring + nx * kUnitBytes;
-  const int n_buf = 4 * np <= 512 ? 2 : 1;
+  const int n_acc = stacked_terms(NT, np) ? NT * np : np, n_rep = stacked_terms(NT, np) ? 1 : NT;
+  const int n_buf = 4 * n_acc <= 512 ? 2 : 1;
   uint32_t tmem_cols = 32;
-  while (tmem_cols < (uint32_t)(n_buf * 2 * np)) tmem_cols <<= 1;
+  while (tmem_cols < (uint32_t)(n_buf * 2 * n_acc)) tmem_cols <<= 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < nx; ++s) { mbar_init(&aux.full[s], 2); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < 2; ++b) {
@@ -591,8 +597,8 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
           const uint32_t bar = q_full0 + qr.stage * 8;
           if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
           __syncwarp();
-          if (lane < 2 * NT)   // lane = (term, half of the columns)
-            tma_load_2d_cta(q_ring + qr.stage * q_bytes + lane * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
+          if (lane < 2 * NT)   // lane = (term, half of the columns); the terms of a half lie one behind the other
+            tma_load_2d_cta(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
           __syncwarp();
           qr.step(nq);
         }
@@ -628,7 +634,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
       } else if (warp == 1) {
         if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, false);
+        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)n_acc, false);
         for (int s = sa; s < sb && ok; ++s) {
           if (!mbar_wait_warp(q_full0 + qr.stage * 8, qr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
           for (int m = 0; m < n_m; ++m) {
@@ -636,15 +642,14 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             tc_fence_after();
             if (elect_one()) {
               const uint32_t a_lo = desc_lo(x_ring + xr.stage * kUnitBytes, 16), b_lo = desc_lo(q_ring + qr.stage * q_bytes, 16);
-              const uint32_t d = tmem + (buf * 2 + m) * np;
+              const uint32_t d = tmem + (buf * 2 + m) * n_acc;
               uint32_t acc = s != sa;
   #pragma unroll
               for (int j = 0; j < 2; ++j)
   #pragma unroll
                 for (int k = 0; k < 4; ++k)
-  #pragma unroll
-                  for (int i = 0; i < NT; ++i) {
-                    tc_mma_cta(d, a_lo + j * 64 + k * 2, desc_hi(2048, true), b_lo + (i * 2 + j) * (np * 8) + k * 2, desc_hi(1024, true), idesc, acc);
+                  for (int i = 0; i < n_rep; ++i) {
+                    tc_mma_cta(d, a_lo + j * 64 + k * 2, desc_hi(2048, true), b_lo + (j * NT + i) * (np * 8) + k * 2, desc_hi(1024, true), idesc, acc);
                     acc = 1u;
                   }
               tc_commit_cta(empty0 + xr.stage * 8);
@@ -664,12 +669,26 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         float* dst = p.scores + (int64_t)(t + piece) * p.heads * kTile;
         for (int m = 0; m < n_m; ++m)
           for (int h0 = 0; h0 < np; h0 += 16) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * np + h0, v);
+            const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * n_acc + h0;
+            uint32_t v[NT][16];
+            tmem_ld16(at, v[0]);
+            if (n_rep == 1) {
+  #pragma unroll
+              for (int i = 1; i < NT; ++i) tmem_ld16(at + i * np, v[i]);
+            }
             tmem_ld_wait();
+            if (n_rep == 1) {   // the smaller terms' sums first
+  #pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                float x = __uint_as_float(v[NT - 1][j]);
+  #pragma unroll
+                for (int i = NT - 2; i >= 0; --i) x += __uint_as_float(v[i][j]);
+                v[0][j] = __float_as_uint(x);
+              }
+            }
   #pragma unroll
             for (int j = 0; j < 16; ++j)
-              if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[j]);
+              if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[0][j]);
           }
         tc_fence_before();
         __syncwarp();
