@@ -51,7 +51,8 @@ constexpr int kSubs = kTile / 16;         // 16-row boxes of the hidden cache pe
 constexpr int kTileCost = 4;              // fixed cost of a tile in boxes (its qt slab), for the work split
 constexpr int kStepTokens = 32;           // tokens per stage of the sum kernel
 constexpr int kMinPiece = 2 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: two full steps
-constexpr int kMaxSlice = 8;              // 128-column blocks of E per work item of the sum kernel
+constexpr int kMaxSlice = 4;              // 128-column blocks of E per work item of the sum kernel
+constexpr int kSumRounds = 2;             // work items per SM below which it takes narrower slices
 constexpr float kProbShift = 15.f;        // p is kept at 2^15 times its value (fp16 range)
 constexpr size_t kRingBytes = 200 * 1024; // shared memory of the operand rings
 
@@ -259,7 +260,11 @@ step_plan_kernel(const PlanArgs a) {
     __syncthreads();
     const int n_tiles = s_toff[n], weight = s_woff[n];
     if (tid == 0) {
-      // sum kernel: the widest slice of E that still gives item_target items
+      // sum kernel: the widest slice of E that still gives item_target items.  Wide slices leave a DRAM page after
+      // up to 1 KB of a row, not 256 bytes, and read the weights less often (a slice of one block reads as many bytes of
+      // weights as of rows); more items even out requests of different lengths.  On one B200, slices of 1 / 2 / 3 /
+      // 4 / 5 blocks: 24 requests of 1800 OPT-13B tokens 127 / 89 / 80 / 87 / - us, 128 of 740 - / 236 / 197 / 186 /
+      // 192, 52 of 950 OPT-66B tp 8 - / 255 / 177 / 167 / 172 (six), 34 of 500 OPT-1.3B 36 / 54 / - / 53 / 68.
       int slice = a.max_slice;
       while (slice > 1 && n * ((a.steps + slice - 1) / slice) < a.item_target) --slice;
       gp->n = n; gp->n_tiles = n_tiles; gp->weight = weight; gp->slice = slice;
@@ -1261,7 +1266,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
   pa.steps = e_blocks; pa.grid_scores = sm_count();
-  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = 8 * sm_count(); pa.wait_last = behind_write ? 1 : 0;
+  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = kSumRounds * sm_count(); pa.wait_last = behind_write ? 1 : 0;
   if ((st = launch_step_plan(pa, cs)) != APS_OK) return st;
   if (have_kv &&
       (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
