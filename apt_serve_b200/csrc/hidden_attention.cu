@@ -480,11 +480,12 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
 // tile.  Warps: 0 qt boxes, 1 MMA issue, 2-5 epilogue, 6-7 boxes of X (eight lanes each).
 constexpr int kScoresThreads = 256;
 constexpr int kMaxStages = 12;
+constexpr int kMaxQUnits = 3;
 constexpr uint32_t kUnitBytes = 128 * 256;
 constexpr size_t kScoresRing = 216 * 1024;
 
 struct RingAux {
-  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], q_full[2], q_empty[2];
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], q_full[kMaxQUnits], q_empty[kMaxQUnits];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -504,9 +505,14 @@ __host__ __device__ inline uint32_t scores_q_bytes(int terms, int np) { return (
 // or 32 cycles of its bandwidth against 12 - 24 of arithmetic, so an instruction per term costs two or three
 // times that.
 __host__ __device__ inline bool stacked_terms(int terms, int np) { return terms * np <= 256; }
-// qt units in the ring: two unless they leave less than two units of X
+// qt units in the ring: a step of a short tile takes less time than a unit's round trip, so three of them where that
+// leaves three units of X (two and two, one otherwise).  Two -> three: scores of 128 OPT-13B requests of 740 tokens
+// 213 -> 207 us, of 64 of 340 71 -> 67, of 52 OPT-66B tp 8 requests 182 -> 170; with four and fewer units of X the
+// bf16 layers lose it again.
 __host__ __device__ inline int scores_q_units(int terms, int np) {
-  return 2 * scores_q_bytes(terms, np) + 2 * kUnitBytes <= kScoresRing ? 2 : 1;
+  for (int n = kMaxQUnits; n > 1; --n)
+    if (n * scores_q_bytes(terms, np) + n * kUnitBytes <= kScoresRing) return n;
+  return 1;
 }
 
 template <typename T>
@@ -537,10 +543,8 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   while (tmem_cols < (uint32_t)(n_buf * 2 * n_acc)) tmem_cols <<= 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < nx; ++s) { mbar_init(&aux.full[s], 2); mbar_init(&aux.empty[s], 1); }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&aux.q_full[b], 1); mbar_init(&aux.q_empty[b], 1);
-      mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4);
-    }
+    for (int b = 0; b < kMaxQUnits; ++b) { mbar_init(&aux.q_full[b], 1); mbar_init(&aux.q_empty[b], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
     for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], kScoresThreads / 32 - 1); }
     aux.abort_flag = 0;
     mbar_init_fence();
