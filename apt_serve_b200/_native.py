@@ -13,6 +13,7 @@ from pathlib import Path
 import torch
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libaptserve_b200.so"
+HOST_LIB_PATH = LIB_PATH.with_name("libaptserve_b200_host.so")
 
 APS_OK = 0
 APS_ERR_NULL_POINTER = 1
@@ -95,6 +96,23 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host_lib = None
+
+
+def host_lib() -> ctypes.PyDLL:
+    """The library that reads Python lists (called with the interpreter lock held); raises if it has not been built."""
+    global _host_lib
+    if _host_lib is None:
+        if not HOST_LIB_PATH.exists():
+            raise RuntimeError(f"{HOST_LIB_PATH} is missing (run `python -m apt_serve_b200.build`)")
+        handle = ctypes.PyDLL(str(HOST_LIB_PATH))
+        handle.aps_pack_block_tables.restype = c_int
+        handle.aps_pack_block_tables.argtypes = [ctypes.py_object, ctypes.py_object, c_void_p, c_int64, c_int64,
+                                                 c_void_p, c_void_p, c_void_p]
+        _host_lib = handle
+    return _host_lib
+
+
 def check(status: int) -> None:
     """Turn a non-zero ``aps_status`` into the exception the reference would
     raise: ``ValueError`` for unsupported head / block sizes and dtypes
@@ -116,7 +134,7 @@ def dtype_enum(t: torch.Tensor) -> int:
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
-    dev = None
+    dev, index = None, -1
     for t in tensors:
         if t is None:
             continue
@@ -124,8 +142,8 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
             raise RuntimeError("aptserve_b200 operators run on CUDA tensors only "
                                "(there is no CPU path)")
         if dev is None:
-            dev = t.device
-        elif t.device != dev:
+            dev, index = t.device, t.get_device()
+        elif t.get_device() != index:
             raise RuntimeError("aptserve_b200: tensors live on different devices")
     return dev
 
@@ -134,5 +152,27 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+class _Nothing:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_nothing = _Nothing()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, which costs a few microseconds a call, only where it is not current already."""
+    return _nothing if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def current_stream(device: torch.device) -> int:
+    """The current stream's handle, without building a Stream object around it where torch offers that."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream

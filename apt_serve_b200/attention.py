@@ -62,7 +62,7 @@ def attention_status(workspace: torch.Tensor) -> int:
     import ctypes
     host = ctypes.c_int(0)
     dev = workspace.device
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_attention_status(N.ptr(workspace), ctypes.addressof(host),
                                              N.current_stream(dev)))
     return host.value
@@ -74,7 +74,7 @@ def reprojection_cycles(workspace: torch.Tensor) -> int:
     import ctypes
     host = ctypes.c_ulonglong(0)
     dev = workspace.device
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_reprojection_cycles(N.ptr(workspace), ctypes.addressof(host),
                                                 N.current_stream(dev)))
     return host.value
@@ -131,7 +131,7 @@ def paged_decode_attention(query: torch.Tensor, key_cache: torch.Tensor,
     sl = _i32(seq_lens, "seq_lens")
     if workspace is None:
         workspace = attention_workspace(dev, b, bt.shape[1], bs, h, d)
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_paged_decode_attention(
             N.ptr(out), N.ptr(query), N.ptr(key_cache), N.ptr(value_cache), N.ptr(bt), N.ptr(sl),
             b, bt.shape[1], h, d, bs, query.stride(0), out.stride(0), key_cache.stride(0),
@@ -168,12 +168,13 @@ def hybrid_decode_attention(query: torch.Tensor, kv_cache: Optional[torch.Tensor
         return out
     if kv_cache is not None:
         _, _, bs, h, d = kv_cache.shape
-        kc, vc, block_stride = kv_cache[0], kv_cache[1], kv_cache.stride(1)
+        kc, block_stride = kv_cache.data_ptr(), kv_cache.stride(1)
+        vc = kc + kv_cache.stride(0) * kv_cache.element_size()
     else:
         if num_heads is None or head_size is None:
             raise RuntimeError("hybrid_decode_attention: num_heads / head_size needed without kv_cache")
         bs, h, d = hidden_cache.shape[2], num_heads, head_size
-        kc = vc = None
+        kc = vc = 0
         block_stride = bs * h * d
     e = w_k.shape[1]
     if w_k.shape != w_v.shape or w_k.stride(0) != w_v.stride(0) or w_k.stride(1) != 1:
@@ -190,9 +191,9 @@ def hybrid_decode_attention(query: torch.Tensor, kv_cache: Optional[torch.Tensor
         # fp32: the layer-step's scratch lets the call attend the hidden rows directly, as the layer-step does
         workspace = (layer_step_workspace(dev, b, bt.shape[1], bs, h, d, e, query.dtype)
                      if query.dtype == torch.float32 else attention_workspace(dev, b, bt.shape[1], bs, h, d))
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_hybrid_decode_attention(
-            N.ptr(out), N.ptr(query), N.ptr(kc), N.ptr(vc), N.ptr(hidden_cache), N.ptr(w_k),
+            N.ptr(out), N.ptr(query), kc, vc, N.ptr(hidden_cache), N.ptr(w_k),
             N.ptr(b_k), N.ptr(w_v), N.ptr(b_v), N.ptr(bt), N.ptr(sl), N.ptr(ct), b, bt.shape[1],
             h, d, e, bs, query.stride(0), out.stride(0), block_stride, row_stride, n_rows,
             w_k.stride(0), float(scale), N.ptr(workspace), workspace.numel(),
@@ -227,12 +228,13 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
         return out
     if kv_cache is not None:
         _, _, bs, h, d = kv_cache.shape
-        kc, vc, block_stride = kv_cache[0], kv_cache[1], kv_cache.stride(1)
+        kc, block_stride = kv_cache.data_ptr(), kv_cache.stride(1)
+        vc = kc + kv_cache.stride(0) * kv_cache.element_size()
     else:
         if num_heads is None or head_size is None:
             raise RuntimeError("decode_layer_step: num_heads / head_size needed without kv_cache")
         bs, h, d = hidden_cache.shape[2], num_heads, head_size
-        kc = vc = None
+        kc = vc = 0
         block_stride = bs * h * d
         new_key = new_value = None
     e = w_k.shape[1]
@@ -252,10 +254,10 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
     ct = _i32(cache_type, "cache_type")
     if workspace is None:
         workspace = layer_step_workspace(dev, b, bt.shape[1], bs, h, d, e, query.dtype)
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_decode_layer_step(
             N.ptr(out), N.ptr(query), N.ptr(hidden_states), N.ptr(new_key), N.ptr(new_value),
-            N.ptr(kc), N.ptr(vc), N.ptr(hidden_cache), N.ptr(w_k), N.ptr(b_k), N.ptr(w_v), N.ptr(b_v),
+            kc, vc, N.ptr(hidden_cache), N.ptr(w_k), N.ptr(b_k), N.ptr(w_v), N.ptr(b_v),
             N.ptr(bt), N.ptr(sl), N.ptr(ct), b, bt.shape[1], h, d, e, bs, query.stride(0), out.stride(0),
             0 if hidden_states is None else hidden_states.stride(0),
             0 if new_key is None else new_key.stride(0), 0 if new_value is None else new_value.stride(0),
@@ -339,7 +341,7 @@ def hybrid_decode_attention_absorbed(query: torch.Tensor, kv_cache: Optional[tor
     rows32 = rows64.to(torch.int32)
     hp = (h + 15) // 16 * 16
     log2e = 1.4426950408889634
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         # fold: qa[h][i] = scale * log2(e) * W_k,h^T q[i][h]  (one batched GEMM over the heads,
         # written in place: the kernels take the head-major layout)
         q_h = (query.index_select(0, rows64).view(n_h, h, d).transpose(0, 1).float() * (scale * log2e)).to(query.dtype)
@@ -390,7 +392,7 @@ def kv_reprojection(x: torch.Tensor, w_k: torch.Tensor, b_k: Optional[torch.Tens
     if out is None:
         out = torch.empty(n, 2 * hd, dtype=x.dtype, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_kv_reprojection(
             N.ptr(out), N.ptr(x), N.ptr(block_ids), n, N.ptr(w_k), N.ptr(b_k), N.ptr(w_v),
             N.ptr(b_v), hd // head_size, head_size, e, row_stride, rows_total, w_k.stride(0),

@@ -31,51 +31,63 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     dev = torch.device(device)
     b = len(seq_lens)
     lens = [int(s) for s in seq_lens]
-    if any(s < 1 for s in lens):
+    if b and min(lens) < 1:
         # the kernels count a length below 1 as 1; the host counts must agree with them
         raise ValueError("expand_decode_metadata: every sequence length must be >= 1 "
                          "(it includes the token being decoded)")
     hid = np.asarray(list(use_hidden), dtype=bool)
-    n_tot = int(sum(s if h else 1 for s, h in zip(lens, hid)))
-    n_hid_tok = int(sum(s for s, h in zip(lens, hid) if h))
-    n_h = int(hid.sum())
+    lens_np = np.asarray(lens, dtype=np.int32)
+    n_h = int(np.count_nonzero(hid))
     n_kv = b - n_h
-    priv = _pad_tables(block_tables)
-    width = priv.shape[1]
-    shared = np.zeros_like(priv)
-    for r, t in enumerate(block_tables_4_shared):
+    n_hid_tok = int(lens_np[hid].sum(dtype=np.int64))
+    n_tot = n_hid_tok + n_kv
+    width = max(1, max(map(len, block_tables)))
+    # everything the device gets, in one buffer and one copy: the K/V-cached rows, three tables (private, shared, and
+    # the reference's: shared for hidden requests, private otherwise), lengths and types; sections of 128 bytes
+    at, words = [], 0
+    for n in (2 * n_kv, b * width, b * width, b * width, b, b):
+        at.append((words, words + n))
+        words += (n + 31) // 32 * 32
+    host = torch.empty(words, dtype=torch.int32, pin_memory=dev.type == "cuda")
+    rows, priv, shared, ref, h_lens, h_type = (host.numpy()[i:j] for i, j in at)
+    if N.host_lib().aps_pack_block_tables(block_tables, block_tables_4_shared, hid.ctypes.data, b, width, priv.ctypes.data,
+                                          shared.ctypes.data, ref.ctypes.data) != 0:
+        _pack_tables(block_tables, block_tables_4_shared, hid, priv.reshape(b, width), shared.reshape(b, width),
+                     ref.reshape(b, width))
+    rows.view(np.int64)[:] = np.flatnonzero(~hid)
+    h_lens[:] = lens_np
+    h_type[:] = hid
+    d = host.to(dev, non_blocking=True)
+    rows, priv, shared, ref, d_lens, d_type = (d[i:j] for i, j in at)
+    priv, shared, ref = priv.view(b, width), shared.view(b, width), ref.view(b, width)
+    # the eight index tensors and the kernels' scratch, again sections of one buffer
+    n_scratch = (N.lib().aps_decode_metadata_scratch_bytes(b) + 7) // 8
+    sizes = (n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h, n_scratch)
+    pitch = [(n + 15) // 16 * 16 for n in sizes]
+    parts = torch.empty(max(1, sum(pitch)), dtype=torch.int64, device=dev)[:sum(pitch)].split(pitch)
+    parts = [t if t.numel() == n else t[:n] for t, n in zip(parts, sizes)]
+    names = ("slot_mapping", "slot_mapping_shared", "hidden_cache_use_tot", "kv_cache_use_tot",
+             "hidden_holder_upd", "hidden_holder_pull", "hidden_cache_store_tot", "hidden_cache_use_input")
+    with N.on_device(dev):
+        N.check(N.lib().aps_expand_decode_metadata(
+            N.ptr(priv), N.ptr(shared), N.ptr(d_lens), N.ptr(d_type), b, width, block_size,
+            *(t.data_ptr() for t in parts[:8]), n_tot, n_hid_tok, None, N.ptr(parts[8]), parts[8].numel() * 8,
+            N.current_stream(dev)))
+    return DecodeMetadata(
+        block_tables=ref, seq_lens_tensor=d_lens, seq_lens=lens,
+        num_hidden_cache_tokens=n_h, num_tot_tokens=n_tot, num_decode_tokens=b,
+        max_decode_seq_len=max(lens, default=0), private_block_tables=priv,
+        cache_type=d_type, kv_request_rows=rows.view(torch.int64), **dict(zip(names, parts)))
+
+
+def _pack_tables(tables, shared_tables, hid, priv, shared, ref):
+    """``aps_pack_block_tables`` for rows of any kind numpy takes."""
+    priv[:] = _pad_tables(tables)
+    shared[:] = 0
+    for r, t in enumerate(shared_tables):
         if hid[r]:
             shared[r, :len(t)] = t
-    host = {
-        "priv": torch.from_numpy(priv), "shared": torch.from_numpy(shared),
-        "lens": torch.tensor(lens, dtype=torch.int32), "ctype": torch.from_numpy(hid.astype(np.int32)),
-    }
-    d = {k: v.to(dev, non_blocking=True) for k, v in host.items()}
-    i64 = dict(dtype=torch.int64, device=dev)
-    out = {
-        "slot_mapping": torch.empty(n_tot, **i64), "slot_mapping_shared": torch.empty(n_hid_tok, **i64),
-        "hidden_cache_use_tot": torch.empty(n_hid_tok, **i64), "kv_cache_use_tot": torch.empty(n_kv, **i64),
-        "hidden_holder_upd": torch.empty(b, **i64), "hidden_holder_pull": torch.empty(n_tot - b, **i64),
-        "hidden_cache_store_tot": torch.empty(n_h, **i64), "hidden_cache_use_input": torch.empty(n_h, **i64),
-    }
-    scratch = torch.empty(max(1, N.lib().aps_decode_metadata_scratch_bytes(b) // 4), dtype=torch.int32,
-                          device=dev)
-    with torch.cuda.device(dev):
-        N.check(N.lib().aps_expand_decode_metadata(
-            N.ptr(d["priv"]), N.ptr(d["shared"]), N.ptr(d["lens"]), N.ptr(d["ctype"]), b, width,
-            block_size, N.ptr(out["slot_mapping"]), N.ptr(out["slot_mapping_shared"]),
-            N.ptr(out["hidden_cache_use_tot"]), N.ptr(out["kv_cache_use_tot"]),
-            N.ptr(out["hidden_holder_upd"]), N.ptr(out["hidden_holder_pull"]),
-            N.ptr(out["hidden_cache_store_tot"]), N.ptr(out["hidden_cache_use_input"]), n_tot,
-            n_hid_tok, None, N.ptr(scratch), scratch.numel() * 4, N.current_stream(dev)))
-    # block_tables of the reference metadata: shared table for hidden requests, private otherwise
-    ref_tables = torch.where(d["ctype"][:, None] != 0, d["shared"], d["priv"])
-    rows = torch.arange(b, device=dev, dtype=torch.int64)
-    return DecodeMetadata(
-        block_tables=ref_tables, seq_lens_tensor=d["lens"], seq_lens=lens,
-        num_hidden_cache_tokens=n_h, num_tot_tokens=n_tot, num_decode_tokens=b,
-        max_decode_seq_len=max(lens, default=0), private_block_tables=d["priv"],
-        cache_type=d["ctype"], kv_request_rows=rows[d["ctype"] == 0], **out)
+    ref[:] = np.where(hid[:, None], shared, priv)
 
 
 def _time_both(config: int = 2, repeats: int = 5):

@@ -303,7 +303,7 @@ def derive_private_block_tables(meta: DecodeMetadata, block_size: int):
         return _derive_with_tensor_ops(meta, block_size)
     tables = torch.empty(b, width, dtype=torch.int32, device=bt.device)
     cache_type = torch.empty(b, dtype=torch.int32, device=bt.device)
-    with torch.cuda.device(bt.device):
+    with N.on_device(bt.device):
         N.check(N.lib().aps_derive_private_tables(
             N.ptr(tables), N.ptr(cache_type), N.ptr(bt), N.ptr(sm), sm.numel(), N.ptr(upd), N.ptr(rows),
             rows.numel(), N.ptr(lens), b, width, max(bt.stride(0), width), block_size, N.current_stream(bt.device)))

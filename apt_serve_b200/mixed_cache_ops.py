@@ -39,7 +39,7 @@ def hidden_to_cache(hidden: torch.Tensor, paged_cache: torch.Tensor, slot_mappin
     if hidden.dtype != paged_cache.dtype:
         raise RuntimeError("hidden_to_cache: hidden and paged_cache dtypes differ")
     n = src_idx.size(0)
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_hidden_to_cache(
             N.ptr(hidden), N.ptr(paged_cache), N.ptr(_idx(slot_mapping, "slot_mapping")),
             N.ptr(_idx(src_idx, "src_idx")), N.ptr(_idx(target_slot_idx, "target_slot_idx")),
@@ -54,7 +54,7 @@ def cache_to_hidden(hidden: torch.Tensor, paged_cache: torch.Tensor, slot_mappin
     dev = N.require_cuda(hidden, paged_cache, slot_mapping, dst_idx)
     if hidden.dtype != paged_cache.dtype:
         raise RuntimeError("cache_to_hidden: hidden and paged_cache dtypes differ")
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_cache_to_hidden(
             N.ptr(hidden), N.ptr(paged_cache), N.ptr(_idx(slot_mapping, "slot_mapping")),
             N.ptr(_idx(dst_idx, "dst_idx")), dst_idx.size(0), hidden.size(1),
@@ -77,7 +77,7 @@ def mixed_kv_to_cache(key: torch.Tensor, value: torch.Tensor, k_cache: torch.Ten
         raise RuntimeError("mixed_kv_to_cache: k_cache.stride(0) != v_cache.stride(0)")
     if shared_k_cache.stride(0) != shared_v_cache.stride(0):
         raise RuntimeError("mixed_kv_to_cache: shared cache strides differ")
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_mixed_kv_to_cache(
             N.ptr(key), N.ptr(value), N.ptr(k_cache), N.ptr(v_cache), N.ptr(shared_k_cache),
             N.ptr(shared_v_cache), N.ptr(_idx(slot_mapping, "slot_mapping")),

@@ -27,7 +27,7 @@ def reshape_and_cache_flash(key: torch.Tensor, value: torch.Tensor, key_cache: t
         raise RuntimeError("reshape_and_cache_flash: cache block strides differ")
     if key.shape[0] > 0 and not (key[0].is_contiguous() and value[0].is_contiguous()):
         raise RuntimeError("reshape_and_cache_flash: token rows must be contiguous")
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_reshape_and_cache(
             N.ptr(key), N.ptr(value), N.ptr(key_cache), N.ptr(value_cache),
             N.ptr(slot_mapping.contiguous()), slot_mapping.size(0), key.size(1), key.size(2),
@@ -67,7 +67,7 @@ def prefill_cache_write(key: Optional[torch.Tensor], value: Optional[torch.Tenso
         raise RuntimeError("prefill_cache_write: dtypes differ")
     heads, head_size, block_size = ((key.size(1), key.size(2), kv_cache.size(2)) if has_kv
                                     else (1, 1, hidden_cache.size(2)))
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_prefill_cache_write(
             N.ptr(key) if has_kv else 0, N.ptr(value) if has_kv else 0, N.ptr(hidden_states) if has_hid else 0,
             N.ptr(kv_cache[0]) if has_kv else 0, N.ptr(kv_cache[1]) if has_kv else 0,
@@ -100,7 +100,7 @@ def copy_blocks(key_caches: List[torch.Tensor], value_caches: List[torch.Tensor]
     n = len(key_caches)
     karr = (ctypes.c_void_p * n)(*[t.data_ptr() for t in key_caches])
     varr = (ctypes.c_void_p * n)(*[t.data_ptr() for t in value_caches])
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_copy_blocks(karr, varr, n, N.ptr(block_mapping.contiguous()),
                                         block_mapping.size(0), block_bytes,
                                         N.current_stream(dev)))
@@ -134,7 +134,7 @@ def swap_blocks(src: torch.Tensor, dst: torch.Tensor, src_to_dst: torch.Tensor) 
         return 0
     es = src.element_size()
     issued = ctypes.c_int64(0)
-    with torch.cuda.device(dev):
+    with N.on_device(dev):
         N.check(N.lib().aps_swap_blocks(
             src.data_ptr(), dst.data_ptr(), pairs.data_ptr(), pairs.size(0), src[0].numel() * es,
             src.stride(0) * es, dst.stride(0) * es, src.size(0), dst.size(0), kind,

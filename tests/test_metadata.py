@@ -100,3 +100,38 @@ def test_prefill_metadata():
     assert m.seq_start_loc.tolist() == [0, 5, 25]
     assert m.slot_mapping_shared.numel() == 0 and m.hidden_holder_upd.numel() == 0
     assert m.num_hidden_cache_tokens == 5 and m.num_prefill_tokens == 25
+
+
+def _pack(tables, shared, hid, width):
+    import ctypes
+    from apt_serve_b200 import _native as N
+    b = len(hid)
+    out = np.full((3, b, width), -9, dtype=np.int32)
+    flags = np.asarray(hid, dtype=bool)
+    st = N.host_lib().aps_pack_block_tables(tables, shared, flags.ctypes.data, b, width,
+                                            *(out[i].ctypes.data for i in range(3)))
+    return st, out
+
+
+def test_packed_tables_equal_numpys():
+    from apt_serve_b200.device_metadata import _pack_tables
+    tables, shared = [[5, 6, 7], (1,), [], [2 ** 31 - 1, -2 ** 31]], [[9], [], [4, 4], [8, 0, 3]]
+    hid = np.array([True, False, True, True])
+    st, out = _pack(tables, shared, hid, 3)
+    want = np.empty((3, 4, 3), dtype=np.int32)
+    _pack_tables(tables, shared, hid, *want)
+    assert st == 0 and np.array_equal(out, want)
+
+
+@pytest.mark.parametrize("tables, shared", [
+    ([np.array([1, 2])], [[3]]),              # rows the general path takes
+    ([[1, np.int64(2)]], [[3]]),
+    ([[True, 2]], [[3]]),
+    ([[1, 2 ** 31]], [[3]]),                  # does not fit
+    ([[1, 2]], [[3, 4, 5, 6]]),               # longer than the width
+    ([[1, 2]], [[3], [4]]),                   # one row too many
+    (([1, 2],), [[3]]),
+])
+def test_packing_leaves_anything_else_to_the_general_path(tables, shared):
+    st, _ = _pack(tables, shared, [True], 3)
+    assert st == 1
