@@ -669,7 +669,7 @@ class FlashAttentionImpl:
                     ops.reshape_and_cache_flash(key, value, shared_k, shared_v,
                                                 m.slot_mapping_shared, self.kv_cache_dtype)
 
-        output = torch.empty_like(query)
+        output = torch.empty_like(query) if n_decode != 0 else query   # prompts alone: their attention's own result
         decode_query = query[n_prefill:]
         query, key, value = query[:n_prefill], key[:n_prefill], value[:n_prefill]
         assert query.shape[0] == n_prefill
@@ -678,15 +678,19 @@ class FlashAttentionImpl:
         if (prefill_meta := m.prefill_metadata) is not None:
             if (kv_cache is None or prefill_meta.block_tables is None
                     or prefill_meta.block_tables.numel() == 0):
-                output[:n_prefill] = _varlen_prefill_attention(
+                prompts = _varlen_prefill_attention(
                     query, key, value, prefill_meta.seq_start_loc,
                     prefill_meta.max_prefill_seq_len, self.scale)
             else:
                 # prefix-enabled attention over the K/V cache (aptserve_flash_attn.py:432-447)
                 assert prefill_meta.seq_lens is not None
-                output[:n_prefill] = _prefix_prefill_attention(
+                prompts = _prefix_prefill_attention(
                     query, key_cache, value_cache, prefill_meta.query_start_loc,
                     prefill_meta.seq_lens, prefill_meta.block_tables, self.scale)
+            if n_decode != 0:
+                output[:n_prefill] = prompts
+            else:
+                output = prompts
 
         if (decode_meta := m.decode_metadata) is not None:
             kc, vc = (key_cache, value_cache) if n_hidden == 0 else (shared_k, shared_v)
@@ -694,7 +698,7 @@ class FlashAttentionImpl:
             o2 = output[n_prefill:].view(n_decode, self.num_heads * self.head_size)
             paged_decode_attention(q2, kc, vc, decode_meta.block_tables,
                                    decode_meta.seq_lens_tensor, self.scale, out=o2)
-        return output.view(num_tokens, hidden_size)
+        return output.reshape(num_tokens, hidden_size)
 
     # -- fused decode ------------------------------------------------------------ #
     def forward_hybrid_decode(self, query: torch.Tensor, kv_cache: Optional[torch.Tensor],
