@@ -832,7 +832,9 @@ softmax_kernel(const Params p) {
 // the copying warp takes the next one when it has requested all of its item and passes it to the other warps.
 // A stage holds 32 tokens: per 16-token cache block and 128 columns one box of (64 columns, 16 rows, 2) =
 // an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
-// K-major B operand).  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
+// K-major B operand).  The rows of a CTA's first stages are requested while the softmax kernel is still running: what a
+// kernel may read before chain_wait() is what was complete when the one before it called chain_next(), here all up
+// to the scores.  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
 constexpr int kSumThreads = 192;
 
 __host__ __device__ inline uint32_t probs_block_bytes(int terms, int np) { return (uint32_t)terms * np * 32; }
@@ -849,13 +851,12 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   __shared__ RingAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   __shared__ ItemRing items;
-  chain_wait();
   GroupPlan* gp = p.plan;
   const int n = gp->n;
-  if (n == 0) return;
+  if (n == 0) { chain_wait(); return; }
   const int np = p.np, e_blocks = p.hidden / 128, slice = gp->slice;
   const int n_slices = (e_blocks + slice - 1) / slice, n_items = n * n_slices;
-  if ((int)blockIdx.x >= n_items) return;
+  if ((int)blockIdx.x >= n_items) { chain_wait(); return; }
   const uint32_t pblk = probs_block_bytes(NT, np), x_bytes = 2u * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   if (threadIdx.x == 0) {
@@ -878,6 +879,9 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   uint32_t n_local = 0;
   Ring ir;
   int next = blockIdx.x;   // the first item needs no counter
+  int ahead = 0;           // stages of the first item whose rows are requested before the wait
+  bool waited = warp != 0;
+  if (waited) chain_wait();
   while (ok) {
     int item;
     if (warp == 0) {
@@ -901,7 +905,10 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
     }
     const int slot = item / n_slices, first = (item % n_slices) * slice;
     const int len = gp->len[slot];
-    if (len <= 0) continue;
+    if (len <= 0) {
+      if (!waited) { chain_wait(); waited = true; }
+      continue;
+    }
     const int n_col = min(slice, e_blocks - first);   // 128-column blocks of this item
     const int n_blk = (len + 15) >> 4;
     const uint32_t buf = n_local & 1u, use = n_local >> 1;
@@ -910,19 +917,34 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       const int32_t* bt = p.block_tables + (int64_t)gp->req[slot] * p.max_blocks;
       const char* probs = static_cast<const char*>(p.probs) + (int64_t)gp->blk_off[slot] * pblk;
       int rows = 0;
-      for (int b = 0; b < n_blk; b += 2) {
+      auto request_rows = [&](int b, uint32_t stage) {   // blocks b, b + 1, after the stage's byte count
         if ((b & 31) == 0) {   // first cache rows of the next 32 blocks
           const int tok = (b + lane) * 16;
           rows = b + lane < n_blk ? bt[tok / p.block_size] * p.block_size + tok % p.block_size : 0;
         }
         const int two = min(2, n_blk - b);
-        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-        const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
+        const uint32_t bar = full0 + stage * 8, dst = ring + stage * stage_bytes;
         if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)two * (n_col * 4096 + pblk));
         __syncwarp();
         const int half = lane >= n_col ? 1 : 0, col = lane - half * n_col;
         const int row = __shfl_sync(0xffffffffu, rows, (b & 31) + half);
         if (lane < two * n_col) tma_load_3d_cta(dst + (half * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2);
+      };
+      if (!waited) {
+        ahead = min(stages, (n_blk + 1) / 2);   // at most 24 blocks: `rows` holds them
+        for (int i = 0; i < ahead; ++i) request_rows(2 * i, i);
+        chain_wait();
+        waited = true;
+      }
+      for (int b = 0; b < n_blk; b += 2) {
+        const int two = min(2, n_blk - b);
+        if (ahead > 0) {
+          --ahead;
+        } else {
+          if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+          request_rows(b, rg.stage);
+        }
+        const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
         if (lane >= 30 && lane - 30 < two)
           bulk_load(dst + x_bytes + (lane - 30) * pblk, probs + (int64_t)(b + lane - 30) * pblk, pblk, bar);
         __syncwarp();
@@ -1013,25 +1035,26 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
 // is wasted.  Partial sums over the ranges of E are added by the combine kernel.
 constexpr int kUnfoldThreads = 192;
 
-__host__ __device__ inline uint32_t unfold_stage_bytes(int terms) { return 16384u + (uint32_t)terms * 16384u; }
+// A stage: 64 columns of 128 rows of W_v and of z in boxes of 16 requests, so that few requests leave room for more
+// stages.
+__host__ __device__ inline uint32_t unfold_stage_bytes(int z_boxes) { return 16384u + (uint32_t)z_boxes * 2048u; }
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kUnfoldThreads, 1)
 unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_z, const Params p) {
   constexpr int NT = kTerms<T>, HT = 128 / D, NC = 128 / HT;   // NC: requests per CTA
-  constexpr uint32_t kZHead = NC * 128;                        // bytes of one (term, head) slab
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  chain_wait();
   const int n = p.plan->n, r0 = blockIdx.z * NC;
-  if (r0 >= n) return;
+  if (r0 >= n) { chain_wait(); return; }
   const int m = min(NC, n - r0), boxes = (m + 15) / 16;
+  const uint32_t z_head = boxes * 2048;   // bytes of one (term, head) slab
   const int head0 = blockIdx.x * HT, n_heads = min(HT, p.heads - head0);
   const int sa = (int)((int64_t)p.slabs * blockIdx.y / gridDim.y), sb = (int)((int64_t)p.slabs * (blockIdx.y + 1) / gridDim.y);
-  const uint32_t stage_bytes = unfold_stage_bytes(NT);
-  constexpr int stages = kRingBytes / (16384 + NT * 16384);
+  const uint32_t stage_bytes = unfold_stage_bytes(NT * HT * boxes);
+  const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     mbar_init(&aux.acc_full[0], 1);
@@ -1050,17 +1073,29 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   Ring rg;
   if (warp == 0) {
     const int n_boxes = NT * n_heads * boxes;
-    for (int s = sa; s < sb; ++s) {
-      if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-      const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
+    auto request_w = [&](int s, uint32_t stage) {
+      const uint32_t bar = full0 + stage * 8;
       if (lane == 0) {
         mbar_expect_tx_addr(bar, (uint32_t)p.w_box_rows * 128 + (uint32_t)n_boxes * 2048);
-        tma_load_2d_cta(dst, &map_w, bar, s * 64, head0 * D);
+        tma_load_2d_cta(ring + stage * stage_bytes, &map_w, bar, s * 64, head0 * D);
       }
       __syncwarp();
+    };
+    // the first stages' rows of W_v are requested while the sum kernel is still running, z once it is complete
+    int ahead = min(stages, sb - sa);
+    for (int i = 0; i < ahead; ++i) request_w(sa + i, i);
+    chain_wait();
+    for (int s = sa; s < sb; ++s) {
+      if (ahead > 0) {
+        --ahead;
+      } else {
+        if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+        request_w(s, rg.stage);
+      }
+      const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
       for (int i = lane; i < n_boxes; i += 32) {   // i = (term, head, box of 16 requests)
         const int b = i % boxes, hh = (i / boxes) % n_heads, t = i / (boxes * n_heads);
-        tma_load_2d_cta(dst + 16384 + (t * HT + hh) * kZHead + b * 2048, &map_z, bar, s * 64,
+        tma_load_2d_cta(dst + 16384 + (t * HT + hh) * z_head + b * 2048, &map_z, bar, s * 64,
                         (t * p.heads + head0 + hh) * p.n_cap + r0 + b * 16);
       }
       __syncwarp();
@@ -1080,7 +1115,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
           for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              tc_mma_cta(tmem + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (kZHead >> 4) + k * 2,
+              tc_mma_cta(tmem + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (z_head >> 4) + k * 2,
                          desc_hi(1024, true), idesc, first);
               first = 1u;
             }
