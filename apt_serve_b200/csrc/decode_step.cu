@@ -20,9 +20,9 @@ namespace {
 // directly (hidden_attention.cu) unless the whole batch, at the longest its block tables allow, is
 // one wave of tile pairs of the re-projection kernel.  One wave costs E / 64 slabs of 520 cycles: 1 us for a
 // 256-wide layer, 22 us for an OPT-13B layer, 40 us at E = 9216, in one launch against five; both forms
-// read W_k and W_v once (16 us for an OPT-13B layer).  The next size up, two waves, is where they meet: one
-// request of 611 tokens of an OPT-13B layer takes 96 us a call in either form (65 us of it the two waves),
-// and every further wave adds to the re-projection only.
+// read W_k and W_v once (16 us for an OPT-13B layer).  At the next size up, two waves, one request of 611 tokens of an
+// OPT-13B layer takes 97 us a call re-projected (65 us of it the two waves) and 67 attended directly, and every
+// further wave adds to the re-projection only.
 bool folded_shape(int batch, int max_blocks, int block_size, int heads, int head_size, int hidden, int dtype) {
   if (!folded_supported(dtype, heads, head_size, hidden)) return false;
   const int64_t pairs = ((int64_t)batch * max_blocks * block_size + 255) / 256;

@@ -13,8 +13,8 @@
 // rows costs 4 T E H D operations; this form costs 4 E H (D + T): D times less for long contexts.
 // What is left is bound by memory: the rows are read twice (scores, weighted sums) and W_k, W_v once.
 // Measured on one B200: a step of 256 requests of an OPT-13B layer, half of them hidden-cached (94.7k rows),
-// 0.91 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
-// requests, 0.53 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.25 ms against 2.5.
+// 0.86 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
+// requests, 0.47 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.20 ms against 2.5.
 //
 //   fold_kernel      qt[r][h] = W_k,h^T q[r][h]                       tcgen05, M = 128 columns of E
 //   scores_kernel    s[t][h] = x_t . qt[r][h]                         tcgen05, M = 128 tokens
@@ -472,8 +472,8 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
 // accumulators that share a qt step).  The work is a line of (tile, 128 columns of E) steps, cut into
 // contiguous pieces (see unit_of_piece): a tile that straddles a cut leaves one partial sum per piece (slot =
 // tile + piece), added by the softmax kernel, so that one long request uses the whole chip and a large
-// batch has no partly filled last wave.  94.7k rows of an OPT-13B layer (0.97 GB): 221 us, 247 us with one
-// equal piece per CTA.
+// batch has no partly filled last wave.  94.7k rows of an OPT-13B layer (0.97 GB): 207 us; one equal piece per
+// CTA took 26 us longer.
 // A box is (64 columns, 8 rows, 2): 256 contiguous bytes of a cached row, so that a DRAM page is left after
 // 256 bytes and not 128, and 8-row groups that lie 2 KB apart, as the K-major operand needs them.  X and qt
 // have a ring each: a unit of X is 128 tokens x 128 columns (32 KB), a unit of qt serves both halves of a
