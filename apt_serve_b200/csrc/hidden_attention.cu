@@ -95,6 +95,7 @@ struct Params {
   int block_size, max_blocks, n_cap;         // n_cap: requests a group can hold here
   int group_first;                           // ordinal of the group's first hidden request
   int n_hidden_cap, splits, grid_scores;
+  uint32_t unfold_ring;                      // bytes of the unfold kernel's ring
   int w_box_rows;                            // rows of a W_v box: 128, fewer when W_v has fewer
   int64_t query_stride;
   float scale_log2;
@@ -1054,7 +1055,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   const int head0 = blockIdx.x * HT, n_heads = min(HT, p.heads - head0);
   const int sa = (int)((int64_t)p.slabs * blockIdx.y / gridDim.y), sb = (int)((int64_t)p.slabs * (blockIdx.y + 1) / gridDim.y);
   const uint32_t stage_bytes = unfold_stage_bytes(NT * HT * boxes);
-  const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
+  const int stages = min(kMaxStages, (int)(p.unfold_ring / stage_bytes));
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     mbar_init(&aux.acc_full[0], 1);
@@ -1159,6 +1160,7 @@ int terms_of(int dtype) { return dtype == APS_BF16 ? 3 : 2; }
 
 struct Layout {
   int np, n_cap, n_groups, splits, max_slice;
+  uint32_t unfold_ring;
   size_t off_groups, off_slot, off_list, off_qscale, off_inv, off_scores, off_probs, off_qz, off_part, total;
 };
 
@@ -1168,9 +1170,14 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.np = (heads + 15) / 16 * 16;
   l.n_cap = ((batch < kGroup ? batch : kGroup) + 15) / 16 * 16;
   l.n_groups = (batch + kGroup - 1) / kGroup;
-  // one wave of unfold CTAs; at least four slabs each
-  const int w_tiles = (heads * head_size + 127) / 128, slabs = hidden / 64;
-  int splits = 148 / w_tiles;
+  // One wave of unfold CTAs; at least four slabs each.  A CTA spends 0.4 us on a slab whatever its requests, so few
+  // requests take two CTAs per SM (half the ring each, three stages at least) and ranges half as long: one OPT-13B
+  // request 14.2 -> 11.4 us, 24 requests 15.6 -> 12.3, 64 requests 20.8 -> 17.1.
+  const int w_tiles = (heads * head_size + 127) / 128, slabs = hidden / 64, ht = 128 / head_size;
+  const int z_boxes = nt * ht * (((batch < head_size ? batch : head_size) + 15) / 16);   // 128 / ht requests per CTA
+  const bool two = 3 * unfold_stage_bytes(z_boxes) <= kRingBytes / 2;
+  l.unfold_ring = (uint32_t)(two ? kRingBytes / 2 : kRingBytes);
+  int splits = (two ? 2 : 1) * 148 / w_tiles;
   if (splits > slabs / 4) splits = slabs / 4;
   l.splits = splits < 1 ? 1 : splits;
   int ms = 256 / l.np;
@@ -1257,8 +1264,8 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv
     auto k = unfold_kernel<T, D>;
     if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
     constexpr int kReqs = 128 / (128 / D);
-    if ((st = launch_chained("unfold_kernel", k, dim3(w_tiles, p.splits, (n_cap + kReqs - 1) / kReqs), kUnfoldThreads, ring,
-                             stream, m.wv, m.z, p)) != APS_OK) return st;
+    if ((st = launch_chained("unfold_kernel", k, dim3(w_tiles, p.splits, (n_cap + kReqs - 1) / kReqs), kUnfoldThreads,
+                             1024 + p.unfold_ring, stream, m.wv, m.z, p)) != APS_OK) return st;
   }
   return APS_OK;
 }
@@ -1338,7 +1345,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_groups * kGroup; p.splits = l.splits; p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_groups * kGroup; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.grid_scores = pa.grid_scores;
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);
