@@ -193,4 +193,30 @@ bool folded32_supported(const HybridCall& c);
 size_t folded32_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size, int hidden);
 int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
 
+// Inclusive prefix sums of a pair over the 1024 threads of a planning CTA, and the totals: shuffles inside the warps,
+// one barrier (a scan through shared memory takes 20, which was 3 us of a K/V-only plan's 8).
+constexpr int kPlanThreads = 1024;
+__device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int2& total) {
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
+    if (lane >= o) { v.x += x; v.y += y; }
+  }
+  if (lane == 31) warp_sums[warp] = v;
+  __syncthreads();
+  int2 s = warp_sums[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, s.x, o), y = __shfl_up_sync(0xffffffffu, s.y, o);
+    if (lane >= o) { s.x += x; s.y += y; }
+  }
+  total.x = __shfl_sync(0xffffffffu, s.x, 31);
+  total.y = __shfl_sync(0xffffffffu, s.y, 31);
+  const int bx = __shfl_sync(0xffffffffu, s.x, warp > 0 ? warp - 1 : 0);
+  const int by = __shfl_sync(0xffffffffu, s.y, warp > 0 ? warp - 1 : 0);
+  if (warp > 0) { v.x += bx; v.y += by; }
+  return v;   // inclusive
+}
+
 }  // namespace aps

@@ -130,31 +130,6 @@ __device__ __forceinline__ void drain() {
 // ---- plan ---------------------------------------------------------------------------
 // One CTA.  K/V-cached requests: the chunk list of the K/V kernel and the partial slots.  Hidden-cached
 // requests: the groups.  Runs of requests per thread, warp-shuffle scans.
-constexpr int kPlanThreads = 1024;
-
-__device__ __forceinline__ int2 block_scan(int2 v, int2* warp_sums, int tid, int2& total) {
-  const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int x = __shfl_up_sync(0xffffffffu, v.x, o), y = __shfl_up_sync(0xffffffffu, v.y, o);
-    if (lane >= o) { v.x += x; v.y += y; }
-  }
-  if (lane == 31) warp_sums[warp] = v;
-  __syncthreads();
-  int2 s = warp_sums[lane];
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int x = __shfl_up_sync(0xffffffffu, s.x, o), y = __shfl_up_sync(0xffffffffu, s.y, o);
-    if (lane >= o) { s.x += x; s.y += y; }
-  }
-  total.x = __shfl_sync(0xffffffffu, s.x, 31);
-  total.y = __shfl_sync(0xffffffffu, s.y, 31);
-  const int bx = __shfl_sync(0xffffffffu, s.x, warp > 0 ? warp - 1 : 0);
-  const int by = __shfl_sync(0xffffffffu, s.y, warp > 0 ? warp - 1 : 0);
-  if (warp > 0) { v.x += bx; v.y += by; }
-  return v;   // inclusive
-}
-
 // Behind the write of the new tokens' cache rows (wait_last) it runs beside it: it reads only the call's
 // arguments, and what it writes (the scratch) was last used by kernels before that write, which were complete when
 // the write let this kernel start.  It waits for the write before it exits.  As a call's first kernel it waits first.

@@ -29,7 +29,6 @@
 namespace aps {
 namespace {
 
-constexpr int kPlanThreads = 1024;
 constexpr int kKvWarps = 8;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -37,26 +36,13 @@ constexpr unsigned kFull = 0xffffffffu;
 // One CTA.  Thread t handles a contiguous run of requests; two block-wide prefix sums:
 // first over (K/V chunks, hidden sub-blocks), which fixes where each hidden request's rows
 // sit in the tile list, then over the number of softmax partials each request will leave.
-__device__ __forceinline__ void block_scan2(int* sa, int* sb, int tid, int& a, int& b) {
-  sa[tid] = a; sb[tid] = b;
-  __syncthreads();
-  for (int off = 1; off < kPlanThreads; off <<= 1) {
-    int x = 0, y = 0;
-    if (tid >= off) { x = sa[tid - off]; y = sb[tid - off]; }
-    __syncthreads();
-    sa[tid] += x; sb[tid] += y;
-    __syncthreads();
-  }
-  a = sa[tid]; b = sb[tid];   // inclusive sums
-}
-
 __global__ void __launch_bounds__(kPlanThreads)
 plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restrict__ kv_chunks,
             int2* __restrict__ hid_tiles, int* __restrict__ first_tile, int2* __restrict__ hid_subs,
             int* __restrict__ hid_rows, const int32_t* __restrict__ seq_lens,
             const int32_t* __restrict__ cache_type, const int32_t* __restrict__ block_tables, int batch,
             int max_tokens, int max_blocks, int block_size, int pack_tiles, int kv_present) {
-  __shared__ int sa[kPlanThreads], sb[kPlanThreads];
+  __shared__ int2 sums_a[32], sums_b[32];
   __shared__ int s_kv_missing;
   const int tid = threadIdx.x;
   if (tid == 0) s_kv_missing = 0;
@@ -80,13 +66,12 @@ plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restr
     if (hidden(r)) sub += subs_of(s);
     else { kv += chunks_of(s); if (!kv_present) s_kv_missing = 1; }
   }
-  int kv_inc = kv, sub_inc = sub;
-  block_scan2(sa, sb, tid, kv_inc, sub_inc);
-  const int total_kv = sa[kPlanThreads - 1], total_sub = sb[kPlanThreads - 1];
-  __syncthreads();
-  int o_kv = kv_inc - kv, o_sub = sub_inc - sub;
+  int2 total;
+  const int2 inc = block_scan(make_int2(kv, sub), sums_a, tid, total);
+  const int total_kv = total.x, total_sub = total.y;
+  int o_kv = inc.x - kv, o_sub = inc.y - sub;
   // pass 2: partial slots per request (K/V: one per chunk; hidden: one per tile it has rows in)
-  int slots = 0, dummy = 0;
+  int slots = 0;
   {
     int g = o_sub;
     for (int r = r0; r < r1; ++r) {
@@ -100,9 +85,8 @@ plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restr
       }
     }
   }
-  int slots_inc = slots;
-  block_scan2(sa, sb, tid, slots_inc, dummy);
-  const int total_slots = sa[kPlanThreads - 1];
+  const int slots_inc = block_scan(make_int2(slots, 0), sums_b, tid, total).x;
+  const int total_slots = total.x;
   int o_slot = slots_inc - slots;
   // write-out.  The per-request words are written by the request's owner thread; the lists
   // (one entry per K/V chunk or per 16-row sub-block, up to 128 per request, each sub-block
