@@ -49,7 +49,6 @@ namespace {
 constexpr int kTile = 256;                // tokens per scores tile: two M128 accumulators share a qt slab
 constexpr int kSubs = kTile / 16;         // 16-row boxes of the hidden cache per tile
 constexpr int kTileCost = 4;              // fixed cost of a tile in boxes (its qt slab), for the work split
-constexpr int kStepTokens = 32;           // tokens per stage of the sum kernel
 constexpr int kMinPiece = 2 * (kSubs + kTileCost);   // least work of a CTA of the scores kernel: two full steps
 constexpr int kMaxSlice = 4;              // 128-column blocks of E per work item of the sum kernel
 constexpr int kSumRounds = 2;             // work items per SM below which it takes narrower slices
@@ -813,7 +812,9 @@ softmax_kernel(const Params p) {
 // columns), the item's accumulators together in half of the tensor memory, so that the epilogue of one item
 // overlaps the next one's main loop.  Items in order of their length, longest first, handed out by a counter:
 // the copying warp takes the next one when it has requested all of its item and passes it to the other warps.
-// A stage holds 32 tokens: per 16-token cache block and 128 columns one box of (64 columns, 16 rows, 2) =
+// A stage holds two cache blocks of 16 tokens, four for slices of one or two column blocks (a stage costs 0.35 us of
+// waits and commits whatever its size: sums of 34 OPT-1.3B requests 36 -> 29 us, of 8 long OPT-13B requests 54 -> 41, of
+// one 12.9 -> 11.0): per cache block and 128 columns one box of (64 columns, 16 rows, 2) =
 // an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
 // K-major B operand).  The rows of a CTA's first stages are requested while the softmax kernel is still running: what a
 // kernel may read before chain_wait() is what was complete when the one before it called chain_next(), here all up
@@ -821,8 +822,12 @@ softmax_kernel(const Params p) {
 constexpr int kSumThreads = 192;
 
 __host__ __device__ inline uint32_t probs_block_bytes(int terms, int np) { return (uint32_t)terms * np * 32; }
+__host__ __device__ inline int sum_stage_blocks(int terms, int np, int slice) {
+  return slice <= 2 && 3 * 4 * (slice * 4096 + probs_block_bytes(terms, np)) <= kRingBytes ? 4 : 2;   // three stages at least
+}
 __host__ __device__ inline uint32_t sum_stage_bytes(int terms, int np, int slice) {
-  return 2u * slice * 4096 + ((2 * probs_block_bytes(terms, np) + 1023) & ~1023u);
+  const uint32_t blocks = sum_stage_blocks(terms, np, slice);
+  return blocks * slice * 4096 + ((blocks * probs_block_bytes(terms, np) + 1023) & ~1023u);
 }
 
 template <typename T>
@@ -840,7 +845,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   const int np = p.np, e_blocks = p.hidden / 128, slice = gp->slice;
   const int n_slices = (e_blocks + slice - 1) / slice, n_items = n * n_slices;
   if ((int)blockIdx.x >= n_items) { chain_wait(); return; }
-  const uint32_t pblk = probs_block_bytes(NT, np), x_bytes = 2u * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
+  const uint32_t pblk = probs_block_bytes(NT, np), per_stage = sum_stage_blocks(NT, np, slice), x_bytes = per_stage * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
@@ -900,27 +905,27 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       const int32_t* bt = p.block_tables + (int64_t)gp->req[slot] * p.max_blocks;
       const char* probs = static_cast<const char*>(p.probs) + (int64_t)gp->blk_off[slot] * pblk;
       int rows = 0;
-      auto request_rows = [&](int b, uint32_t stage) {   // blocks b, b + 1, after the stage's byte count
+      auto request_rows = [&](int b, uint32_t stage) {   // the stage's byte count, then the rows of the blocks from b on
         if ((b & 31) == 0) {   // first cache rows of the next 32 blocks
           const int tok = (b + lane) * 16;
           rows = b + lane < n_blk ? bt[tok / p.block_size] * p.block_size + tok % p.block_size : 0;
         }
-        const int two = min(2, n_blk - b);
+        const int nb = min((int)per_stage, n_blk - b);
         const uint32_t bar = full0 + stage * 8, dst = ring + stage * stage_bytes;
-        if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)two * (n_col * 4096 + pblk));
+        if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)nb * (n_col * 4096 + pblk));
         __syncwarp();
-        const int half = lane >= n_col ? 1 : 0, col = lane - half * n_col;
-        const int row = __shfl_sync(0xffffffffu, rows, (b & 31) + half);
-        if (lane < two * n_col) tma_load_3d_cta(dst + (half * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2);
+        const int k = lane / n_col, col = lane - k * n_col;
+        const int row = __shfl_sync(0xffffffffu, rows, ((b & 31) + k) & 31);
+        if (lane < nb * n_col) tma_load_3d_cta(dst + (k * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2);
       };
       if (!waited) {
-        ahead = min(stages, (n_blk + 1) / 2);   // at most 24 blocks: `rows` holds them
-        for (int i = 0; i < ahead; ++i) request_rows(2 * i, i);
+        ahead = min(min(stages, 32 / (int)per_stage), (n_blk + (int)per_stage - 1) / (int)per_stage);   // `rows` holds 32 blocks
+        for (int i = 0; i < ahead; ++i) request_rows(i * (int)per_stage, i);
         chain_wait();
         waited = true;
       }
-      for (int b = 0; b < n_blk; b += 2) {
-        const int two = min(2, n_blk - b);
+      for (int b = 0; b < n_blk; b += (int)per_stage) {
+        const int nb = min((int)per_stage, n_blk - b);
         if (ahead > 0) {
           --ahead;
         } else {
@@ -928,8 +933,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
           request_rows(b, rg.stage);
         }
         const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
-        if (lane >= 30 && lane - 30 < two)
-          bulk_load(dst + x_bytes + (lane - 30) * pblk, probs + (int64_t)(b + lane - 30) * pblk, pblk, bar);
+        if (lane == 31) bulk_load(dst + x_bytes, probs + (int64_t)b * pblk, nb * pblk, bar);   // blocks lie one behind the other
         __syncwarp();
         rg.step(stages);
       }
@@ -937,15 +941,15 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
       tc_fence_after();
       const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
-      for (int b = 0; b < n_blk; b += 2) {
-        const int two = min(2, n_blk - b);
+      for (int b = 0; b < n_blk; b += (int)per_stage) {
+        const int nb = min((int)per_stage, n_blk - b);
         if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
         const uint32_t x_at = ring + rg.stage * stage_bytes, p_at = x_at + x_bytes;
-        const int valid = len - (b + two - 1) * 16;   // tokens of the stage's last block
+        const int valid = len - (b + nb - 1) * 16;   // tokens of the stage's last block
         if (valid < 16) {
           // rows past the sequence length hold whatever the cache block holds; their weights are zero,
           // but zero times NaN is not
-          const uint32_t at = x_at + (two - 1) * slice * 4096;
+          const uint32_t at = x_at + (nb - 1) * slice * 4096;
           const int pieces = (16 - valid) * 8;
           for (int i = lane; i < pieces * 2 * n_col; i += 32) {
             const int r = valid + (i % pieces) / 8, piece = i % 8, hc = i / pieces;
@@ -956,7 +960,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         }
         tc_fence_after();
         if (elect_one()) {
-          for (int k = 0; k < two; ++k) {
+          for (int k = 0; k < nb; ++k) {
             const uint32_t acc = (b + k) != 0;
             const uint32_t a_lo = desc_lo(x_at + k * slice * 4096, 2048), b_lo = desc_lo(p_at + k * pblk, (uint32_t)np * 16);
             for (int col = 0; col < n_col; ++col)
