@@ -27,7 +27,8 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
                            device) -> DecodeMetadata:
     """Same arguments and result as ``metadata.build_decode_metadata``, with the tensors
     created on ``device`` by the expansion kernels.  Host work is O(number of blocks):
-    padding the two block tables."""
+    padding the two block tables.  Nothing waits for the device: one copy from pinned memory and two launches on
+    the current stream.  The tensors are sections of two allocations (what came from the host, what the kernels wrote)."""
     dev = torch.device(device)
     b = len(seq_lens)
     lens = [int(s) for s in seq_lens]
