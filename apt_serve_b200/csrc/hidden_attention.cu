@@ -237,9 +237,10 @@ step_plan_kernel(const PlanArgs a) {
     if (tid == 0) {
       // sum kernel: the widest slice of E that still gives item_target items.  Wide slices leave a DRAM page after
       // up to 1 KB of a row, not 256 bytes, and read the weights less often (a slice of one block reads as many bytes of
-      // weights as of rows); more items even out requests of different lengths.  On one B200, slices of 1 / 2 / 3 /
-      // 4 / 5 blocks: 24 requests of 1800 OPT-13B tokens 127 / 89 / 80 / 87 / - us, 128 of 740 - / 236 / 197 / 186 /
-      // 192, 52 of 950 OPT-66B tp 8 - / 255 / 177 / 167 / 172 (six), 34 of 500 OPT-1.3B 36 / 54 / - / 53 / 68.
+      // weights as of rows); more items even out requests of different lengths.  On one B200, slices of 1 / 2 / 3 / 4
+      // blocks: 24 requests of 1800 OPT-13B tokens 95 / 76 / 79 / 87 us, 128 of 740 - / - / 197 / 186; before the
+      // narrow slices had stages of four cache blocks 52 of 950 OPT-66B tp 8 - / 255 / 177 / 167, 34 of 500 OPT-1.3B
+      // 36 / 54 / - / 53.
       int slice = a.max_slice;
       while (slice > 1 && n * ((a.steps + slice - 1) / slice) < a.item_target) --slice;
       gp->n = n; gp->n_tiles = n_tiles; gp->weight = weight; gp->slice = slice;
