@@ -25,10 +25,16 @@
 //
 // Precision.  x, W and q are used as they are stored.  The three intermediates that meet a tensor-core
 // operand (qt, p, z) are fp32 values carried as a sum of 16-bit TERMS (value = hi + rest, rest again
-// rounded): two for fp16 (22 bits), three for bf16 (24 bits), each multiplied separately into the same
-// fp32 accumulator.  fp16 has a narrow exponent, so q is normalised by a power of two before it is folded
-// (|q| < 2, undone in the softmax) and p is kept at 2^15 times its value (undone by the
-// normalisation); both then sit well inside the range and the second term keeps its bits.
+// rounded): two for fp16 (22 bits), three for bf16 (24 bits), each multiplied separately into fp32
+// accumulators.  fp16 has a narrow exponent:
+//   - q is normalised by a power of two before it is folded (|q| < 2) and the folded query is kept at 1 / 2D of its
+//     value (both undone in the softmax): |qt| <= sum_d |q_d W_d| < 2 D 65504 always fits;
+//   - p is kept at 2^15 times its value (undone by the normalisation), so that what its second term loses below
+//     2^-24 is 2^-39 of the largest weight;
+//   - the rests of qt and z are kept at 2^11 times their value and multiplied into accumulators of their own, which
+//     the epilogues add with 2^-11.  Kept as they are they are subnormal as soon as the value is below 0.1: the weighted
+//     sums then had an absolute error of 2^-26, 3.6 units of the output's last place for cached rows of N(0, 0.01) and
+//     W_v of N(0, 1).  Now the value's error is 2^-23 of it or 2^-36, whichever is more.
 //
 // Requests are taken in groups of at most kGroup, so that the scratch (qt, z: kGroup x H x E terms)
 // does not grow with the batch; inside a group they are sorted by length, longest first.
@@ -100,14 +106,28 @@ struct Params {
   float scale_log2;
 };
 
-template <typename T>
+// SCALED: fp16's second term at kRestUp times its value, for products that have accumulators of their own.
+constexpr float kRestUp = 2048.f;
+template <typename T, bool SCALED>
 __device__ __forceinline__ void split_terms(float v, T (&t)[kTerms<T>]) {
 #pragma unroll
   for (int i = 0; i < kTerms<T>; ++i) {
     t[i] = Elem<T>::from_float(v);
     v -= Elem<T>::to_float(t[i]);
+    if (SCALED && kTerms<T> == 2) v *= kRestUp;
   }
 }
+// The value whose terms' products are v, the smaller ones added first.
+template <int NT, int N>
+__device__ __forceinline__ float add_terms(const uint32_t (&v)[NT][N], int j) {
+  if (NT == 2) return fmaf(__uint_as_float(v[NT - 1][j]), 1.f / kRestUp, __uint_as_float(v[0][j]));
+  float x = __uint_as_float(v[NT - 1][j]);
+#pragma unroll
+  for (int i = NT - 2; i >= 0; --i) x += __uint_as_float(v[i][j]);
+  return x;
+}
+// The folded query is kept at this fraction of its value.
+template <typename T, int D> constexpr float kFoldDown = kTerms<T> == 2 ? 0.5f / D : 1.f;
 template <typename T>
 __device__ __forceinline__ uint32_t pack_pair(T a, T b) {
   return (uint32_t)reinterpret_cast<const unsigned short&>(a) | ((uint32_t)reinterpret_cast<const unsigned short&>(b) << 16);
@@ -332,7 +352,7 @@ __device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, in
       if constexpr (EPL == 4) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)), "r"((uint32_t)w[2] | ((uint32_t)w[3] << 16)) : "memory");
       else if constexpr (EPL == 2) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"((uint32_t)w[0] | ((uint32_t)w[1] << 16)) : "memory");
       else asm volatile("st.shared.b16 [%0], %1;" ::"r"(dst), "h"(w[0]) : "memory");
-      if (keep_scale && lane == 0 && rr < m) p.qscale[(int64_t)(r0 + rr) * p.heads + head] = p.scale_log2 * down;
+      if (keep_scale && lane == 0 && rr < m) p.qscale[(int64_t)(r0 + rr) * p.heads + head] = p.scale_log2 * (down * (1.f / kFoldDown<T, D>));
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // read by the tensor cores next
@@ -423,8 +443,8 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
           const float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
           if (c + j + (lane & 1) < m) {
             T x[NT], y[NT];
-            split_terms<T>(f.x, x);
-            split_terms<T>(f.y, y);
+            split_terms<T, true>(f.x * kFoldDown<T, D>, x);
+            split_terms<T, true>(f.y * kFoldDown<T, D>, y);
 #pragma unroll
             for (int k = 0; k < NT; ++k) *reinterpret_cast<uint32_t*>(dst + k * term_stride) = pack_pair<T>(x[k], y[k]);
           }
@@ -481,6 +501,9 @@ __host__ __device__ inline uint32_t scores_q_bytes(int terms, int np) { return (
 // or 32 cycles of its bandwidth against 12 - 24 of arithmetic, so an instruction per term costs two or three
 // times that.
 __host__ __device__ inline bool stacked_terms(int terms, int np) { return terms * np <= 256; }
+// Heads too many for that: an instruction per term, into accumulators of its own for fp16 (its second term has a
+// scale of its own) and, if those of a tile's two halves do not fit the tensor memory, the halves one after the
+// other, with a second copy of qt.
 // qt units in the ring: a step of a short tile takes less time than a unit's round trip, so three of them where that
 // leaves three units of X (two and two, one otherwise).  Two -> three: scores of 128 OPT-13B requests of 740 tokens
 // 213 -> 207 us, of 64 of 340 71 -> 67, of 52 OPT-66B tp 8 requests 182 -> 170; with four and fewer units of X the
@@ -513,10 +536,11 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   const uint32_t q_bytes = scores_q_bytes(NT, np);
   const int nq = scores_q_units(NT, np), nx = min(kMaxStages, (int)((kScoresRing - nq * q_bytes) / kUnitBytes));
   const uint32_t q_ring = x_ring + nx * kUnitBytes;
-  const int n_acc = stacked_terms(NT, np) ? NT * np : np, n_rep = stacked_terms(NT, np) ? 1 : NT;
-  const int n_buf = 4 * n_acc <= 512 ? 2 : 1;
+  const bool stacked = stacked_terms(NT, np), own_acc = NT == 2 || stacked;   // own_acc: an accumulator per term
+  const int n_acc = own_acc ? NT * np : np, n_rep = stacked ? 1 : NT, m_step = 2 * n_acc <= 512 ? 2 : 1;
+  const int n_buf = 2 * m_step * n_acc <= 512 ? 2 : 1;
   uint32_t tmem_cols = 32;
-  while (tmem_cols < (uint32_t)(n_buf * 2 * n_acc)) tmem_cols <<= 1;
+  while (tmem_cols < (uint32_t)(n_buf * m_step * n_acc)) tmem_cols <<= 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < nx; ++s) { mbar_init(&aux.full[s], 2); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < kMaxQUnits; ++b) { mbar_init(&aux.q_full[b], 1); mbar_init(&aux.q_empty[b], 1); }
@@ -574,26 +598,13 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
       const int tok0 = (t - s_toff[slot]) * kTile;
       const int n_sub = min(kSubs, (s_len[slot] - tok0 + 15) >> 4);
       const int n_m = n_sub > 8 ? 2 : 1;
-      const uint32_t buf = n_local % n_buf, use = n_local / n_buf;
-      ++n_local;
-      if (warp == 0) {
-        for (int s = sa; s < sb; ++s) {
-          if (!mbar_wait_warp(q_empty0 + qr.stage * 8, qr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-          const uint32_t bar = q_full0 + qr.stage * 8;
-          if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
-          __syncwarp();
-          if (lane < 2 * NT)   // lane = (term, half of the columns); the terms of a half lie one behind the other
-            tma_load_2d_cta(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
-          __syncwarp();
-          qr.step(nq);
-        }
-      } else if (warp >= 6) {
-        // box g of a unit: rows 8 g ... of its 128 tokens; warp 6 the first eight, warp 7 the others
-        const int g = (warp - 6) * 8 + lane;
-        int row[2] = {0, 0};
-        bool has[2] = {false, false};
-        int boxes[2];
-  #pragma unroll
+      // box g of a unit: rows 8 g ... of its 128 tokens; warp 6 the first eight, warp 7 the others
+      const int g = (warp - 6) * 8 + lane;
+      int row[2] = {0, 0};
+      bool has[2] = {false, false};
+      int boxes[2] = {0, 0};
+      if (warp >= 6) {
+#pragma unroll
         for (int m = 0; m < 2; ++m) {
           const int sub = m * 8 + (g >> 1);
           has[m] = lane < 8 && sub < n_sub;
@@ -603,81 +614,94 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             row[m] = p.block_tables[(int64_t)s_req[slot] * p.max_blocks + tok / p.block_size] * p.block_size + tok % p.block_size + (g & 1) * 8;
           }
         }
-        for (int s = sa; s < sb && ok; ++s) {
-  #pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            if (m >= n_m) break;
-            if (!mbar_wait_warp(empty0 + xr.stage * 8, xr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-            const uint32_t bar = full0 + xr.stage * 8;
-            if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)boxes[m] * 2048);
+      }
+      for (int m0 = 0; m0 < n_m && ok; m0 += m_step) {   // halves m0 ... m1 - 1 of the tile, one set of accumulators
+        const int m1 = min(n_m, m0 + m_step);
+        const uint32_t buf = n_local % n_buf, use = n_local / n_buf;
+        ++n_local;
+        if (warp == 0) {
+          for (int s = sa; s < sb; ++s) {
+            if (!mbar_wait_warp(q_empty0 + qr.stage * 8, qr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+            const uint32_t bar = q_full0 + qr.stage * 8;
+            if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
             __syncwarp();
-            if (has[m]) tma_load_3d_cta(x_ring + xr.stage * kUnitBytes + g * 2048, &map_x, bar, 0, row[m], s * 2);
+            if (lane < 2 * NT)   // lane = (term, half of the columns); the terms of a half lie one behind the other
+              tma_load_2d_cta(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
             __syncwarp();
-            xr.step(nx);
+            qr.step(nq);
           }
-        }
-      } else if (warp == 1) {
-        if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)n_acc, false);
-        for (int s = sa; s < sb && ok; ++s) {
-          if (!mbar_wait_warp(q_full0 + qr.stage * 8, qr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
-          for (int m = 0; m < n_m; ++m) {
-            if (!mbar_wait_warp(full0 + xr.stage * 8, xr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
-            tc_fence_after();
-            if (elect_one()) {
-              const uint32_t a_lo = desc_lo(x_ring + xr.stage * kUnitBytes, 16), b_lo = desc_lo(q_ring + qr.stage * q_bytes, 16);
-              const uint32_t d = tmem + (buf * 2 + m) * n_acc;
-              uint32_t acc = s != sa;
-  #pragma unroll
-              for (int j = 0; j < 2; ++j)
-  #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  for (int i = 0; i < n_rep; ++i) {
-                    tc_mma_cta(d, a_lo + j * 64 + k * 2, desc_hi(2048, true), b_lo + (j * NT + i) * (np * 8) + k * 2, desc_hi(1024, true), idesc, acc);
+        } else if (warp >= 6) {
+          for (int s = sa; s < sb && ok; ++s) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              if (m < m0 || m >= m1) continue;
+              if (!mbar_wait_warp(empty0 + xr.stage * 8, xr.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+              const uint32_t bar = full0 + xr.stage * 8;
+              if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)boxes[m] * 2048);
+              __syncwarp();
+              if (has[m]) tma_load_3d_cta(x_ring + xr.stage * kUnitBytes + g * 2048, &map_x, bar, 0, row[m], s * 2);
+              __syncwarp();
+              xr.step(nx);
+            }
+          }
+        } else if (warp == 1) {
+          if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)(stacked ? NT * np : np), false);
+          const uint32_t rep_acc = own_acc ? (uint32_t)np : 0u;
+          for (int s = sa; s < sb && ok; ++s) {
+            if (!mbar_wait_warp(q_full0 + qr.stage * 8, qr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+            for (int m = m0; m < m1; ++m) {
+              if (!mbar_wait_warp(full0 + xr.stage * 8, xr.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
+              tc_fence_after();
+              if (elect_one()) {
+                const uint32_t a_lo = desc_lo(x_ring + xr.stage * kUnitBytes, 16), b_lo = desc_lo(q_ring + qr.stage * q_bytes, 16);
+                const uint32_t d = tmem + (buf * m_step + m - m0) * n_acc;
+                uint32_t acc = s != sa;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) {
+                    for (int i = 0; i < n_rep; ++i) {
+                      tc_mma_cta(d + i * rep_acc, a_lo + j * 64 + k * 2, desc_hi(2048, true), b_lo + (j * NT + i) * (np * 8) + k * 2, desc_hi(1024, true), idesc, acc);
+                      if (rep_acc == 0) acc = 1u;
+                    }
                     acc = 1u;
                   }
-              tc_commit_cta(empty0 + xr.stage * 8);
-              if (m == n_m - 1) tc_commit_cta(q_empty0 + qr.stage * 8);
-            }
-            __syncwarp();
-            xr.step(nx);
-          }
-          qr.step(nq);
-        }
-        if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
-        __syncwarp();
-      } else {
-        const int quarter = warp & 3;
-        if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
-        tc_fence_after();
-        float* dst = p.scores + (int64_t)(t + piece) * p.heads * kTile;
-        for (int m = 0; m < n_m; ++m)
-          for (int h0 = 0; h0 < np; h0 += 16) {
-            const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (buf * 2 + m) * n_acc + h0;
-            uint32_t v[NT][16];
-            tmem_ld16(at, v[0]);
-            if (n_rep == 1) {
-  #pragma unroll
-              for (int i = 1; i < NT; ++i) tmem_ld16(at + i * np, v[i]);
-            }
-            tmem_ld_wait();
-            if (n_rep == 1) {   // the smaller terms' sums first
-  #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                float x = __uint_as_float(v[NT - 1][j]);
-  #pragma unroll
-                for (int i = NT - 2; i >= 0; --i) x += __uint_as_float(v[i][j]);
-                v[0][j] = __float_as_uint(x);
+                tc_commit_cta(empty0 + xr.stage * 8);
+                if (m == m1 - 1) tc_commit_cta(q_empty0 + qr.stage * 8);
               }
+              __syncwarp();
+              xr.step(nx);
             }
-  #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (h0 + j < p.heads) dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = __uint_as_float(v[0][j]);
+            qr.step(nq);
           }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+          if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
+          __syncwarp();
+        } else {
+          const int quarter = warp & 3;
+          if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
+          tc_fence_after();
+          float* dst = p.scores + (int64_t)(t + piece) * p.heads * kTile;
+          for (int m = m0; m < m1; ++m)
+            for (int h0 = 0; h0 < np; h0 += 16) {
+              const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (buf * m_step + m - m0) * n_acc + h0;
+              uint32_t v[NT][16];
+              tmem_ld16(at, v[0]);
+              if (own_acc) {
+#pragma unroll
+                for (int i = 1; i < NT; ++i) tmem_ld16(at + i * np, v[i]);
+              }
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (h0 + j < p.heads)
+                  dst[(int64_t)(h0 + j) * kTile + m * 128 + quarter * 32 + lane] = own_acc ? add_terms(v, j) : __uint_as_float(v[0][j]);
+            }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_addr(smem_u32(&aux.acc_empty[buf]));
+        }
       }
     }
   }
@@ -772,7 +796,7 @@ softmax_kernel(const Params p) {
       for (int e = 0; e < 8; ++e) {
         const float w = exp2f(s[e] - mx + kProbShift);
         sum += w;
-        split_terms<T>(w, terms[e]);
+        split_terms<T, false>(w, terms[e]);
       }
       const int blk = k * kSubs + (lane >> 1);
       if (blk < n_blk) {
@@ -996,8 +1020,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
             if (h < p.heads) {
               const float w = inv[h];
               T a[NT], b[NT];
-              split_terms<T>(f.x * w, a);
-              split_terms<T>(f.y * w, b);
+              split_terms<T, true>(f.x * w, a);
+              split_terms<T, true>(f.y * w, b);
 #pragma unroll
               for (int t = 0; t < NT; ++t)
                 *reinterpret_cast<uint32_t*>(z + (((int64_t)t * p.heads + h) * p.n_cap + slot) * p.hidden + (e & ~1)) = pack_pair<T>(a[t], b[t]);
@@ -1020,7 +1044,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
 // D[row of W_v][request] = sum_e W_v[row][e] z[request][head of the row][e]: one CTA per (128 rows of W_v,
 // range of E, 128 / HT requests), HT = 128 / D heads per 128 rows.  Rows of every head are multiplied with
 // every one of the HT heads' z and the epilogue keeps the matching quarter (half): for D = 128 nothing
-// is wasted.  Partial sums over the ranges of E are added by the combine kernel.
+// is wasted.  fp16's second term has accumulators of its own.  Partial sums over the ranges of E are added by the
+// combine kernel.
 constexpr int kUnfoldThreads = 192;
 
 // A stage: 64 columns of 128 rows of W_v and of z in boxes of 16 requests, so that few requests leave room for more
@@ -1031,6 +1056,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kUnfoldThreads, 1)
 unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_z, const Params p) {
   constexpr int NT = kTerms<T>, HT = 128 / D, NC = 128 / HT;   // NC: requests per CTA
+  constexpr uint32_t kTermAcc = NT == 2 ? 128 : 0, kCols = 128 + kTermAcc;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
@@ -1049,7 +1075,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     aux.abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 1) tmem_alloc(&aux.tmem_base, 128);
+  if (warp == 1) tmem_alloc(&aux.tmem_base, kCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1103,9 +1129,9 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
           for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              tc_mma_cta(tmem + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (z_head >> 4) + k * 2,
+              tc_mma_cta(tmem + t * kTermAcc + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (z_head >> 4) + k * 2,
                          desc_hi(1024, true), idesc, first);
-              first = 1u;
+              if (kTermAcc == 0 || t == NT - 1) first = 1u;
             }
         }
         tc_commit_cta(empty0 + rg.stage * 8);
@@ -1126,12 +1152,14 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int width = p.heads * D;
         float* dst = p.out_part + ((int64_t)blockIdx.y * p.n_hidden_cap + p.group_first + r0) * width + head0 * D + row;
         for (int c = 0; c < m; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + hh * NC + c, v);
+          uint32_t v[NT][16];
+          const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + hh * NC + c;
+          tmem_ld16(at, v[0]);
+          if (kTermAcc != 0) tmem_ld16(at + kTermAcc, v[1]);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c + j < m) dst[(int64_t)(c + j) * width] = __uint_as_float(v[j]);
+            if (c + j < m) dst[(int64_t)(c + j) * width] = kTermAcc != 0 ? add_terms(v, j) : __uint_as_float(v[0][j]);
         }
       }
     }
@@ -1139,7 +1167,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   if (!ok) drain();
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_free(tmem, 128); }
+  if (warp == 1) { tc_fence_after(); tmem_free(tmem, kCols); }
 }
 
 // ---- scratch and host side --------------------------------------------------------------

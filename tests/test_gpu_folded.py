@@ -107,6 +107,47 @@ def test_small_and_large_queries_keep_their_bits():
     check(w, "query sizes")
 
 
+def attention64(w, r):
+    """Hidden-cached request r (its new row written) in 64 bits."""
+    m, s, h, d, bs = w.meta, w.seq_lens[r], w.heads, w.shape.head_dim, w.shape.block_size
+    t = torch.arange(s)
+    rows = m.private_block_tables[r].cpu().long()[t // bs] * bs + t % bs
+    x = O.flat_rows(w.hidden_cache.cpu())[rows].double()
+    wk, bk, wv, bv = (y.cpu().double() for y in w.kv_weights())
+    k, v = (x @ wk.T + bk).view(s, h, d), (x @ wv.T + bv).view(s, h, d)
+    p = torch.softmax(torch.einsum("hd,thd->ht", w.query[r].cpu().double().view(h, d), k) * w.scale, dim=1)
+    return torch.einsum("ht,thd->hd", p, v).reshape(-1)
+
+
+# (heads, head size, hidden): one instruction per step for both terms of the folded query, and one for each
+@pytest.mark.parametrize("heads,d,e", [(8, 128, 1024), (160, 32, 128)])
+@pytest.mark.parametrize("rows,w_k", [(1.0, 0.02), (0.1, 0.02), (1e-2, 0.02), (1e-3, 0.02), (1.0, 1e-3), (1.0, 1e-4), (1e-4, "large")])
+def test_rows_and_weights_of_any_size_keep_their_bits(rows, w_k, heads, d, e):
+    """fp16 has few exponents: cached rows N(0, rows) against W_v of N(0, 1), W_k from N(0, 1e-4) up to entries whose
+    folded queries (2 sum |W_k| over a head's rows) pass the largest fp16.  The bound is that of the oracle's
+    cases, and half the spacing of the subnormal numbers for an output among them."""
+    w = make_decode_workload(LayerShape("t", heads, d, e, F), [300, 17, 600, 1], [True] * 4, seed=9, device="cpu")
+    hd = heads * d
+    w.kv_cache.mul_(rows)
+    if w.hidden_cache.data_ptr() != w.kv_cache.data_ptr():
+        w.hidden_cache.mul_(rows)
+    w.hidden_states.mul_(rows)
+    w.qkv_weight[2 * hd:].mul_(50.0)
+    w.qkv_bias.zero_()
+    if w_k == "large":
+        w.query.abs_().clamp_(max=0.4).add_(1.5)
+        w.qkv_weight[hd:2 * hd].add_(1.0).mul_(51200.0 / d)
+        assert float((w.query[0, :d].double() @ w.qkv_weight[hd:hd + d].double()).min()) > 65504
+    else:
+        w.qkv_weight[hd:2 * hd].mul_(w_k / 0.02)
+    w = w.to("cuda")
+    out = run_step(w).cpu().double()
+    for r in range(4):
+        y = attention64(w, r)
+        bad = ~((out[r] - y).abs() <= 2.0 ** -11 * y.abs() + 2.0 ** -14 * y.pow(2).mean().sqrt() + 2.0 ** -25)
+        assert not bad.any(), (r, int(bad.sum()), float(((out[r] - y).abs() / y.pow(2).mean().sqrt()).max()))
+
+
 def _step_into(w, out, ws):
     m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
     return A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache, wk, bk, wv,
