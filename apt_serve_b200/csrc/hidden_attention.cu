@@ -108,6 +108,7 @@ struct Params {
 
 // SCALED: fp16's second term at kRestUp times its value, for products that have accumulators of their own.
 constexpr float kRestUp = 2048.f;
+template <typename T> constexpr float kRestDown = kTerms<T> == 2 ? 1.f / kRestUp : 1.f;
 template <typename T, bool SCALED>
 __device__ __forceinline__ void split_terms(float v, T (&t)[kTerms<T>]) {
 #pragma unroll
@@ -120,7 +121,7 @@ __device__ __forceinline__ void split_terms(float v, T (&t)[kTerms<T>]) {
 // The value whose terms' products are v, the smaller ones added first.
 template <int NT, int N>
 __device__ __forceinline__ float add_terms(const uint32_t (&v)[NT][N], int j) {
-  if (NT == 2) return fmaf(__uint_as_float(v[NT - 1][j]), 1.f / kRestUp, __uint_as_float(v[0][j]));
+  if constexpr (NT == 2) return fmaf(__uint_as_float(v[1][j]), 1.f / kRestUp, __uint_as_float(v[0][j]));
   float x = __uint_as_float(v[NT - 1][j]);
 #pragma unroll
   for (int i = NT - 2; i >= 0; --i) x += __uint_as_float(v[i][j]);
@@ -844,6 +845,14 @@ softmax_kernel(const Params p) {
 // K-major B operand).  The rows of a CTA's first stages are requested while the softmax kernel is still running: what a
 // kernel may read before chain_wait() is what was complete when the one before it called chain_next(), here all up
 // to the scores.  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
+// The tensor cores drop what falls below the accumulator's last place at every instruction, so a sum's error grows with
+// the number of instructions that went into one accumulator (terms x cache blocks).  Where few heads leave the
+// tensor memory for it, the rests have accumulators of their own and the cache blocks' first terms take turns among two
+// or four, added in fp32; slices are narrow enough for the rests'.  Error before the output's rounding, 2048 tokens
+// among 150 requests, all terms in one -> this (the re-projection's for comparison): OPT-13B fp16 8.5e-6 -> 4.3e-6
+// (6.2e-6), bf16 1.15e-5 -> 3.8e-6 (6.1e-6), OPT-1.3B bf16 7.3e-6 -> 2.8e-6 (3.1e-6); OPT-66B tp 8 bf16, three requests,
+// 7.3e-6 -> 2.7e-6 (1.1e-5).  It costs 2 - 3 % of a step of 256 OPT-13B requests (slices of two blocks instead of four), 2 %
+// of 128 OPT-66B tp 8 requests, 1 % of 48 OPT-1.3B requests; 24 long OPT-13B requests gain 1 %.
 constexpr int kSumThreads = 192;
 
 __host__ __device__ inline uint32_t probs_block_bytes(int terms, int np) { return (uint32_t)terms * np * 32; }
@@ -872,6 +881,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   if ((int)blockIdx.x >= n_items) { chain_wait(); return; }
   const uint32_t pblk = probs_block_bytes(NT, np), per_stage = sum_stage_blocks(NT, np, slice), x_bytes = per_stage * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
+  // sets of accumulators: n_hi for the first terms, one for the rests (or all terms in one)
+  const uint32_t n_hi = 5 * slice * np <= 256 ? 4 : 3 * slice * np <= 256 ? 2 : 1, rest_set = 2 * slice * np <= 256 ? n_hi : 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
@@ -986,13 +997,13 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         tc_fence_after();
         if (elect_one()) {
           for (int k = 0; k < nb; ++k) {
-            const uint32_t acc = (b + k) != 0;
+            const uint32_t hi_set = (uint32_t)(b + k) & (n_hi - 1), hi_acc = (uint32_t)(b + k) >= n_hi;
             const uint32_t a_lo = desc_lo(x_at + k * slice * 4096, 2048), b_lo = desc_lo(p_at + k * pblk, (uint32_t)np * 16);
             for (int col = 0; col < n_col; ++col)
 #pragma unroll
               for (int i = 0; i < NT; ++i)
-                tc_mma_cta(tmem + buf * 256 + col * np, a_lo + col * 256, desc_hi(1024, true), b_lo + i * (np * 2),
-                           desc_hi(128, false), idesc, i == 0 ? acc : 1u);
+                tc_mma_cta(tmem + buf * 256 + ((i == 0 ? hi_set : rest_set) * slice + col) * np, a_lo + col * 256, desc_hi(1024, true),
+                           b_lo + i * (np * 2), desc_hi(128, false), idesc, i == 0 ? hi_acc : i > 1 || rest_set == 0 || b + k > 0);
           }
           tc_commit_cta(empty0 + rg.stage * 8);
         }
@@ -1007,12 +1018,28 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       T* z = static_cast<T*>(p.z);
       if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
       tc_fence_after();
+      const uint32_t used = min(n_hi, (uint32_t)n_blk);
       for (int col = 0; col < n_col; ++col) {
         const int e = (first + col) * 128 + quarter * 32 + lane;
         for (int h0 = 0; h0 < np; h0 += 16) {
           uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0, v);
+          const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0;
+          tmem_ld16(at, v);
+          uint32_t more[3][16], rest[16];
+#pragma unroll
+          for (uint32_t i = 0; i < 3; ++i)
+            if (i + 1 < used) tmem_ld16(at + (i + 1) * slice * np, more[i]);
+          if (rest_set != 0) tmem_ld16(at + rest_set * slice * np, rest);
           tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            float x = __uint_as_float(v[j]);
+#pragma unroll
+            for (uint32_t i = 0; i < 3; ++i)
+              if (i + 1 < used) x += __uint_as_float(more[i][j]);
+            if (rest_set != 0) x += __uint_as_float(rest[j]);
+            v[j] = __float_as_uint(x);
+          }
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {
             float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
@@ -1044,8 +1071,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
 // D[row of W_v][request] = sum_e W_v[row][e] z[request][head of the row][e]: one CTA per (128 rows of W_v,
 // range of E, 128 / HT requests), HT = 128 / D heads per 128 rows.  Rows of every head are multiplied with
 // every one of the HT heads' z and the epilogue keeps the matching quarter (half): for D = 128 nothing
-// is wasted.  fp16's second term has accumulators of its own.  Partial sums over the ranges of E are added by the
-// combine kernel.
+// is wasted.  The first term and the rests have accumulators of their own (see sum_kernel).  Partial sums over the
+// ranges of E are added by the combine kernel.
 constexpr int kUnfoldThreads = 192;
 
 // A stage: 64 columns of 128 rows of W_v and of z in boxes of 16 requests, so that few requests leave room for more
@@ -1056,7 +1083,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kUnfoldThreads, 1)
 unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_z, const Params p) {
   constexpr int NT = kTerms<T>, HT = 128 / D, NC = 128 / HT;   // NC: requests per CTA
-  constexpr uint32_t kTermAcc = NT == 2 ? 128 : 0, kCols = 128 + kTermAcc;
+  constexpr uint32_t kRestAcc = 128, kCols = 256;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
@@ -1129,9 +1156,9 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
           for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              tc_mma_cta(tmem + t * kTermAcc + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (z_head >> 4) + k * 2,
+              tc_mma_cta(tmem + (t == 0 ? 0 : kRestAcc) + hh * NC, a_lo + k * 2, desc_hi(1024, true), b_lo + (t * HT + hh) * (z_head >> 4) + k * 2,
                          desc_hi(1024, true), idesc, first);
-              if (kTermAcc == 0 || t == NT - 1) first = 1u;
+              if (t > 0) first = 1u;
             }
         }
         tc_commit_cta(empty0 + rg.stage * 8);
@@ -1152,14 +1179,14 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int width = p.heads * D;
         float* dst = p.out_part + ((int64_t)blockIdx.y * p.n_hidden_cap + p.group_first + r0) * width + head0 * D + row;
         for (int c = 0; c < m; c += 16) {
-          uint32_t v[NT][16];
+          uint32_t v[16], rest[16];
           const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + hh * NC + c;
-          tmem_ld16(at, v[0]);
-          if (kTermAcc != 0) tmem_ld16(at + kTermAcc, v[1]);
+          tmem_ld16(at, v);
+          tmem_ld16(at + kRestAcc, rest);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            if (c + j < m) dst[(int64_t)(c + j) * width] = kTermAcc != 0 ? add_terms(v, j) : __uint_as_float(v[0][j]);
+            if (c + j < m) dst[(int64_t)(c + j) * width] = fmaf(__uint_as_float(rest[j]), kRestDown<T>, __uint_as_float(v[j]));
         }
       }
     }
@@ -1197,6 +1224,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.splits = splits < 1 ? 1 : splits;
   int ms = 256 / l.np;
   if (ms > kMaxSlice) ms = kMaxSlice;
+  while (ms > 1 && 2 * ms * l.np > 256) --ms;   // room for the rests' accumulators (see sum_kernel)
   while (ms > 1 && 3 * sum_stage_bytes(nt, l.np, ms) > kRingBytes) --ms;   // at least three stages
   l.max_slice = ms;
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
