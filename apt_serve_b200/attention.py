@@ -85,19 +85,36 @@ def raise_on_device_status(workspace: Optional[torch.Tensor] = None,
     """Raise ``RuntimeError`` if the last attention call on ``workspace`` (default: the
     per-device workspace of ``device``) left a non-zero status word: 1..7 = a bounded wait
     of the re-projection kernel ran out and the call's output is NaN, 8 = K/V-cached
-    requests in a batch that was given no K/V cache.  Synchronises the current stream, so
-    call it where a synchronisation is cheap (once per engine step, beside the sampler's
-    device-to-host copy), not per layer."""
-    if workspace is None:
-        workspace = _workspaces.get(torch.device(device) if device is not None
-                                    else torch.device("cuda", torch.cuda.current_device()))
-        if workspace is None:
-            return
-    code = attention_status(workspace)
+    requests in a batch that was given no K/V cache; or if the cache operations on the device
+    left one: a cache write that was not finished, metadata that points outside its tensors.
+    Synchronises the current stream, so call it where a synchronisation is cheap (once per engine
+    step, beside the sampler's device-to-host copy), not per layer."""
+    if workspace is not None:
+        dev = workspace.device
+    else:
+        dev = (torch.device(device) if device is not None
+               else torch.device("cuda", torch.cuda.current_device()))
+        workspace = _workspaces.get(dev)
+    code = 0 if workspace is None else attention_status(workspace)
     if code != 0:
         what = ("a bounded device-side wait ran out; the output was filled with NaN" if code < 8 else
                 "the batch holds K/V-cached requests but no K/V cache was passed; their rows are zero")
         raise RuntimeError(f"aptserve_b200: attention status {code}: {what}")
+    code = cache_ops_status(dev)
+    if code != 0:
+        what = ("a bounded device-side wait of a cache write ran out; rows are missing in the cache" if code == 1 else
+                "decode metadata pointed outside its tensors; the requests concerned were left out of the step")
+        raise RuntimeError(f"aptserve_b200: cache operations status {code}: {what}")
+
+
+def cache_ops_status(device: torch.device) -> int:
+    """Status word of the cache operations on ``device`` (0 = fine; ``aps_cache_ops_status``).  Synchronises the
+    current stream."""
+    import ctypes
+    host = ctypes.c_int(0)
+    with N.on_device(device):
+        N.check(N.lib().aps_cache_ops_status(ctypes.addressof(host), N.current_stream(device)))
+    return host.value
 
 
 def _i32(t: torch.Tensor, name: str) -> torch.Tensor:

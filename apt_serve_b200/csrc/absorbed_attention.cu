@@ -123,7 +123,7 @@ scores_kernel(const AbsorbedArgs a) {
     const int piece = threadIdx.x + i * kScoreThreads, row = piece >> 3, j = piece & 7;
     const int tok = tok0 + row;
     const int64_t xr = tok < seq ? token_row(bt, tok, a.block_size) : 0;
-    x_ok[i] = tok < seq && xr < a.num_x_rows;
+    x_ok[i] = tok < seq && xr >= 0 && xr < a.num_x_rows;
     x_src[i] = x + xr * a.x_row_stride + j * 8;
     x_dst[i] = (uint32_t)(row * 128 + ((j ^ (row & 7)) << 4));
   }
@@ -321,7 +321,7 @@ weighted_sum_kernel(const AbsorbedArgs a) {
       for (int i = 0; i < 4; ++i) {
         const int row = half * 16 + r0 + i * 4;
         const int64_t xr = row_first + r0 + i * 4;
-        const bool ok = sub * kSumTokens + row < seq && xr < a.num_x_rows;
+        const bool ok = sub * kSumTokens + row < seq && row_first >= 0 && xr < a.num_x_rows;
         cp_async16(s + row * 1024 + (((j & ~7) | ((j ^ row) & 7)) << 4), x + (ok ? xr : 0) * a.x_row_stride + j * 8, ok);
       }
     }

@@ -44,6 +44,9 @@ inline int launch_status(const char* what) {
   return APS_OK;
 }
 
+// cache_type of a request that has no usable tables (derive_tables_kernel): it is neither written nor attended.
+constexpr int32_t kCacheTypeNone = INT32_MIN;
+
 // ---- chained launches ----------------------------------------------------------------
 // The kernels of one call run one after the other on the caller's stream, most of them for 5 - 30 us; a plain
 // launch leaves 2 us between two of them and starts every one with cold CTAs.  They are therefore launched as

@@ -558,7 +558,7 @@ struct NewTokenJobs {
     const bool second = (row & 1) != 0;
     BulkJob j{nullptr, nullptr, nullptr, 0u};
     const int pos = min(seq_lens[r], max_blocks * block_size) - 1;
-    if (pos < 0) return j;
+    if (pos < 0 || cache_type[r] == kCacheTypeNone) return j;
     const int64_t blk = block_tables[r * max_blocks + pos / block_size];
     if (cache_type[r] != 0) {
       if (second || piece >= pc_hid.pieces || hidden == nullptr) return j;

@@ -169,21 +169,22 @@ step_plan_kernel(const PlanArgs a) {
   auto chunks_of = [&](int s) { return a.kv_present ? (s + kChunkTokens - 1) / kChunkTokens : 0; };
   int2 mine = make_int2(0, 0);
   for (int r = r0; r < r1; ++r) {
-    const int s = max(0, min(a.seq_lens[r], a.max_tokens));
-    if (a.cache_type[r] != 0) ++mine.y;
+    const int s = max(0, min(a.seq_lens[r], a.max_tokens)), type = a.cache_type[r];
+    if (type == kCacheTypeNone) continue;
+    if (type != 0) ++mine.y;
     else { mine.x += chunks_of(s); if (!a.kv_present) s_missing = 1; }
   }
   int2 total;
   const int2 inc = block_scan(mine, warp_sums, tid, total);
   int o_kv = inc.x - mine.x, o_hid = inc.y - mine.y;
   for (int r = r0; r < r1; ++r) {
-    const int s = max(0, min(a.seq_lens[r], a.max_tokens));
+    const int s = max(0, min(a.seq_lens[r], a.max_tokens)), type = a.cache_type[r];
     a.part_offset[r] = o_kv;
-    if (a.cache_type[r] != 0) {
+    if (type != 0 && type != kCacheTypeNone) {
       a.hid_list[o_hid++] = make_int2(r, s);
     } else {
       a.hid_slot[r] = -1;
-      const int c = chunks_of(s);
+      const int c = type != 0 ? 0 : chunks_of(s);
       for (int j = 0; j < c; ++j) a.kv_chunks[o_kv + j] = make_int2(r, j);
       o_kv += c;
     }

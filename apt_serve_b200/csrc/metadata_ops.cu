@@ -129,7 +129,10 @@ fill_kernel(MetaLayout L, MetaOut O, const int32_t* __restrict__ block_tables,
 // those.  What is left is
 // one dependent chain of loads (hidden_rows, holder_upd, slot_mapping), about 4 us.  Every CTA scans
 // hidden_rows itself: at most 8 bytes per request and CTA, from L2.
-// An index outside its tensor is never followed: the entry is 0 and g_metadata_status is set.
+// An index outside its tensor is never followed, and no block is made up for it: a request whose run of slot_mapping leaves
+// the tensor or holds a negative slot gets kCacheTypeNone and a table of -1 (no cache write, no attention, a zero
+// output row), every request does if hidden_rows names one that does not exist (the request it was meant for would
+// pass for a K/V-cached one), and g_metadata_status is set.
 __device__ int g_metadata_status = 0;
 constexpr int kDeriveThreads = 128;
 constexpr int kStatusBadIndex = 2;   // value of the cache-operation status word
@@ -141,15 +144,15 @@ derive_tables_kernel(int32_t* __restrict__ tables, int32_t* __restrict__ cache_t
                      const int64_t* __restrict__ hidden_rows, int64_t num_hidden, const int32_t* __restrict__ seq_lens,
                      int batch, int max_blocks, int64_t table_stride, int block_size) {
   const int r = blockIdx.x;
-  bool mine = false, bad = false;
+  bool mine = false, lost = false;
   for (int64_t i = threadIdx.x; i < num_hidden; i += kDeriveThreads) {
     int64_t row = hidden_rows[i];
     if (row < 0) row += batch;   // an index counts from the end when it is negative, as in the tensor form
-    bad |= row < 0 || row >= batch;
+    lost |= row < 0 || row >= batch;
     mine |= row == r;
   }
   const bool hidden = __syncthreads_or(mine) != 0;
-  if (threadIdx.x == 0) cache_type[r] = hidden ? 1 : 0;
+  bool bad = lost;
   const int64_t len = seq_lens[r], start = hidden ? holder_upd[r] - (len - 1) : 0;
   for (int j = threadIdx.x; j < max_blocks; j += kDeriveThreads) {
     int32_t id = 0;
@@ -158,16 +161,19 @@ derive_tables_kernel(int32_t* __restrict__ tables, int32_t* __restrict__ cache_t
     } else if ((int64_t)j * block_size < len) {
       int64_t pos = start + (int64_t)j * block_size;
       if (pos < 0) pos += num_slots;
-      if (pos < 0 || pos >= num_slots) {
-        bad = true;
-      } else {
-        const int64_t slot = slot_mapping[pos];
-        id = (int32_t)(slot >= 0 ? slot / block_size : -((block_size - 1 - slot) / block_size));
-      }
+      const int64_t slot = pos >= 0 && pos < num_slots ? slot_mapping[pos] : -1;
+      bad |= slot < 0;
+      id = (int32_t)(slot / block_size);
     }
     tables[(int64_t)r * max_blocks + j] = id;
   }
-  if (bad) g_metadata_status = kStatusBadIndex;
+  bad = __syncthreads_or(bad) != 0;
+  if (bad)
+    for (int j = threadIdx.x; j < max_blocks; j += kDeriveThreads) tables[(int64_t)r * max_blocks + j] = -1;
+  if (threadIdx.x == 0) {
+    cache_type[r] = bad ? kCacheTypeNone : hidden ? 1 : 0;
+    if (bad) g_metadata_status = kStatusBadIndex;
+  }
 }
 
 }  // namespace
@@ -177,6 +183,7 @@ int read_metadata_status(int* host_status, cudaStream_t stream) {
   APS_CUDA(cudaGetSymbolAddress(&addr, g_metadata_status));
   APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, stream));
   APS_CUDA(cudaStreamSynchronize(stream));
+  if (*host_status != 0) APS_CUDA(cudaMemsetAsync(addr, 0, sizeof(int), stream));   // reported once
   return APS_OK;
 }
 

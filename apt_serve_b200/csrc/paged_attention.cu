@@ -51,8 +51,9 @@ plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restr
   __syncthreads();
   const int per = (batch + kPlanThreads - 1) / kPlanThreads;
   const int r0 = min(batch, tid * per), r1 = min(batch, r0 + per);
-  auto seq_of = [&](int r) { return max(0, min(seq_lens[r], max_tokens)); };
-  auto hidden = [&](int r) { return cache_type != nullptr && cache_type[r] != 0; };
+  auto none = [&](int r) { return cache_type != nullptr && cache_type[r] == kCacheTypeNone; };
+  auto seq_of = [&](int r) { return none(r) ? 0 : max(0, min(seq_lens[r], max_tokens)); };
+  auto hidden = [&](int r) { return cache_type != nullptr && cache_type[r] != 0 && !none(r); };
   // without a K/V cache a K/V-cached request gets no chunks and no partials: its output row is zero
   auto chunks_of = [&](int s) { return kv_present ? (s + kChunkTokens - 1) / kChunkTokens : 0; };
   auto subs_of = [&](int s) {   // sub-blocks a hidden request of s tokens occupies in the tile list
@@ -64,7 +65,7 @@ plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restr
   for (int r = r0; r < r1; ++r) {
     const int s = seq_of(r);
     if (hidden(r)) sub += subs_of(s);
-    else { kv += chunks_of(s); if (!kv_present) s_kv_missing = 1; }
+    else { kv += chunks_of(s); if (!kv_present && !none(r)) s_kv_missing = 1; }
   }
   int2 total;
   const int2 inc = block_scan(make_int2(kv, sub), sums_a, tid, total);

@@ -287,7 +287,10 @@ def derive_private_block_tables(meta: DecodeMetadata, block_size: int):
     Returns ``(private_block_tables int32 [B, max_blocks], cache_type int32 [B])``.
 
     One kernel launch (``aps_derive_private_tables``) when the metadata lies on a GPU in the types the
-    model runner gives it, tensor operations for anything else.
+    model runner gives it, tensor operations for anything else.  Metadata that points outside its own tensors
+    stops the tensor operations with an index error; the kernel takes the requests concerned out of the step
+    (cache type ``INT32_MIN``, tables of -1: no cache write, a zero output row) and
+    ``attention.raise_on_device_status`` raises.
     """
     bt, sm, upd = meta.block_tables, meta.slot_mapping, meta.hidden_holder_upd
     rows, lens = meta.hidden_cache_use_input, meta.seq_lens_tensor

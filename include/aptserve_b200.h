@@ -240,7 +240,9 @@ int aps_paged_decode_attention_static(void* out, const void* query, const void* 
  *                       (row id = block_tables[r][t / BS] * BS + t % BS, row
  *                       stride hidden_row_stride, first hidden_size elements);
  *                       K = X_r W_k^T + b_k, V = X_r W_v^T + b_v on the tensor
- *                       cores, fp32 accumulation, then the same softmax.
+ *                       cores, fp32 accumulation, then the same softmax;
+ *   cache_type[r] == INT32_MIN: not attended, the output row is zero (see
+ *                       aps_derive_private_tables).
  * w_k / w_v: [H*D, hidden_size] row-major with row stride w_stride (the K and V
  * thirds of the fused QKV weight, lin.py:123-125); b_k / b_v: [H*D] or NULL.
  * num_hidden_rows is the number of addressable rows of hidden_cache
@@ -347,8 +349,8 @@ int aps_reprojection_cycles(const void* workspace, unsigned long long* host_cycl
 
 /*
  * Status of the cache operations on the current device: 0, 1 once a bounded wait on a bulk load
- * ran out (the launch then stopped copying), or 2 once aps_derive_private_tables met an index
- * outside its tensor.  Synchronises `stream`.
+ * ran out (the launch then stopped copying), or 2 if aps_derive_private_tables has met an index
+ * outside its tensor since the last call that returned 2.  Synchronises `stream`.
  */
 int aps_cache_ops_status(int* host_status, void* stream);
 
@@ -412,8 +414,10 @@ int aps_expand_decode_metadata(const int32_t* block_tables, const int32_t* block
  * cache_type: int32 [B]; block_tables: int32 rows of block_tables_stride elements; slot_mapping [num_slots],
  * hidden_holder_upd [B], hidden_cache_use_input [num_hidden]: the reference's int64 tensors;
  * seq_lens: int32 [B].  A hidden-cached request's entries past its length are 0.  Negative indices
- * count from the end; an index outside its tensor gives a 0 entry and sets the status word that
- * aps_cache_ops_status reads.
+ * count from the end.  A request whose run leaves slot_mapping or holds a negative slot gets
+ * cache_type INT32_MIN and a table of -1, and so does every request if hidden_cache_use_input names
+ * one that does not exist: the calls that take the tables neither write nor attend such a request
+ * (its output row is zero), and the status word that aps_cache_ops_status reads is set.
  */
 int aps_derive_private_tables(int32_t* tables, int32_t* cache_type, const int32_t* block_tables,
                               const int64_t* slot_mapping, int64_t num_slots, const int64_t* hidden_holder_upd,

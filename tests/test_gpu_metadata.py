@@ -132,18 +132,75 @@ def test_derived_tables_equal_the_tensor_form(lens, hid, bs):
 
 
 def test_derived_tables_bound_their_indices():
-    """A claim that points outside slot_mapping: nothing is read there, the entries are 0, the status says so."""
+    """A claim that points outside slot_mapping: nothing is read there, the request is taken out of the step, the status
+    says so once."""
     import ctypes
     from apt_serve_b200 import _native as N
     lib, host = N.lib(), ctypes.c_int(0)
     i32 = dict(dtype=torch.int32, device="cuda")
     i64 = dict(dtype=torch.int64, device="cuda")
-    tables, ctype = torch.full((2, 4), -5, **i32), torch.full((2,), -5, **i32)
-    bt, lens = torch.arange(8, **i32).view(2, 4), torch.tensor([40, 7], **i32)
-    slots, upd, rows = torch.arange(32, 64, **i64), torch.tensor([39, 40], **i64), torch.tensor([0], **i64)
-    stream = N.current_stream(tables.device)
-    N.check(lib.aps_derive_private_tables(N.ptr(tables), N.ptr(ctype), N.ptr(bt), N.ptr(slots), 32, N.ptr(upd),
-                                          N.ptr(rows), 1, N.ptr(lens), 2, 4, 4, 16, stream))
-    N.check(lib.aps_cache_ops_status(ctypes.addressof(host), stream))
-    assert tables.tolist() == [[2, 3, 0, 0], [4, 5, 6, 7]] and ctype.tolist() == [1, 0]
-    assert host.value == 2
+    none = -2 ** 31
+    for upd, rows, want, types in [([39, 40], [0], [[-1] * 4, [4, 5, 6, 7]], [none, 0]),
+                                   ([31, 40], [0, 2], [[-1] * 4] * 2, [none] * 2),
+                                   ([31, 40], [-3], [[-1] * 4] * 2, [none] * 2)]:
+        tables, ctype = torch.full((2, 4), -5, **i32), torch.full((2,), -5, **i32)
+        bt, lens = torch.arange(8, **i32).view(2, 4), torch.tensor([40, 7], **i32)
+        slots, upd, rows = torch.arange(32, 64, **i64), torch.tensor(upd, **i64), torch.tensor(rows, **i64)
+        stream = N.current_stream(tables.device)
+        N.check(lib.aps_derive_private_tables(N.ptr(tables), N.ptr(ctype), N.ptr(bt), N.ptr(slots), 32, N.ptr(upd),
+                                              N.ptr(rows), rows.numel(), N.ptr(lens), 2, 4, 4, 16, stream))
+        for status in (2, 0):
+            N.check(lib.aps_cache_ops_status(ctypes.addressof(host), stream))
+            assert host.value == status
+        assert tables.tolist() == want and ctype.tolist() == types
+
+
+# direct path (fp16, fp32), re-projection on the tensor cores (few requests) and on the CUDA cores (three heads)
+@pytest.mark.parametrize("heads,d,e,dtype", [(8, 128, 1024, torch.float16), (12, 64, 768, torch.float32),
+                                             (2, 128, 256, torch.float16), (3, 64, 192, torch.float16)])
+@pytest.mark.parametrize("fault", ["run", "slot", "list"])
+def test_a_step_on_bad_metadata_touches_no_other_request(heads, d, e, dtype, fault):
+    from apt_serve_b200 import attention as A
+    from apt_serve_b200.metadata import derive_private_block_tables
+    from apt_serve_b200.workloads import LayerShape, make_decode_workload
+    from dataclasses import replace
+    w = make_decode_workload(LayerShape("t", heads, d, e, dtype), [300, 40, 129, 33, 260], [True, False, True, True, False],
+                             seed=5, device="cuda")
+    two_caches = w.hidden_cache.data_ptr() != w.kv_cache.data_ptr()
+
+    def step(meta):
+        tables, types = derive_private_block_tables(meta, 16)
+        return A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache,
+                                   *w.kv_weights(), tables, meta.seq_lens_tensor, types, w.scale)
+
+    before = w.kv_cache.clone(), w.hidden_cache.clone()
+    want = step(w.meta)
+    A.raise_on_device_status()
+    rows = w.hidden_cache.reshape(-1, e)
+    bad = 2
+    at = w.block_tables[bad][-1] * 16 + (w.seq_lens[bad] - 1) % 16   # its new row
+    rows[at] = before[1].reshape(-1, e)[at]
+    after = w.kv_cache.clone(), w.hidden_cache.clone()
+    w.kv_cache.copy_(before[0])
+    if two_caches:
+        w.hidden_cache.copy_(before[1])
+    m = w.meta
+    if fault == "run":
+        m = replace(m, hidden_holder_upd=m.hidden_holder_upd + torch.tensor([0, 0, 5000, 0, 0], device="cuda"))
+    elif fault == "slot":
+        slots = m.slot_mapping.clone()
+        slots[m.hidden_holder_upd[bad] - 128] = -1
+        m = replace(m, slot_mapping=slots)
+    else:
+        m = replace(m, hidden_cache_use_input=torch.tensor([0, 3, 17], device="cuda"))
+        after = before
+    out = step(m)
+    with pytest.raises(RuntimeError, match="outside its tensors"):
+        A.raise_on_device_status()
+    A.raise_on_device_status()   # said once
+    assert torch.equal(w.kv_cache, after[0]) and torch.equal(w.hidden_cache, after[1])
+    good = [] if fault == "list" else [0, 1, 3, 4]
+    assert not out[[r for r in range(5) if r not in good]].any()
+    if good:
+        tol = 1e-4 if dtype == torch.float32 else 4e-3
+        assert torch.allclose(out[good].float(), want[good].float(), rtol=tol, atol=tol)
