@@ -123,6 +123,14 @@ def _i32(t: torch.Tensor, name: str) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _plane_pointers(kv_cache: torch.Tensor) -> Tuple[int, int]:
+    """Addresses of ``kv_cache[0]`` and ``kv_cache[1]``, without building the two tensors."""
+    if kv_cache.shape[0] < 2:
+        raise IndexError(f"kv_cache holds {kv_cache.shape[0]} plane(s), the K and the V plane are needed")
+    k = kv_cache.data_ptr()
+    return k, k + kv_cache.stride(0) * kv_cache.element_size()
+
+
 # ----------------------------------------------------------------------------- #
 # functional entry points
 # ----------------------------------------------------------------------------- #
@@ -185,8 +193,8 @@ def hybrid_decode_attention(query: torch.Tensor, kv_cache: Optional[torch.Tensor
         return out
     if kv_cache is not None:
         _, _, bs, h, d = kv_cache.shape
-        kc, block_stride = kv_cache.data_ptr(), kv_cache.stride(1)
-        vc = kc + kv_cache.stride(0) * kv_cache.element_size()
+        kc, vc = _plane_pointers(kv_cache)
+        block_stride = kv_cache.stride(1)
     else:
         if num_heads is None or head_size is None:
             raise RuntimeError("hybrid_decode_attention: num_heads / head_size needed without kv_cache")
@@ -245,8 +253,8 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
         return out
     if kv_cache is not None:
         _, _, bs, h, d = kv_cache.shape
-        kc, block_stride = kv_cache.data_ptr(), kv_cache.stride(1)
-        vc = kc + kv_cache.stride(0) * kv_cache.element_size()
+        kc, vc = _plane_pointers(kv_cache)
+        block_stride = kv_cache.stride(1)
     else:
         if num_heads is None or head_size is None:
             raise RuntimeError("decode_layer_step: num_heads / head_size needed without kv_cache")

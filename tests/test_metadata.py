@@ -135,3 +135,13 @@ def test_packed_tables_equal_numpys():
 def test_packing_leaves_anything_else_to_the_general_path(tables, shared):
     st, _ = _pack(tables, shared, [True], 3)
     assert st == 1
+
+
+def test_plane_pointers_are_those_of_the_two_planes():
+    """What the fused calls hand to the kernels as K and V plane; a cache with one plane is refused, not read past."""
+    from apt_serve_b200.attention import _plane_pointers
+    whole = torch.zeros(3, 5, 16, 2, 4, dtype=torch.float16)
+    for t in (whole, whole[:2], whole[1:], whole[:, 1:4], whole[::2]):
+        assert _plane_pointers(t) == (t[0].data_ptr(), t[1].data_ptr())
+    with pytest.raises(IndexError):
+        _plane_pointers(whole[:1])
