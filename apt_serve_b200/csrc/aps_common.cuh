@@ -58,6 +58,8 @@ constexpr int32_t kCacheTypeNone = INT32_MIN;
 //     still implies that of everything before it;
 //   - chain_next() comes after the CTA's tensor memory is allocated: a CTA of the next kernel cannot take
 //     columns that this kernel still has to get.
+//   - its pointer parameters are not __restrict__: that would let the compiler take what is read through them for constant
+//     over the whole kernel and load it before the wait.
 // chain_wait() returns at once in a kernel launched the plain way, and work enqueued the plain way behind a
 // chained kernel waits for it as always.
 // Measured on one B200, plain -> chained: a step of one OPT-13B request 89 -> 67 us, of 48 OPT-1.3B requests 149 -> 127,

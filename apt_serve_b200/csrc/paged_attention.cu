@@ -37,10 +37,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // first over (K/V chunks, hidden sub-blocks), which fixes where each hidden request's rows
 // sit in the tile list, then over the number of softmax partials each request will leave.
 __global__ void __launch_bounds__(kPlanThreads)
-plan_kernel(int* __restrict__ plan, int* __restrict__ part_offset, int2* __restrict__ kv_chunks,
-            int2* __restrict__ hid_tiles, int* __restrict__ first_tile, int2* __restrict__ hid_subs,
-            int* __restrict__ hid_rows, const int32_t* __restrict__ seq_lens,
-            const int32_t* __restrict__ cache_type, const int32_t* __restrict__ block_tables, int batch,
+plan_kernel(int* plan, int* part_offset, int2* kv_chunks,
+            int2* hid_tiles, int* first_tile, int2* hid_subs,
+            int* hid_rows, const int32_t* seq_lens,
+            const int32_t* cache_type, const int32_t* block_tables, int batch,
             int max_tokens, int max_blocks, int block_size, int pack_tiles, int kv_present) {
   __shared__ int2 sums_a[32], sums_b[32];
   __shared__ int s_kv_missing;
@@ -181,11 +181,11 @@ struct KvCfg {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kKvWarps * 32, 2)
-kv_attention_kernel(int* __restrict__ plan, const int* __restrict__ part_offset,
-                    const int2* __restrict__ kv_chunks, float* __restrict__ part_ml,
-                    float* __restrict__ part_acc, const T* __restrict__ query,
-                    const T* __restrict__ key_cache, const T* __restrict__ value_cache,
-                    const int32_t* __restrict__ block_tables, const int32_t* __restrict__ seq_lens,
+kv_attention_kernel(int* plan, const int* part_offset,
+                    const int2* kv_chunks, float* part_ml,
+                    float* part_acc, const T* query,
+                    const T* key_cache, const T* value_cache,
+                    const int32_t* block_tables, const int32_t* seq_lens,
                     int max_blocks_per_seq, int heads, int block_size, int64_t query_stride,
                     int64_t block_stride, float scale_log2) {
   using C = KvCfg<T, D>;
@@ -381,10 +381,10 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 template <typename T, int D, int S>
 __global__ void __launch_bounds__(kTmaWarps * 32, (384 / (kTmaWarps * 32)) > 0 ? (384 / (kTmaWarps * 32)) : 1)
 kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                        int* __restrict__ plan, const int* __restrict__ part_offset,
-                        const int2* __restrict__ kv_chunks, float* __restrict__ part_ml,
-                        float* __restrict__ part_acc, const T* __restrict__ query,
-                        const int32_t* __restrict__ block_tables, const int32_t* __restrict__ seq_lens,
+                        int* plan, const int* part_offset,
+                        const int2* kv_chunks, float* part_ml,
+                        float* part_acc, const T* query,
+                        const int32_t* block_tables, const int32_t* seq_lens,
                         int max_blocks_per_seq, int heads, int block_size, int64_t query_stride,
                         float scale_log2) {
   static_assert(sizeof(T) == 2 && (D == 64 || D == 128), "2-byte types, head size 64 or 128");
@@ -626,8 +626,8 @@ __device__ __forceinline__ void store4(T* dst, const float (&v)[4]) {
 // written: the whole output is filled with NaN instead of numbers that look plausible.
 template <typename T>
 __global__ void __launch_bounds__(256)
-combine_kernel(const int* __restrict__ plan, const int* __restrict__ part_offset, const float* __restrict__ part_ml,
-               const float* __restrict__ part_acc, T* __restrict__ out, int batch, int heads,
+combine_kernel(const int* plan, const int* part_offset, const float* part_ml,
+               const float* part_acc, T* out, int batch, int heads,
                int head_size, int64_t out_stride, const HiddenOutputs hid) {
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
