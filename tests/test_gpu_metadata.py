@@ -106,6 +106,21 @@ def test_zero_length_is_refused_on_the_host():
         expand_decode_metadata([5, 0], [True, False], [[0], [1]], [[2], []], 16, "cuda")
 
 
+def test_expansion_during_capture_is_refused():
+    """A replay would copy from a staging buffer that is no longer this call's."""
+    tables, shared = batch([40, 7], [True, False])
+    expand_decode_metadata([40, 7], [True, False], tables, shared, 16, "cuda")
+    x, g = torch.zeros(4, device="cuda"), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        with pytest.raises(RuntimeError, match="capture"):
+            expand_decode_metadata([40, 7], [True, False], tables, shared, 16, "cuda")
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4
+    check([40, 7], [True, False])
+
+
 @pytest.mark.parametrize("bs", [16, 32])
 @pytest.mark.parametrize("lens,hid", [
     ([1], [True]),
