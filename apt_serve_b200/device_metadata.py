@@ -36,6 +36,8 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         # the kernels count a length below 1 as 1; the host counts must agree with them
         raise ValueError("expand_decode_metadata: every sequence length must be >= 1 "
                          "(it includes the token being decoded)")
+    if len(block_tables) != b:
+        raise ValueError(f"expand_decode_metadata: {len(block_tables)} block tables for {b} sequences")
     if dev.type == "cuda" and torch.cuda.is_current_stream_capturing():
         # the graph would read the staging buffer again on every replay, long after it has been given back
         raise RuntimeError("expand_decode_metadata: not during stream capture (the tables come from host memory)")

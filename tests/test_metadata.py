@@ -145,3 +145,11 @@ def test_plane_pointers_are_those_of_the_two_planes():
         assert _plane_pointers(t) == (t[0].data_ptr(), t[1].data_ptr())
     with pytest.raises(IndexError):
         _plane_pointers(whole[:1])
+
+
+@pytest.mark.parametrize("tables", [[[1]], [[1], [2], [3]], []])
+def test_expansion_wants_one_table_per_sequence(tables):
+    """One table too few used to be repeated for every sequence by the general packing path."""
+    from apt_serve_b200.device_metadata import expand_decode_metadata
+    with pytest.raises(ValueError, match="block tables for 2 sequences"):
+        expand_decode_metadata([5, 6], [True, False], tables, [[4], []], BS, "cuda")
