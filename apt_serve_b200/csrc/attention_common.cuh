@@ -182,6 +182,7 @@ int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t stream);
 // output (hidden_attention.cu).
 constexpr int kGroup = 256;   // hidden requests per pass (bounds the scratch)
 bool folded_supported(int dtype, int heads, int head_size, int hidden);
+bool folded_takes(const HybridCall& c);   // pointers and strides; what it does not take is re-projected
 size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
                               int hidden, int dtype);
 // behind_write: the kernel enqueued last on the stream is launch_new_token_write's.

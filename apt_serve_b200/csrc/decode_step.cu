@@ -32,7 +32,7 @@ bool folded_shape(int batch, int max_blocks, int block_size, int heads, int head
 
 bool use_folded(const HybridCall& c) {
   const AttnShape& s = c.shape;
-  return folded_shape(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size, s.dtype) &&
+  return folded_takes(c) && folded_shape(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size, s.dtype) &&
          c.workspace_bytes >= folded_workspace_bytes(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size,
                                                      c.hidden_size, s.dtype);
 }

@@ -1332,14 +1332,16 @@ size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size,
          layout_of(batch, max_blocks_per_seq, block_size, heads, head_size, hidden, dtype).total;
 }
 
+// Tensor maps: 16-byte aligned bases and row strides.  The CUDA-core re-projection, which serves the head counts that do not
+// fill a tile, takes any others, so they are left to it and not refused.
+bool folded_takes(const HybridCall& c) {
+  return c.hidden_cache && c.w_k && c.w_v && c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size &&
+         c.w_stride >= c.hidden_size && c.hidden_row_stride % 8 == 0 && c.w_stride % 8 == 0 && aligned_to(c.hidden_cache, 16) &&
+         aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16) && sm_count() <= kMaxGrid;   // kMaxGrid: bounds the plan keeps
+}
+
 int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t cs) {
   const AttnShape& s = c.shape;
-  APS_REQUIRE(c.hidden_cache && c.w_k && c.w_v, APS_ERR_NULL_POINTER, "decode_layer_step: null pointer");
-  APS_REQUIRE(c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size && c.w_stride >= c.hidden_size,
-              APS_ERR_SHAPE, "decode_layer_step: bad hidden sizes / strides");
-  APS_REQUIRE(c.hidden_row_stride % 8 == 0 && c.w_stride % 8 == 0 && aligned_to(c.hidden_cache, 16) &&
-                  aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16),
-              APS_ERR_MISALIGNED, "decode_layer_step: hidden cache and weights must be 16-byte aligned with 16-byte row strides");
   const WorkspaceLayout w = workspace_layout(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size);
   const WorkspacePtrs ws = workspace_ptrs(c.workspace, w);
   const Layout l = layout_of(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size, s.dtype);
@@ -1348,7 +1350,6 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   const bool have_kv = c.key_cache != nullptr && c.value_cache != nullptr;
   const int nt = terms_of(s.dtype), e_blocks = c.hidden_size / 128;
   int st;
-  APS_REQUIRE(sm_count() <= kMaxGrid, APS_ERR_UNSUPPORTED, "decode_layer_step: more SMs than the plan keeps bounds for");
 
   PlanArgs pa{};
   pa.plan = ws.plan; pa.part_offset = ws.part_offset; pa.kv_chunks = ws.kv_chunks;

@@ -334,7 +334,8 @@ bool folded32_shape(int dtype, int heads, int head_size, int hidden) {
 bool folded32_supported(const HybridCall& c) {
   const AttnShape& s = c.shape;
   return folded32_shape(s.dtype, s.heads, s.head_size, c.hidden_size) && c.hidden_row_stride % 4 == 0 && c.w_stride % 4 == 0 &&
-         aligned_to(c.hidden_cache, 16) && aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16) &&
+         c.hidden_cache && c.w_k && c.w_v && c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size &&
+         c.w_stride >= c.hidden_size && aligned_to(c.hidden_cache, 16) && aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16) &&
          c.workspace_bytes >= folded32_workspace_bytes(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size);
 }
 
@@ -345,9 +346,6 @@ size_t folded32_workspace_bytes(int batch, int max_blocks_per_seq, int block_siz
 
 int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStream_t cs) {
   const AttnShape& s = c.shape;
-  APS_REQUIRE(c.hidden_cache && c.w_k && c.w_v, APS_ERR_NULL_POINTER, "decode_layer_step: null pointer");
-  APS_REQUIRE(c.num_hidden_rows > 0 && c.hidden_row_stride >= c.hidden_size && c.w_stride >= c.hidden_size,
-              APS_ERR_SHAPE, "decode_layer_step: bad hidden sizes / strides");
   const WorkspaceLayout w = workspace_layout(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size);
   const WorkspacePtrs ws = workspace_ptrs(c.workspace, w);
   const Layout l = layout_of(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size, c.hidden_size);

@@ -107,6 +107,22 @@ def test_small_and_large_queries_keep_their_bits():
     check(w, "query sizes")
 
 
+@pytest.mark.parametrize("dtype", [F, B, torch.float32])
+def test_unaligned_weights_are_re_projected(dtype):
+    """Head counts that do not fill a tile take weights of any alignment and row stride, as the CUDA-core kernel always has."""
+    w = make_decode_workload(LayerShape("t", 5, 64, 384, dtype), [300, 17, 640, 1], [True, True, False, True], seed=3, device="cuda")
+    m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
+    wide = torch.zeros(2, wk.shape[0], wk.shape[1] + 3, dtype=dtype, device="cuda")[:, :, 1:-2]
+    wide[0], wide[1] = wk, wv
+    assert wide[0].data_ptr() % 16 and wide.stride(1) % 4
+    step = lambda k, v: A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache, k,
+                                            bk, v, bv, m.private_block_tables, m.seq_lens_tensor, m.cache_type, w.scale)
+    want, got = step(wk, wv), step(wide[0], wide[1])
+    A.raise_on_device_status()
+    u = {F: 2.0 ** -10, B: 2.0 ** -7, torch.float32: 1e-5}[dtype]   # both roundings of the output
+    assert torch.allclose(got.float(), want.float(), rtol=u, atol=u * float(want.float().pow(2).mean().sqrt()))
+
+
 def attention64(w, r):
     """Hidden-cached request r (its new row written) in 64 bits."""
     m, s, h, d, bs = w.meta, w.seq_lens[r], w.heads, w.shape.head_dim, w.shape.block_size
