@@ -82,7 +82,8 @@ class QKVParallelLinear(torch.nn.Module):
 class RowParallelLinear(torch.nn.Module):
     """o_proj: this rank's columns of W_o; partial GEMM, all-reduce, then the bias
     once (aptserve_linear.py:815-839).  Without a reduction between them the bias is added by the GEMM
-    (in fp32, before the one rounding; as a pass of its own it took 36 us of a 3300-token OPT-13B prompt batch)."""
+    (in fp32, before the one rounding; as a pass of its own it took 36 us of a 3300-token OPT-13B prompt batch),
+    if it is one the GEMM takes: a value per output, of the weight's type."""
 
     def __init__(self, weight_shard: torch.Tensor, bias: Optional[torch.Tensor], group=None):
         super().__init__()
@@ -91,8 +92,9 @@ class RowParallelLinear(torch.nn.Module):
         self.group = group
 
     def forward(self, input_: torch.Tensor):
-        if not _reduces(self.group):
-            return F.linear(input_, self.weight, self.bias), None
+        b = self.bias
+        if (b is None or (b.dtype == self.weight.dtype and b.shape == self.weight.shape[:1])) and not _reduces(self.group):
+            return F.linear(input_, self.weight, b), None
         out = tensor_model_parallel_all_reduce(F.linear(input_, self.weight), self.group)
         if self.bias is not None:
             out = out + self.bias
