@@ -8,12 +8,14 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
+import sysconfig
 from pathlib import Path
 
 import torch
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libaptserve_b200.so"
-HOST_LIB_PATH = LIB_PATH.with_name("libaptserve_b200_host.so")
+# reads Python objects with the layout of the interpreter it was compiled for, whose tag it carries in its name
+HOST_LIB_PATH = LIB_PATH.with_name("libaptserve_b200_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 APS_OK = 0
 APS_ERR_NULL_POINTER = 1

@@ -1,7 +1,7 @@
 """Build the sm_100a shared library in-tree: ``python -m apt_serve_b200.build``.
 
 One ``nvcc`` invocation over ``csrc/*.cu`` producing ``lib/libaptserve_b200.so``.
-(Beside it ``lib/libaptserve_b200_host.so`` from ``csrc/host_tables.cpp``, by the host compiler.)
+(Beside it ``lib/libaptserve_b200_host.<interpreter's tag>.so`` from ``csrc/host_tables.cpp``, by the host compiler.)
 The library exports the C ABI declared in ``include/aptserve_b200.h`` and links
 the CUDA runtime dynamically, so that it shares the runtime PyTorch has loaded.
 """
@@ -18,7 +18,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libaptserve_b200.so"
-HOST_LIB_PATH = LIB_DIR / "libaptserve_b200_host.so"   # reads Python objects: not part of the C-ABI library
+# reads Python objects: not part of the C-ABI library, and one per interpreter (as in _native.py)
+HOST_LIB_PATH = LIB_DIR / ("libaptserve_b200_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 SOURCES = ["c_api.cu", "cache_ops.cu", "paged_attention.cu", "hybrid_attention.cu", "hidden_simt.cu", "metadata_ops.cu",
            "tp_comm.cu", "absorbed_attention.cu", "hidden_attention.cu", "hidden_fp32.cu", "decode_step.cu", "tensor_maps.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -37,7 +38,7 @@ def build_host(force: bool = False) -> Path:
     if not force and HOST_LIB_PATH.exists() and HOST_LIB_PATH.stat().st_mtime >= src.stat().st_mtime:
         return HOST_LIB_PATH
     LIB_DIR.mkdir(exist_ok=True)
-    tmp = HOST_LIB_PATH.with_suffix(".so.tmp")
+    tmp = HOST_LIB_PATH.with_name(HOST_LIB_PATH.name + ".tmp")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"],
            str(src), "-o", str(tmp)]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
