@@ -2,7 +2,8 @@
 ``include/aptserve_b200.h``).
 
 There is no fallback: if the library is missing, every operator of this package
-raises.  Build it with ``python -m apt_serve_b200.build``.
+raises.  Build it with ``python -m apt_serve_b200.build``.  (The small host library beside it only
+packs lists faster than numpy does and may be missing.)
 """
 from __future__ import annotations
 
@@ -101,12 +102,10 @@ def lib() -> ctypes.CDLL:
 _host_lib = None
 
 
-def host_lib() -> ctypes.PyDLL:
-    """The library that reads Python lists (called with the interpreter lock held); raises if it has not been built."""
+def host_lib():
+    """The library that reads Python lists (called with the interpreter lock held), or None where it has not been built."""
     global _host_lib
-    if _host_lib is None:
-        if not HOST_LIB_PATH.exists():
-            raise RuntimeError(f"{HOST_LIB_PATH} is missing (run `python -m apt_serve_b200.build`)")
+    if _host_lib is None and HOST_LIB_PATH.exists():
         handle = ctypes.PyDLL(str(HOST_LIB_PATH))
         handle.aps_pack_block_tables.restype = c_int
         handle.aps_pack_block_tables.argtypes = [ctypes.py_object, ctypes.py_object, c_void_p, c_int64, c_int64,

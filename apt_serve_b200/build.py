@@ -33,7 +33,9 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
 
 
-def build_host(force: bool = False) -> Path:
+def build_host(force: bool = False):
+    """Compiles the host library; None, with a word on stderr, where there is no host compiler or no ``Python.h`` (numpy then
+    packs the block tables)."""
     src = CSRC / "host_tables.cpp"
     if not force and HOST_LIB_PATH.exists() and HOST_LIB_PATH.stat().st_mtime >= src.stat().st_mtime:
         return HOST_LIB_PATH
@@ -41,9 +43,15 @@ def build_host(force: bool = False) -> Path:
     tmp = HOST_LIB_PATH.with_name(HOST_LIB_PATH.name + ".tmp")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"],
            str(src), "-o", str(tmp)]
-    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"{cmd[0]} failed on {src.name}:\n{r.stdout}")
+    try:
+        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        failure = None if r.returncode == 0 else r.stdout
+    except OSError as exc:
+        failure = str(exc)
+    if failure is not None:
+        print(f"host library not built, {cmd[0]} failed on {src.name}:\n{failure}", file=sys.stderr)
+        HOST_LIB_PATH.unlink(missing_ok=True)   # an older one may not fit its callers any more
+        return None
     os.replace(tmp, HOST_LIB_PATH)
     return HOST_LIB_PATH
 
@@ -58,7 +66,12 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
+    path = build_cuda(force, verbose)
     build_host(force)
+    return path
+
+
+def build_cuda(force: bool = False, verbose: bool = False) -> Path:
     if not force and not needs_build():
         return LIB_PATH
     LIB_DIR.mkdir(exist_ok=True)

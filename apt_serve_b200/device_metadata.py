@@ -56,10 +56,8 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         words += (n + 31) // 32 * 32
     host = torch.empty(words, dtype=torch.int32, pin_memory=dev.type == "cuda")
     rows, priv, shared, ref, h_lens, h_type = (host.numpy()[i:j] for i, j in at)
-    if N.host_lib().aps_pack_block_tables(block_tables, block_tables_4_shared, hid.ctypes.data, b, width, priv.ctypes.data,
-                                          shared.ctypes.data, ref.ctypes.data) != 0:
-        _pack_tables(block_tables, block_tables_4_shared, hid, priv.reshape(b, width), shared.reshape(b, width),
-                     ref.reshape(b, width))
+    pack_tables(block_tables, block_tables_4_shared, hid, priv.reshape(b, width), shared.reshape(b, width),
+                ref.reshape(b, width))
     rows.view(np.int64)[:] = np.flatnonzero(~hid)
     h_lens[:] = lens_np
     h_type[:] = hid
@@ -84,6 +82,16 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         num_hidden_cache_tokens=n_h, num_tot_tokens=n_tot, num_decode_tokens=b,
         max_decode_seq_len=max(lens, default=0), private_block_tables=priv,
         cache_type=d_type, kv_request_rows=rows.view(torch.int64), **dict(zip(names, parts)))
+
+
+def pack_tables(tables, shared_tables, hid, priv, shared, ref):
+    """Pads the tables into three contiguous int32 arrays ``[sequences, width]``: private, shared (zero for K/V-cached requests)
+    and the reference's (the one that the request's type selects).  Natively for lists of lists or tuples of plain
+    integers where the host library has been built, by numpy otherwise."""
+    lib = N.host_lib()
+    if lib is None or lib.aps_pack_block_tables(tables, shared_tables, hid.ctypes.data, len(hid), priv.shape[1],
+                                                priv.ctypes.data, shared.ctypes.data, ref.ctypes.data) != 0:
+        _pack_tables(tables, shared_tables, hid, priv, shared, ref)
 
 
 def _pack_tables(tables, shared_tables, hid, priv, shared, ref):
