@@ -32,28 +32,30 @@ from .metadata import derive_private_block_tables
 _workspaces: Dict[torch.device, torch.Tensor] = {}
 
 
-def attention_workspace(device: torch.device, batch: int, max_blocks: int, block_size: int,
-                        heads: int, head_size: int) -> torch.Tensor:
-    """A per-device scratch tensor large enough for the given batch (grown on
-    demand, reused by later calls on the same stream)."""
-    need = N.lib().aps_attention_workspace_bytes(batch, max_blocks, block_size, heads, head_size)
+def _workspace(device: torch.device, need: int) -> torch.Tensor:
+    """The first bytes of the per-device scratch tensor (grown on demand, reused by later calls on the same stream): as
+    many as asked for and not all there are, because a layer-step chooses its path by the size of its scratch and must
+    not depend on what other calls have asked for before."""
+    need = max(need, 1 << 20)
     ws = _workspaces.get(device)
     if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
+        ws = torch.empty(need, dtype=torch.uint8, device=device)
         _workspaces[device] = ws
-    return ws
+    return ws[:need]
+
+
+def attention_workspace(device: torch.device, batch: int, max_blocks: int, block_size: int,
+                        heads: int, head_size: int) -> torch.Tensor:
+    """Scratch large enough for the attention calls on the given batch.  A layer-step that is given it re-projects the
+    cached hidden rows, at many times the cost for a large batch (see ``layer_step_workspace``)."""
+    return _workspace(device, N.lib().aps_attention_workspace_bytes(batch, max_blocks, block_size, heads, head_size))
 
 
 def layer_step_workspace(device: torch.device, batch: int, max_blocks: int, block_size: int,
                          heads: int, head_size: int, hidden: int, dtype: torch.dtype) -> torch.Tensor:
-    """The same per-device scratch tensor, large enough for ``decode_layer_step``."""
-    need = N.lib().aps_decode_layer_step_workspace_bytes(batch, max_blocks, block_size, heads, head_size,
-                                                         hidden, N.DTYPE_ENUM[dtype])
-    ws = _workspaces.get(device)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[device] = ws
-    return ws
+    """Scratch with which ``decode_layer_step`` can attend the cached hidden rows directly."""
+    return _workspace(device, N.lib().aps_decode_layer_step_workspace_bytes(batch, max_blocks, block_size, heads, head_size,
+                                                                            hidden, N.DTYPE_ENUM[dtype]))
 
 
 def attention_status(workspace: torch.Tensor) -> int:
