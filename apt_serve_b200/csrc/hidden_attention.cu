@@ -1202,7 +1202,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 int terms_of(int dtype) { return dtype == APS_BF16 ? 3 : 2; }
 
 struct Layout {
-  int np, n_cap, n_groups, splits, max_slice;
+  int np, n_cap, n_groups, n_hidden_cap, splits, max_slice;
   uint32_t unfold_ring;
   size_t off_groups, off_slot, off_list, off_qscale, off_inv, off_scores, off_probs, off_qz, off_part, total;
 };
@@ -1213,6 +1213,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.np = (heads + 15) / 16 * 16;
   l.n_cap = ((batch < kGroup ? batch : kGroup) + 15) / 16 * 16;
   l.n_groups = (batch + kGroup - 1) / kGroup;
+  l.n_hidden_cap = l.n_groups == 1 ? l.n_cap : l.n_groups * kGroup;
   // One wave of unfold CTAs; at least four slabs each.  A CTA spends 0.4 us on a slab whatever its requests, so few
   // requests take two CTAs per SM (half the ring each, three stages at least) and ranges half as long: one OPT-13B
   // request 14.2 -> 11.4 us, 24 requests 15.6 -> 12.3, 64 requests 20.8 -> 17.1.
@@ -1220,7 +1221,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   const int z_boxes = nt * ht * (((batch < head_size ? batch : head_size) + 15) / 16);   // 128 / ht requests per CTA
   const bool two = 3 * unfold_stage_bytes(z_boxes) <= kRingBytes / 2;
   l.unfold_ring = (uint32_t)(two ? kRingBytes / 2 : kRingBytes);
-  int splits = (two ? 2 : 1) * 148 / w_tiles;
+  int splits = (two ? 2 : 1) * sm_count() / w_tiles;
   if (splits > slabs / 4) splits = slabs / 4;
   l.splits = splits < 1 ? 1 : splits;
   int ms = 256 / l.np;
@@ -1229,8 +1230,10 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   while (ms > 1 && 3 * sum_stage_bytes(nt, l.np, ms) > kRingBytes) --ms;   // at least three stages
   l.max_slice = ms;
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
-  const int64_t tiles = (int64_t)l.n_cap * ((max_tokens + kTile - 1) / kTile) + kMaxPieces;
-  const int64_t blks = (int64_t)l.n_cap * ((max_tokens + 15) / 16);
+  const int64_t reqs = batch < kGroup ? batch : kGroup, blks = reqs * ((max_tokens + 15) / 16);
+  int64_t tiles = reqs * ((max_tokens + kTile - 1) / kTile);
+  const int64_t pieces = (blks + tiles * kTileCost) * (hidden / 128) / kMinPiece;   // none is smaller than kMinPiece
+  tiles += pieces < 1 ? 1 : pieces < kMaxPieces ? pieces : kMaxPieces;
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o = align_up(o + bytes, 256); return at; };
   l.off_groups = take((size_t)l.n_groups * sizeof(GroupPlan));
@@ -1242,7 +1245,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.off_probs = take((size_t)blks * probs_block_bytes(nt, l.np));
   // qt is dead once the scores are there, z is written after them: one buffer
   l.off_qz = take((size_t)l.n_cap * nt * heads * hidden * 2);
-  l.off_part = take((size_t)l.splits * l.n_groups * kGroup * heads * head_size * sizeof(float));
+  l.off_part = take((size_t)l.splits * l.n_hidden_cap * heads * head_size * sizeof(float));
   l.total = o;
   return l;
 }
@@ -1390,7 +1393,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_groups * kGroup; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.grid_scores = pa.grid_scores;
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);

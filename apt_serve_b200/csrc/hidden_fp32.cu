@@ -278,7 +278,7 @@ unfold32_kernel(const Params p) {
 }
 
 struct Layout {
-  int n_groups, count, chunk, chunks, splits;
+  int n_groups, n_hidden_cap, count, chunk, chunks, splits;
   size_t off_groups, off_slot, off_list, off_qt, off_ml, off_z, off_part, total;
 };
 
@@ -289,13 +289,14 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
   const size_t row = (size_t)heads * hidden * sizeof(float);
   l.n_groups = (batch + kGroup - 1) / kGroup;
+  l.n_hidden_cap = l.n_groups == 1 ? batch : l.n_groups * kGroup;
   l.count = batch < kGroup ? batch : kGroup;
   l.chunk = kMinChunk;
   auto per_request = [&] { return (size_t)((max_tokens + l.chunk - 1) / l.chunk) * row; };
   while (l.chunk < kMaxChunk && (size_t)l.count * per_request() > kScratch) l.chunk *= 2;
   l.chunks = (int)((max_tokens + l.chunk - 1) / l.chunk);
   while (l.count > 1 && (size_t)l.count * per_request() > kScratch) l.count = (l.count + 1) / 2;
-  l.splits = 148 / heads;   // one wave of unfold CTAs for one group of R requests
+  l.splits = sm_count() / heads;   // one wave of unfold CTAs for one group of R requests
   const int steps = (hidden + 255) / 256;
   l.splits = l.splits < 1 ? 1 : l.splits > steps ? steps : l.splits;
   size_t o = 0;
@@ -306,7 +307,7 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.off_qt = take((size_t)l.count * row);
   l.off_ml = take((size_t)l.count * l.chunks * heads * 2 * sizeof(float));
   l.off_z = take((size_t)l.count * l.chunks * row);
-  l.off_part = take((size_t)l.splits * l.n_groups * kGroup * heads * head_size * sizeof(float));
+  l.off_part = take((size_t)l.splits * l.n_hidden_cap * heads * head_size * sizeof(float));
   l.total = o;
   return l;
 }
@@ -370,7 +371,7 @@ int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStrea
   p.qt = reinterpret_cast<float*>(b + l.off_qt); p.ml = reinterpret_cast<float*>(b + l.off_ml);
   p.z = reinterpret_cast<float*>(b + l.off_z); p.out_part = reinterpret_cast<float*>(b + l.off_part);
   p.heads = s.heads; p.hidden = c.hidden_size; p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq;
-  p.chunk = l.chunk; p.chunks = l.chunks; p.n_hidden_cap = l.n_groups * kGroup;
+  p.chunk = l.chunk; p.chunks = l.chunks; p.n_hidden_cap = l.n_hidden_cap;
   p.query_stride = s.query_stride; p.x_stride = c.hidden_row_stride; p.w_stride = c.w_stride;
   p.scale_log2 = s.scale * 1.4426950408889634f;
   ScopedProfile prof(1, cs);
