@@ -5,10 +5,11 @@
 // with additional_designs/attention/backends/aptserve_flash_attn.py:331-387, 449-475):
 // write the new token's layer-input row for hidden-cached requests (hidden_to_cache), write
 // the new token's K/V rows for K/V-cached requests (mixed_kv_to_cache / reshape_and_cache_flash),
-// then attend.  Here that is one host call that enqueues three launches on the caller's
+// then attend.  Here that is one host call that enqueues its launches on the caller's
 // stream: a bulk-copy launch for all new-token rows, addressed straight from the private
 // block tables, the sequence lengths and the cache-type mask (no int64 index tensors), and
-// the hybrid decode attention (plan, K/V streaming, re-projection, combine).
+// the hybrid decode attention: plan, K/V streaming, the hidden path (five launches per 256 requests when the
+// cached rows are attended directly, three in fp32, one when they are re-projected), combine.
 
 #include "attention_common.cuh"
 

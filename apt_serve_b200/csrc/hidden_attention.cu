@@ -11,7 +11,8 @@
 //     sum_t p_t (W_v,h x_t + b_v) = W_v,h (sum_t p_t x_t) + b_v
 // so the rows are attended as they are, with K = V = X and a head dimension of E.  Re-projecting T
 // rows costs 4 T E H D operations; this form costs 4 E H (D + T): D times less for long contexts.
-// What is left is bound by memory: the rows are read twice (scores, weighted sums) and W_k, W_v once.
+// What is left is bound by memory: the rows are read twice (scores, weighted sums), W_k once per 128 requests and W_v once
+// per D requests (128, 64 or 32) of a group.
 // Measured on one B200: a step of 256 requests of an OPT-13B layer, half of them hidden-cached (94.7k rows),
 // 0.86 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
 // requests, 0.47 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.20 ms against 2.5.
@@ -36,8 +37,10 @@
 //     sums then had an absolute error of 2^-26, 3.6 units of the output's last place for cached rows of N(0, 0.01) and
 //     W_v of N(0, 1).  Now the value's error is 2^-23 of it or 2^-36, whichever is more.
 //
-// Requests are taken in groups of at most kGroup, so that the scratch (qt, z: kGroup x H x E terms)
-// does not grow with the batch; inside a group they are sorted by length, longest first.
+// Requests are taken in groups of at most kGroup, so that most of the scratch (qt and z: kGroup x H x E terms, scores and
+// weights) does not grow with the batch beyond one group (the projected outputs, splits x H x D per request, do); inside a
+// group they are sorted by length, longest first.  The host does not know how many requests are hidden-cached and
+// enqueues the five kernels for every group there could be; one that finds nothing to do takes 1 us.
 //
 // Every mbarrier wait is bounded by a clock budget; a wait that runs out records a code in the plan's
 // status word, tells the other warps through shared memory, and the CTA drains and returns.

@@ -18,9 +18,10 @@ struct TensorMapSpec {
   uint32_t box[3];
 };
 
-// A tensor map is a pure function of its spec: the encoded maps are kept in a small per-thread
-// table (the library has one calling thread), so a layer that is called every step with the
-// same caches and weights encodes each of its maps once.
+// A tensor map is a pure function of its spec: the last encoded maps are kept in a small per-thread table (the library
+// has one calling thread).  A layer called again and again finds its up to eight maps there; the layers of a model
+// called in turn have more than the table holds and encode theirs every time, beside the GPU's work: 40 OPT-13B
+// layers of one request each in turn 57 us a layer, one layer 58; 24 OPT-1.3B layers of eight requests 43 and 43.
 int cached_tensor_map(CUtensorMap* out, const TensorMapSpec& spec, const char* what);
 
 }  // namespace aps

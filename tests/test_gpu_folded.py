@@ -1,7 +1,7 @@
 """The layer-step's hidden path with the projections moved to the query and the output
 (csrc/hidden_attention.cu) at the sizes where its tiles, stages, groups and splits end.
 
-Tolerance of the hidden-cached requests' rows: the intermediates carry at least 22 bits, so what is left
+Tolerance of the hidden-cached requests' rows: the intermediates carry at least 22 bits (fp16: down to 2^-36), so what is left
 is the rounding of the output, half a unit of its last place (u = 2^-11 of the value in fp16, 2^-8 in bf16),
 and an eighth of that, relative to the rows' root mean square, for the sums and the oracle's own fp32.
 K/V-cached requests: the 2e-2 of the other attention tests (their weights are rounded to the cache type)."""
@@ -100,7 +100,7 @@ def test_larger_cache_blocks_and_garbage_behind_the_sequences():
 
 
 def test_small_and_large_queries_keep_their_bits():
-    """The folded query is normalised per request and head: queries and hidden rows of very different sizes."""
+    """The folded query is normalised per request and head: queries of very different sizes.  (Rows and weights: below.)"""
     w = make_decode_workload(LayerShape("t", 8, 128, 1024, F), [300] * 12, [True] * 12, seed=8, device="cpu")
     for r, s in enumerate((1e-6, 1e-4, 1e-2, 1.0, 8.0, 30.0, 1e-6, 1e-4, 1e-2, 1.0, 8.0, 0.0)):
         w.query[r] *= s
