@@ -15,7 +15,8 @@ context lengths, half of them hidden-cached).  Prints ONE JSON line on rank 0.  
 timed region the default run adds, each with its own clock sample:
 
   roofline_kv_path_pure / roofline_reprojection_pure   the K/V-only and the hidden-only
-        sub-batch of configuration 2, each kernel running alone;
+        sub-batch of configuration 2 through ``attention.hybrid_decode_attention``, which re-projects
+        the cached hidden rows on the tensor cores, each kernel running alone;
   roofline_cache_writes   configuration 3's prefill cache writes + block copies, alone and
         inside the loaded step;
   config5_sweep           configuration 5 at 0 / 25 / 50 / 75 / 100 % hidden-cached;
@@ -264,8 +265,10 @@ class LayerStep:
         self.wk, self.bk, self.wv, self.bv = w.kv_weights()
         self.out = torch.empty_like(w.query)
         self.prefill_events = None   # (start, stop) recorded around prefill_writes when set
-        self.workspace = A.attention_workspace(w.query.device, w.query.shape[0],
-                                               m.private_block_tables.shape[1], w.shape.block_size, h, d)
+        # the scratch decode_layer_step takes by itself; `direct`: it lets the step attend the hidden rows as they are
+        sizes = (w.query.shape[0], m.private_block_tables.shape[1], w.shape.block_size, h, d)
+        self.workspace = A.layer_step_workspace(w.query.device, *sizes, w.shape.hidden, w.shape.dtype)
+        self.direct = self.workspace.numel() > max(1 << 20, A.N.lib().aps_attention_workspace_bytes(*sizes))
 
     def layer_step(self, query, hidden_states, new_key, new_value, tables, seq_lens, cache_type, out=None):
         """New-token cache writes + hybrid decode attention: one native call."""
@@ -421,8 +424,9 @@ class Timer:
         return res
 
 
-def kernel_rooflines(work, res, peaks):
-    """The two attention kernels' roofline blocks from per-kernel event times."""
+def kernel_rooflines(work, res, peaks, direct=False):
+    """The two attention paths' roofline blocks from event times around their kernels.  direct: the cached hidden rows
+    are attended as they are (bound by reading them and W once), not re-projected (bound by the tensor cores)."""
     hid_ms, kv_ms = res["hid_ms"], res["kv_ms"]
     tflops = work["reprojection_flops"] / (hid_ms * 1e-3) / 1e12 if hid_ms > 0 and work["t_hidden"] else 0.0
     kv_gbs = work["kv_attention_bytes"] / (kv_ms * 1e-3) / 1e9 if kv_ms > 0 and work["t_kv"] else 0.0
@@ -432,6 +436,13 @@ def kernel_rooflines(work, res, peaks):
               "frac_of_burst_peak": round(tflops / peaks["tflops_burst"], 4),
               "peak_source": peaks["source"] + " (sustained bf16 figure: the kernel runs inside a long step)",
               "ms_per_launch": round(hid_ms, 4), "flops_per_launch": work["reprojection_flops"]}
+    if direct:
+        gbs = work["hidden_bytes"] / (hid_ms * 1e-3) / 1e9 if hid_ms > 0 and work["t_hidden"] else 0.0
+        hidden = {"kernel": "fold, scores, softmax, sum, unfold and combine kernels (cached hidden rows attended directly)",
+                  "bound": "hbm", "achieved": round(gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                  "frac": round(gbs / peaks["hbm_gbs"], 4), "peak_source": peaks["source"],
+                  "ms_per_launch": round(hid_ms, 4), "bytes_per_launch": work["hidden_bytes"],
+                  "note": "bytes: hidden rows, W_k and W_v once; the kernels read the rows twice (scores, weighted sums)"}
     kv = {"kernel": "kv_attention_tma_kernel (K/V streaming)", "bound": "hbm",
           "achieved": round(kv_gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
           "frac": round(kv_gbs / peaks["hbm_gbs"], 4), "peak_source": peaks["source"],
@@ -595,14 +606,17 @@ def run_ours(args):
     res = timer.run(st.step, K, W, preload_s=0.5, step_obj=st)
     ms_per_step = res["ms_per_step"]
     status = st.A.attention_status(st.workspace)
-    roof_hidden, roof_kv = kernel_rooflines(work, res, peaks)
-    if work["t_hidden"] > 0 and shape.dtype != torch.float32:
+    roof_hidden, roof_kv = kernel_rooflines(work, res, peaks, st.direct)
+    if work["t_hidden"] > 0 and shape.dtype != torch.float32 and not st.direct:
         roof_hidden.update(tensor_cycle_block(st, shape, lens, hid, tp))
-    if shape.dtype == torch.float32:
+    if shape.dtype == torch.float32 and st.direct:
+        roof_hidden["kernel"] = "fold32, attend32, unfold32 and combine kernels (cached hidden rows attended directly, fp32)"
+    elif shape.dtype == torch.float32:
         # fp32 runs the CUDA-core re-projection (tcgen05 has no fp32 MMA): the tensor peak is not its bound
         roof_hidden.update({"kernel": "hidden_simt_kernel (fp32 CUDA-core re-projection + softmax partials)",
                             "bound": "fp32 CUDA cores (no measured peak on file)", "peak": None, "frac": None,
                             "frac_of_burst_peak": None, "peak_source": None})
+    if shape.dtype == torch.float32:
         roof_kv["kernel"] = "kv_attention_kernel (K/V streaming, CUDA-core arithmetic: fp32)"
 
     per_rank = per_rank_block(st, res, tp, dev, B, shape) if tp > 1 else None
@@ -616,8 +630,8 @@ def run_ours(args):
     status |= st.A.attention_status(st.workspace)
 
     line_extra = {}
-    # ---- for information: the same step with absorbed projections (not the path the metric
-    # is quoted on: the headline step re-projects on the tensor cores) ----
+    # ---- for information: the opt-in variant with absorbed projections (not the path the metric
+    # is quoted on) ----
     if (extras and tp == 1 and work["t_hidden"] > 0 and st.A.absorbed_supported(w.heads, shape.hidden, shape.dtype)
             and shape.head_dim == 128 and w.prefill is None):
         ref_out = st.step().float().clone()
@@ -649,6 +663,7 @@ def run_ours(args):
             blk = rk if name == "roofline_kv_path_pure" else rh
             if name == "roofline_reprojection_pure":
                 blk["traffic"] = None
+                blk.update(tensor_cycle_block(st, shape, lens, hid, tp))
             blk.update({"requests": int(rows.numel()), "call_ms": round(r["ms_per_step"], 4),
                         "clocks": r.get("clocks"), "kernel_ms_x_sm_mhz":
                             round(blk["ms_per_launch"] * r["clocks"]["sm_mhz"], 1)
@@ -661,7 +676,7 @@ def run_ours(args):
     # tensor peak was measured with, on THIS box in THIS run ----
     if extras and cfg == 2 and tp == 1:
         line_extra["hbm_copy_yardstick"] = copy_yardstick(st, peaks, max(5, K // 2))
-        line_extra["gemm_yardstick"] = gemm_yardstick(timer, peaks, roof_hidden)
+        line_extra["gemm_yardstick"] = gemm_yardstick(timer, peaks, line_extra.get("roofline_reprojection_pure", {}))
 
     # ---- host-core baseline on a bounded sample (rank 0, N = 1 only) ----
     cpu_baseline = None
@@ -671,6 +686,7 @@ def run_ours(args):
     pf_block = None
     if w.prefill is not None and res["pf_ms"]:
         pf_block = cache_write_block(st, res["pf_ms"], peaks, "inside the loaded step")
+    direct = st.direct
     del e2e, st, w
     torch.cuda.empty_cache()
 
@@ -703,11 +719,11 @@ def run_ours(args):
             st5 = LayerStep(w5)
             r = timer.run(st5.step, max(5, K // 2), 3, preload_s=0.3)
             wk5 = algorithmic_work(CONFIG_SHAPES[5], l5, h5, tp)
-            rh, rk = kernel_rooflines(wk5, r, peaks)
+            rh, rk = kernel_rooflines(wk5, r, peaks, st5.direct)
             sweep.append({"hidden_fraction": frac, "ms_per_step": round(r["ms_per_step"], 4),
                           "tokens_per_s": round(len(l5) / (r["ms_per_step"] * 1e-3), 1),
-                          "reprojection_tflops": rh["achieved"] if wk5["t_hidden"] else None,
-                          "reprojection_frac": rh["frac"] if wk5["t_hidden"] else None,
+                          "hidden_path_gbs": rh["achieved"] if wk5["t_hidden"] else None,
+                          "hidden_path_frac": rh["frac"] if wk5["t_hidden"] else None,
                           "kv_path_gbs": rk["achieved"] if wk5["t_kv"] else None,
                           "kv_path_frac": rk["frac"] if wk5["t_kv"] else None,
                           "clocks": r.get("clocks"), "ms_x_sm_mhz": r.get("ms_x_sm_mhz")})
@@ -724,7 +740,7 @@ def run_ours(args):
         k4 = max(3, K // 4) if tp == 1 else K
         r = timer.run(st4.step, k4, 3, preload_s=0.4)
         wk4 = algorithmic_work(CONFIG_SHAPES[4], l4, h4, tp)
-        rh, rk = kernel_rooflines(wk4, r, peaks)
+        rh, rk = kernel_rooflines(wk4, r, peaks, st4.direct)
         e4 = EndToEnd(st4, dev, tp, (len(l4), CONFIG_SHAPES[4].hidden) if tp > 1 else tuple(w4.query.shape),
                       CONFIG_SHAPES[4].dtype)
         e4_s = e4.run(k4, timer.barrier)
@@ -735,7 +751,7 @@ def run_ours(args):
             "steps": k4, "ms_per_step": round(r["ms_per_step"], 4),
             "tokens_per_s": round(len(l4) / (r["ms_per_step"] * 1e-3), 1),
             "e2e_ms_per_step": round(e4_s * 1e3, 4), "e2e_tokens_per_s": round(len(l4) / e4_s, 1),
-            "reprojection_ms": round(r["hid_ms"], 4), "reprojection_tflops_per_gpu": rh["achieved"],
+            "hidden_path_ms": round(r["hid_ms"], 4), "hidden_path_gbs_per_gpu": rh["achieved"],
             "kv_path_ms": round(r["kv_ms"], 4), "kv_path_gbs_per_gpu": rk["achieved"],
             "clocks": r.get("clocks"), "ms_x_sm_mhz": r.get("ms_x_sm_mhz")}
         del e4, st4, w4
@@ -757,35 +773,33 @@ def run_ours(args):
     capture = ("`ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:%s -s 3 -c 2 "
                "python bench.py --steps 2 --warmup 3 --no-cpu-baseline --no-extras` (1 pass per launch), two launches: ")
     if default_workload:
-        roofline["traffic"] = 9_650_000_000
-        roofline["traffic_source"] = (capture % "hidden_path" + "9.61 + 0.037 GB and 9.47 + 0.033 GB read + written, 8.9 x the "
-                                      "mandatory bytes (hidden rows and W once: 1.08 GB): W and the hidden rows are re-streamed "
-                                      "from HBM per round of work items, 1.2 TB/s = 18 % of the copy bandwidth; the figure moves "
-                                      "with the GPU (7.4 - 7.6 GB, 9.3 - 10.5 GB and 13.0 GB on others for the same binary and "
-                                      "inputs: the live set sits at the ~60 MB of L2 that serve data read from both dies), the "
-                                      "kernel's time x clock does not")
+        roofline["traffic"] = None
+        roofline["traffic_source"] = "not captured: the path is six launches per group of requests, and the figure is per launch"
         roof_kv["traffic"] = 2_040_000_000
         roof_kv["traffic_source"] = capture % "kv_attention_tma" + "2.02 + 0.02 GB, 1.02 x the algorithmic bytes"
     else:
         roofline["traffic"] = None
-        roofline["traffic_source"] = ("not captured for this workload (captured for the default one: configuration 2, one GPU); "
-                                      "the re-projection kernel's DRAM traffic depends on the work-order groups, not on the "
-                                      "cached tokens alone, so it is not scaled from another case")
+        roofline["traffic_source"] = "not captured for this workload"
         roof_kv["traffic"] = int(1.02 * work["kv_attention_bytes"]) if work["t_kv"] else None
         roof_kv["traffic_source"] = ("1.02 x the algorithmic bytes, the ratio ncu measured on configuration 2 and on the "
                                      "16-request all-K/V case, scaled by the cached tokens")
-    # the mixed step against its two lower bounds: every K/V byte at the measured copy bandwidth,
-    # every re-projection FLOP at the measured sustained tensor rate; the step cannot beat the
-    # larger of the two and would equal their sum if the two paths did not overlap at all
+    # the mixed step against its lower bounds: every K/V byte, and every hidden row and weight once, at the measured copy
+    # bandwidth (directly attended), or every re-projection FLOP at the measured sustained tensor rate.  Both paths read
+    # the same memory when attended directly: the sum is the bound then, the larger of the two otherwise
     t_kv = work["kv_attention_bytes"] / (peaks["hbm_gbs"] * 1e9) * 1e3 if work["t_kv"] else 0.0
-    t_tc = work["reprojection_flops"] / (peaks["tflops_sustained"] * 1e12) * 1e3 if work["t_hidden"] else 0.0
-    mixed = {"kv_bytes_at_copy_bandwidth_ms": round(t_kv, 4), "reprojection_flops_at_sustained_peak_ms": round(t_tc, 4),
+    if direct:
+        t_hid = work["hidden_bytes"] / (peaks["hbm_gbs"] * 1e9) * 1e3 if work["t_hidden"] else 0.0
+    else:
+        t_hid = work["reprojection_flops"] / (peaks["tflops_sustained"] * 1e12) * 1e3 if work["t_hidden"] else 0.0
+    mixed = {"kv_bytes_at_copy_bandwidth_ms": round(t_kv, 4),
+             ("hidden_bytes_at_copy_bandwidth_ms" if direct else "reprojection_flops_at_sustained_peak_ms"): round(t_hid, 4),
              "step_ms": round(ms_per_step, 4),
-             "frac_of_max_bound": round(max(t_kv, t_tc) / ms_per_step, 4),
-             "frac_of_sum_bound": round((t_kv + t_tc) / ms_per_step, 4),
+             "frac_of_max_bound": round(max(t_kv, t_hid) / ms_per_step, 4),
+             "frac_of_sum_bound": round((t_kv + t_hid) / ms_per_step, 4),
              "note": "lower bounds over the step's device time: max = the slower path alone, sum = both paths "
-                     "back to back (they run back to back here: one stream, the re-projection kernel fills the SMs)"}
-    launches = 5 + (2 if cfg == 3 else 0)
+                     "back to back (they run back to back here, on one stream)"}
+    per_group = 3 if shape.dtype == torch.float32 else 5
+    launches = (4 + per_group * -(-B // 256) if direct else 5) + (2 if cfg == 3 else 0)
     line = {
         "metric": METRIC, "value": round(B / (ms_per_step * 1e-3), 2), "unit": UNIT, "n_gpus": n_gpus,
         "steps": K, "warmup": W, "ms_per_step": round(ms_per_step, 4),
@@ -812,8 +826,12 @@ def run_ours(args):
                             "the host waits for step i - 1's result before it enqueues step i + 1"},
         "gpu_launches": launches * K,
         "gpu_launches_per_step": {"count": launches,
-                                  "kernels": "bulk_copy_kernel (new-token rows), plan_kernel, kv_attention_tma_kernel, "
-                                             "hidden_path_kernel, combine_kernel" +
+                                  "kernels": "bulk_copy_kernel (new-token rows), " +
+                                             ("step_plan_kernel, kv_attention_kernel, fold32_kernel, attend32_kernel, unfold32_kernel, "
+                                              if direct and shape.dtype == torch.float32 else
+                                              "step_plan_kernel, kv_attention_tma_kernel, fold_kernel, scores_kernel, softmax_kernel, "
+                                              "sum_kernel, unfold_kernel, " if direct else
+                                              "plan_kernel, kv_attention_tma_kernel, hidden_path_kernel, ") + "combine_kernel" +
                                              (" + 2 bulk_copy_kernel launches of the prefill part" if cfg == 3 else "")},
         "roofline": roofline, "roofline_kv_path": roof_kv, "roofline_mixed_step": mixed,
         "device_status": status,
@@ -831,8 +849,8 @@ def run_ours(args):
 
 
 def per_rank_block(st, res, tp, dev, batch, shape):
-    """What every rank measured for its own two attention kernels in the timed region, the
-    re-projection kernel's cycle count per rank, and the all-reduce of the step's [B, E] tensor
+    """What every rank measured for its own two attention paths in the timed region, the
+    re-projection kernel's cycle count per rank where it ran, and the all-reduce of the step's [B, E] tensor
     timed alone (20 back-to-back calls): the step is as long as its slowest rank plus the
     exchange, and the ranks' GPUs do not sit at the same clock under the power cap."""
     import torch.distributed as dist
@@ -854,9 +872,9 @@ def per_rank_block(st, res, tp, dev, batch, shape):
     torch.cuda.synchronize()
     t = torch.tensor([e0.elapsed_time(e1) / 20], device=dev, dtype=torch.float64)
     dist.all_reduce(t, op=dist.ReduceOp.MAX)
-    return {"reprojection_ms": [round(float(x[0]), 4) for x in allr],
+    return {"hidden_path_ms": [round(float(x[0]), 4) for x in allr],
             "kv_path_ms": [round(float(x[1]), 4) for x in allr],
-            "reprojection_sm_cycles_cta0": [int(x[2]) for x in allr],
+            **({} if st.direct else {"reprojection_sm_cycles_cta0": [int(x[2]) for x in allr]}),
             "all_reduce_alone_ms": round(float(t.item()), 4),
             "all_reduce_bytes": int(y.numel() * y.element_size())}
 
@@ -880,7 +898,7 @@ def tensor_cycle_block(st, shape, lens, hid, tp):
             "work_items_per_cta_pair": round(items / (sms // 2), 2)}
 
 
-def gemm_yardstick(timer, peaks, roof_hidden):
+def gemm_yardstick(timer, peaks, reprojection):
     """The measured tensor peak is `torch.matmul` on 8192^3 bf16 (cuBLAS) in a seconds-long loop
     on one B200 of the pool; the power cap makes that figure move with the box.  The same GEMM
     (fp16, like the step) run here as a loaded loop, so that the re-projection kernel's TFLOP/s
@@ -895,8 +913,8 @@ def gemm_yardstick(timer, peaks, roof_hidden):
     out = {"what": "torch.matmul 8192 x 8192 x 8192 fp16 (cuBLAS, yardstick only), 60 back-to-back calls after "
                    "half a second of the same", "tflops": round(tflops, 1), "ms_per_call": round(r["ms_per_step"], 4),
            "measured_sustained_peak": peaks["tflops_sustained"], "clocks": r.get("clocks")}
-    if roof_hidden.get("achieved"):
-        out["reprojection_kernel_over_this_gemm"] = round(roof_hidden["achieved"] / tflops, 4)
+    if reprojection.get("achieved"):
+        out["reprojection_kernel_over_this_gemm"] = round(reprojection["achieved"] / tflops, 4)
     return out
 
 
