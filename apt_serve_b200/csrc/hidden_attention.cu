@@ -473,12 +473,15 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
 // accumulators that share a qt step).  The work is a line of (tile, 128 columns of E) steps, cut into
 // contiguous pieces (see unit_of_piece): a tile that straddles a cut leaves one partial sum per piece (slot =
 // tile + piece), added by the softmax kernel, so that one long request uses the whole chip and a large
-// batch has no partly filled last wave.  94.7k rows of an OPT-13B layer (0.97 GB): 207 us; one equal piece per
+// batch has no partly filled last wave.  94.7k rows of an OPT-13B layer (0.97 GB): 190 us; one equal piece per
 // CTA took 26 us longer.
 // A box is (64 columns, 8 rows, 2): 256 contiguous bytes of a cached row, so that a DRAM page is left after
 // 256 bytes and not 128, and 8-row groups that lie 2 KB apart, as the K-major operand needs them.  X and qt
 // have a ring each: a unit of X is 128 tokens x 128 columns (32 KB), a unit of qt serves both halves of a
-// tile.  Warps: 0 qt boxes, 1 MMA issue, 2-5 epilogue, 6-7 boxes of X (eight lanes each).
+// tile.  L2: qt (105 MB for 128 OPT-13B requests) is read once per tile and was fetched from memory almost every time,
+// because the rows, which are read once by this kernel, pushed it out (1.25 GB of DRAM traffic for 0.97 GB of rows).  The
+// rows are the first to go (evict_first), qt stays (evict_last): 205 -> 190 us for 128 OPT-13B requests, 172 -> 155 for 52
+// OPT-66B tp 8 requests, 69 -> 63 for 24 of 1800 OPT-13B tokens, 313 -> 283 for 100 OPT-66B tp 2.  Warps: 0 qt boxes, 1 MMA issue, 2-5 epilogue, 6-7 boxes of X (eight lanes each).
 constexpr int kScoresThreads = 256;
 constexpr int kMaxStages = 12;
 constexpr int kMaxQUnits = 3;
@@ -563,6 +566,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   volatile int* abort_flag = &aux.abort_flag;
   const uint32_t full0 = smem_u32(&aux.full[0]), empty0 = smem_u32(&aux.empty[0]);
   const uint32_t q_full0 = smem_u32(&aux.q_full[0]), q_empty0 = smem_u32(&aux.q_empty[0]);
+  const uint64_t once = l2_policy_evict_first(), again = l2_policy_evict_last();
   bool ok = true;
   Ring xr, qr, ir;
   uint32_t n_local = 0;
@@ -631,7 +635,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
             __syncwarp();
             if (lane < 2 * NT)   // lane = (term, half of the columns); the terms of a half lie one behind the other
-              tma_load_2d_cta(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads);
+              tma_load_2d_hint(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads, again);
             __syncwarp();
             qr.step(nq);
           }
@@ -644,7 +648,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
               const uint32_t bar = full0 + xr.stage * 8;
               if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)boxes[m] * 2048);
               __syncwarp();
-              if (has[m]) tma_load_3d_cta(x_ring + xr.stage * kUnitBytes + g * 2048, &map_x, bar, 0, row[m], s * 2);
+              if (has[m]) tma_load_3d_hint(x_ring + xr.stage * kUnitBytes + g * 2048, &map_x, bar, 0, row[m], s * 2, once);
               __syncwarp();
               xr.step(nx);
             }
@@ -907,6 +911,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   uint32_t n_local = 0;
   Ring ir;
   int next = blockIdx.x;   // the first item needs no counter
+  const uint64_t once = l2_policy_evict_first();
   int ahead = 0;           // stages of the first item whose rows are requested before the wait
   bool waited = warp != 0;
   if (waited) chain_wait();
@@ -956,7 +961,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         __syncwarp();
         const int k = lane / n_col, col = lane - k * n_col;
         const int row = __shfl_sync(0xffffffffu, rows, ((b & 31) + k) & 31);
-        if (lane < nb * n_col) tma_load_3d_cta(dst + (k * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2);
+        if (lane < nb * n_col) tma_load_3d_hint(dst + (k * slice + col) * 4096, &map_x, bar, 0, row, (first + col) * 2, once);
       };
       if (!waited) {
         ahead = min(min(stages, 32 / (int)per_stage), (n_blk + (int)per_stage - 1) / (int)per_stage);   // `rows` holds 32 blocks
