@@ -19,7 +19,7 @@
 //
 //   fold_kernel      qt[r][h] = W_k,h^T q[r][h]                       tcgen05, M = 128 columns of E
 //   scores_kernel    s[t][h] = x_t . qt[r][h]                         tcgen05, M = 128 tokens
-//   softmax_kernel   p[t][h] = 2^(scale s - max)                      one warp per (request, head)
+//   softmax_kernel   p[t][h] = 2^(scale s - max)                      four warps per (request, two heads)
 //   sum_kernel       z[r][h] = sum_t p[t][h] x_t / sum_t p[t][h]      tcgen05, M = 128 columns of E
 //   unfold_kernel    y[r][h] = W_v,h z[r][h]                          tcgen05, M = 128 rows of W_v
 // and the combine kernel adds b_v.
@@ -73,19 +73,10 @@ template <typename T> constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::
 // idle for a fifth of the kernel (they do not get equal shares of the memory bandwidth).  In units of the
 // smallest size there are per_level << (levels - 1) of them; piece c starts at unit_of_piece(c), position
 // X * unit / units.
-__host__ __device__ inline int unit_of_piece(int c, int levels, int per_level) {
+__device__ inline int unit_of_piece(int c, int levels, int per_level) {
   const int l = c / per_level, k = c - l * per_level;
   const int size = l >= levels - 2 ? 1 : 1 << (levels - 2 - l);
   return l >= levels ? per_level << (levels - 1) : per_level * ((1 << (levels - 1)) - (1 << (levels - 1 - l))) + k * size;
-}
-// The last piece that starts at or before `unit`.
-__host__ __device__ inline int piece_of_unit(int unit, int levels, int per_level) {
-  int l = 0;
-  for (; l < levels - 1; ++l)
-    if (unit < per_level * ((1 << (levels - 1)) - (1 << (levels - 2 - l)))) break;
-  const int size = l >= levels - 2 ? 1 : 1 << (levels - 2 - l);
-  const int k = (unit - per_level * ((1 << (levels - 1)) - (1 << (levels - 1 - l)))) / size;
-  return l * per_level + (k < per_level ? k : per_level - 1);
 }
 
 struct Params {
@@ -94,6 +85,7 @@ struct Params {
   void* qt;              // [request][term][head][E]
   float* qscale;         // [request][head] scale * log2(e) / (power of two q was multiplied with)
   float* scores;         // [tile + piece][head][kTile] partial scores over a range of E
+  int2* tile_pieces;     // [tile] the first and the last piece with a part of it
   void* probs;           // [16-token block][term][K half][heads padded][8 tokens]
   float* inv_sum;        // [request][head]
   void* z;               // [term][head][request capacity][E]
@@ -692,6 +684,10 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
           if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
           tc_fence_after();
           float* dst = p.scores + (int64_t)(t + piece) * p.heads * kTile;
+          if (quarter == 0 && lane == 0) {
+            if (sa == 0) p.tile_pieces[t].x = piece;
+            if (sb == steps) p.tile_pieces[t].y = piece;
+          }
           for (int m = m0; m < m1; ++m)
             for (int h0 = 0; h0 < np; h0 += 16) {
               const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (buf * m_step + m - m0) * n_acc + h0;
@@ -721,100 +717,114 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
 }
 
 // ---- softmax ------------------------------------------------------------------------
-// One CTA per (request, head) at a time, one warp per tile.  A lane takes eight consecutive tokens of the
-// tile: it adds the tile's partial sums, and after the maximum is known writes the eight weights of each
-// term as one 16-byte piece of the sum kernel's B operand.  The scores of kHold tiles per warp stay in
-// registers (2048 tokens); those of longer requests are added up twice.
+// One CTA per (request, two heads) at a time, one warp per tile.  A lane takes eight consecutive tokens of the
+// tile for both heads: it adds the tile's partial sums, and after the maxima are known writes the eight weights of each
+// term and head as one 16-byte piece of the sum kernel's B operand, the two heads' pieces together as one 32-byte sector.
+// The scores of kHold tiles per warp stay in registers (2048 tokens); those of longer requests are added up twice.
+// What bounds it is the chain of round trips of a unit (plan, pieces, scores, two reductions): two heads share it
+// and the address arithmetic, and which pieces have a part of a tile is left there by the scores kernel (finding it from the
+// cut's formula took two 64-bit divisions per tile).  A batch of no more than two (request, head) per SM takes single
+// heads (one OPT-13B request 7.7 -> 6.1).  26.5 -> 17.3 us for 128 OPT-13B requests, 31.5 -> 22.5 in bf16, 14.0 -> 11.6 for 24 of 1800 tokens.
 constexpr int kSoftmaxWarps = 4;
 constexpr int kHold = 2;
 
-template <typename T>
-__global__ void __launch_bounds__(kSoftmaxWarps * 32)
-softmax_kernel(const Params p) {
+template <typename T, int PER>
+__device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kSoftmaxWarps], float (*s_sum)[kSoftmaxWarps]) {
   constexpr int NT = kTerms<T>;
-  __shared__ float s_max[kSoftmaxWarps], s_sum[kSoftmaxWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  chain_wait();
-  chain_next();
   const GroupPlan* gp = p.plan;
-  const int n_units = gp->n * p.heads, levels = gp->levels, per_level = gp->per_level, steps = p.hidden / 128;
-  const int64_t units = (int64_t)per_level << (levels - 1);
-  const int64_t work = (int64_t)gp->weight * steps;
-  // x / work by a reciprocal and one correction: a 64-bit division is a loop of a hundred instructions, and every warp
-  // has two per tile (softmax of 128 bf16 OPT-13B requests 33.2 -> 31.2 us, of one 7.0 -> 6.1).  Exact below 2^53.
-  const double inv_work = 1.0 / (double)work;
-  auto over_work = [&](int64_t x) {
-    const int64_t q = (int64_t)((double)x * inv_work), r = x - q * work;
-    return (int)(r < 0 ? q - 1 : r >= work ? q + 1 : q);
-  };
+  const int units_of = (p.heads + PER - 1) / PER, n_units = gp->n * units_of;
   T* probs = static_cast<T*>(p.probs);
   for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
-    const int slot = unit / p.heads, h = unit - slot * p.heads;
+    const int slot = unit / units_of, h = (unit - slot * units_of) * PER;
+    const bool two = PER == 2 && h + 1 < p.heads;
     const int len = gp->len[slot];
     const int tile0 = gp->tile_off[slot], n_tiles = gp->tile_off[slot + 1] - tile0;
-    const float scale = p.qscale[(int64_t)slot * p.heads + h];
-    const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot], w0 = gp->w_off[slot];
+    const float* scales = p.qscale + (int64_t)slot * p.heads + h;
+    const float scale[2] = {scales[0], two ? scales[1] : 0.f};
+    const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot];
     // scores of this lane's eight tokens of tile k
-    auto load = [&](int k, float (&s)[8]) {
-      // the pieces of the line of (tile, step) that touch this tile: c0 is the last that starts at or
-      // before its first step, c1 the last that starts at or before its last one
-      const int w = min(kSubs, n_blk - k * kSubs) + kTileCost;
-      const int64_t at = (int64_t)(w0 + k * (kSubs + kTileCost)) * steps;
-      const int c0 = piece_of_unit(over_work((at + w) * units - 1), levels, per_level);
-      const int c1 = piece_of_unit(over_work((at + (int64_t)w * steps) * units - 1), levels, per_level);
+    auto load = [&](int k, float (&s)[PER][8]) {
+      const int2 c = p.tile_pieces[tile0 + k];   // the first and the last piece with a part of the tile
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s[e] = 0.f;
-      const float4* src = reinterpret_cast<const float4*>(p.scores + ((int64_t)(tile0 + k + c0) * p.heads + h) * kTile + lane * 8);
-#pragma unroll 4
-      for (int c = c0; c <= c1; ++c) {
-        const float4 x = src[0], y = src[1];
+      for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[i][e] = 0.f;
+      const float4* src = reinterpret_cast<const float4*>(p.scores + ((int64_t)(tile0 + k + c.x) * p.heads + h) * kTile + lane * 8);
+#pragma unroll (4 / PER)
+      for (int j = c.x; j <= c.y; ++j) {
+        float4 x[PER], y[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const bool in = i == 0 || two;
+          x[i] = in ? src[i * (kTile / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+          y[i] = in ? src[i * (kTile / 4) + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         src += p.heads * (kTile / 4);
-        s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
-        s[4] += y.x; s[5] += y.y; s[6] += y.z; s[7] += y.w;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          s[i][0] += x[i].x; s[i][1] += x[i].y; s[i][2] += x[i].z; s[i][3] += x[i].w;
+          s[i][4] += y[i].x; s[i][5] += y[i].y; s[i][6] += y[i].z; s[i][7] += y[i].w;
+        }
       }
       const int tok = k * kTile + lane * 8;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s[e] = tok + e < len ? s[e] * scale : -INFINITY;
+      for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[i][e] = tok + e < len ? s[i][e] * scale[i] : -INFINITY;
     };
-    float held[kHold][8], mx = -INFINITY;
+    float held[kHold][PER][8], mx[2] = {-INFINITY, -INFINITY};
+    auto take_max = [&](const float (&s)[PER][8]) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mx[i] = fmaxf(mx[i], s[i][e]);
+    };
 #pragma unroll
     for (int j = 0; j < kHold; ++j) {
       const int k = warp + j * kSoftmaxWarps;
-      if (k < n_tiles) {
-        load(k, held[j]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) mx = fmaxf(mx, held[j][e]);
-      }
+      if (k < n_tiles) { load(k, held[j]); take_max(held[j]); }
     }
     for (int k = warp + kHold * kSoftmaxWarps; k < n_tiles; k += kSoftmaxWarps) {
-      float s[8];
+      float s[PER][8];
       load(k, s);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, s[e]);
+      take_max(s);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s_max[warp] = mx;
+    for (int o = 16; o > 0; o >>= 1) {
+      mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], o));
+      mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], o));
+    }
+    if (lane < 2) s_max[lane][warp] = lane == 0 ? mx[0] : mx[1];
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kSoftmaxWarps; ++w) mx = fmaxf(mx, s_max[w]);
-    float sum = 0.f;
-    auto store = [&](int k, const float (&s)[8]) {
-      T terms[8][NT];
+    for (int w = 0; w < kSoftmaxWarps; ++w) { mx[0] = fmaxf(mx[0], s_max[0][w]); mx[1] = fmaxf(mx[1], s_max[1][w]); }
+    float sum[2] = {0.f, 0.f};
+    auto store = [&](int k, const float (&s)[PER][8]) {
+      T terms[PER][8][NT];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float w = exp2f(s[e] - mx + kProbShift);
-        sum += w;
-        split_terms<T, false>(w, terms[e]);
-      }
+      for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float w = exp2f(s[i][e] - mx[i] + kProbShift);
+          sum[i] += w;
+          split_terms<T, false>(w, terms[i][e]);
+        }
       const int blk = k * kSubs + (lane >> 1);
       if (blk < n_blk) {
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          uint4 v;
-          v.x = pack_pair<T>(terms[0][t], terms[1][t]); v.y = pack_pair<T>(terms[2][t], terms[3][t]);
-          v.z = pack_pair<T>(terms[4][t], terms[5][t]); v.w = pack_pair<T>(terms[6][t], terms[7][t]);
-          *reinterpret_cast<uint4*>(probs + ((((int64_t)(blk0 + blk) * NT + t) * 2 + (lane & 1)) * p.np + h) * 8) = v;
+          uint32_t v[2][4] = {};
+#pragma unroll
+          for (int i = 0; i < PER; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[i][e] = pack_pair<T>(terms[i][2 * e][t], terms[i][2 * e + 1][t]);
+          T* dst = probs + ((((int64_t)(blk0 + blk) * NT + t) * 2 + (lane & 1)) * p.np + h) * 8;   // 32-byte aligned: np and h are even
+          if (two)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]),
+                         "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]) : "memory");
+          else
+            *reinterpret_cast<uint4*>(dst) = make_uint4(v[0][0], v[0][1], v[0][2], v[0][3]);
         }
       }
     };
@@ -824,21 +834,34 @@ softmax_kernel(const Params p) {
       if (k < n_tiles) store(k, held[j]);
     }
     for (int k = warp + kHold * kSoftmaxWarps; k < n_tiles; k += kSoftmaxWarps) {
-      float s[8];
+      float s[PER][8];
       load(k, s);
       store(k, s);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) s_sum[warp] = sum;
+    for (int o = 16; o > 0; o >>= 1) {
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+      sum[1] += __shfl_xor_sync(0xffffffffu, sum[1], o);
+    }
+    if (lane < 2) s_sum[lane][warp] = lane == 0 ? sum[0] : sum[1];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < (two ? 2 : 1)) {
       float total = 0.f;
 #pragma unroll
-      for (int w = 0; w < kSoftmaxWarps; ++w) total += s_sum[w];
-      p.inv_sum[(int64_t)slot * p.heads + h] = 1.f / total;
+      for (int w = 0; w < kSoftmaxWarps; ++w) total += s_sum[threadIdx.x][w];
+      p.inv_sum[(int64_t)slot * p.heads + h + threadIdx.x] = 1.f / total;
     }
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSoftmaxWarps * 32, kTerms<T> == 2 ? 6 : 5)
+softmax_kernel(const Params p) {
+  __shared__ float s_max[2][kSoftmaxWarps], s_sum[2][kSoftmaxWarps];
+  chain_wait();
+  chain_next();
+  if (p.plan->n * p.heads <= 2 * p.grid_scores) softmax_units<T, 1>(p, s_max, s_sum);
+  else softmax_units<T, 2>(p, s_max, s_sum);
 }
 
 // ---- weighted sums ------------------------------------------------------------------
@@ -1212,7 +1235,7 @@ int terms_of(int dtype) { return dtype == APS_BF16 ? 3 : 2; }
 struct Layout {
   int np, n_cap, n_groups, n_hidden_cap, splits, max_slice;
   uint32_t unfold_ring;
-  size_t off_groups, off_slot, off_list, off_qscale, off_inv, off_scores, off_probs, off_qz, off_part, total;
+  size_t off_groups, off_slot, off_list, off_qscale, off_inv, off_scores, off_pieces, off_probs, off_qz, off_part, total;
 };
 
 Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_size, int hidden, int dtype) {
@@ -1239,11 +1262,13 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.max_slice = ms;
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
   const int64_t reqs = batch < kGroup ? batch : kGroup, blks = reqs * ((max_tokens + 15) / 16);
-  int64_t tiles = reqs * ((max_tokens + kTile - 1) / kTile);
+  const int64_t all_tiles = reqs * ((max_tokens + kTile - 1) / kTile);
+  int64_t tiles = all_tiles;
   const int64_t pieces = (blks + tiles * kTileCost) * (hidden / 128) / kMinPiece;   // none is smaller than kMinPiece
   tiles += pieces < 1 ? 1 : pieces < kMaxPieces ? pieces : kMaxPieces;
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o = align_up(o + bytes, 256); return at; };
+  l.off_pieces = take((size_t)all_tiles * sizeof(int2));
   l.off_groups = take((size_t)l.n_groups * sizeof(GroupPlan));
   l.off_slot = take((size_t)batch * sizeof(int));
   l.off_list = take((size_t)batch * sizeof(int2));
@@ -1397,6 +1422,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   p.qt = qz; p.z = qz;
   p.qscale = reinterpret_cast<float*>(b + l.off_qscale); p.inv_sum = reinterpret_cast<float*>(b + l.off_inv);
   p.scores = reinterpret_cast<float*>(b + l.off_scores); p.probs = b + l.off_probs;
+  p.tile_pieces = reinterpret_cast<int2*>(b + l.off_pieces);
   p.out_part = reinterpret_cast<float*>(b + l.off_part);
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
