@@ -163,7 +163,7 @@ struct HybridCall {
   int64_t hidden_row_stride, num_hidden_rows, w_stride;
   void* workspace; size_t workspace_bytes;
 };
-// New-token cache writes of a decode batch addressed from the block tables (cache_ops.cu).
+// New-token cache writes of a decode batch addressed from the block tables (launch_step_plan).
 // key == NULL: no K/V rows are written; hidden == NULL: no hidden rows are written.
 struct NewTokenWrite {
   const void* hidden; const void* key; const void* value; void* key_cache; void* value_cache; void* hidden_cache;
@@ -172,7 +172,6 @@ struct NewTokenWrite {
   int64_t hidden_stride, key_stride, value_stride, block_stride, slot_stride;
   int dtype;
 };
-int launch_new_token_write(const NewTokenWrite& a, cudaStream_t stream);
 int read_metadata_status(int* host_status, cudaStream_t stream);   // metadata_ops.cu
 
 int check_hybrid_call(const char* op, const HybridCall& c);
@@ -185,14 +184,14 @@ bool folded_supported(int dtype, int heads, int head_size, int hidden);
 bool folded_takes(const HybridCall& c);   // pointers and strides; what it does not take is re-projected
 size_t folded_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size,
                               int hidden, int dtype);
-// behind_write: the kernel enqueued last on the stream is launch_new_token_write's.
-int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
+// The new-token writes and the attention.
+int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& n, cudaStream_t stream);
 
 // Its fp32 counterpart on the CUDA cores (hidden_fp32.cu).
 bool folded32_shape(int dtype, int heads, int head_size, int hidden);
 bool folded32_supported(const HybridCall& c);
 size_t folded32_workspace_bytes(int batch, int max_blocks_per_seq, int block_size, int heads, int head_size, int hidden);
-int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStream_t stream);
+int enqueue_folded32_attention(const HybridCall& c, const NewTokenWrite& n, cudaStream_t stream);
 
 // Inclusive prefix sums of a pair over the 1024 threads of a planning CTA, and the totals: shuffles inside the warps,
 // one barrier (a scan through shared memory takes 20, which was 3 us of a K/V-only plan's 8).

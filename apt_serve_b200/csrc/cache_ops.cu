@@ -325,8 +325,8 @@ bulk_copy_kernel(const Resolver R, int64_t n_jobs, uint32_t stage_bytes) {
 }
 
 // One-warp CTAs, all resident: as many per SM as the occupancy query grants for this ring size
-// with the shared-memory carve-out at its maximum (at most 16).  chained: a decode step's write, which takes
-// microseconds and other kernels of the step follow.  The bulk moves (prefill rows, block copies) are launched the
+// with the shared-memory carve-out at its maximum (at most 16).  chained: the writes of a decode batch, which take
+// microseconds and other kernels follow.  The bulk moves (prefill rows, block copies) are launched the
 // plain way: chained, the CTAs of the next one start wherever an SM has run dry, and a prefill write of 32 prompts
 // with its block copies takes 175 us instead of 170.
 template <class Resolver>
@@ -538,76 +538,6 @@ inline int threads_for(int64_t n_vec) {
   }
 
 }  // namespace
-}  // namespace aps
-
-namespace aps {
-namespace {
-
-// New-token writes of a decode batch, addressed from the block tables: row r*2 is the K row
-// (K/V-cached request) or the layer-input row (hidden-cached request) of request r, row
-// r*2 + 1 its V row (K/V-cached requests only).  The token's position is seq_lens[r] - 1.
-struct NewTokenJobs {
-  const char* hidden; const char* key; const char* value; char* key_cache; char* value_cache; char* hidden_cache;
-  const int32_t* block_tables; const int32_t* seq_lens; const int32_t* cache_type;
-  int max_blocks, block_size;
-  int64_t hidden_stride_b, key_stride_b, value_stride_b, block_stride_b, slot_stride_b, kv_row_bytes, hidden_row_bytes;
-  Pieces pc_kv, pc_hid; uint32_t pieces;
-  __device__ BulkJob operator()(int64_t job) const {
-    const uint32_t piece = (uint32_t)(job % pieces);
-    const int64_t row = job / pieces, r = row >> 1;
-    const bool second = (row & 1) != 0;
-    BulkJob j{nullptr, nullptr, nullptr, 0u};
-    const int pos = min(seq_lens[r], max_blocks * block_size) - 1;
-    if (pos < 0 || cache_type[r] == kCacheTypeNone) return j;
-    const int64_t blk = block_tables[r * max_blocks + pos / block_size];
-    if (cache_type[r] != 0) {
-      if (second || piece >= pc_hid.pieces || hidden == nullptr) return j;
-      j.src = hidden + r * hidden_stride_b + pc_hid.offset(piece);
-      j.dst0 = hidden_cache + (blk * block_size + pos % block_size) * slot_stride_b + pc_hid.offset(piece);
-      j.bytes = pc_hid.length(piece, (uint32_t)hidden_row_bytes);
-    } else {
-      if (piece >= pc_kv.pieces || key == nullptr) return j;
-      const int64_t off = blk * block_stride_b + (pos % block_size) * kv_row_bytes + pc_kv.offset(piece);
-      j.src = (second ? value + r * value_stride_b : key + r * key_stride_b) + pc_kv.offset(piece);
-      j.dst0 = (second ? value_cache : key_cache) + off;
-      j.bytes = pc_kv.length(piece, (uint32_t)kv_row_bytes);
-    }
-    return j;
-  }
-};
-
-}  // namespace
-
-int launch_new_token_write(const NewTokenWrite& a, cudaStream_t stream) {
-  const int es = dtype_size(a.dtype);
-  const int64_t row = (int64_t)a.heads * a.head_size;
-  const bool kv = a.key != nullptr, hid = a.hidden != nullptr;
-  if (!kv && !hid) return APS_OK;
-  APS_REQUIRE(!kv || (a.value && a.key_cache && a.value_cache), APS_ERR_NULL_POINTER,
-              "decode_layer_step: new_key given without new_value / K/V cache");
-  APS_REQUIRE(!hid || a.hidden_cache, APS_ERR_NULL_POINTER, "decode_layer_step: hidden_states given without hidden cache");
-  int vb = 16;
-  if (kv) vb = common_vector_bytes({(uint64_t)(uintptr_t)a.key, (uint64_t)(uintptr_t)a.value, (uint64_t)(uintptr_t)a.key_cache,
-                                    (uint64_t)(uintptr_t)a.value_cache, (uint64_t)row * es, (uint64_t)a.key_stride * es,
-                                    (uint64_t)a.value_stride * es, (uint64_t)a.block_stride * es});
-  if (hid) {
-    const int vh = common_vector_bytes({(uint64_t)(uintptr_t)a.hidden, (uint64_t)(uintptr_t)a.hidden_cache,
-                                        (uint64_t)a.hidden_size * es, (uint64_t)a.hidden_stride * es,
-                                        (uint64_t)a.slot_stride * es});
-    vb = vh < vb ? vh : vb;
-  }
-  APS_REQUIRE(vb == 16, APS_ERR_MISALIGNED,
-              "decode_layer_step: step inputs and caches must be 16-byte aligned with 16-byte rows and strides");
-  const Pieces pk = pieces_for((uint64_t)row * es), ph = pieces_for((uint64_t)a.hidden_size * es);
-  const uint32_t pieces = !kv ? ph.pieces : !hid ? pk.pieces : (pk.pieces > ph.pieces ? pk.pieces : ph.pieces);
-  const uint32_t stage = !kv ? ph.piece : !hid ? pk.piece : (pk.piece > ph.piece ? pk.piece : ph.piece);
-  NewTokenJobs R{(const char*)a.hidden, (const char*)a.key, (const char*)a.value, (char*)a.key_cache,
-                 (char*)a.value_cache, (char*)a.hidden_cache, a.block_tables, a.seq_lens, a.cache_type,
-                 a.max_blocks_per_seq, a.block_size, a.hidden_stride * es, a.key_stride * es, a.value_stride * es,
-                 a.block_stride * es, a.slot_stride * es, row * es, (int64_t)a.hidden_size * es, pk, ph, pieces};
-  return launch_bulk(R, (int64_t)a.batch * 2 * pieces, stage, stream, "new-token cache write (bulk copy)", true);
-}
-
 }  // namespace aps
 
 using namespace aps;

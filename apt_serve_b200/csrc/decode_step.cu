@@ -6,12 +6,12 @@
 // write the new token's layer-input row for hidden-cached requests (hidden_to_cache), write
 // the new token's K/V rows for K/V-cached requests (mixed_kv_to_cache / reshape_and_cache_flash),
 // then attend.  Here that is one host call that enqueues its launches on the caller's
-// stream: a bulk-copy launch for all new-token rows, addressed straight from the private
-// block tables, the sequence lengths and the cache-type mask (no int64 index tensors), and
-// the hybrid decode attention: plan, K/V streaming, the hidden path (five launches per 256 requests when the
+// stream: the new-token rows, addressed straight from the private
+// block tables, the sequence lengths and the cache-type mask (no int64 index tensors), with the plan
+// (a launch of its own when the rows are re-projected), K/V streaming, the hidden path (five launches per 256 requests when the
 // cached rows are attended directly, three in fp32, one when they are re-projected), combine.
 
-#include "attention_common.cuh"
+#include "step_plan.cuh"
 
 using namespace aps;
 
@@ -75,10 +75,9 @@ extern "C" int aps_decode_layer_step(void* out, const void* query, const void* h
                    block_tables, seq_lens, cache_type, batch, max_blocks_per_seq, block_size,
                    num_heads, head_size, hidden_size, hidden_states_stride, new_key_stride,
                    new_value_stride, block_stride, hidden_row_stride, dtype};
-  if ((st = launch_new_token_write(nw, cs)) != APS_OK) return st;
-  const bool behind_write = hidden_states != nullptr || new_key != nullptr;
-  if (use_folded(c)) return enqueue_folded_attention(c, behind_write, cs);
-  if (folded32_supported(c)) return enqueue_folded32_attention(c, behind_write, cs);
+  if (use_folded(c)) return enqueue_folded_attention(c, nw, cs);
+  if (folded32_supported(c)) return enqueue_folded32_attention(c, nw, cs);
+  if ((st = launch_step_plan(nullptr, nw, cs)) != APS_OK) return st;
   return enqueue_hybrid_attention(c, cs);
 }
 

@@ -17,6 +17,7 @@
 // 0.86 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
 // requests, 0.47 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.20 ms against 2.5.
 //
+//   step_plan_kernel the plan, and the new tokens' cache rows
 //   fold_kernel      qt[r][h] = W_k,h^T q[r][h]                       tcgen05, M = 128 columns of E
 //   scores_kernel    s[t][h] = x_t . qt[r][h]                         tcgen05, M = 128 tokens
 //   softmax_kernel   p[t][h] = 2^(scale s - max)                      four warps per (request, two heads)
@@ -50,6 +51,7 @@
 #include "step_plan.cuh"
 #include "tensor_maps.cuh"
 
+#include <initializer_list>
 #include <type_traits>
 
 namespace aps {
@@ -81,7 +83,7 @@ __device__ inline int unit_of_piece(int c, int levels, int per_level) {
 
 struct Params {
   GroupPlan* plan;
-  const void* query; const void* b_k; const int32_t* block_tables;
+  const void* query; const int32_t* block_tables; const int32_t* cache_type;
   void* qt;              // [request][term][head][E]
   float* qscale;         // [request][head] scale * log2(e) / (power of two q was multiplied with)
   float* scores;         // [tile + piece][head][kTile] partial scores over a range of E
@@ -91,7 +93,7 @@ struct Params {
   void* z;               // [term][head][request capacity][E]
   float* out_part;       // [split][hidden request][H * D]
   int* status;
-  int heads, np, head_size, hidden, slabs;   // np: heads padded to a multiple of 16; slabs: E / 64
+  int batch, heads, np, head_size, hidden, slabs;   // np: heads padded to a multiple of 16; slabs: E / 64
   int block_size, max_blocks, n_cap;         // n_cap: requests a group can hold here
   int group_first;                           // ordinal of the group's first hidden request
   int n_hidden_cap, splits, grid_scores;
@@ -142,22 +144,66 @@ __device__ __forceinline__ void drain() {
   while (clock64() - t0 < 2000000LL) { }
 }
 
-// ---- plan ---------------------------------------------------------------------------
-// One CTA.  K/V-cached requests: the chunk list of the K/V kernel and the partial slots.  Hidden-cached
-// requests: the groups.  Runs of requests per thread, warp-shuffle scans.
-// Behind the write of the new tokens' cache rows (wait_last) it runs beside it: it reads only the call's
-// arguments, and what it writes (the scratch) was last used by kernels before that write, which were complete when
-// the write let this kernel start.  It waits for the write before it exits.  As a call's first kernel it waits first.
+// ---- plan and new-token writes --------------------------------------------------------
+// The first kernel of a layer-step.  CTA 0 plans: K/V-cached requests: the chunk list of the K/V kernel and the partial
+// slots.  Hidden-cached requests: the groups.  Runs of requests per thread, warp-shuffle scans.  The other CTAs write the
+// step's new rows, addressed straight from the block tables: a warp per 2 KB of a row, three round trips (length and
+// type, block, row).  One launch instead of two one after the other, and the fold
+// beside it: a step of one OPT-13B request 70 -> 60 us, of 48 OPT-1.3B requests 118 -> 108, of 8 in fp32 52 -> 45.
+
+constexpr uint32_t kWriteChunk = 2048;   // bytes of a row per warp: four 16-byte vectors per lane
+
+struct StepWrite {
+  const char* hidden; const char* key; const char* value; char* key_cache; char* value_cache; char* hidden_cache;
+  const int32_t* block_tables; const int32_t* seq_lens; const int32_t* cache_type;
+  int batch, max_blocks, block_size, chunks;   // chunks: per row, of the longer kind
+  uint32_t kv_row_bytes, hidden_row_bytes;
+  int64_t hidden_stride_b, key_stride_b, value_stride_b, block_stride_b, slot_stride_b;
+};
+
+// Row 2 r is the K row (K/V-cached request) or the layer-input row (hidden-cached request) of request r, row 2 r + 1 its
+// V row (K/V-cached requests only).  The token's position is seq_lens[r] - 1.
+__device__ __forceinline__ void write_new_rows(const StepWrite& w, int64_t job, int lane) {
+  const int64_t row = job / w.chunks, r = row >> 1;
+  if (r >= w.batch) return;
+  const uint32_t at = (uint32_t)(job - row * w.chunks) * kWriteChunk;
+  const bool second = (row & 1) != 0;
+  const int pos = min(w.seq_lens[r], w.max_blocks * w.block_size) - 1, type = w.cache_type[r];
+  if (pos < 0 || type == kCacheTypeNone) return;
+  const bool hid = type != 0;
+  const uint32_t bytes = hid ? w.hidden_row_bytes : w.kv_row_bytes;
+  const char* base = hid ? w.hidden : second ? w.value : w.key;
+  if (base == nullptr || (hid && second) || at >= bytes) return;
+  const int64_t blk = w.block_tables[r * w.max_blocks + pos / w.block_size];
+  const char* src = base + r * (hid ? w.hidden_stride_b : second ? w.value_stride_b : w.key_stride_b);
+  char* dst = hid ? w.hidden_cache + (blk * w.block_size + pos % w.block_size) * w.slot_stride_b
+                  : (second ? w.value_cache : w.key_cache) + blk * w.block_stride_b + (int64_t)(pos % w.block_size) * bytes;
+  uint4 v[kWriteChunk / 512];
+#pragma unroll
+  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
+    const uint32_t o = at + k * 512 + lane * 16;
+    if (o < bytes) v[k] = *reinterpret_cast<const uint4*>(src + o);
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
+    const uint32_t o = at + k * 512 + lane * 16;
+    if (o < bytes) *reinterpret_cast<uint4*>(dst + o) = v[k];
+  }
+}
 
 __global__ void __launch_bounds__(kPlanThreads)
-step_plan_kernel(const PlanArgs a) {
+step_plan_kernel(const PlanArgs a, const StepWrite w, const int plan_ctas) {
   __shared__ int2 warp_sums[32];
   __shared__ int s_missing;
   __shared__ int s_req[kGroup], s_len[kGroup], s_toff[kGroup + 1], s_woff[kGroup + 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_missing = 0;
-  if (!a.wait_last) chain_wait();
+  chain_wait();
   chain_next();
+  if ((int)blockIdx.x >= plan_ctas) {
+    write_new_rows(w, (int64_t)((int)blockIdx.x - plan_ctas) * (kPlanThreads / 32) + warp, lane);
+    return;
+  }
   __syncthreads();
   const int per = (a.batch + kPlanThreads - 1) / kPlanThreads;
   const int r0 = min(a.batch, tid * per), r1 = min(a.batch, r0 + per);
@@ -215,7 +261,7 @@ step_plan_kernel(const PlanArgs a) {
     __syncthreads();
     if (i < n && part == 0) {
       s_req[rank] = rec.x; s_len[rank] = rec.y;
-      gp->req[rank] = rec.x; gp->len[rank] = rec.y;
+      gp->req[rank] = rec.x; gp->len[rank] = rec.y; gp->ord[rank] = i;
       a.hid_slot[rec.x] = g * kGroup + rank;
     }
     __syncthreads();
@@ -285,7 +331,6 @@ step_plan_kernel(const PlanArgs a) {
       gp->bound_tile[c] = t; gp->bound_step[c] = step;
     }
   }
-  chain_wait();
 }
 
 // ---- fold ---------------------------------------------------------------------------
@@ -293,9 +338,9 @@ step_plan_kernel(const PlanArgs a) {
 // One CTA per (range of E, head, 128 requests): q is gathered once by all threads into a K-major B operand
 // and stays; W_k,h streams past it in tiles of 128 columns (two boxes of 64 columns x D rows, an MN-major
 // A operand) through a two-stage ring, the accumulators are double-buffered.  Two CTAs per SM.
-// Behind the K/V kernel it does not wait for that kernel (wait_last): it needs the plan, which was complete when the
-// K/V kernel let it start, and writes qt, which no kernel since the plan touches; its CTAs fill the SMs that the
-// K/V kernel leaves.  It waits before it exits.
+// It takes the group's requests in batch order, which it finds in cache_type by itself, so that it needs neither the plan
+// nor the new rows: the first group's fold runs beside the step's first kernel (wait_last; what was enqueued before that
+// one is complete, since it waits before it lets this one start) and waits before it exits.
 // Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
 constexpr int kFoldThreads = 192;
 constexpr int kFoldReqs = 128;
@@ -311,10 +356,10 @@ template <int D> constexpr size_t fold_smem() {
   return 1024 + (size_t)kFoldStages * 2 * D * 128 + (size_t)((D + 63) / 64) * kFoldReqs * 128;
 }
 
-// Gathers q[request][head] of m requests from ordinal r0 on (zero rows up to np) into shared memory: slabs of
+// Gathers q[request][head] of m requests, reqs, of ordinals from r0 on (zero rows up to np) into shared memory: slabs of
 // 64 elements, rows of 128 bytes, 128-byte swizzle.  All warps of the CTA.
 template <typename T, int D>
-__device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, int r0, int m, int np, int head, bool keep_scale) {
+__device__ __forceinline__ void stage_queries(const Params& p, const int* reqs, uint32_t q_at, int r0, int m, int np, int head, bool keep_scale) {
   constexpr int kWarps = kFoldThreads / 32, U = 4, EPL = D / 32;   // U requests at a time, EPL elements per lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* query = static_cast<const T*>(p.query);
@@ -324,7 +369,7 @@ __device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, in
     for (int u = 0; u < U; ++u) {
       const int rr = r + u * kWarps;
       const bool in = rr < m;
-      const T* src = query + (in ? (int64_t)p.plan->req[r0 + rr] * p.query_stride + head * D + lane * EPL : 0);
+      const T* src = query + (in ? (int64_t)reqs[rr] * p.query_stride + head * D + lane * EPL : 0);
 #pragma unroll
       for (int e = 0; e < EPL; ++e) v[u][e] = in ? src[e] : Elem<T>::from_float(0.f);
     }
@@ -355,6 +400,31 @@ __device__ __forceinline__ void stage_queries(const Params& p, uint32_t q_at, in
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // read by the tensor cores next
 }
 
+// The batch rows of hidden-cached requests first ... first + kFoldReqs - 1 (counted over the batch); returns how many there
+// are of them.  All warps of the CTA; a warp counts 32 rows at a time.
+__device__ __forceinline__ int find_requests(const int32_t* cache_type, int batch, int first, int* reqs, int* counts) {
+  constexpr int kWarps = kFoldThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int before = 0;
+  for (int b = 0; b < batch && before < first + kFoldReqs; b += kFoldThreads) {
+    const int r = b + threadIdx.x, type = r < batch ? cache_type[r] : 0;
+    const bool hid = type != 0 && type != kCacheTypeNone;
+    const uint32_t mask = __ballot_sync(0xffffffffu, hid);
+    __syncthreads();   // the last round's counts have been read
+    if (lane == 0) counts[warp] = __popc(mask);
+    __syncthreads();
+    int at = before + __popc(mask & ((1u << lane) - 1)) - first;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) {
+      at += k < warp ? counts[k] : 0;
+      before += counts[k];
+    }
+    if (hid && at >= 0 && at < kFoldReqs) reqs[at] = r;
+  }
+  __syncthreads();
+  return max(0, min(kFoldReqs, before - first));
+}
+
 template <typename T, int D>
 __global__ void __launch_bounds__(kFoldThreads, 2)
 fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int wait_last) {
@@ -365,9 +435,10 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
   __shared__ FoldAux aux;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (!wait_last) chain_wait();
-  const int n = p.plan->n, r0 = blockIdx.z * kFoldReqs, head = blockIdx.y;
-  if (r0 >= n) { chain_wait(); return; }
-  const int m = min(kFoldReqs, n - r0), np = (m + 15) & ~15;
+  __shared__ int s_reqs[kFoldReqs], s_counts[kFoldThreads / 32];
+  const int r0 = blockIdx.z * kFoldReqs, head = blockIdx.y;
+  const int m = find_requests(p.cache_type, p.batch, p.group_first + r0, s_reqs, s_counts), np = (m + 15) & ~15;
+  if (m == 0) { chain_wait(); return; }
   const int blocks = p.hidden / 128;
   const int ta = blocks * blockIdx.x / gridDim.x, tb = blocks * (blockIdx.x + 1) / gridDim.x;
   volatile int* abort_flag = &aux.abort_flag;
@@ -384,7 +455,7 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
     }
   }
   if (warp == 1) tmem_alloc(&aux.tmem_base, 2 * kFoldReqs);
-  stage_queries<T, D>(p, q_at, r0, m, np, head, blockIdx.x == 0);
+  stage_queries<T, D>(p, s_reqs, q_at, r0, m, np, head, blockIdx.x == 0);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -470,7 +541,8 @@ fold_kernel(const __grid_constant__ CUtensorMap map_w, const Params p, const int
 // A box is (64 columns, 8 rows, 2): 256 contiguous bytes of a cached row, so that a DRAM page is left after
 // 256 bytes and not 128, and 8-row groups that lie 2 KB apart, as the K-major operand needs them.  X and qt
 // have a ring each: a unit of X is 128 tokens x 128 columns (32 KB), a unit of qt serves both halves of a
-// tile.  L2: qt (105 MB for 128 OPT-13B requests) is read once per tile and was fetched from memory almost every time,
+// tile.  Behind the K/V kernel it does not wait for that one (wait_last): plan and folded queries were complete when the K/V
+// kernel let it start, and its CTAs fill the SMs which that one leaves; it waits before it exits.  L2: qt (105 MB for 128 OPT-13B requests) is read once per tile and was fetched from memory almost every time,
 // because the rows, which are read once by this kernel, pushed it out (1.25 GB of DRAM traffic for 0.97 GB of rows).  The
 // rows are the first to go (evict_first), qt stays (evict_last): 205 -> 190 us for 128 OPT-13B requests, 172 -> 155 for 52
 // OPT-66B tp 8 requests, 69 -> 63 for 24 of 1800 OPT-13B tokens, 313 -> 283 for 100 OPT-66B tp 2.  Warps: 0 qt boxes, 1 MMA issue, 2-5 epilogue, 6-7 boxes of X (eight lanes each).
@@ -516,21 +588,21 @@ __host__ __device__ inline int scores_q_units(int terms, int np) {
 
 template <typename T>
 __global__ void __launch_bounds__(kScoresThreads, 1)
-scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q, const Params p) {
+scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q, const Params p, const int wait_last) {
   constexpr int NT = kTerms<T>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t x_ring = (smem_u32(smem_raw) + 1023) & ~1023u;
   __shared__ RingAux aux;
-  __shared__ int s_toff[kGroup + 1], s_len[kGroup], s_req[kGroup];
+  __shared__ int s_toff[kGroup + 1], s_len[kGroup], s_req[kGroup], s_ord[kGroup];
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   __shared__ ItemRing items;
-  chain_wait();
+  if (!wait_last) chain_wait();
   GroupPlan* gp = p.plan;
   const int n = gp->n, n_pieces = gp->levels * gp->per_level;
-  if (n == 0 || (int)blockIdx.x >= n_pieces) return;
+  if (n == 0 || (int)blockIdx.x >= n_pieces) { chain_wait(); return; }
   for (int i = threadIdx.x; i <= n; i += kScoresThreads) {
     s_toff[i] = gp->tile_off[i];
-    if (i < n) { s_len[i] = gp->len[i]; s_req[i] = gp->req[i]; }
+    if (i < n) { s_len[i] = gp->len[i]; s_req[i] = gp->req[i]; s_ord[i] = gp->ord[i]; }
   }
   const int np = p.np, steps = p.hidden / 128;
   const uint32_t q_bytes = scores_q_bytes(NT, np);
@@ -627,7 +699,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)(NT * 2 * p.heads * 128));
             __syncwarp();
             if (lane < 2 * NT)   // lane = (term, half of the columns); the terms of a half lie one behind the other
-              tma_load_2d_hint(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (slot * NT + (lane >> 1)) * p.heads, again);
+              tma_load_2d_hint(q_ring + qr.stage * q_bytes + ((lane & 1) * NT + (lane >> 1)) * np * 128, &map_q, bar, s * 128 + (lane & 1) * 64, (s_ord[slot] * NT + (lane >> 1)) * p.heads, again);
             __syncwarp();
             qr.step(nq);
           }
@@ -714,6 +786,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_free(tmem, tmem_cols); }
+  chain_wait();
 }
 
 // ---- softmax ------------------------------------------------------------------------
@@ -740,7 +813,7 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
     const bool two = PER == 2 && h + 1 < p.heads;
     const int len = gp->len[slot];
     const int tile0 = gp->tile_off[slot], n_tiles = gp->tile_off[slot + 1] - tile0;
-    const float* scales = p.qscale + (int64_t)slot * p.heads + h;
+    const float* scales = p.qscale + (int64_t)gp->ord[slot] * p.heads + h;
     const float scale[2] = {scales[0], two ? scales[1] : 0.f};
     const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot];
     // scores of this lane's eight tokens of tile k
@@ -1309,8 +1382,9 @@ int allow_smem(K kernel, size_t bytes, bool* done) {
 struct Maps { CUtensorMap x_scores, x_sum, q, wk, wv, z; };
 
 template <typename T, int D>
-int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv, cudaStream_t stream) {
+int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCall* kv, const WorkspacePtrs& ws, cudaStream_t stream) {
   const size_t ring = 1024 + kRingBytes;
+  const int first = p.group_first == 0 ? 1 : 0;
   int st;
   {
     static bool done[64] = {false};
@@ -1321,14 +1395,16 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv
     int splits = 2 * sm_count() / p.heads;   // one wave at two CTAs per SM when one chunk of requests is in use
     splits = splits < 1 ? 1 : splits > blocks ? blocks : splits;
     if ((st = launch_chained("fold_kernel", k, dim3(splits, p.heads, chunks), kFoldThreads, smem, stream, m.wk, p,
-                             behind_kv ? 1 : 0)) != APS_OK) return st;
+                             first)) != APS_OK) return st;
   }
+  if (kv != nullptr && (st = launch_kv_attention(ws, kv->query, kv->key_cache, kv->value_cache, kv->block_tables, kv->seq_lens,
+                                                 kv->shape, stream)) != APS_OK) return st;
   {
     static bool done[64] = {false};
     auto k = scores_kernel<T>;
     if ((st = allow_smem(k, 1024 + kScoresRing, done)) != APS_OK) return st;
     if ((st = launch_chained("scores_kernel", k, p.grid_scores, kScoresThreads, 1024 + kScoresRing, stream, m.x_scores,
-                             m.q, p)) != APS_OK) return st;
+                             m.q, p, kv != nullptr ? 1 : 0)) != APS_OK) return st;
   }
   const int units = n_cap * p.heads, resident = sm_count() * 12;
   if ((st = launch_chained("softmax_kernel", softmax_kernel<T>, units < resident ? units : resident, kSoftmaxWarps * 32, 0,
@@ -1352,8 +1428,38 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, bool behind_kv
 
 }  // namespace
 
-int launch_step_plan(const PlanArgs& a, cudaStream_t stream) {
-  return launch_chained("step_plan_kernel", step_plan_kernel, 1, kPlanThreads, 0, stream, a);
+// plan may be NULL: the new-token writes alone.
+int launch_step_plan(const PlanArgs* plan, const NewTokenWrite& n, cudaStream_t stream) {
+  const int64_t es = dtype_size(n.dtype), row = (int64_t)n.heads * n.head_size;
+  const bool kv = n.key != nullptr, hid = n.hidden != nullptr;
+  if (plan == nullptr && !kv && !hid) return APS_OK;
+  APS_REQUIRE(!kv || (n.value && n.key_cache && n.value_cache), APS_ERR_NULL_POINTER,
+              "decode_layer_step: new_key given without new_value / K/V cache");
+  APS_REQUIRE(!hid || n.hidden_cache, APS_ERR_NULL_POINTER, "decode_layer_step: hidden_states given without hidden cache");
+  auto fits = [](std::initializer_list<const void*> p, std::initializer_list<int64_t> bytes) {
+    for (const void* x : p) if (!aligned_to(x, 16)) return false;
+    for (int64_t x : bytes) if (x % 16 != 0) return false;
+    return true;
+  };
+  APS_REQUIRE((!kv || fits({n.key, n.value, n.key_cache, n.value_cache}, {row * es, n.key_stride * es, n.value_stride * es, n.block_stride * es})) &&
+                  (!hid || fits({n.hidden, n.hidden_cache}, {n.hidden_size * es, n.hidden_stride * es, n.slot_stride * es})),
+              APS_ERR_MISALIGNED,
+              "decode_layer_step: step inputs and caches must be 16-byte aligned with 16-byte rows and strides");
+  StepWrite w{};
+  w.hidden = (const char*)n.hidden; w.key = (const char*)n.key; w.value = (const char*)n.value;
+  w.key_cache = (char*)n.key_cache; w.value_cache = (char*)n.value_cache; w.hidden_cache = (char*)n.hidden_cache;
+  w.block_tables = n.block_tables; w.seq_lens = n.seq_lens; w.cache_type = n.cache_type;
+  w.batch = n.batch; w.max_blocks = n.max_blocks_per_seq; w.block_size = n.block_size;
+  w.kv_row_bytes = (uint32_t)(row * es); w.hidden_row_bytes = (uint32_t)(n.hidden_size * es);
+  w.hidden_stride_b = n.hidden_stride * es; w.key_stride_b = n.key_stride * es; w.value_stride_b = n.value_stride * es;
+  w.block_stride_b = n.block_stride * es; w.slot_stride_b = n.slot_stride * es;
+  const uint32_t widest = !kv ? w.hidden_row_bytes : !hid ? w.kv_row_bytes : w.kv_row_bytes > w.hidden_row_bytes ? w.kv_row_bytes : w.hidden_row_bytes;
+  w.chunks = (int)((widest + kWriteChunk - 1) / kWriteChunk);
+  const int64_t jobs = kv || hid ? 2 * (int64_t)n.batch * w.chunks : 0, ctas = (jobs + kPlanThreads / 32 - 1) / (kPlanThreads / 32);
+  const int plan_ctas = plan != nullptr ? 1 : 0;
+  APS_REQUIRE(ctas + plan_ctas < (int64_t(1) << 31), APS_ERR_SHAPE, "decode_layer_step: batch too large");
+  return launch_chained("step_plan_kernel", step_plan_kernel, dim3((unsigned)(ctas + plan_ctas)), kPlanThreads, 0, stream,
+                        plan != nullptr ? *plan : PlanArgs{}, w, plan_ctas);
 }
 
 bool folded_supported(int dtype, int heads, int head_size, int hidden) {
@@ -1376,7 +1482,7 @@ bool folded_takes(const HybridCall& c) {
          aligned_to(c.w_k, 16) && aligned_to(c.w_v, 16) && sm_count() <= kMaxGrid;   // kMaxGrid: bounds the plan keeps
 }
 
-int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_t cs) {
+int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaStream_t cs) {
   const AttnShape& s = c.shape;
   const WorkspaceLayout w = workspace_layout(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size);
   const WorkspacePtrs ws = workspace_ptrs(c.workspace, w);
@@ -1393,10 +1499,8 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
   pa.steps = e_blocks; pa.grid_scores = sm_count();
-  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = kSumRounds * sm_count(); pa.wait_last = behind_write ? 1 : 0;
-  if ((st = launch_step_plan(pa, cs)) != APS_OK) return st;
-  if (have_kv &&
-      (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
+  pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = kSumRounds * sm_count();
+  if ((st = launch_step_plan(&pa, nw, cs)) != APS_OK) return st;
 
   Maps m;
   const uint64_t hd = (uint64_t)s.heads * s.head_size;
@@ -1418,7 +1522,7 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
   if ((st = map_2d(&m.z, qz, s.dtype, c.hidden_size, (uint64_t)nt * s.heads * l.n_cap, c.hidden_size, 16, "weighted sums")) != APS_OK) return st;
 
   Params p{};
-  p.query = c.query; p.block_tables = c.block_tables;
+  p.query = c.query; p.block_tables = c.block_tables; p.cache_type = c.cache_type; p.batch = s.batch;
   p.qt = qz; p.z = qz;
   p.qscale = reinterpret_cast<float*>(b + l.off_qscale); p.inv_sum = reinterpret_cast<float*>(b + l.off_inv);
   p.scores = reinterpret_cast<float*>(b + l.off_scores); p.probs = b + l.off_probs;
@@ -1436,10 +1540,11 @@ int enqueue_folded_attention(const HybridCall& c, bool behind_write, cudaStream_
     p.plan = groups + g;
     p.group_first = g * kGroup;
     const bool bf16 = s.dtype == APS_BF16;
+    const HybridCall* kv = have_kv && g == 0 ? &c : nullptr;   // the K/V kernel runs between the first fold and its scores
     switch (s.head_size) {
-      case 128: st = bf16 ? launch_group<__nv_bfloat16, 128>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 128>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
-      case 64: st = bf16 ? launch_group<__nv_bfloat16, 64>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 64>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
-      default: st = bf16 ? launch_group<__nv_bfloat16, 32>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs) : launch_group<__half, 32>(m, p, l.n_cap, w_tiles, have_kv && g == 0, cs); break;
+      case 128: st = bf16 ? launch_group<__nv_bfloat16, 128>(m, p, l.n_cap, w_tiles, kv, ws, cs) : launch_group<__half, 128>(m, p, l.n_cap, w_tiles, kv, ws, cs); break;
+      case 64: st = bf16 ? launch_group<__nv_bfloat16, 64>(m, p, l.n_cap, w_tiles, kv, ws, cs) : launch_group<__half, 64>(m, p, l.n_cap, w_tiles, kv, ws, cs); break;
+      default: st = bf16 ? launch_group<__nv_bfloat16, 32>(m, p, l.n_cap, w_tiles, kv, ws, cs) : launch_group<__half, 32>(m, p, l.n_cap, w_tiles, kv, ws, cs); break;
     }
     if (st != APS_OK) return st;
   }

@@ -345,7 +345,7 @@ size_t folded32_workspace_bytes(int batch, int max_blocks_per_seq, int block_siz
          layout_of(batch, max_blocks_per_seq, block_size, heads, head_size, hidden).total;
 }
 
-int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStream_t cs) {
+int enqueue_folded32_attention(const HybridCall& c, const NewTokenWrite& nw, cudaStream_t cs) {
   const AttnShape& s = c.shape;
   const WorkspaceLayout w = workspace_layout(s.batch, s.max_blocks_per_seq, s.block_size, s.heads, s.head_size);
   const WorkspacePtrs ws = workspace_ptrs(c.workspace, w);
@@ -360,8 +360,9 @@ int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStrea
   pa.hid_slot = reinterpret_cast<int*>(b + l.off_slot); pa.hid_list = reinterpret_cast<int2*>(b + l.off_list);
   pa.groups = groups; pa.seq_lens = c.seq_lens; pa.cache_type = c.cache_type; pa.batch = s.batch;
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
-  pa.steps = 1; pa.grid_scores = 1; pa.max_slice = 1; pa.item_target = 1; pa.wait_last = behind_write ? 1 : 0;
-  if ((st = launch_step_plan(pa, cs)) != APS_OK) return st;
+  pa.steps = 1; pa.grid_scores = 1; pa.max_slice = 1; pa.item_target = 1;
+  if ((st = launch_step_plan(&pa, nw, cs)) != APS_OK) return st;
+  ScopedProfile prof(1, cs);   // with the K/V kernel's events inside, as in hidden_attention.cu
   if (have_kv &&
       (st = launch_kv_attention(ws, c.query, c.key_cache, c.value_cache, c.block_tables, c.seq_lens, s, cs)) != APS_OK) return st;
 
@@ -374,7 +375,6 @@ int enqueue_folded32_attention(const HybridCall& c, bool behind_write, cudaStrea
   p.chunk = l.chunk; p.chunks = l.chunks; p.n_hidden_cap = l.n_hidden_cap;
   p.query_stride = s.query_stride; p.x_stride = c.hidden_row_stride; p.w_stride = c.w_stride;
   p.scale_log2 = s.scale * 1.4426950408889634f;
-  ScopedProfile prof(1, cs);
   for (int first = 0; first < s.batch; first += l.count) {
     p.first = first;
     p.count = s.batch - first < l.count ? s.batch - first : l.count;

@@ -926,7 +926,7 @@ extern "C" int aps_hybrid_decode_attention(void* out, const void* query, const v
   if (st != APS_OK || batch == 0) return st;
   // fp32 has no tensor-core form of the re-projection to prefer: with the layer-step's scratch the hidden rows
   // are attended directly here too
-  if (folded32_supported(c)) return enqueue_folded32_attention(c, false, (cudaStream_t)stream);
+  if (folded32_supported(c)) return enqueue_folded32_attention(c, NewTokenWrite{}, (cudaStream_t)stream);
   return enqueue_hybrid_attention(c, (cudaStream_t)stream);
 }
 

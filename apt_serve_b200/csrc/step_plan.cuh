@@ -19,6 +19,7 @@ struct GroupPlan {
   int levels, per_level;      // pieces of the scores work: levels x per_level
   int next_piece, next_item;  // work counters of the scores and the sum kernel
   int req[kGroup];            // batch row of each request, longest first
+  int ord[kGroup];            // its place in the group in batch order (folded queries)
   int len[kGroup];            // its length in tokens
   int tile_off[kGroup + 1];   // first scores tile
   int blk_off[kGroup + 1];    // first 16-token block of p
@@ -30,8 +31,8 @@ struct GroupPlan {
 struct PlanArgs {
   int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
   const int32_t* seq_lens; const int32_t* cache_type;
-  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target, wait_last;
+  int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target;
 };
-int launch_step_plan(const PlanArgs& a, cudaStream_t stream);
+int launch_step_plan(const PlanArgs* plan, const NewTokenWrite& n, cudaStream_t stream);   // plan may be NULL: the new-token writes alone
 
 }  // namespace aps

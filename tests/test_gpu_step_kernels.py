@@ -3,12 +3,14 @@ against the oracle with the tolerances of test_gpu_folded.py."""
 import pytest
 import torch
 
+from apt_serve_b200 import attention as A
 from apt_serve_b200.workloads import LayerShape, make_decode_workload
 
 from test_gpu_folded import check
 
 pytestmark = pytest.mark.gpu
 F, B = torch.float16, torch.bfloat16
+NONE = -2 ** 31   # cache type of a request without usable tables
 
 
 def workload(heads, d, e, dtype, lens, hidden, device="cpu"):
@@ -22,3 +24,53 @@ def workload(heads, d, e, dtype, lens, hidden, device="cpu"):
 ])
 def test_softmax_units(heads, dtype, lens):
     check(workload(heads, 64, 128, dtype, list(lens), [True] * len(lens)), f"{heads} heads, {len(lens)} requests")
+
+
+def test_requests_without_tables_are_left_out():
+    lens = [40, 17, 900, 1, 129, 64, 33, 200]
+    w = workload(4, 128, 512, F, lens, [True, False] * 4, device="cuda")
+    m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
+
+    def step(types, kv):
+        out = torch.full_like(w.query, float("nan"))
+        return A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, kv, kv, wk, bk, wv, bv,
+                                   m.private_block_tables, m.seq_lens_tensor, types, w.scale, out=out)
+    kv_all, kv_some = w.kv_cache.clone(), w.kv_cache.clone()
+    want = step(m.cache_type, kv_all)
+    types = m.cache_type.clone()
+    types[2] = types[5] = NONE
+    got = step(types, kv_some)
+    assert torch.equal(got[[1, 3, 7]], want[[1, 3, 7]])   # K/V-cached
+    # hidden-cached: another batch is cut into other pieces; both within check()'s bound of the oracle
+    x, y = got[[0, 4, 6]].float(), want[[0, 4, 6]].float()
+    rms = y.pow(2).mean(dim=1, keepdim=True).sqrt()
+    assert ((x - y).abs() <= 2 * (2.0 ** -11 * y.abs() + 2.0 ** -14 * rms)).all()
+    assert not got[[2, 5]].any()
+    rows = kv_some.reshape(2, -1, 4 * 128)
+    slot = int(m.private_block_tables[5][63 // 16]) * 16 + 63 % 16   # request 5 is K/V-cached: its new rows are not written
+    assert torch.equal(rows[:, slot], w.kv_cache.reshape(2, -1, 4 * 128)[:, slot])
+
+
+# new-token rows: a row shorter than a warp's 2 KB, one of several, K/V rows and layer-input rows of different lengths
+@pytest.mark.parametrize("heads,d,e,dtype", [(1, 64, 128, F), (3, 128, 1152, B), (2, 64, 2560, F), (9, 128, 9216, B)])
+def test_new_rows_are_written(heads, d, e, dtype):
+    lens, hidden = [1, 16, 17, 40, 33, 128], [True, False, False, True, False, True]
+    full = e % d == 0 and heads * d != e
+    w = make_decode_workload(LayerShape("t", e // d if full else heads, d, e, dtype), lens, hidden, seed=7, device="cuda",
+                             **({"tp_rank": 0, "tp_size": (e // d) // heads} if full else {}))
+    m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
+    kv, hid = w.kv_cache.clone(), w.hidden_cache.clone()
+    alias = w.hidden_cache.data_ptr() == w.kv_cache.data_ptr()
+    A.decode_layer_step(w.query, w.hidden_states, w.new_key, w.new_value, w.kv_cache, w.hidden_cache, wk, bk, wv, bv,
+                        m.private_block_tables, m.seq_lens_tensor, m.cache_type, w.scale)
+    width = w.new_key.reshape(len(lens), -1).shape[1]
+    if alias:
+        hid = kv
+    flat, planes = hid.view(-1, e), kv.view(2, -1, width)
+    for r, (s, u) in enumerate(zip(lens, hidden)):
+        slot = int(m.private_block_tables[r][(s - 1) // 16]) * 16 + (s - 1) % 16
+        if u:
+            flat[slot] = w.hidden_states[r]
+        else:
+            planes[0, slot], planes[1, slot] = w.new_key.reshape(len(lens), -1)[r], w.new_value.reshape(len(lens), -1)[r]
+    assert torch.equal(w.hidden_cache, hid) and torch.equal(w.kv_cache, kv)
