@@ -26,6 +26,14 @@ def test_softmax_units(heads, dtype, lens):
     check(workload(heads, 64, 128, dtype, list(lens), [True] * len(lens)), f"{heads} heads, {len(lens)} requests")
 
 
+# fold: one turn and several turns of 16 requests per epilogue warp, a second chunk of 128; it finds the requests by itself
+@pytest.mark.parametrize("n,every", [(16, 1), (17, 1), (33, 2), (129, 1), (400, 3)])
+@pytest.mark.parametrize("dtype", [F, B])
+def test_fold_finds_its_requests(n, every, dtype):
+    lens = [1 + 7 * i % 61 for i in range(n - 1)] + [450]
+    check(workload(3, 128, 256, dtype, lens, [i % every == 0 for i in range(n)]), f"{n} requests, one in {every} hidden-cached")
+
+
 def test_requests_without_tables_are_left_out():
     lens = [40, 17, 900, 1, 129, 64, 33, 200]
     w = workload(4, 128, 512, F, lens, [True, False] * 4, device="cuda")
