@@ -98,6 +98,7 @@ struct Params {
   int group_first;                           // ordinal of the group's first hidden request
   int n_hidden_cap, splits, grid_scores;
   uint32_t unfold_ring;                      // bytes of the unfold kernel's ring
+  int sum_threads;                           // of the sum kernel
   int w_box_rows;                            // rows of a W_v box: 128, fewer when W_v has fewer
   int64_t query_stride;
   float scale_log2;
@@ -952,7 +953,7 @@ softmax_kernel(const Params p) {
 // an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
 // K-major B operand).  The rows of a CTA's first stages are requested while the softmax kernel is still running: what a
 // kernel may read before chain_wait() is what was complete when the one before it called chain_next(), here all up
-// to the scores.  Warps: 0 copies, 1 MMA issue, 2-5 epilogue.
+// to the scores.  Warps: 0 copies, 1 MMA issue, 2-9 epilogue.
 // The tensor cores drop what falls below the accumulator's last place at every instruction, so a sum's error grows with
 // the number of instructions that went into one accumulator (terms x cache blocks).  Where few heads leave the
 // tensor memory for it, the rests have accumulators of their own and the cache blocks' first terms take turns among two
@@ -961,7 +962,14 @@ softmax_kernel(const Params p) {
 // (6.2e-6), bf16 1.15e-5 -> 3.8e-6 (6.1e-6), OPT-1.3B bf16 7.3e-6 -> 2.8e-6 (3.1e-6); OPT-66B tp 8 bf16, three requests,
 // 7.3e-6 -> 2.7e-6 (1.1e-5).  It costs 2 - 3 % of a step of 256 OPT-13B requests (slices of two blocks instead of four), 2 %
 // of 128 OPT-66B tp 8 requests, 1 % of 48 OPT-1.3B requests; 24 long OPT-13B requests gain 1 %.
-constexpr int kSumThreads = 192;
+// Two epilogue warps per quarter of the accumulators' lanes take turns at an item's groups of 16 heads and 128 columns, from six
+// groups on: with one, an item of a short request (300 tokens) takes as long to be split into terms and written as to be read.
+// 64 OPT-13B requests of 340 tokens 77 -> 65 us, 128 of 740 198 -> 191, in bf16 228 -> 217; with fewer groups the second warp
+// costs more than it takes over (52 OPT-66B tp 8 requests, four groups, 170 -> 175; 8 long OPT-13B requests, three, 40 -> 43).
+constexpr int kSumThreads = 320;
+// Where no item of the batch can have six, the kernel is launched without the second ones: their registers keep its CTAs from
+// starting beside the softmax's.
+__host__ __device__ inline int sum_epilogue_warps(int slice, int np) { return slice * np >= 96 ? 8 : 4; }
 
 __host__ __device__ inline uint32_t probs_block_bytes(int terms, int np) { return (uint32_t)terms * np * 32; }
 __host__ __device__ inline int sum_stage_blocks(int terms, int np, int slice) {
@@ -991,10 +999,11 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   // sets of accumulators: n_hi for the first terms, one for the rests (or all terms in one)
   const uint32_t n_hi = 5 * slice * np <= 256 ? 4 : 3 * slice * np <= 256 ? 2 : 1, rest_set = 2 * slice * np <= 256 ? n_hi : 0;
+  const int n_epilogue = sum_epilogue_warps(slice, np);   // the others only wait
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], 4); }
-    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 5); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], n_epilogue); }
+    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 1 + n_epilogue); }
     aux.abort_flag = 0;
     mbar_init_fence();
   }
@@ -1015,7 +1024,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   int ahead = 0;           // stages of the first item whose rows are requested before the wait
   bool waited = warp != 0;
   if (waited) chain_wait();
-  while (ok) {
+  while (ok && warp < 2 + n_epilogue) {
     int item;
     if (warp == 0) {
       item = next;
@@ -1122,46 +1131,46 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       if (ok && elect_one()) tc_commit_cta(smem_u32(&aux.acc_full[buf]));
       __syncwarp();
     } else {
-      const int quarter = warp & 3;
+      const int quarter = warp & 3, turn = (warp - 2) >> 2;
       const float* inv = p.inv_sum + (int64_t)slot * p.heads;
       T* z = static_cast<T*>(p.z);
       if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
       tc_fence_after();
       const uint32_t used = min(n_hi, (uint32_t)n_blk);
-      for (int col = 0; col < n_col; ++col) {
+      const int h_steps = np / 16;
+      for (int it = turn; it < n_col * h_steps; it += n_epilogue / 4) {
+        const int col = it / h_steps, h0 = (it - col * h_steps) * 16;
         const int e = (first + col) * 128 + quarter * 32 + lane;
-        for (int h0 = 0; h0 < np; h0 += 16) {
-          uint32_t v[16];
-          const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0;
-          tmem_ld16(at, v);
-          uint32_t more[3][16], rest[16];
+        uint32_t v[16];
+        const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0;
+        tmem_ld16(at, v);
+        uint32_t more[3][16], rest[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 3; ++i)
+          if (i + 1 < used) tmem_ld16(at + (i + 1) * slice * np, more[i]);
+        if (rest_set != 0) tmem_ld16(at + rest_set * slice * np, rest);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          float x = __uint_as_float(v[j]);
 #pragma unroll
           for (uint32_t i = 0; i < 3; ++i)
-            if (i + 1 < used) tmem_ld16(at + (i + 1) * slice * np, more[i]);
-          if (rest_set != 0) tmem_ld16(at + rest_set * slice * np, rest);
-          tmem_ld_wait();
+            if (i + 1 < used) x += __uint_as_float(more[i][j]);
+          if (rest_set != 0) x += __uint_as_float(rest[j]);
+          v[j] = __float_as_uint(x);
+        }
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float x = __uint_as_float(v[j]);
+        for (int j = 0; j < 16; j += 2) {
+          float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
+          const int h = h0 + j + (lane & 1);
+          if (h < p.heads) {
+            const float w = inv[h];
+            T a[NT], b[NT];
+            split_terms<T, true>(f.x * w, a);
+            split_terms<T, true>(f.y * w, b);
 #pragma unroll
-            for (uint32_t i = 0; i < 3; ++i)
-              if (i + 1 < used) x += __uint_as_float(more[i][j]);
-            if (rest_set != 0) x += __uint_as_float(rest[j]);
-            v[j] = __float_as_uint(x);
-          }
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            float2 f = pair_rows(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), lane);
-            const int h = h0 + j + (lane & 1);
-            if (h < p.heads) {
-              const float w = inv[h];
-              T a[NT], b[NT];
-              split_terms<T, true>(f.x * w, a);
-              split_terms<T, true>(f.y * w, b);
-#pragma unroll
-              for (int t = 0; t < NT; ++t)
-                *reinterpret_cast<uint32_t*>(z + (((int64_t)t * p.heads + h) * p.n_cap + slot) * p.hidden + (e & ~1)) = pack_pair<T>(a[t], b[t]);
-            }
+            for (int t = 0; t < NT; ++t)
+              *reinterpret_cast<uint32_t*>(z + (((int64_t)t * p.heads + h) * p.n_cap + slot) * p.hidden + (e & ~1)) = pack_pair<T>(a[t], b[t]);
           }
         }
       }
@@ -1417,7 +1426,7 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCa
     static bool done[64] = {false};
     auto k = sum_kernel<T>;
     if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
-    if ((st = launch_chained("sum_kernel", k, sm_count(), kSumThreads, ring, stream, m.x_sum, p)) != APS_OK) return st;
+    if ((st = launch_chained("sum_kernel", k, sm_count(), p.sum_threads, ring, stream, m.x_sum, p)) != APS_OK) return st;
   }
   {
     static bool done[64] = {false};
@@ -1535,7 +1544,7 @@ int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaS
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_threads = 64 + 32 * sum_epilogue_warps(pa.max_slice, l.np); p.grid_scores = pa.grid_scores;
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);
