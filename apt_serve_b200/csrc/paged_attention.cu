@@ -179,6 +179,11 @@ struct KvCfg {
   static_assert(LPR >= 1 && LPR <= 32 && (LPR & (LPR - 1)) == 0, "unsupported head size");
 };
 
+// A batch of few units (a quarter of the warps could take them all) is a chain of a unit's round trips, eight groups one after
+// the other: four warps then share a unit, each a quarter of its tokens, and merge their partials in shared
+// memory, in token order (8 OPT-125M requests in fp32, half of them K/V-cached, 15.2 -> 7.0 us).
+constexpr int kKvShare = 4;
+
 template <typename T, int D>
 __global__ void __launch_bounds__(kKvWarps * 32, 2)
 kv_attention_kernel(int* plan, const int* part_offset,
@@ -190,28 +195,34 @@ kv_attention_kernel(int* plan, const int* part_offset,
                     int64_t block_stride, float scale_log2) {
   using C = KvCfg<T, D>;
   __shared__ int s_base;
+  __shared__ __align__(16) float s_acc[kKvWarps][D];
+  __shared__ float2 s_ml[kKvWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % C::LPR, tsel = lane / C::LPR;
   chain_wait();
   chain_next();
   const int total = plan[kPlanNumKvChunks] * heads;
   const int64_t row_stride = (int64_t)heads * D;
+  const int share = total * kKvShare <= (int)gridDim.x * kKvWarps ? kKvShare : 1;   // warps per unit
 
   while (true) {
-    if (threadIdx.x == 0) s_base = atomicAdd(&plan[kPlanKvCounter], (int)(blockDim.x >> 5));
+    if (threadIdx.x == 0) s_base = atomicAdd(&plan[kPlanKvCounter], kKvWarps / share);
     __syncthreads();
     const int base = s_base;
     __syncthreads();
     if (base >= total) break;
-    const int unit = base + warp;
-    if (unit >= total) continue;
+    // past the last unit the warps of a shared one only keep the others company at the barrier
+    const int unit = min(base + warp / share, total - 1);
+    const bool mine = base + warp / share < total;
+    if (!mine && share == 1) continue;
 
     const int2 rc = kv_chunks[unit / heads];
     const int h = unit % heads;
     const int req = rc.x;
     const int seq = min(seq_lens[req], max_blocks_per_seq * block_size);
-    const int tok_begin = rc.y * kChunkTokens;
-    const int tok_end = min(seq, tok_begin + kChunkTokens);
+    const int part = kChunkTokens / share;   // a multiple of C::GT
+    const int tok_begin = rc.y * kChunkTokens + warp % share * part;
+    const int tok_end = min(seq, tok_begin + part);   // a sharing warp may have none
     const int32_t* bt = block_tables + (int64_t)req * max_blocks_per_seq;
 
     float qf[C::EPL];
@@ -242,7 +253,7 @@ kv_attention_kernel(int* plan, const int* part_offset,
       }
     };
 
-    load_group(kreg, key_cache, tok_begin);
+    if (tok_begin < tok_end) load_group(kreg, key_cache, tok_begin);
     for (int tb = tok_begin; tb < tok_end; tb += C::GT) {
       load_group(vreg, value_cache, tb);
       float s[C::NL];
@@ -284,6 +295,28 @@ kv_attention_kernel(int* plan, const int* part_offset,
       l += __shfl_xor_sync(kFull, l, o);
 #pragma unroll
       for (int e = 0; e < C::EPL; ++e) acc[e] += __shfl_xor_sync(kFull, acc[e], o);
+    }
+    if (share > 1) {
+      if (tsel == 0) {
+#pragma unroll
+        for (int e = 0; e < C::EPL; ++e) s_acc[warp][sub * C::EPL + e] = acc[e];
+        if (lane == 0) s_ml[warp] = make_float2(m, l);
+      }
+      __syncthreads();   // the next one before these are written again: s_base
+      if (warp % share != 0 || !mine) continue;
+      float w[kKvShare], top = m;   // the first warp of a unit always has tokens
+#pragma unroll
+      for (int i = 1; i < kKvShare; ++i) top = fmaxf(top, s_ml[warp + i].x);
+      l = 0.f;
+#pragma unroll
+      for (int i = 0; i < kKvShare; ++i) { w[i] = exp2f(s_ml[warp + i].x - top); l = fmaf(w[i], s_ml[warp + i].y, l); }
+#pragma unroll
+      for (int e = 0; e < C::EPL; ++e) {
+        acc[e] = 0.f;
+#pragma unroll
+        for (int i = 0; i < kKvShare; ++i) acc[e] = fmaf(w[i], s_acc[warp + i][sub * C::EPL + e], acc[e]);
+      }
+      m = top;
     }
     const int64_t slot = (int64_t)(part_offset[req] + rc.y) * heads + h;
     if (tsel == 0) {

@@ -3,9 +3,11 @@ against the oracle with the tolerances of test_gpu_folded.py."""
 import pytest
 import torch
 
+from oracle import hybrid_cache_oracle as O
 from apt_serve_b200 import attention as A
 from apt_serve_b200.workloads import LayerShape, make_decode_workload
 
+from helpers import assert_close
 from test_gpu_folded import check
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +84,21 @@ def test_new_rows_are_written(heads, d, e, dtype):
         else:
             planes[0, slot], planes[1, slot] = w.new_key.reshape(len(lens), -1)[r], w.new_value.reshape(len(lens), -1)[r]
     assert torch.equal(w.hidden_cache, hid) and torch.equal(w.kv_cache, kv)
+
+
+# K/V path: units shared by four warps (CUDA cores, few of them) or not; units from a warp's place, from the counter, and from
+# the counter without a look at the plan's total (long block tables); tolerances of test_gpu_attention.py
+@pytest.mark.parametrize("heads,d,dtype,lens", [
+    (3, 64, torch.float32, [1, 31, 32, 33, 127, 128, 129, 300]), (12, 64, torch.float32, [300] * 20 + [7] * 20),
+    (2, 128, torch.float32, [96, 97, 513]), (2, 256, F, [96, 97, 513]), (2, 32, B, [33, 640]),
+    (5, 64, F, [1, 90, 128, 129]), (40, 128, F, [130] * 40), (40, 64, B, [40] * 60 + [1300]), (40, 128, F, [40] * 60 + [1300]),
+])
+def test_kv_units(heads, d, dtype, lens):
+    w = make_decode_workload(LayerShape("t", heads, d, heads * d, dtype), lens, [False] * len(lens), seed=len(lens))
+    ref = O.paged_decode_attention(w.query, w.kv_cache[0], w.kv_cache[1], w.meta.block_tables, w.meta.seq_lens_tensor, w.scale)
+    g = w.to("cuda")
+    args = (g.query, g.kv_cache[0], g.kv_cache[1], g.meta.block_tables, g.meta.seq_lens_tensor, g.scale)
+    out = A.paged_decode_attention(*args)
+    assert torch.equal(out, A.paged_decode_attention(*args))
+    tol = 1e-4 if dtype == torch.float32 else 2e-2
+    assert_close(out, ref, f"{len(lens)} requests of {heads} heads", tol, tol)
