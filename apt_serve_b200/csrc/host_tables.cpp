@@ -3,7 +3,8 @@
 // The reference pads them in its model runner (additional_designs/worker/aptserve_model_runner.py:601-609).
 // Nineteen thousand list elements (256 OPT-13B requests) cost numpy 30 ns each; read through the interpreter's own
 // list and integer accessors they cost 3.  With one copy to the device and one allocation for the outputs a
-// call of device_metadata.expand_decode_metadata went from 855 to 218 us.  A library of its own, because this one needs
+// call of device_metadata.expand_decode_metadata went from 855 to 218 us, and with lengths, types and counts read here too and
+// the tensors cut out of their buffers by one call from 222 to 160.  A library of its own, because this one needs
 // the Python process it is loaded into; called with the interpreter lock held (ctypes.PyDLL).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -13,26 +14,30 @@
 
 namespace {
 
+// A plain integer of 32 bits; false for anything else.
+inline bool read_int(PyObject* x, int32_t* out) {
+  if (!PyLong_CheckExact(x)) return false;
+#if PY_VERSION_HEX >= 0x030C0000
+  if (PyUnstable_Long_IsCompact((PyLongObject*)x)) {   // one digit: below 2^30, read without a call
+    *out = (int32_t)PyUnstable_Long_CompactValue((PyLongObject*)x);
+    return true;
+  }
+#endif
+  int overflow = 0;
+  const long v = PyLong_AsLongAndOverflow(x, &overflow);
+  if (overflow != 0 || v < INT32_MIN || v > INT32_MAX) return false;
+  *out = (int32_t)v;
+  return true;
+}
+
 // One row; false for anything but a list or tuple of plain integers of 32 bits that fits the width.
 bool pack_row(PyObject* row, int64_t width, int32_t* out) {
   const bool list = PyList_CheckExact(row);
   if (!list && !PyTuple_CheckExact(row)) return false;
   const Py_ssize_t n = list ? PyList_GET_SIZE(row) : PyTuple_GET_SIZE(row);
   if (n > width) return false;
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* x = list ? PyList_GET_ITEM(row, i) : PyTuple_GET_ITEM(row, i);
-    if (!PyLong_CheckExact(x)) return false;
-#if PY_VERSION_HEX >= 0x030C0000
-    if (PyUnstable_Long_IsCompact((PyLongObject*)x)) {   // one digit: below 2^30, read without a call
-      out[i] = (int32_t)PyUnstable_Long_CompactValue((PyLongObject*)x);
-      continue;
-    }
-#endif
-    int overflow = 0;
-    const long v = PyLong_AsLongAndOverflow(x, &overflow);
-    if (overflow != 0 || v < INT32_MIN || v > INT32_MAX) return false;
-    out[i] = (int32_t)v;
-  }
+  for (Py_ssize_t i = 0; i < n; ++i)
+    if (!read_int(list ? PyList_GET_ITEM(row, i) : PyTuple_GET_ITEM(row, i), out + i)) return false;
   memset(out + n, 0, (size_t)(width - n) * sizeof(int32_t));
   return true;
 }
@@ -59,5 +64,61 @@ extern "C" int aps_pack_block_tables(PyObject* tables, PyObject* shared_tables, 
     }
     memcpy(ref + r * width, use_hidden[r] ? s : p, bytes);
   }
+  return 0;
+}
+
+// What the tables' buffer is sized by, in one pass over the lists: counts = {hidden-cached requests, their tokens, the
+// widest private table, the shortest and the longest length}; the lengths as they are in lens, the types (0 or 1) in types.
+// Returns 0, or 1 for arguments that are not lists: lengths and tables of `batch`, plain integers and booleans.
+extern "C" int aps_measure_decode_batch(PyObject* seq_lens, PyObject* use_hidden, PyObject* tables, int64_t batch,
+                                        int32_t* lens, int32_t* types, int64_t* counts) {
+  if (!PyList_CheckExact(seq_lens) || !PyList_CheckExact(use_hidden) || !PyList_CheckExact(tables) ||
+      PyList_GET_SIZE(seq_lens) != batch || PyList_GET_SIZE(use_hidden) != batch || PyList_GET_SIZE(tables) != batch)
+    return 1;
+  int64_t n_hidden = 0, tokens = 0, width = 0, least = INT32_MAX, most = 0;
+  for (int64_t r = 0; r < batch; ++r) {
+    PyObject *h = PyList_GET_ITEM(use_hidden, r), *t = PyList_GET_ITEM(tables, r);
+    if ((h != Py_True && h != Py_False) || !read_int(PyList_GET_ITEM(seq_lens, r), lens + r)) return 1;
+    const bool list = PyList_CheckExact(t);
+    if (!list && !PyTuple_CheckExact(t)) return 1;
+    const int64_t n = list ? PyList_GET_SIZE(t) : PyTuple_GET_SIZE(t);
+    types[r] = h == Py_True ? 1 : 0;
+    n_hidden += types[r];
+    tokens += types[r] ? lens[r] : 0;
+    if (n > width) width = n;
+    if (lens[r] < least) least = lens[r];
+    if (lens[r] > most) most = lens[r];
+  }
+  counts[0] = n_hidden; counts[1] = tokens; counts[2] = width; counts[3] = least; counts[4] = most;
+  return 0;
+}
+
+// The buffer's sections, each a multiple of 32 words: the K/V-cached rows (int64), the private, shared and the reference's
+// tables, lengths, types.  Returns as aps_pack_block_tables does.
+extern "C" int aps_pack_decode_batch(PyObject* tables, PyObject* shared_tables, const int32_t* lens, const int32_t* types,
+                                     int64_t batch, int64_t width, int64_t n_hidden, int32_t* out) {
+  auto padded = [](int64_t n) { return (n + 31) / 32 * 32; };
+  if (!PyList_CheckExact(tables) || !PyList_CheckExact(shared_tables) || PyList_GET_SIZE(tables) != batch ||
+      PyList_GET_SIZE(shared_tables) != batch)
+    return 1;
+  int64_t* rows = (int64_t*)out;
+  int32_t* priv = out + padded(2 * (batch - n_hidden));
+  int32_t* shared = priv + padded(batch * width);
+  int32_t* ref = shared + padded(batch * width);
+  int32_t* d_lens = ref + padded(batch * width);
+  const size_t bytes = (size_t)width * sizeof(int32_t);
+  for (int64_t r = 0; r < batch; ++r) {
+    int32_t *p = priv + r * width, *s = shared + r * width;
+    if (!pack_row(PyList_GET_ITEM(tables, r), width, p)) return 1;
+    if (types[r]) {
+      if (!pack_row(PyList_GET_ITEM(shared_tables, r), width, s)) return 1;
+    } else {
+      *rows++ = r;
+      memset(s, 0, bytes);
+    }
+    memcpy(ref + r * width, types[r] ? s : p, bytes);
+  }
+  memcpy(d_lens, lens, (size_t)batch * sizeof(int32_t));
+  memcpy(d_lens + padded(batch), types, (size_t)batch * sizeof(int32_t));
   return 0;
 }

@@ -31,8 +31,8 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     the current stream.  The tensors are sections of two allocations (what came from the host, what the kernels wrote)."""
     dev = torch.device(device)
     b = len(seq_lens)
-    lens = [int(s) for s in seq_lens]
-    if b and min(lens) < 1:
+    lens, types, (n_h, n_hid_tok, width, least, most) = _measure(seq_lens, use_hidden, block_tables, b)
+    if b and least < 1:
         # the kernels count a length below 1 as 1; the host counts must agree with them
         raise ValueError("expand_decode_metadata: every sequence length must be >= 1 "
                          "(it includes the token being decoded)")
@@ -41,47 +41,68 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     if dev.type == "cuda" and torch.cuda.is_current_stream_capturing():
         # the graph would read the staging buffer again on every replay, long after it has been given back
         raise RuntimeError("expand_decode_metadata: not during stream capture (the tables come from host memory)")
-    hid = np.asarray(list(use_hidden), dtype=bool)
-    lens_np = np.asarray(lens, dtype=np.int32)
-    n_h = int(np.count_nonzero(hid))
     n_kv = b - n_h
-    n_hid_tok = int(lens_np[hid].sum(dtype=np.int64))
     n_tot = n_hid_tok + n_kv
-    width = max(1, max(map(len, block_tables)))
     # everything the device gets, in one buffer and one copy: the K/V-cached rows, three tables (private, shared, and
     # the reference's: shared for hidden requests, private otherwise), lengths and types; sections of 128 bytes
-    at, words = [], 0
-    for n in (2 * n_kv, b * width, b * width, b * width, b, b):
-        at.append((words, words + n))
-        words += (n + 31) // 32 * 32
-    host = torch.empty(words, dtype=torch.int32, pin_memory=dev.type == "cuda")
-    rows, priv, shared, ref, h_lens, h_type = (host.numpy()[i:j] for i, j in at)
-    pack_tables(block_tables, block_tables_4_shared, hid, priv.reshape(b, width), shared.reshape(b, width),
-                ref.reshape(b, width))
-    rows.view(np.int64)[:] = np.flatnonzero(~hid)
-    h_lens[:] = lens_np
-    h_type[:] = hid
-    d = host.to(dev, non_blocking=True)
-    rows, priv, shared, ref, d_lens, d_type = (d[i:j] for i, j in at)
+    cuts = _cuts((2 * n_kv, b * width, b * width, b * width, b, b), 32)
+    host = torch.empty(sum(cuts), dtype=torch.int32, pin_memory=dev.type == "cuda")
+    _fill_host(host, cuts, block_tables, block_tables_4_shared, lens, types, width, n_h)
+    rows, priv, shared, ref, d_lens, d_type = host.to(dev, non_blocking=True).split(cuts)[::2]
     priv, shared, ref = priv.view(b, width), shared.view(b, width), ref.view(b, width)
     # the eight index tensors and the kernels' scratch, again sections of one buffer
-    n_scratch = (N.lib().aps_decode_metadata_scratch_bytes(b) + 7) // 8
-    sizes = (n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h, n_scratch)
-    pitch = [(n + 15) // 16 * 16 for n in sizes]
-    parts = torch.empty(max(1, sum(pitch)), dtype=torch.int64, device=dev)[:sum(pitch)].split(pitch)
-    parts = [t if t.numel() == n else t[:n] for t, n in zip(parts, sizes)]
+    lib = N.lib()
+    cuts = _cuts((n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h, (lib.aps_decode_metadata_scratch_bytes(b) + 7) // 8), 16)
+    parts = torch.empty(sum(cuts), dtype=torch.int64, device=dev).split(cuts)[::2]
     names = ("slot_mapping", "slot_mapping_shared", "hidden_cache_use_tot", "kv_cache_use_tot",
              "hidden_holder_upd", "hidden_holder_pull", "hidden_cache_store_tot", "hidden_cache_use_input")
     with N.on_device(dev):
-        N.check(N.lib().aps_expand_decode_metadata(
+        N.check(lib.aps_expand_decode_metadata(
             N.ptr(priv), N.ptr(shared), N.ptr(d_lens), N.ptr(d_type), b, width, block_size,
             *(t.data_ptr() for t in parts[:8]), n_tot, n_hid_tok, None, N.ptr(parts[8]), parts[8].numel() * 8,
             N.current_stream(dev)))
     return DecodeMetadata(
-        block_tables=ref, seq_lens_tensor=d_lens, seq_lens=lens,
+        block_tables=ref, seq_lens_tensor=d_lens, seq_lens=lens.tolist(),
         num_hidden_cache_tokens=n_h, num_tot_tokens=n_tot, num_decode_tokens=b,
-        max_decode_seq_len=max(lens, default=0), private_block_tables=priv,
+        max_decode_seq_len=most, private_block_tables=priv,
         cache_type=d_type, kv_request_rows=rows.view(torch.int64), **dict(zip(names, parts)))
+
+
+def _cuts(sizes, pitch):
+    """Sizes to split a buffer by: each section and then what pads it to a multiple of ``pitch``."""
+    return [n for size in sizes for n in (size, -size % pitch)]
+
+
+def _measure(seq_lens, use_hidden, tables, b):
+    """Lengths and types as int32 arrays, and (hidden-cached requests, their tokens, the widest table or 1, the shortest length,
+    the longest): natively for plain lists where the host library has been built."""
+    lib = N.host_lib()
+    if lib is not None and b:
+        both = np.empty((2, b), dtype=np.int32)
+        counts = np.empty(5, dtype=np.int64)
+        at = both.ctypes.data
+        if lib.aps_measure_decode_batch(seq_lens, use_hidden, tables, b, at, at + 4 * b, counts.ctypes.data) == 0:
+            n_h, tokens, width, least, most = counts.tolist()
+            return both[0], both[1], (n_h, tokens, max(1, width), least, most)
+    lens = [int(s) for s in seq_lens]
+    least, most = min(lens, default=0), max(lens, default=0)
+    hid = np.asarray(list(use_hidden), dtype=bool)
+    lens = np.asarray(lens, dtype=np.int32)
+    width = max(1, max(map(len, tables))) if len(tables) == b else 1
+    return lens, hid.astype(np.int32), (int(np.count_nonzero(hid)), int(lens[hid].sum(dtype=np.int64)), width, least, most)
+
+
+def _fill_host(host, cuts, tables, shared_tables, lens, types, width, n_hidden):
+    """The sections of the buffer that goes to the device."""
+    lib, b = N.host_lib(), len(lens)
+    if lib is not None and lib.aps_pack_decode_batch(tables, shared_tables, lens.ctypes.data, types.ctypes.data, b, width,
+                                                     n_hidden, host.data_ptr()) == 0:
+        return
+    rows, priv, shared, ref, h_lens, h_type = (t.numpy() for t in host.split(cuts)[::2])
+    pack_tables(tables, shared_tables, types != 0, priv.reshape(b, width), shared.reshape(b, width), ref.reshape(b, width))
+    rows.view(np.int64)[:] = np.flatnonzero(types == 0)
+    h_lens[:] = lens
+    h_type[:] = types
 
 
 def pack_tables(tables, shared_tables, hid, priv, shared, ref):
