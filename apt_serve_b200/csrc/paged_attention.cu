@@ -26,6 +26,8 @@
 #include "attention_common.cuh"
 #include "tensor_maps.cuh"
 
+#include <initializer_list>
+
 namespace aps {
 namespace {
 
@@ -411,7 +413,7 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
-template <typename T, int D, int S>
+template <typename T, int D, int S, bool MANY>
 __global__ void __launch_bounds__(kTmaWarps * 32, (384 / (kTmaWarps * 32)) > 0 ? (384 / (kTmaWarps * 32)) : 1)
 kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         int* plan, const int* part_offset,
@@ -513,8 +515,14 @@ kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     return got;
   };
 
-  Unit cur = load_unit(next_index());
-  Unit nxt = load_unit(next_index());
+  // Few units (two per warp at most): a warp's are known from its place.  The counter costs every warp two round trips to the
+  // same address before its first copies (five OPT-1.3B requests 9.3 -> 7.2 us, none 3.1 -> 1.6); with more units it evens out
+  // the warps' different speeds.  MANY: the block tables are so long that there will be more; without the test the kernel
+  // of a large batch is 1 % faster.
+  const int warps = gridDim.x * kTmaWarps, mine = blockIdx.x * kTmaWarps + warp;
+  const bool few = !MANY && total <= 2 * warps;
+  Unit cur = load_unit(few ? mine : next_index());
+  Unit nxt = load_unit(few ? warps + mine : next_index());
   int issue_in_nxt = 0, issue_g = 0;       // the request cursor: unit (cur / nxt) and group
   uint32_t issued = 0, consumed = 0;       // groups requested / used so far (ring stage = count % S)
   auto refill = [&]() {
@@ -627,7 +635,7 @@ kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     // the next unit becomes the current one; the request cursor keeps its place in it
     cur = nxt;
     if (issue_in_nxt) issue_in_nxt = 0; else issue_g = 0;
-    nxt = load_unit(cur.n_groups > 0 ? next_index() : total);
+    nxt = load_unit(cur.n_groups > 0 && !few ? next_index() : total);
     refill();
   }
   if (!ok) {
@@ -780,23 +788,27 @@ int launch_kv_typed(const WorkspacePtrs& ws, const void* query, const void* key_
     if (s.block_stride == (int64_t)s.block_size * s.heads * D) {
       constexpr int kStages = APS_KV_STAGES;
       constexpr int kSmem = 1024 + kTmaWarps * kStages * (2 * 16 * D * 2);
-      auto kernel = kv_attention_tma_kernel<T, D, kStages>;
+      auto kernel = kv_attention_tma_kernel<T, D, kStages, false>, kernel_many = kv_attention_tma_kernel<T, D, kStages, true>;
       static bool attr_set[64] = {false};
       int dev = 0;
       APS_CUDA(cudaGetDevice(&dev));
       APS_REQUIRE(dev >= 0 && dev < 64, APS_ERR_CUDA, "device index %d out of range", dev);
       if (!attr_set[dev]) {
-        APS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        APS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        for (auto k : {kernel, kernel_many}) {
+          APS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+          APS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        }
         attr_set[dev] = true;
       }
       CUtensorMap mk, mv;
       int st = kv_plane_maps<D>(key_cache, value_cache, s, &mk, &mv);
       if (st != APS_OK) return st;
       ScopedProfile prof(0, stream);
+      const int64_t most = (int64_t)s.batch * s.heads * (((int64_t)s.max_blocks_per_seq * s.block_size + kChunkTokens - 1) / kChunkTokens);
       int per_sm = 0;
       APS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTmaWarps * 32, kSmem));
       APS_REQUIRE(per_sm > 0, APS_ERR_CUDA, "the K/V streaming kernel does not fit on this device");
+      if (most > (int64_t)12 * sm_count() * per_sm * kTmaWarps) kernel = kernel_many;
       return launch_chained("kv_attention_tma_kernel", kernel, sm_count() * per_sm, kTmaWarps * 32, kSmem, stream,
                             mk, mv, ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query,
                             block_tables, seq_lens, s.max_blocks_per_seq, s.heads, s.block_size, s.query_stride, scale_log2);
