@@ -581,10 +581,31 @@ class FlashAttentionMetadata:
                    use_cuda_graph=False)
 
 
+def _prefill_supported(q, k, v, bounds, scale) -> bool:
+    """Whether ``aps_prefill_attention`` takes the packed prompts: 16-bit, head size 64 or 128, rows of back-to-back heads
+    with 16-byte aligned rows."""
+    if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not scale > 0 or bounds is None:
+        return False
+    t, h, d = q.shape
+    return (d in (64, 128) and 0 < t < (1 << 31) - 128 and 0 < h <= 65535 and k.shape == q.shape and v.shape == q.shape
+            and bounds.dtype == torch.int32 and bounds.dim() == 1 and 1 < bounds.shape[0] <= 65536 and bounds.is_contiguous()
+            and all(x.is_cuda and x.get_device() == q.get_device() for x in (q, k, v, bounds))
+            and all(x.dtype == q.dtype and x.stride(2) == 1 and x.stride(1) == d and x.stride(0) % 8 == 0 and x.stride(0) >= h * d
+                    and x.data_ptr() % 16 == 0 for x in (q, k, v)))
+
+
 def _varlen_prefill_attention(q, k, v, seq_start_loc, max_len, scale):
-    """Causal var-len self-attention over packed prompts.  Prefill attention is
-    not one of the rewritten kernels: it stays a library call, as in the
-    reference (flash_attn_varlen_func, aptserve_flash_attn.py:414-426)."""
+    """Causal var-len self-attention over packed prompts (flash_attn_varlen_func in the reference,
+    aptserve_flash_attn.py:414-426): ``aps_prefill_attention`` where it takes the tensors, the library call otherwise."""
+    if _prefill_supported(q, k, v, seq_start_loc, scale):
+        out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+        t, h, d = q.shape
+        with N.on_device(q.device):
+            N.check(N.lib().aps_prefill_attention(
+                out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), seq_start_loc.data_ptr(), seq_start_loc.shape[0] - 1,
+                max_len, t, h, d, q.stride(0), k.stride(0), v.stride(0), h * d, scale, N.DTYPE_ENUM[q.dtype],
+                N.current_stream(q.device)))
+        return out
     try:
         from flash_attn import flash_attn_varlen_func
         if q.dtype in (torch.float16, torch.bfloat16):

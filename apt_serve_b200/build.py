@@ -21,7 +21,8 @@ LIB_PATH = LIB_DIR / "libaptserve_b200.so"
 # reads Python objects: not part of the C-ABI library, and one per interpreter (as in _native.py)
 HOST_LIB_PATH = LIB_DIR / ("libaptserve_b200_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 SOURCES = ["c_api.cu", "cache_ops.cu", "paged_attention.cu", "hybrid_attention.cu", "hidden_simt.cu", "metadata_ops.cu",
-           "tp_comm.cu", "absorbed_attention.cu", "hidden_attention.cu", "hidden_fp32.cu", "decode_step.cu", "tensor_maps.cu"]
+           "tp_comm.cu", "absorbed_attention.cu", "hidden_attention.cu", "hidden_fp32.cu", "decode_step.cu", "tensor_maps.cu",
+           "prefill_attention.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-cudart", "shared"]
 

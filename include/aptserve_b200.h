@@ -196,6 +196,16 @@ int aps_paged_decode_attention(void* out, const void* query, const void* key_cac
                                void* workspace, size_t workspace_bytes, int dtype,
                                void* stream);
 
+/* Causal self-attention of packed prompts (fp16 / bf16, head sizes 64 and 128): out[t] of prompt i for rows
+ * bounds[i] <= t < bounds[i + 1] (device int32, num_prompts + 1 entries), query rows of a prompt attending to its rows up to
+ * their own.  query / key / value: rows of num_heads * head_size elements, strides in elements (multiples of 8), 16-byte
+ * aligned; max_prompt_len: no prompt is longer.  Stands in for flash_attn_varlen_func
+ * (additional_designs/attention/backends/aptserve_flash_attn.py:414-426). */
+int aps_prefill_attention(void* out, const void* query, const void* key, const void* value, const int32_t* bounds,
+                          int num_prompts, int max_prompt_len, int64_t num_tokens, int num_heads, int head_size,
+                          int64_t query_stride, int64_t key_stride, int64_t value_stride, int64_t out_stride,
+                          float scale, int dtype, void* stream);
+
 /*
  * aps_paged_decode_attention for callers that cannot allocate device memory.
  * This one has no counterpart in the reference.  Same arguments and result as

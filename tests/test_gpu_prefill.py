@@ -1,0 +1,82 @@
+"""aps_prefill_attention against causal attention of every prompt in fp64.
+
+Tolerance: the weights and the output are rounded to the inputs' type (u: half a unit of the last place, relative), the sums
+are fp32: |x - y| <= u |y| + u sum_k p_k |v_k|, half of the latter again for the products' and exponentials' own rounding.  fp16
+below its normal range: 2^-25 for the output and for every weight, times the |v_k| of the keys the row sees."""
+import pytest
+import torch
+
+from apt_serve_b200 import attention as A
+
+pytestmark = pytest.mark.gpu
+F, B = torch.float16, torch.bfloat16
+U = {F: 2.0 ** -11, B: 2.0 ** -8}
+
+
+def prompts(lens, heads, d, dtype, seed=0, spread=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    qkv = torch.randn(sum(lens), 3 * heads * d, generator=g, device="cuda").mul_(spread).to(dtype)
+    q, k, v = (t.view(-1, heads, d) for t in qkv.chunk(3, dim=1))   # row strides of the projection
+    bounds = torch.tensor([0] + lens, device="cuda").cumsum(0).to(torch.int32)
+    return q, k, v, bounds
+
+
+def reference(q, k, v, lens, scale):
+    out, size, least = (torch.empty(q.shape, dtype=torch.double, device="cuda") for _ in range(3))
+    a = 0
+    for n in lens:
+        s = torch.einsum("qhd,khd->hqk", q[a:a + n].double(), k[a:a + n].double()) * scale
+        p = torch.softmax(s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), float("-inf")), dim=2)
+        out[a:a + n] = torch.einsum("hqk,khd->qhd", p, v[a:a + n].double())
+        size[a:a + n] = torch.einsum("hqk,khd->qhd", p, v[a:a + n].double().abs())
+        least[a:a + n] = 2.0 ** -25 * (1 + v[a:a + n].double().abs().cumsum(0)) if q.dtype == F else 0.0
+        a += n
+    return out, size, least
+
+
+def attend(q, k, v, bounds, lens, scale):
+    assert A._prefill_supported(q, k, v, bounds, scale), "this size does not take the kernel under test"
+    return A._varlen_prefill_attention(q, k, v, bounds, max(lens), scale)
+
+
+@pytest.mark.parametrize("dtype", [F, B])
+@pytest.mark.parametrize("heads,d,lens,spread", [
+    (2, 128, [1, 127, 128, 129, 255, 256, 257, 2, 640], 1.0), (3, 64, [1, 127, 128, 129, 255, 256, 257, 2, 640], 1.0),
+    (1, 128, [2048], 1.0), (5, 64, [700, 33], 3.0), (2, 128, [300] * 20, 4.0),
+])
+def test_against_fp64(heads, d, lens, spread, dtype):
+    scale = d ** -0.5
+    q, k, v, bounds = prompts(lens, heads, d, dtype, spread=spread)
+    out = attend(q, k, v, bounds, lens, scale)
+    assert torch.equal(out, attend(q, k, v, bounds, lens, scale))
+    ref, size, least = reference(q, k, v, lens, scale)
+    bad = ~((out.double() - ref).abs() <= U[dtype] * (ref.abs() + 1.5 * size) + least)
+    assert not bad.any(), (int(bad.sum()), float(((out.double() - ref).abs() / size).max() / U[dtype]))
+
+
+def test_growing_scores_move_the_maximum():
+    """Scores that grow by more than 2^8 per tile: what has been accumulated is rescaled."""
+    lens, d = [900], 128
+    q, k, v, bounds = prompts(lens, 2, d, F, seed=1)
+    k *= torch.linspace(0.0, 4.0, 900, device="cuda").view(-1, 1, 1).half()
+    q.copy_(k * 0.5 + q * 0.1)
+    out = attend(q, k, v, bounds, lens, d ** -0.5)
+    ref, size, least = reference(q, k, v, lens, d ** -0.5)
+    assert ((out.double() - ref).abs() <= U[F] * (ref.abs() + 1.5 * size) + least).all()
+
+
+def test_prompts_do_not_see_each_other():
+    lens = [130, 40, 7]
+    q, k, v, bounds = prompts(lens, 2, 64, F, seed=2)
+    want = attend(q, k, v, bounds, lens, 0.125)
+    k[170:], v[170:] = float("nan"), float("inf")
+    got = attend(q, k, v, bounds, lens, 0.125)
+    assert torch.equal(got[:170], want[:170]) and torch.isfinite(got[:170]).all()
+
+
+def test_what_it_does_not_take_goes_to_the_library():
+    q, k, v, bounds = prompts([40, 9], 2, 32, F, seed=3)
+    assert not A._prefill_supported(q, k, v, bounds, 0.2)
+    out = A._varlen_prefill_attention(q, k, v, bounds, 40, 0.2)
+    ref, size, least = reference(q, k, v, [40, 9], 0.2)
+    assert ((out.double() - ref).abs() <= U[F] * (ref.abs() + 4 * size) + least).all()
