@@ -788,13 +788,12 @@ int launch_kv_typed(const WorkspacePtrs& ws, const void* query, const void* key_
     if (s.block_stride == (int64_t)s.block_size * s.heads * D) {
       constexpr int kStages = APS_KV_STAGES;
       constexpr int kSmem = 1024 + kTmaWarps * kStages * (2 * 16 * D * 2);
-      auto kernel = kv_attention_tma_kernel<T, D, kStages, false>, kernel_many = kv_attention_tma_kernel<T, D, kStages, true>;
       static bool attr_set[64] = {false};
       int dev = 0;
       APS_CUDA(cudaGetDevice(&dev));
       APS_REQUIRE(dev >= 0 && dev < 64, APS_ERR_CUDA, "device index %d out of range", dev);
       if (!attr_set[dev]) {
-        for (auto k : {kernel, kernel_many}) {
+        for (auto k : {kv_attention_tma_kernel<T, D, kStages, false>, kv_attention_tma_kernel<T, D, kStages, true>}) {
           APS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
           APS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         }
@@ -805,10 +804,11 @@ int launch_kv_typed(const WorkspacePtrs& ws, const void* query, const void* key_
       if (st != APS_OK) return st;
       ScopedProfile prof(0, stream);
       const int64_t most = (int64_t)s.batch * s.heads * (((int64_t)s.max_blocks_per_seq * s.block_size + kChunkTokens - 1) / kChunkTokens);
+      auto kernel = kv_attention_tma_kernel<T, D, kStages, false>;
       int per_sm = 0;
       APS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTmaWarps * 32, kSmem));
       APS_REQUIRE(per_sm > 0, APS_ERR_CUDA, "the K/V streaming kernel does not fit on this device");
-      if (most > (int64_t)12 * sm_count() * per_sm * kTmaWarps) kernel = kernel_many;
+      if (most > (int64_t)12 * sm_count() * per_sm * kTmaWarps) kernel = kv_attention_tma_kernel<T, D, kStages, true>;
       return launch_chained("kv_attention_tma_kernel", kernel, sm_count() * per_sm, kTmaWarps * 32, kSmem, stream,
                             mk, mv, ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query,
                             block_tables, seq_lens, s.max_blocks_per_seq, s.heads, s.block_size, s.query_stride, scale_log2);
