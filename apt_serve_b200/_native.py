@@ -60,6 +60,8 @@ PROTOTYPES = {
     "aps_decode_layer_step": (c_int, [c_void_p] * 15 + [c_int] * 6 + [c_int64] * 9 +
                               [c_float, c_void_p, c_size_t, c_int, c_void_p]),
     "aps_decode_layer_step_workspace_bytes": (c_size_t, [c_int] * 7),
+    "aps_plain_decode_step": (c_int, [c_void_p] * 7 + [c_int64] + [c_void_p] * 2 + [c_int] * 5 + [c_int64] * 5 +
+                              [c_float, c_void_p, c_size_t, c_int, c_void_p]),
     "aps_prefill_attention": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int64, c_int, c_int] + [c_int64] * 4 +
                               [c_float, c_int, c_void_p]),
     "aps_attention_status": (c_int, [c_void_p, c_void_p, c_void_p]),

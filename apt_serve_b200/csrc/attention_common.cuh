@@ -108,6 +108,31 @@ struct AttnShape {
   int dtype;
 };
 
+// New rows of a decode batch that a planning kernel's other CTAs write: a warp per kWriteChunk bytes of a row, four 16-byte
+// vectors per lane.
+constexpr uint32_t kWriteChunk = 2048;
+__device__ __forceinline__ void move_chunk(char* dst, const char* src, uint32_t at, uint32_t bytes, int lane) {
+  uint4 v[kWriteChunk / 512];
+#pragma unroll
+  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
+    const uint32_t o = at + k * 512 + lane * 16;
+    if (o < bytes) v[k] = *reinterpret_cast<const uint4*>(src + o);
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
+    const uint32_t o = at + k * 512 + lane * 16;
+    if (o < bytes) *reinterpret_cast<uint4*>(dst + o) = v[k];
+  }
+}
+
+// K and V rows of tokens into the slots of a paged cache; a negative slot is skipped.  Everything in multiples of 16 bytes.
+struct SlotWrite {
+  const char* key; const char* value; char* key_cache; char* value_cache; const int64_t* slots;
+  int64_t tokens, key_stride_b, value_stride_b, block_stride_b;
+  uint32_t row_bytes;
+  int block_size, chunks;   // chunks per row
+};
+
 // cache_type may be NULL (all requests K/V-cached).  The M tiles of the hidden requests are
 // described in 16-row sub-blocks (hid_subs, 8 per tile).  pack_tiles = false: every request
 // starts a new tile (tile = 128-token chunk, hid_tiles is filled too); pack_tiles = true:
@@ -115,9 +140,10 @@ struct AttnShape {
 // rows of several requests and only the last tile is partly empty.
 // kv_present = false: the call has no K/V cache; K/V-cached requests then get no work and no
 // partials (zero output rows) and the status word is set to kStatusNoKvCache.
+// w: rows that the launch writes besides.
 int launch_plan(const WorkspacePtrs& ws, const int32_t* seq_lens, const int32_t* cache_type,
                 const int32_t* block_tables, int batch, int max_blocks_per_seq, int block_size,
-                bool pack_tiles, bool kv_present, cudaStream_t stream);
+                bool pack_tiles, bool kv_present, cudaStream_t stream, const SlotWrite& w = SlotWrite{});
 
 int launch_kv_attention(const WorkspacePtrs& ws, const void* query, const void* key_cache,
                         const void* value_cache, const int32_t* block_tables,

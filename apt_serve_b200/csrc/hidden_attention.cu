@@ -152,8 +152,6 @@ __device__ __forceinline__ void drain() {
 // type, block, row).  One launch instead of two one after the other, and the fold
 // beside it: a step of one OPT-13B request 70 -> 60 us, of 48 OPT-1.3B requests 118 -> 108, of 8 in fp32 52 -> 45.
 
-constexpr uint32_t kWriteChunk = 2048;   // bytes of a row per warp: four 16-byte vectors per lane
-
 struct StepWrite {
   const char* hidden; const char* key; const char* value; char* key_cache; char* value_cache; char* hidden_cache;
   const int32_t* block_tables; const int32_t* seq_lens; const int32_t* cache_type;
@@ -179,17 +177,7 @@ __device__ __forceinline__ void write_new_rows(const StepWrite& w, int64_t job, 
   const char* src = base + r * (hid ? w.hidden_stride_b : second ? w.value_stride_b : w.key_stride_b);
   char* dst = hid ? w.hidden_cache + (blk * w.block_size + pos % w.block_size) * w.slot_stride_b
                   : (second ? w.value_cache : w.key_cache) + blk * w.block_stride_b + (int64_t)(pos % w.block_size) * bytes;
-  uint4 v[kWriteChunk / 512];
-#pragma unroll
-  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
-    const uint32_t o = at + k * 512 + lane * 16;
-    if (o < bytes) v[k] = *reinterpret_cast<const uint4*>(src + o);
-  }
-#pragma unroll
-  for (uint32_t k = 0; k < kWriteChunk / 512; ++k) {
-    const uint32_t o = at + k * 512 + lane * 16;
-    if (o < bytes) *reinterpret_cast<uint4*>(dst + o) = v[k];
-  }
+  move_chunk(dst, src, at, bytes, lane);
 }
 
 __global__ void __launch_bounds__(kPlanThreads)

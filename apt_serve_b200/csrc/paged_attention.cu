@@ -35,7 +35,22 @@ constexpr int kKvWarps = 8;
 constexpr unsigned kFull = 0xffffffffu;
 
 // ---- planning ------------------------------------------------------------------
-// One CTA.  Thread t handles a contiguous run of requests; two block-wide prefix sums:
+// The rows a K/V-only step adds, beside the plan instead of in a bulk-copy launch before it: at a decode batch's 20 KB a
+// request both are a round trip and a launch, and the planning CTA leaves 147 SMs idle (five OPT-1.3B requests through
+// FlashAttentionImpl.forward 24.3 -> 21.3 us, 128 OPT-13B requests 347 -> 345).
+// Row 2 t is the K row of token t, row 2 t + 1 its V row.
+__device__ __forceinline__ void write_slots(const SlotWrite& w, int64_t job, int lane) {
+  const int64_t row = job / w.chunks, t = row >> 1;
+  if (t >= w.tokens) return;
+  const int64_t slot = w.slots[t];
+  if (slot < 0) return;
+  const int64_t to = slot / w.block_size * w.block_stride_b + slot % w.block_size * w.row_bytes;
+  const bool v = (row & 1) != 0;
+  move_chunk((v ? w.value_cache : w.key_cache) + to, v ? w.value + t * w.value_stride_b : w.key + t * w.key_stride_b,
+             (uint32_t)(job - row * w.chunks) * kWriteChunk, w.row_bytes, lane);
+}
+
+// CTA 0 plans, the others write rows.  Thread t handles a contiguous run of requests; two block-wide prefix sums:
 // first over (K/V chunks, hidden sub-blocks), which fixes where each hidden request's rows
 // sit in the tile list, then over the number of softmax partials each request will leave.
 __global__ void __launch_bounds__(kPlanThreads)
@@ -43,13 +58,17 @@ plan_kernel(int* plan, int* part_offset, int2* kv_chunks,
             int2* hid_tiles, int* first_tile, int2* hid_subs,
             int* hid_rows, const int32_t* seq_lens,
             const int32_t* cache_type, const int32_t* block_tables, int batch,
-            int max_tokens, int max_blocks, int block_size, int pack_tiles, int kv_present) {
+            int max_tokens, int max_blocks, int block_size, int pack_tiles, int kv_present, const SlotWrite rows) {
   __shared__ int2 sums_a[32], sums_b[32];
   __shared__ int s_kv_missing;
   const int tid = threadIdx.x;
   if (tid == 0) s_kv_missing = 0;
   chain_wait();
   chain_next();
+  if (blockIdx.x > 0) {
+    write_slots(rows, (int64_t)(blockIdx.x - 1) * (kPlanThreads / 32) + (tid >> 5), tid & 31);
+    return;
+  }
   __syncthreads();
   const int per = (batch + kPlanThreads - 1) / kPlanThreads;
   const int r0 = min(batch, tid * per), r1 = min(batch, r0 + per);
@@ -849,11 +868,13 @@ bool kv_attention_supported(int dtype, int head_size) {
 
 int launch_plan(const WorkspacePtrs& ws, const int32_t* seq_lens, const int32_t* cache_type,
                 const int32_t* block_tables, int batch, int max_blocks_per_seq, int block_size,
-                bool pack_tiles, bool kv_present, cudaStream_t stream) {
-  return launch_chained("plan_kernel", plan_kernel, 1, kPlanThreads, 0, stream, ws.plan, ws.part_offset, ws.kv_chunks,
+                bool pack_tiles, bool kv_present, cudaStream_t stream, const SlotWrite& w) {
+  const int64_t jobs = 2 * w.tokens * w.chunks, ctas = 1 + (jobs + kPlanThreads / 32 - 1) / (kPlanThreads / 32);
+  APS_REQUIRE(ctas < (int64_t(1) << 31), APS_ERR_SHAPE, "decode attention: too many rows to write");
+  return launch_chained("plan_kernel", plan_kernel, (unsigned)ctas, kPlanThreads, 0, stream, ws.plan, ws.part_offset, ws.kv_chunks,
                         ws.hid_tiles, ws.first_tile, ws.hid_subs, ws.hid_rows, seq_lens, cache_type, block_tables,
                         batch, max_blocks_per_seq * block_size, max_blocks_per_seq, block_size, pack_tiles ? 1 : 0,
-                        kv_present ? 1 : 0);
+                        kv_present ? 1 : 0, w);
 }
 
 int launch_kv_attention(const WorkspacePtrs& ws, const void* query, const void* key_cache,
@@ -945,6 +966,39 @@ extern "C" int aps_paged_decode_attention(void* out, const void* query, const vo
   const WorkspacePtrs ws = workspace_ptrs(workspace, w);
   cudaStream_t cs = (cudaStream_t)stream;
   if ((st = launch_plan(ws, seq_lens, nullptr, block_tables, batch, max_blocks_per_seq, block_size, false, true, cs)) != APS_OK) return st;
+  if ((st = launch_kv_attention(ws, query, key_cache, value_cache, block_tables, seq_lens, s, cs)) != APS_OK) return st;
+  return launch_combine(ws, out, nullptr, s, cs);
+}
+
+extern "C" int aps_plain_decode_step(void* out, const void* query, const void* key, const void* value, void* key_cache,
+                                     void* value_cache, const int64_t* slot_mapping, int64_t num_slots,
+                                     const int32_t* block_tables, const int32_t* seq_lens, int batch, int max_blocks_per_seq,
+                                     int num_heads, int head_size, int block_size, int64_t query_stride, int64_t key_stride,
+                                     int64_t value_stride, int64_t out_stride, int64_t block_stride, float scale,
+                                     void* workspace, size_t workspace_bytes, int dtype, void* stream) {
+  const int64_t es = dtype_size(dtype), row = (int64_t)num_heads * head_size;
+  auto by_16 = [&](const void* p, int64_t stride) { return aligned_to(p, 16) && stride * es % 16 == 0; };
+  const bool rows = es != 0 && num_slots > 0 && slot_mapping && key && value && key_cache && value_cache && row > 0 && block_size > 0 &&
+                    key_stride >= row && value_stride >= row && block_stride >= row * block_size && row * es % 16 == 0 &&
+                    by_16(key, key_stride) && by_16(value, value_stride) && by_16(key_cache, block_stride) &&
+                    by_16(value_cache, block_stride) && aligned_to(slot_mapping, 8) && batch > 0;
+  int st;
+  if (!rows) {   // what the two calls take, or what they say is wrong with it
+    if ((st = aps_reshape_and_cache(key, value, key_cache, value_cache, slot_mapping, num_slots, num_heads, head_size, block_size,
+                                    key_stride, value_stride, block_stride, dtype, stream)) != APS_OK) return st;
+    return aps_paged_decode_attention(out, query, key_cache, value_cache, block_tables, seq_lens, batch, max_blocks_per_seq, num_heads,
+                                      head_size, block_size, query_stride, out_stride, block_stride, scale, workspace,
+                                      workspace_bytes, dtype, stream);
+  }
+  const AttnShape s{batch, max_blocks_per_seq, num_heads, head_size, block_size, query_stride, out_stride, block_stride, scale, dtype};
+  if ((st = check_attention_args("plain_decode_step", out, query, key_cache, value_cache, block_tables, seq_lens, s, workspace,
+                                 workspace_bytes, true)) != APS_OK) return st;
+  const WorkspacePtrs ws = workspace_ptrs(workspace, workspace_layout(batch, max_blocks_per_seq, block_size, num_heads, head_size));
+  const SlotWrite w{(const char*)key, (const char*)value, (char*)key_cache, (char*)value_cache, slot_mapping, num_slots, key_stride * es,
+                    value_stride * es, block_stride * es, (uint32_t)(row * es), block_size,
+                    (int)((row * es + kWriteChunk - 1) / kWriteChunk)};
+  cudaStream_t cs = (cudaStream_t)stream;
+  if ((st = launch_plan(ws, seq_lens, nullptr, block_tables, batch, max_blocks_per_seq, block_size, false, true, cs, w)) != APS_OK) return st;
   if ((st = launch_kv_attention(ws, query, key_cache, value_cache, block_tables, seq_lens, s, cs)) != APS_OK) return st;
   return launch_combine(ws, out, nullptr, s, cs);
 }

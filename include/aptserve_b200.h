@@ -196,6 +196,16 @@ int aps_paged_decode_attention(void* out, const void* query, const void* key_cac
                                void* workspace, size_t workspace_bytes, int dtype,
                                void* stream);
 
+/* aps_reshape_and_cache followed by aps_paged_decode_attention over the same caches (a decode batch without hidden-cached
+ * requests, aptserve_flash_attn.py:338-345, 449-461), the rows written by the attention's planning launch where everything is
+ * in multiples of 16 bytes.  num_slots: entries of slot_mapping, rows of key and value. */
+int aps_plain_decode_step(void* out, const void* query, const void* key, const void* value, void* key_cache,
+                          void* value_cache, const int64_t* slot_mapping, int64_t num_slots,
+                          const int32_t* block_tables, const int32_t* seq_lens, int batch, int max_blocks_per_seq,
+                          int num_heads, int head_size, int block_size, int64_t query_stride, int64_t key_stride,
+                          int64_t value_stride, int64_t out_stride, int64_t block_stride, float scale,
+                          void* workspace, size_t workspace_bytes, int dtype, void* stream);
+
 /* Causal self-attention of packed prompts (fp16 / bf16, head sizes 64 and 128): out[t] of prompt i for rows
  * bounds[i] <= t < bounds[i + 1] (device int32, num_prompts + 1 entries), query rows of a prompt attending to its rows up to
  * their own.  query / key / value: rows of num_heads * head_size elements, strides in elements (multiples of 8), 16-byte

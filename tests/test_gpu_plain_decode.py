@@ -24,14 +24,18 @@ def forward(impl, w, meta, q, k, v, general, monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("strided", [False, True])
+@pytest.mark.parametrize("strided", ["no", "columns of one projection", "rows of no multiple of 16 bytes", "a slot left out"])
 def test_equals_the_general_path(monkeypatch, dtype, strided):
     w, impl, meta = setup(dtype)
     q, k, v = w.query, w.new_key, w.new_value
     n = q.shape[0]
     q, k, v = q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)
-    if strided:
+    if strided == "columns of one projection":
         q, k, v = torch.cat([q, k, v], dim=1).chunk(3, dim=1)
+    elif strided == "rows of no multiple of 16 bytes":
+        k, v = (torch.nn.functional.pad(t, (0, 1))[:, :-1] for t in (k, v))
+    elif strided == "a slot left out":
+        meta.slot_mapping[2] = -1
     assert impl._plain_decode(q, k, v, w.kv_cache.clone(), meta) is not None
     short, general = (forward(impl, w, meta, q, k, v, g, monkeypatch) for g in (False, True))
     assert torch.equal(short[0], general[0]) and torch.equal(short[1], general[1])
