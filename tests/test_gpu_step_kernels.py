@@ -28,8 +28,9 @@ def test_softmax_units(heads, dtype, lens):
     check(workload(heads, 64, 128, dtype, list(lens), [True] * len(lens)), f"{heads} heads, {len(lens)} requests")
 
 
-# fold: one turn and several turns of 16 requests per epilogue warp, a second chunk of 128; it finds the requests by itself
-@pytest.mark.parametrize("n,every", [(16, 1), (17, 1), (33, 2), (129, 1), (400, 3)])
+# fold: one turn and several turns of 16 requests per epilogue warp, a second chunk of 128; it finds the requests by itself,
+# those past 256 in the plan
+@pytest.mark.parametrize("n,every", [(16, 1), (17, 1), (33, 2), (129, 1), (400, 3), (450, 1), (600, 2)])
 @pytest.mark.parametrize("dtype", [F, B])
 def test_fold_finds_its_requests(n, every, dtype):
     lens = [1 + 7 * i % 61 for i in range(n - 1)] + [450]
