@@ -813,7 +813,7 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
   constexpr int NT = kTerms<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const GroupPlan* gp = p.plan;
-  const int units_of = (p.heads + PER - 1) / PER, n_units = gp->n * units_of;
+  const int units_of = (p.heads + PER - 1) / PER, n_units = gp->n * units_of, n_pieces = gp->levels * gp->per_level;
   T* probs = static_cast<T*>(p.probs);
   for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
     const int slot = unit / units_of, h = (unit - slot * units_of) * PER;
@@ -825,7 +825,7 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
     const int n_blk = (len + 15) / 16, blk0 = gp->blk_off[slot];
     // scores of this lane's eight tokens of tile k
     auto load = [&](int k, float (&s)[PER][8]) {
-      const int2 c = p.tile_pieces[tile0 + k];   // the first and the last piece with a part of the tile
+      const int2 c = clamp_pieces(p.tile_pieces[tile0 + k], n_pieces);   // the first and the last piece with a part of the tile
 #pragma unroll
       for (int i = 0; i < PER; ++i)
 #pragma unroll
@@ -1442,6 +1442,18 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCa
 }
 
 }  // namespace
+}  // namespace aps
+
+extern "C" int aps_selftest_tile_pieces(int first, int last, int num_pieces, int* pieces_out) {
+  APS_REQUIRE(num_pieces > 0 && num_pieces <= aps::kMaxPieces, APS_ERR_SHAPE, "selftest_tile_pieces: no such number of pieces");
+  APS_REQUIRE(pieces_out != nullptr, APS_ERR_NULL_POINTER, "selftest_tile_pieces: null pointer");
+  const int2 c = aps::clamp_pieces(make_int2(first, last), num_pieces);
+  pieces_out[0] = c.x;
+  pieces_out[1] = c.y;
+  return APS_OK;
+}
+
+namespace aps {
 
 // plan may be NULL: the new-token writes alone.
 int launch_step_plan(const PlanArgs* plan, const NewTokenWrite& n, cudaStream_t stream) {

@@ -28,6 +28,16 @@ struct GroupPlan {
   int bound_step[kMaxPieces + 1];
 };
 
+// The pieces [x, y] that left partial sums of a scores tile, as the scores kernel noted them, kept within those there are.  When
+// one of that kernel's waits has run out, the entries of the tiles it did not reach are what the scratch held before: the
+// output is then NaN by the status word, but the softmax in between must not follow them out of the scratch.
+__host__ __device__ inline int2 clamp_pieces(int2 c, int n_pieces) {
+  const int last = n_pieces - 1;
+  c.x = c.x < 0 ? 0 : c.x > last ? last : c.x;
+  c.y = c.y < 0 ? 0 : c.y > last ? last : c.y;
+  return c;
+}
+
 struct PlanArgs {
   int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
   const int32_t* seq_lens; const int32_t* cache_type;

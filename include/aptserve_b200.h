@@ -388,6 +388,12 @@ int aps_selftest_bounded_wait(void* workspace, size_t workspace_bytes, long long
                               int head_size, int block_size, int64_t out_stride, int dtype,
                               void* stream);
 
+/*
+ * Test aid, host only (no counterpart in the reference): the pieces of the scores work that the softmax of the directly
+ * attended rows reads for a tile whose entry in the scratch holds (first, last), with num_pieces pieces in all.
+ */
+int aps_selftest_tile_pieces(int first, int last, int num_pieces, int* pieces_out);
+
 /* ------------------------------------------------------------------------ */
 /* Index tensors                                                             */
 /* ------------------------------------------------------------------------ */

@@ -100,6 +100,28 @@ def test_status_and_cycle_readers_check_their_pointers():
     assert lib.aps_reprojection_cycles(ctypes.addressof(buf), 0, 0) == N.APS_ERR_NULL_POINTER
 
 
+def test_tile_pieces_stay_within_those_there_are():
+    """The softmax of the directly attended rows reads which pieces left a part of a tile from scratch that a scores kernel
+    whose wait ran out has not written: whatever is there, it stays inside the partial scores and ends."""
+    lib, out = N.lib(), (ctypes.c_int * 2)()
+    ints = [-2 ** 31, -2 ** 31 + 1, -1, 0, 1, 2, 146, 147, 148, 739, 740, 959, 960, 2 ** 30, 2 ** 31 - 1]
+    for n in (1, 2, 148, 740, 960):
+        for first in ints:
+            for last in ints:
+                assert lib.aps_selftest_tile_pieces(first, last, n, ctypes.addressof(out)) == N.APS_OK
+                assert 0 <= out[0] < n and 0 <= out[1] < n
+                if 0 <= first < n:
+                    assert out[0] == first
+                if 0 <= last < n:
+                    assert out[1] == last
+    assert lib.aps_selftest_tile_pieces(0, 0, 0, ctypes.addressof(out)) == N.APS_ERR_SHAPE
+    # and the kernel has no other way to them
+    text = (HEADER.parents[1] / "apt_serve_b200" / "csrc" / "hidden_attention.cu").read_text()
+    uses = [m.group(0) for m in re.finditer(r"[^\n]*\btile_pieces\[[^\n]*", text)]
+    reads = [u for u in uses if not re.search(r"tile_pieces\[t\]\.[xy] = piece;", u)]
+    assert len(uses) == 3 and len(reads) == 1 and "clamp_pieces(p.tile_pieces[" in reads[0]
+
+
 def test_python_shims_refuse_cpu_tensors_and_map_errors():
     from apt_serve_b200 import mixed_cache_ops, ops
     z = torch.zeros(2, 8)
