@@ -780,6 +780,9 @@ class FlashAttentionImpl:
                 or lens.dtype != torch.int32 or query.stride(1) != 1 or key.stride(1) != 1 or value.stride(1) != 1
                 or not (slots.is_contiguous() and tables.is_contiguous() and lens.is_contiguous())):
             return None
+        if n == 1 and not query.stride(0) == key.stride(0) == value.stride(0) == width:
+            # a single row has the first stride of whatever it was cut from; the views would give it a row's
+            query, key, value = (t.as_strided(shape, (width, 1)) for t in (query, key, value))
         out = torch.empty_like(query)
         if out.stride(1) != 1:
             return None

@@ -42,6 +42,16 @@ def test_equals_the_general_path(monkeypatch, dtype, strided):
     assert short[0].shape == general[0].shape and short[0].stride() == general[0].stride()
 
 
+@pytest.mark.parametrize("pitch", [4 * 64, 4 * 64 + 1, 1, 0])
+def test_a_single_row_of_any_stride(monkeypatch, pitch):
+    w, impl, meta = setup(lens=(40,))
+    q, k, v = (t.reshape(-1).as_strided((1, 4 * 64), (pitch, 1)) for t in (w.query, w.new_key, w.new_value))
+    assert impl._plain_decode(q, k, v, w.kv_cache.clone(), meta) is not None
+    short, general = (forward(impl, w, meta, q, k, v, g, monkeypatch) for g in (False, True))
+    assert torch.equal(short[0], general[0]) and torch.equal(short[1], general[1])
+    assert short[0].stride() == general[0].stride()
+
+
 @pytest.mark.parametrize("what", ["slots", "dtype", "rows", "lengths"])
 def test_refuses_what_the_general_path_refuses(monkeypatch, what):
     w, impl, meta = setup()
