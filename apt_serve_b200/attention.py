@@ -581,10 +581,23 @@ class FlashAttentionMetadata:
                    use_cuda_graph=False)
 
 
+def _only_values(*tensors) -> bool:
+    """Whether a call wants nothing of the tensors but their values: no graph for a backward pass, no tangents, trace, batching
+    or other transform, no fake tensors or modes that watch the operators.  A native call would leave all of these out in
+    silence, the library call is an operator that torch knows."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing()
+                or any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter for t in tensors)
+                or (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
+                or torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch._C._len_torch_dispatch_stack() > 0)
+
+
 def _prefill_supported(q, k, v, bounds, scale) -> bool:
     """Whether ``aps_prefill_attention`` takes the packed prompts: 16-bit, head size 64 or 128, rows of back-to-back heads
-    with 16-byte aligned rows."""
-    if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not scale > 0 or bounds is None:
+    with 16-byte aligned rows, of which nothing but the values is wanted."""
+    if bounds is None or not _only_values(q, k, v, bounds):
+        return False
+    if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not scale > 0:
         return False
     t, h, d = q.shape
     return (d in (64, 128) and 0 < t < (1 << 31) - 128 and 0 < h <= 65535 and k.shape == q.shape and v.shape == q.shape

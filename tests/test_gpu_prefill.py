@@ -80,3 +80,25 @@ def test_what_it_does_not_take_goes_to_the_library():
     out = A._varlen_prefill_attention(q, k, v, bounds, 40, 0.2)
     ref, size, least = reference(q, k, v, [40, 9], 0.2)
     assert ((out.double() - ref).abs() <= U[F] * (ref.abs() + 4 * size) + least).all()
+
+
+def test_gradients_flow_where_they_are_wanted():
+    lens = [70, 33]
+    q, k, v, bounds = prompts(lens, 2, 64, B, seed=6)
+    plain = attend(q, k, v, bounds, lens, 0.125)
+    assert not plain.requires_grad
+    q, k, v = (t.detach().clone().requires_grad_() for t in (q, k, v))
+    out = A._varlen_prefill_attention(q, k, v, bounds, max(lens), 0.125)
+    g = torch.randn(out.shape, generator=torch.Generator(device="cuda").manual_seed(7), device="cuda").to(B)
+    got = torch.autograd.grad(out, (q, k, v), g)
+    qd, kd, vd = (t.detach().double().requires_grad_() for t in (q, k, v))
+    rows = []
+    for a, n in ((0, 70), (70, 33)):
+        s = torch.einsum("qhd,khd->hqk", qd[a:a + n], kd[a:a + n]) * 0.125
+        p = torch.softmax(s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), float("-inf")), dim=2)
+        rows.append(torch.einsum("hqk,khd->qhd", p, vd[a:a + n]))
+    want = torch.autograd.grad(torch.cat(rows), (qd, kd, vd), g.double())
+    for x, y in zip(got, want):   # sums of products of factors rounded to bf16: a few units of 2^-8 in the 2-norm
+        assert float((x.double() - y).norm() / y.norm()) < 4 * U[B]
+    with torch.no_grad():
+        assert torch.equal(A._varlen_prefill_attention(q, k, v, bounds, max(lens), 0.125), plain)
