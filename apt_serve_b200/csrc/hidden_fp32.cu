@@ -167,8 +167,9 @@ attend32_kernel(const Params p) {
     for (int t = lane; t < n; t += 32) m = fmaxf(m, s_p[t][warp]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float ref = m == -INFINITY ? 0.f : m;   // scores of -infinity alone: no weights, the other chunks have them
     for (int t = lane; t < n; t += 32) {
-      const float w = exp2f(s_p[t][warp] - m);
+      const float w = exp2f(s_p[t][warp] - ref);
       s_p[t][warp] = w;
       l += w;
     }

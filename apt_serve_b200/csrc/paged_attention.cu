@@ -295,14 +295,16 @@ kv_attention_kernel(int* plan, const int* part_offset,
       for (int i = 1; i < C::NL; ++i) gm = fmaxf(gm, s[i]);
 #pragma unroll
       for (int o = C::LPR; o < 32; o <<= 1) gm = fmaxf(gm, __shfl_xor_sync(kFull, gm, o));
-      const float m_new = fmaxf(m, gm);  // finite: every group holds at least one valid token
-      const float corr = exp2f(m - m_new);
+      const float m_new = fmaxf(m, gm);
+      // scores of -infinity alone so far: nothing has a weight yet (a warp that shares a unit begins anywhere in it)
+      const float ref = m_new == -INFINITY ? 0.f : m_new;
+      const float corr = exp2f(m - ref);
       l *= corr;
 #pragma unroll
       for (int e = 0; e < C::EPL; ++e) acc[e] *= corr;
 #pragma unroll
       for (int i = 0; i < C::NL; ++i) {
-        const float p = exp2f(s[i] - m_new);
+        const float p = exp2f(s[i] - ref);
         l += p;
         float vf[C::EPL];
         Vec16<T>::unpack(vreg[i], vf);
@@ -329,8 +331,9 @@ kv_attention_kernel(int* plan, const int* part_offset,
 #pragma unroll
       for (int i = 1; i < kKvShare; ++i) top = fmaxf(top, s_ml[warp + i].x);
       l = 0.f;
+      const float ref = top == -INFINITY ? 0.f : top;
 #pragma unroll
-      for (int i = 0; i < kKvShare; ++i) { w[i] = exp2f(s_ml[warp + i].x - top); l = fmaf(w[i], s_ml[warp + i].y, l); }
+      for (int i = 0; i < kKvShare; ++i) { w[i] = exp2f(s_ml[warp + i].x - ref); l = fmaf(w[i], s_ml[warp + i].y, l); }
 #pragma unroll
       for (int e = 0; e < C::EPL; ++e) {
         acc[e] = 0.f;

@@ -103,3 +103,52 @@ def test_kv_units(heads, d, dtype, lens):
     assert torch.equal(out, A.paged_decode_attention(*args))
     tol = 1e-4 if dtype == torch.float32 else 2e-2
     assert_close(out, ref, f"{len(lens)} requests of {heads} heads", tol, tol)
+
+
+# scores of -infinity: such tokens have no weight, wherever the work of a request is cut (fp32: four warps per K/V unit, a quarter
+# of its 128 tokens each; chunks of 32 cached rows); tolerances of test_gpu_attention.py
+@pytest.mark.parametrize("first,last", [(32, 64), (0, 32), (96, 128), (0, 128), (40, 300)])
+def test_scores_of_minus_infinity(first, last):
+    w = make_decode_workload(LayerShape("t", 3, 64, 192, torch.float32), [300], [False], seed=4)
+    m, q = w.meta, w.query.view(1, 3, 64)
+    q[..., 0] = 1.0
+    if last == 300:   # all of them
+        first = 0
+    slots = torch.tensor([int(m.block_tables[0][t // 16]) * 16 + t % 16 for t in range(300)])
+    key, value = (w.kv_cache[i].reshape(-1, 3, 64)[slots].double() for i in (0, 1))
+    key[first:last, :, 0] = float("-inf")
+    w.kv_cache[0].view(-1, 3, 64)[slots] = key.float()
+    p = torch.softmax(torch.einsum("hd,thd->ht", q[0].double(), key) * w.scale, dim=1)
+    ref = torch.einsum("ht,thd->hd", p, value).reshape(1, 192)
+    g = w.to("cuda")
+    out = A.paged_decode_attention(g.query, g.kv_cache[0], g.kv_cache[1], g.meta.block_tables, g.meta.seq_lens_tensor, g.scale)
+    if last == 300:
+        assert torch.isnan(out).all() and torch.isnan(ref).all()
+    else:
+        assert_close(out, ref, f"tokens {first} to {last}", 1e-4, 1e-4)
+
+
+@pytest.mark.parametrize("first,last", [(32, 64), (0, 32), (96, 128), (0, 128)])
+def test_scores_of_minus_infinity_of_cached_rows(first, last):
+    e = 64
+    w = make_decode_workload(LayerShape("t", 1, 64, e, torch.float32), [300], [True], seed=4)
+    m, (wk, bk, wv, bv) = w.meta, w.kv_weights()
+    w.query.mul_(100.0)
+    slots = torch.tensor([int(m.private_block_tables[0][t // 16]) * 16 + t % 16 for t in range(300)])
+    x = w.hidden_cache.reshape(-1, e)[slots]
+    qt = wk.double().t() @ w.query[0].double() * w.scale   # scores are x . qt
+    col = int(qt.abs().argmax())
+    x[first:last] = 0.0
+    x[first:last, col] = -3e38 * float(qt[col].sign())
+    w.hidden_cache.view(-1, e)[slots] = x
+    x = x.double()
+    assert float(qt[col].abs()) > 1.2   # the product is out of fp32's range
+    s = x @ qt
+    s[first:last] = float("-inf")
+    p = torch.softmax(s, dim=0)
+    ref = (p @ torch.where(p[:, None] > 0, x, torch.zeros_like(x))) @ wv.double().t() + (0 if bv is None else bv.double())
+    g = w.to("cuda")
+    wk, bk, wv, bv = g.kv_weights()
+    out = A.hybrid_decode_attention(g.query, g.kv_cache, g.hidden_cache, wk, bk, wv, bv, g.meta.private_block_tables,
+                                    g.meta.seq_lens_tensor, g.meta.cache_type, g.scale)
+    assert_close(out, ref[None], f"tokens {first} to {last}", 1e-4, 1e-4)
