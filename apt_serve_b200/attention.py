@@ -162,6 +162,8 @@ def paged_decode_attention(query: torch.Tensor, key_cache: torch.Tensor,
         raise RuntimeError("paged_decode_attention: cache block strides differ")
     bt = _i32(block_tables, "block_tables")
     sl = _i32(seq_lens, "seq_lens")
+    if bt.shape[0] < b or sl.shape[0] < b:
+        raise RuntimeError(f"paged_decode_attention: {bt.shape[0]} block tables and {sl.shape[0]} lengths for {b} requests")
     if workspace is None:
         workspace = attention_workspace(dev, b, bt.shape[1], bs, h, d)
     with N.on_device(dev):
@@ -783,10 +785,12 @@ class FlashAttentionImpl:
         n, width = m.num_decode_tokens, self.num_heads * self.head_size
         if (n == 0 or m.num_prefills != 0 or self.kv_cache_dtype != "auto" or not isinstance(kv_cache, torch.Tensor)
                 or not isinstance(tables, torch.Tensor) or not isinstance(lens, torch.Tensor) or not isinstance(slots, torch.Tensor)
-                or kv_cache.dim() != 5 or kv_cache.shape[0] < 2 or tables.dim() != 2):
+                or kv_cache.dim() != 5 or kv_cache.shape[0] < 2 or tables.dim() != 2 or slots.dim() != 1):
             return None
-        shape, dtype = (n, width), query.dtype
-        _, _, bs, h, d = kv_cache.shape
+        shape, dtype, n_slots = (n, width), query.dtype, slots.numel()
+        (_, _, bs, h, d), (n_tables, max_blocks) = kv_cache.shape, tables.shape
+        if n_tables < n or lens.numel() < n:
+            return None
         if (query.shape != shape or key.shape != shape or value.shape != shape or h != self.num_heads or d != self.head_size
                 or key.dtype != kv_cache.dtype or value.dtype != key.dtype or dtype != key.dtype
                 or dtype not in N.DTYPE_ENUM or slots.dtype != torch.int64 or tables.dtype != torch.int32
@@ -800,13 +804,13 @@ class FlashAttentionImpl:
         if out.stride(1) != 1:
             return None
         dev = N.require_cuda(query, key, value, kv_cache, slots, tables, lens)
-        lib, max_blocks, block_stride = N.lib(), tables.shape[1], kv_cache.stride(1)
+        lib, block_stride = N.lib(), kv_cache.stride(1)
         kc, vc = _plane_pointers(kv_cache)
         with N.on_device(dev):
             stream = N.current_stream(dev)
             ws, ws_bytes = _scratch_of(dev, lib.aps_attention_workspace_bytes(n, max_blocks, bs, h, d))
             N.check(lib.aps_plain_decode_step(
-                out.data_ptr(), query.data_ptr(), key.data_ptr(), value.data_ptr(), kc, vc, slots.data_ptr(), slots.shape[0],
+                out.data_ptr(), query.data_ptr(), key.data_ptr(), value.data_ptr(), kc, vc, slots.data_ptr(), n_slots if n_slots < n else n,
                 tables.data_ptr(), lens.data_ptr(), n, max_blocks, h, d, bs, query.stride(0), key.stride(0), value.stride(0),
                 out.stride(0), block_stride, self.scale, ws.data_ptr(), ws_bytes, N.DTYPE_ENUM[dtype], stream))
         return out

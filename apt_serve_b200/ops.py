@@ -15,7 +15,8 @@ def reshape_and_cache_flash(key: torch.Tensor, value: torch.Tensor, key_cache: t
                             value_cache: torch.Tensor, slot_mapping: torch.Tensor,
                             kv_cache_dtype: str = "auto") -> None:
     """``key_cache[slot // BS, slot % BS] = key[t]`` (and value) for ``slot >= 0``.
-    ``key`` / ``value``: ``[T, H, D]``; caches ``[NB, BS, H, D]``."""
+    ``key`` / ``value``: ``[T, H, D]``; caches ``[NB, BS, H, D]``.  Slots past the last row (a padded mapping) have
+    nothing to store, rows past the last slot nowhere to go."""
     if kv_cache_dtype != "auto":  # aptserve_flash_attn.py:311-312: no FP8 cache here
         raise ValueError(f"kv_cache_dtype {kv_cache_dtype!r} is not supported")
     dev = N.require_cuda(key, value, key_cache, value_cache, slot_mapping)
@@ -30,7 +31,7 @@ def reshape_and_cache_flash(key: torch.Tensor, value: torch.Tensor, key_cache: t
     with N.on_device(dev):
         N.check(N.lib().aps_reshape_and_cache(
             N.ptr(key), N.ptr(value), N.ptr(key_cache), N.ptr(value_cache),
-            N.ptr(slot_mapping.contiguous()), slot_mapping.size(0), key.size(1), key.size(2),
+            N.ptr(slot_mapping.contiguous()), min(slot_mapping.size(0), key.size(0), value.size(0)), key.size(1), key.size(2),
             key_cache.size(1), key.stride(0), value.stride(0), key_cache.stride(0),
             N.dtype_enum(key), N.current_stream(dev)))
 

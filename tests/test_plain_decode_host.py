@@ -70,3 +70,34 @@ def test_a_single_row_has_the_stride_of_a_row(lib, kind):
     assert name == "aps_plain_decode_step"
     assert a[15:19] == (WIDTH,) * 4   # of query, key, value and output
     assert out.shape == (1, WIDTH) and out.stride() == (WIDTH, 1)
+
+
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("slots", [2, 3, 5])
+def test_no_slot_without_a_row(lib, monkeypatch, general, slots):
+    """A padded slot mapping names rows of key and value that do not exist."""
+    impl, cache = impl_and_cache()
+    if general:
+        monkeypatch.setattr(impl, "_plain_decode", lambda *a: None)
+    meta, (q, k, v) = batch(3, slots=slots)
+    impl.forward(q, k, v, cache, None, meta)
+    name, a = lib.calls[0]
+    assert (name, a[5 + 2 * (not general)]) == (("aps_reshape_and_cache", min(slots, 3)) if general else
+                                                ("aps_plain_decode_step", min(slots, 3)))
+
+
+@pytest.mark.parametrize("what", [dict(table_rows=2), dict(lens=2)])
+def test_tables_and_lengths_of_fewer_requests_are_refused(lib, what):
+    impl, cache = impl_and_cache()
+    meta, (q, k, v) = batch(3, **what)
+    assert impl._plain_decode(q, k, v, cache, meta) is None
+    with pytest.raises(RuntimeError, match="for 3 requests"):
+        impl.forward(q, k, v, cache, None, meta)
+    assert not any("attention" in name or "plain" in name for name, _ in lib.calls)
+
+
+def test_tables_and_lengths_of_more_requests_are_taken(lib):
+    impl, cache = impl_and_cache()
+    meta, (q, k, v) = batch(3, table_rows=5, lens=4)
+    impl.forward(q, k, v, cache, None, meta)
+    assert [name for name, _ in lib.calls] == ["aps_plain_decode_step"]
