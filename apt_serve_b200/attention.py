@@ -596,10 +596,10 @@ def _only_values(*tensors) -> bool:
 
 def _prefill_supported(q, k, v, bounds, scale) -> bool:
     """Whether ``aps_prefill_attention`` takes the packed prompts: 16-bit, head size 64 or 128, rows of back-to-back heads
-    with 16-byte aligned rows, of which nothing but the values is wanted."""
+    with 16-byte aligned rows, of which nothing but the values is wanted, a scale that is positive in fp32."""
     if bounds is None or not _only_values(q, k, v, bounds):
         return False
-    if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not scale > 0:
+    if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not 2.0 ** -126 <= scale < 2.0 ** 127:
         return False
     t, h, d = q.shape
     return (d in (64, 128) and 0 < t < (1 << 31) - 128 and 0 < h <= 65535 and k.shape == q.shape and v.shape == q.shape

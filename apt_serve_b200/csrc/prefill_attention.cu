@@ -311,6 +311,9 @@ extern "C" int aps_prefill_attention(void* out, const void* query, const void* k
               APS_ERR_SHAPE, "prefill_attention: bad sizes");
   if (num_prompts == 0 || max_prompt_len == 0 || num_tokens == 0) return APS_OK;
   APS_REQUIRE(out && query && key && value && bounds, APS_ERR_NULL_POINTER, "prefill_attention: null pointer");
+  // the running maximum is that of the raw scores, and a masked score stays -infinity only times a positive number
+  APS_REQUIRE(scale >= 1.17549435e-38f && scale < 1.70141183e38f, APS_ERR_UNSUPPORTED,
+              "prefill_attention: the scale must be positive and below 2^127 (got %g)", (double)scale);
   const int64_t row = (int64_t)num_heads * head_size;
   APS_REQUIRE(query_stride >= row && key_stride >= row && value_stride >= row && out_stride >= row, APS_ERR_SHAPE,
               "prefill_attention: strides smaller than a row");

@@ -209,7 +209,7 @@ int aps_plain_decode_step(void* out, const void* query, const void* key, const v
 /* Causal self-attention of packed prompts (fp16 / bf16, head sizes 64 and 128): out[t] of prompt i for rows
  * bounds[i] <= t < bounds[i + 1] (device int32, num_prompts + 1 entries), query rows of a prompt attending to its rows up to
  * their own.  query / key / value: rows of num_heads * head_size elements, strides in elements (multiples of 8), 16-byte
- * aligned; max_prompt_len: no prompt is longer.  Stands in for flash_attn_varlen_func
+ * aligned; max_prompt_len: no prompt is longer; scale: positive (not below 2^-126) and below 2^127.  Stands in for flash_attn_varlen_func
  * (additional_designs/attention/backends/aptserve_flash_attn.py:414-426). */
 int aps_prefill_attention(void* out, const void* query, const void* key, const void* value, const int32_t* bounds,
                           int num_prompts, int max_prompt_len, int64_t num_tokens, int num_heads, int head_size,

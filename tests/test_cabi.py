@@ -100,6 +100,16 @@ def test_status_and_cycle_readers_check_their_pointers():
     assert lib.aps_reprojection_cycles(ctypes.addressof(buf), 0, 0) == N.APS_ERR_NULL_POINTER
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.0, -0.125, 1e-40, float("inf"), float("-inf"), float("nan"), 2.0 ** 127])
+def test_prompt_attention_refuses_scales_it_is_wrong_for(scale):
+    lib = N.lib()
+    buf = (ctypes.c_char * 4096)()
+    p16 = (ctypes.addressof(buf) + 15) // 16 * 16
+    call = lambda prompts, s: lib.aps_prefill_attention(p16, p16, p16, p16, p16, prompts, 5, 5, 2, 64, 128, 128, 128, 128, s, 1, 0)
+    assert call(1, scale) == N.APS_ERR_UNSUPPORTED and b"scale" in lib.aps_last_error()
+    assert call(0, scale) == N.APS_OK   # nothing to do
+
+
 def test_tile_pieces_stay_within_those_there_are():
     """The softmax of the directly attended rows reads which pieces left a part of a tile from scratch that a scores kernel
     whose wait ran out has not written: whatever is there, it stays inside the partial scores and ends."""

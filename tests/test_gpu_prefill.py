@@ -102,3 +102,10 @@ def test_gradients_flow_where_they_are_wanted():
         assert float((x.double() - y).norm() / y.norm()) < 4 * U[B]
     with torch.no_grad():
         assert torch.equal(A._varlen_prefill_attention(q, k, v, bounds, max(lens), 0.125), plain)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.125, 1e-40, float("inf"), float("nan")])
+def test_scales_it_is_wrong_for_go_to_the_library(scale):
+    q, k, v, bounds = prompts([40, 9], 2, 64, F, seed=8)
+    assert A._prefill_supported(q, k, v, bounds, 0.125) and not A._prefill_supported(q, k, v, bounds, scale)
+    assert A._varlen_prefill_attention(q, k, v, bounds, 40, scale).shape == q.shape
