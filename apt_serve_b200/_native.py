@@ -69,6 +69,7 @@ PROTOTYPES = {
     "aps_cache_ops_status": (c_int, [c_void_p, c_void_p]),
     "aps_selftest_bounded_wait": (c_int, [c_void_p, c_size_t, ctypes.c_longlong, c_void_p] + [c_int] * 5 +
                                   [c_int64, c_int, c_void_p]),
+    "aps_selftest_prefill_wait": (c_int, [ctypes.c_longlong, c_void_p]),
     "aps_selftest_tile_pieces": (c_int, [c_int, c_int, c_int, c_void_p]),
     "aps_set_profile_events": (c_int, [c_int, c_void_p, c_void_p]),
     "aps_absorbed_hidden_attention": (c_int, [c_void_p] * 9 + [c_int] * 5 + [c_int64, c_int64, c_int, c_void_p]),

@@ -93,8 +93,9 @@ def raise_on_device_status(workspace: Optional[torch.Tensor] = None,
     """Raise ``RuntimeError`` if the last attention call on ``workspace`` (default: the
     per-device workspace of ``device``) left a non-zero status word: 1..7 = a bounded wait
     of the re-projection kernel ran out and the call's output is NaN, 8 = K/V-cached
-    requests in a batch that was given no K/V cache; or if the cache operations on the device
-    left one: a cache write that was not finished, metadata that points outside its tensors.
+    requests in a batch that was given no K/V cache; or if the operations without a workspace left one on the
+    device: a cache write that was not finished, metadata that points outside its tensors, prompt attention
+    that was not finished (rows of NaN).
     Synchronises the current stream, so call it where a synchronisation is cheap (once per engine
     step, beside the sampler's device-to-host copy), not per layer."""
     if workspace is not None:
@@ -111,12 +112,13 @@ def raise_on_device_status(workspace: Optional[torch.Tensor] = None,
     code = cache_ops_status(dev)
     if code != 0:
         what = ("a bounded device-side wait of a cache write ran out; rows are missing in the cache" if code == 1 else
-                "decode metadata pointed outside its tensors; the requests concerned were left out of the step")
+                "decode metadata pointed outside its tensors; the requests concerned were left out of the step" if code == 2 else
+                "a bounded device-side wait of the prompts' attention ran out; the rows concerned were filled with NaN")
         raise RuntimeError(f"aptserve_b200: cache operations status {code}: {what}")
 
 
 def cache_ops_status(device: torch.device) -> int:
-    """Status word of the cache operations on ``device`` (0 = fine; ``aps_cache_ops_status``).  Synchronises the
+    """Status of the operations without a workspace on ``device`` (0 = fine; ``aps_cache_ops_status``).  Synchronises the
     current stream."""
     import ctypes
     host = ctypes.c_int(0)

@@ -199,6 +199,7 @@ struct NewTokenWrite {
   int dtype;
 };
 int read_metadata_status(int* host_status, cudaStream_t stream);   // metadata_ops.cu
+int read_prefill_status(int* host_status, cudaStream_t stream);    // prefill_attention.cu
 
 int check_hybrid_call(const char* op, const HybridCall& c);
 int enqueue_hybrid_attention(const HybridCall& c, cudaStream_t stream);

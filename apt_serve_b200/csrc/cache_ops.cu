@@ -26,7 +26,7 @@
 // third-party reshape_and_cache_flash / copy_blocks in additional_designs/
 // attention/backends/aptserve_flash_attn.py:58-65, 338-385.
 
-#include "attention_common.cuh"   // NewTokenWrite
+#include "attention_common.cuh"   // read_metadata_status, read_prefill_status
 
 #include <initializer_list>
 #include <stdlib.h>
@@ -548,7 +548,9 @@ extern "C" int aps_cache_ops_status(int* host_status, void* stream) {
   APS_CUDA(cudaGetSymbolAddress(&addr, g_copy_status));
   APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   APS_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-  return *host_status != 0 ? APS_OK : read_metadata_status(host_status, (cudaStream_t)stream);
+  if (*host_status != 0) return APS_OK;
+  const int st = read_metadata_status(host_status, (cudaStream_t)stream);
+  return st != APS_OK || *host_status != 0 ? st : read_prefill_status(host_status, (cudaStream_t)stream);
 }
 
 // Block moves between one plane of a GPU cache and one plane of the pinned CPU cache (or

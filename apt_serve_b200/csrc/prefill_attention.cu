@@ -21,8 +21,10 @@
 // With one buffer of S and tiles of 128 keys, where scores, weights and P V are one chain, 93 and 429 us.
 //
 // Warps: 0 copies, 1 MMA issue, 2-5 softmax (a warp's tensor-memory lanes are given by its number modulo four).
-// Every mbarrier wait is bounded by a clock budget; one that runs out leaves the CTA's rows as NaN.
+// Every mbarrier wait is bounded by a clock budget; one that runs out leaves the CTA's rows as NaN and a status that
+// aps_cache_ops_status reports.
 
+#include "attention_common.cuh"   // read_prefill_status
 #include "sm100.cuh"
 #include "tensor_maps.cuh"
 
@@ -34,6 +36,8 @@ namespace {
 constexpr int kThreads = 192, kRows = 128, kKeys = 64;
 constexpr float kSlack = 8.f;   // log2 of how much the maximum may have grown before O is rescaled
 constexpr float kUp = 7.f;      // log2 of what the weights are kept at
+
+__device__ int g_prefill_status = 0;   // a wait has run out since this was read last; the calls have no scratch to hold it
 
 struct Args {
   const int32_t* bounds; void* out;
@@ -120,7 +124,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   volatile int* abort_flag = &aux.abort_flag;
   const int n_tiles = (min(len, row0 + kRows) + kKeys - 1) / kKeys;
   auto wait = [&](uint64_t* bars, int tile, int code) {
-    return mbar_wait_warp(smem_u32(&bars[tile & 1]), (uint32_t)(tile >> 1) & 1u, abort_flag, nullptr, code, lane);
+    return mbar_wait_warp(smem_u32(&bars[tile & 1]), (uint32_t)(tile >> 1) & 1u, abort_flag, &g_prefill_status, code, lane);
   };
   bool ok = true;
   if (warp == 0) {
@@ -157,7 +161,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       __syncwarp();
       return true;
     };
-    ok = mbar_wait_warp(smem_u32(&aux.q_full), 0, abort_flag, nullptr, 3, lane) && scores(0);
+    ok = mbar_wait_warp(smem_u32(&aux.q_full), 0, abort_flag, &g_prefill_status, 3, lane) && scores(0);
     for (int j = 0; j < n_tiles && ok; ++j) {
       const int i = j & 1;
       if ((j + 1 < n_tiles && !scores(j + 1)) || !wait(aux.v_full, j, 3) || !wait(aux.p_full, j, 4)) { ok = false; break; }
@@ -279,6 +283,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   if (warp == 1) { tc_fence_after(); tmem_free(tmem, kCols); }
 }
 
+// A wait on a barrier that nothing arrives on, as the kernel's waits.
+__global__ void prefill_wait_selftest_kernel(long long budget) {
+  __shared__ uint64_t bar;
+  __shared__ int abort_flag;
+  if (threadIdx.x != 0) return;
+  abort_flag = 0;
+  mbar_init(&bar, 1);
+  mbar_init_fence();
+  mbar_wait_addr(smem_u32(&bar), 0, &abort_flag, &g_prefill_status, 1, budget);
+}
+
 template <typename T, int D>
 int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Args& a, int blocks, int heads, int prompts,
            cudaStream_t stream) {
@@ -296,9 +311,29 @@ int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, con
 }
 
 }  // namespace
+
+int read_prefill_status(int* host_status, cudaStream_t stream) {
+  void* addr = nullptr;
+  APS_CUDA(cudaGetSymbolAddress(&addr, g_prefill_status));
+  APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  APS_CUDA(cudaStreamSynchronize(stream));
+  if (*host_status != 0) {
+    *host_status = 3;
+    APS_CUDA(cudaMemsetAsync(addr, 0, sizeof(int), stream));   // reported once
+  }
+  return APS_OK;
+}
+
 }  // namespace aps
 
 using namespace aps;
+
+extern "C" int aps_selftest_prefill_wait(long long budget_cycles, void* stream) {
+  APS_REQUIRE(budget_cycles > 0 && budget_cycles <= 100000000LL, APS_ERR_SHAPE,
+              "selftest_prefill_wait: the budget must be between 1 and 1e8 clock cycles");
+  prefill_wait_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(budget_cycles);
+  return launch_status("prefill_wait_selftest_kernel");
+}
 
 extern "C" int aps_prefill_attention(void* out, const void* query, const void* key, const void* value, const int32_t* bounds,
                                      int num_prompts, int max_prompt_len, int64_t num_tokens, int num_heads, int head_size,

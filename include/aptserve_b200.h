@@ -368,9 +368,10 @@ int aps_attention_status(const void* workspace, int* host_status, void* stream);
 int aps_reprojection_cycles(const void* workspace, unsigned long long* host_cycles, void* stream);
 
 /*
- * Status of the cache operations on the current device: 0, 1 once a bounded wait on a bulk load
- * ran out (the launch then stopped copying), or 2 if aps_derive_private_tables has met an index
- * outside its tensor since the last call that returned 2.  Synchronises `stream`.
+ * Status of the operations without a workspace on the current device: 0, 1 once a bounded wait on a bulk load of a
+ * cache operation ran out (the launch then stopped copying), 2 if aps_derive_private_tables has met an index
+ * outside its tensor since the last call that returned 2, or 3 if a bounded wait of aps_prefill_attention has run out
+ * (up to 128 rows of a head are then NaN) since the last call that returned 3.  Synchronises `stream`.
  */
 int aps_cache_ops_status(int* host_status, void* stream);
 
@@ -387,6 +388,13 @@ int aps_selftest_bounded_wait(void* workspace, size_t workspace_bytes, long long
                               void* out, int batch, int max_blocks_per_seq, int num_heads,
                               int head_size, int block_size, int64_t out_stride, int dtype,
                               void* stream);
+
+/*
+ * Test aid (no counterpart in the reference): one thread waits on an mbarrier that nothing arrives on and gives up after
+ * budget_cycles clock cycles (1 .. 1e8), exactly as the bounded waits of aps_prefill_attention do;
+ * aps_cache_ops_status then reports 3, once.  Nothing hangs or faults and the context stays usable.
+ */
+int aps_selftest_prefill_wait(long long budget_cycles, void* stream);
 
 /*
  * Test aid, host only (no counterpart in the reference): the pieces of the scores work that the softmax of the directly

@@ -96,6 +96,12 @@ def test_status_and_cycle_readers_check_their_pointers():
     host = ctypes.c_ulonglong(0)
     assert lib.aps_reprojection_cycles(0, ctypes.addressof(host), 0) == N.APS_ERR_NULL_POINTER
     assert lib.aps_attention_status(0, ctypes.addressof(host), 0) == N.APS_ERR_NULL_POINTER
+    assert lib.aps_selftest_prefill_wait(0, 0) == N.APS_ERR_SHAPE
+    assert lib.aps_selftest_prefill_wait(10 ** 9, 0) == N.APS_ERR_SHAPE
+    # every wait of the prompts' attention says where it leaves word that it ran out
+    text = (HEADER.parents[1] / "apt_serve_b200" / "csrc" / "prefill_attention.cu").read_text()
+    waits = re.findall(r"mbar_wait\w*\([^;]*;", text)
+    assert len(waits) == 3 and all("&g_prefill_status" in w for w in waits)
     buf = (ctypes.c_char * 512)()
     assert lib.aps_reprojection_cycles(ctypes.addressof(buf), 0, 0) == N.APS_ERR_NULL_POINTER
 

@@ -6,6 +6,7 @@ below its normal range: 2^-25 for the output and for every weight, times the |v_
 import pytest
 import torch
 
+from apt_serve_b200 import _native as N
 from apt_serve_b200 import attention as A
 
 pytestmark = pytest.mark.gpu
@@ -109,3 +110,14 @@ def test_scales_it_is_wrong_for_go_to_the_library(scale):
     q, k, v, bounds = prompts([40, 9], 2, 64, F, seed=8)
     assert A._prefill_supported(q, k, v, bounds, 0.125) and not A._prefill_supported(q, k, v, bounds, scale)
     assert A._varlen_prefill_attention(q, k, v, bounds, 40, scale).shape == q.shape
+
+
+def test_a_wait_that_runs_out_is_reported():
+    A.raise_on_device_status()
+    N.check(N.lib().aps_selftest_prefill_wait(200000, N.current_stream(torch.device("cuda", 0))))
+    with pytest.raises(RuntimeError, match="status 3"):
+        A.raise_on_device_status()
+    A.raise_on_device_status()   # said once
+    q, k, v, bounds = prompts([40], 2, 64, F)
+    attend(q, k, v, bounds, [40], 0.125)
+    A.raise_on_device_status()
