@@ -231,7 +231,7 @@ step_plan_kernel(const PlanArgs a, const StepWrite w, const int plan_ctas) {
     GroupPlan* gp = a.groups + g;
     const int n = max(0, min(kGroup, total.y - g * kGroup));
     if (n == 0) {
-      if (tid == 0) { gp->n = 0; gp->n_tiles = 0; }
+      if (tid == 0) gp->n = 0;
       continue;
     }
     // sort by length, longest first: rank = requests that come before (four threads per request)
@@ -274,14 +274,14 @@ step_plan_kernel(const PlanArgs a, const StepWrite w, const int plan_ctas) {
         const int s = lane * (kGroup / 32) + k;
         if (s > n) break;
         s_toff[s] = to; s_woff[s] = wo;
-        gp->tile_off[s] = to; gp->blk_off[s] = bo; gp->w_off[s] = wo;
+        gp->tile_off[s] = to; gp->blk_off[s] = bo;
         if (s == n) break;
         const int blocks = (s_len[s] + 15) / 16, tiles = (blocks + kSubs - 1) / kSubs;
         to += tiles; bo += blocks; wo += blocks + tiles * kTileCost;
       }
       if (lane == 31 && n == kGroup) {
         s_toff[n] = to; s_woff[n] = wo;
-        gp->tile_off[n] = to; gp->blk_off[n] = bo; gp->w_off[n] = wo;
+        gp->tile_off[n] = to; gp->blk_off[n] = bo;
       }
     }
     __syncthreads();
@@ -295,7 +295,7 @@ step_plan_kernel(const PlanArgs a, const StepWrite w, const int plan_ctas) {
       // 36 / 54 / - / 53.
       int slice = a.max_slice;
       while (slice > 1 && n * ((a.steps + slice - 1) / slice) < a.item_target) --slice;
-      gp->n = n; gp->n_tiles = n_tiles; gp->weight = weight; gp->slice = slice;
+      gp->n = n; gp->slice = slice;
     }
     // cut the scores work.  No piece is smaller than kMinPiece (more than a full step), so that none is empty
     // and the partial sums of a tile stay few.

@@ -13,8 +13,6 @@ constexpr int kMaxPieces = kMaxGrid * kMaxLevels;
 // ---- the plan of one group of hidden requests (device memory) --------------------------
 struct GroupPlan {
   int n;                      // requests of the group
-  int n_tiles;                // scores tiles
-  int weight;                 // total cost of the tiles, in boxes
   int slice;                  // 128-column blocks per item of the sum kernel
   int levels, per_level;      // pieces of the scores work: levels x per_level
   int next_piece, next_item;  // work counters of the scores and the sum kernel
@@ -23,7 +21,6 @@ struct GroupPlan {
   int len[kGroup];            // its length in tokens
   int tile_off[kGroup + 1];   // first scores tile
   int blk_off[kGroup + 1];    // first 16-token block of p
-  int w_off[kGroup + 1];      // cost of the tiles before it
   int bound_tile[kMaxPieces + 1];   // piece c: from (bound_tile[c], bound_step[c]) to the next bound
   int bound_step[kMaxPieces + 1];
 };
