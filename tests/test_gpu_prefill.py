@@ -83,6 +83,30 @@ def test_what_it_does_not_take_goes_to_the_library():
     assert ((out.double() - ref).abs() <= U[F] * (ref.abs() + 4 * size) + least).all()
 
 
+def test_prompts_of_no_tokens():
+    lens = [0, 40, 0, 0, 130, 0]
+    q, k, v, bounds = prompts(lens, 2, 64, F, seed=4)
+    want = attend(q, k, v, torch.tensor([0, 40, 170], device="cuda", dtype=torch.int32), [40, 130], 0.125)
+    assert torch.equal(attend(q, k, v, bounds, lens, 0.125), want)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("which", ["query", "key", "value"])
+@pytest.mark.parametrize("where", [3, 130, 255, 399])
+def test_nan_inside_a_prompt(which, where, d):
+    """A row is not finite where it attends to the bad row, and at most in the bad row's 128 query rows before it (weights of
+    zero there, times the bad value); the rows of other prompts and of earlier query tiles are as they were."""
+    lens = [400, 70]
+    q, k, v, bounds = prompts(lens, 2, d, B, seed=5)
+    want = attend(q, k, v, bounds, lens, d ** -0.5)
+    {"query": q, "key": k, "value": v}[which][where, :, 5] = float("nan")
+    got = attend(q, k, v, bounds, lens, d ** -0.5)
+    same = [t for t in range(470) if t < where // 128 * 128 or t >= 400 or (which == "query" and t != where)]
+    assert torch.equal(got[same], want[same])
+    bad = got[where if which == "query" else slice(where, 400)]
+    assert torch.isnan(bad[..., 5] if which == "value" else bad).all()
+
+
 def test_gradients_flow_where_they_are_wanted():
     lens = [70, 33]
     q, k, v, bounds = prompts(lens, 2, 64, B, seed=6)
