@@ -19,6 +19,8 @@
 
 #include "step_plan.cuh"
 
+#include <cfloat>
+
 namespace aps {
 namespace {
 
@@ -163,13 +165,13 @@ attend32_kernel(const Params p) {
   }
   __syncthreads();
   if (warp < kHeads) {
-    float m = -INFINITY, l = 0.f;
+    // not -infinity: where all scores are, the chunk has no weights and no NaN, the other chunks have them
+    float m = -FLT_MAX, l = 0.f;
     for (int t = lane; t < n; t += 32) m = fmaxf(m, s_p[t][warp]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const float ref = m == -INFINITY ? 0.f : m;   // scores of -infinity alone: no weights, the other chunks have them
     for (int t = lane; t < n; t += 32) {
-      const float w = exp2f(s_p[t][warp] - ref);
+      const float w = exp2f(s_p[t][warp] - m);
       s_p[t][warp] = w;
       l += w;
     }
@@ -224,7 +226,8 @@ unfold32_kernel(const Params p) {
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) { s_max[r] = m; s_inv[r] = l > 0.f || l != l ? 1.f / l : 0.f; s_chunks[r] = n; }
+    // no weight in any chunk (all scores -infinity): NaN, as 0 / 0 is
+    if (lane == 0) { s_max[r] = m; s_inv[r] = n == 0 ? 0.f : l > 0.f || l != l ? 1.f / l : __int_as_float(0x7fc00000); s_chunks[r] = n; }
   }
   const int steps = (p.hidden + kStep - 1) / kStep;
   const int sa = steps * blockIdx.y / gridDim.y, sb = steps * (blockIdx.y + 1) / gridDim.y;
