@@ -92,7 +92,7 @@ def raise_on_device_status(workspace: Optional[torch.Tensor] = None,
                            device: Optional[torch.device] = None) -> None:
     """Raise ``RuntimeError`` if the last attention call on ``workspace`` (default: the
     per-device workspace of ``device``) left a non-zero status word: 1..7 = a bounded wait
-    of the re-projection kernel ran out and the call's output is NaN, 8 = K/V-cached
+    of one of its kernels ran out and the call's output is NaN, 8 = K/V-cached
     requests in a batch that was given no K/V cache; or if the operations without a workspace left one on the
     device: a cache write that was not finished, metadata that points outside its tensors, prompt attention
     that was not finished (rows of NaN).
@@ -646,7 +646,7 @@ def _prefix_prefill_attention(query, key_cache, value_cache, query_start_loc, se
     """Prefix-enabled prefill (aptserve_flash_attn.py:432-447): the new prompt tokens of each
     sequence attend to the sequence's whole context, read through its block table from the
     cache the step has just written; causal with the query rows aligned to the END of the
-    context.  Like the prefill attention without a prefix it stays a composition of library
+    context.  Unlike the prefill attention without a prefix it is a composition of library
     calls (a gather by block id and scaled_dot_product_attention per sequence); the reference
     calls flash_attn_varlen_func with ``block_table``."""
     out = torch.empty_like(query)

@@ -3,11 +3,12 @@
 //
 // A decode batch is cut into CHUNKS of kChunkTokens consecutive tokens of one
 // request.  Every chunk of a K/V-cached request is streamed by warps of the
-// K/V kernel (one warp per head); every chunk of a hidden-cached request is one
+// K/V kernel (one warp per head; on the CUDA cores four where the batch is small); every chunk of a hidden-cached request is one
 // 128-row M tile of the re-projection GEMM.  Each (chunk, head) leaves a softmax
 // partial (running max and sum in the log2 domain, un-normalised fp32
 // accumulator) in the scratch buffer; a combine kernel merges a request's
-// partials in chunk order, so the result does not depend on scheduling.
+// partials in chunk order, so the result does not depend on scheduling (its last bits can
+// depend on the rest of the batch, by whose size the work is cut).
 #pragma once
 
 #include "aps_common.cuh"
@@ -30,7 +31,7 @@ enum PlanWord {
   kPlanWords = 64
 };
 
-// Values of the status word.  1..7: a bounded mbarrier wait of the re-projection kernel ran
+// Values of the status word.  1..7: a bounded mbarrier wait of one of the attention kernels ran
 // out (the code names the waiting role); the combine kernel then fills the whole output with
 // NaN.  8: the batch holds K/V-cached requests but the call was given no K/V cache; their
 // output rows are zero, the hidden-cached requests' rows are valid.

@@ -418,7 +418,7 @@ __device__ __forceinline__ int find_requests(const int32_t* cache_type, int batc
 }
 
 // The same from the plan, where it is complete: the first group's fold runs beside the planning, the others behind it.  Counting
-// there too, an empty group's fold took 9 us instead of 4 (700 OPT-1.3B requests without hidden-cached ones, three groups).
+// in these too, an empty group's fold took 9 us instead of 4 (700 OPT-1.3B requests without hidden-cached ones, three groups).
 __device__ __forceinline__ int planned_requests(const GroupPlan* gp, int first, int* reqs) {
   static_assert(kFoldThreads >= kGroup, "a thread per request of the group");
   const int n = gp->n;
@@ -1412,6 +1412,10 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCa
     if ((st = launch_chained("fold_kernel", k, dim3(splits, p.heads, chunks), kFoldThreads, smem, stream, m.wk, p,
                              first)) != APS_OK) return st;
   }
+  // Behind the fold whatever the batch.  Before it, K/V-only steps of more than 700 requests would be 0.5 - 1.3 % faster (their empty
+  // fold holds the K/V kernel back: 1100 OPT-1.3B requests 291 -> 287 us, 1500 374 -> 370), but the host does not know the
+  // types, and steps with hidden-cached requests would lose what the fold beside the plan gives (400, 30 % of them
+  // hidden-cached, 243 -> 249, 700 half 462 -> 471, 1500 half 717 -> 735, all 1061 -> 1091).
   if (kv != nullptr && (st = launch_kv_attention(ws, kv->query, kv->key_cache, kv->value_cache, kv->block_tables, kv->seq_lens,
                                                  kv->shape, stream)) != APS_OK) return st;
   {

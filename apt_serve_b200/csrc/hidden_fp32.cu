@@ -12,8 +12,8 @@
 // reads the cached rows once from memory and twice more per four heads from L1 / L2, which is what it then runs at.
 // The re-projecting kernel (hidden_simt.cu) does D times the arithmetic for a long request.  A step of an OPT-125M
 // layer in fp32, half of the requests hidden-cached, on one B200, that kernel -> this path: 8 requests of about 230 tokens
-// 340 -> 51 us (at 51 the calls' host side is what shows), 64 of 700 2.74 -> 0.14 ms, 200 of 1200, three quarters of them
-// hidden-cached, 20.2 -> 0.71 ms.  Its distance from 64 bits is a quarter of the re-projection's.
+// 340 -> 38 us (the host side of six launches; the device needs 32), 64 of 700 2.74 -> 0.16 ms, 200 of 1200, three quarters of
+// them hidden-cached, 20.2 -> 0.74 ms.  Its distance from 64 bits is a quarter of the re-projection's.
 //
 // Requests are taken in groups, so that the scratch (z: one row of E per request, chunk and head) stays bounded.
 
@@ -76,8 +76,9 @@ __device__ __forceinline__ float transpose_sum(float (&v)[N], int lane) {
 }
 
 // One CTA per (128 columns of E, head, kFoldReqs requests); warp w takes rows w, w + 8, ... of W_k,h (its loads are
-// independent: one round trip), the warps' sums are added through shared memory.  Like the tensor-core fold it
-// does not wait for the K/V kernel it is launched behind (wait_last).
+// independent: one round trip), the warps' sums are added through shared memory.  It
+// takes its requests from the plan, which is complete when the K/V kernel lets it start; behind that one it does not wait
+// for it before it begins but before it exits (wait_last).
 template <int D>
 __global__ void __launch_bounds__(kThreads)
 fold32_kernel(const Params p, const int wait_last) {
@@ -297,8 +298,9 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.count = batch < kGroup ? batch : kGroup;
   l.chunk = kMinChunk;
   auto per_request = [&] { return (size_t)((max_tokens + l.chunk - 1) / l.chunk) * row; };
-  // chunks of 32 tokens only while those of 64 leave SMs without a CTA: a CTA's time is its tokens' round trips, but every
-  // chunk's partial sums are read again (four OPT-125M requests 13.2 -> 8.4 us)
+  // chunks of 32 tokens only where those of 64 make no more than two CTAs per SM, counting every request as hidden-cached and as
+  // long as its table (the host knows no more): a CTA's time is its tokens' round trips, but every chunk's partial sums are
+  // read again (four OPT-125M requests 13.2 -> 8.4 us)
   if ((int64_t)l.count * ((max_tokens + 63) / 64) * ((heads + kHeads - 1) / kHeads) > 2 * sm_count()) l.chunk = 64;
   while (l.chunk < kMaxChunk && (size_t)l.count * per_request() > kScratch) l.chunk *= 2;
   l.chunks = (int)((max_tokens + l.chunk - 1) / l.chunk);

@@ -37,7 +37,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // ---- planning ------------------------------------------------------------------
 // The rows a K/V-only step adds, beside the plan instead of in a bulk-copy launch before it: at a decode batch's 20 KB a
 // request both are a round trip and a launch, and the planning CTA leaves 147 SMs idle (five OPT-1.3B requests through
-// FlashAttentionImpl.forward 24.3 -> 21.3 us, 128 OPT-13B requests 347 -> 345).
+// FlashAttentionImpl.forward 24.3 -> 21.3 us, 128 OPT-13B requests 346 either way).
 // Row 2 t is the K row of token t, row 2 t + 1 its V row.
 __device__ __forceinline__ void write_slots(const SlotWrite& w, int64_t job, int lane) {
   const int64_t row = job / w.chunks, t = row >> 1;
@@ -202,7 +202,8 @@ struct KvCfg {
 
 // A batch of few units (a quarter of the warps could take them all) is a chain of a unit's round trips, eight groups one after
 // the other: four warps then share a unit, each a quarter of its tokens, and merge their partials in shared
-// memory, in token order (8 OPT-125M requests in fp32, half of them K/V-cached, 15.2 -> 7.0 us).
+// memory, in token order (8 OPT-125M requests in fp32, half of them K/V-cached, 15.2 -> 7.0 us).  Whether they share follows
+// the batch's total work, so a request's last bits can be others in another batch; within a batch they are always the same.
 constexpr int kKvShare = 4;
 
 template <typename T, int D>
@@ -539,8 +540,9 @@ kv_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
   // Few units (two per warp at most): a warp's are known from its place.  The counter costs every warp two round trips to the
   // same address before its first copies (five OPT-1.3B requests 9.3 -> 7.2 us, none 3.1 -> 1.6); with more units it evens out
-  // the warps' different speeds.  MANY: the block tables are so long that there will be more; without the test the kernel
-  // of a large batch is 1 % faster.
+  // the warps' different speeds.  MANY: the block tables are so long that there may be many more, and the test is left out: a
+  // large batch is 1 % faster without it (336 us against 339, 350 against 355).  The host knows the tables' width, not the
+  // lengths: a batch of few units in tables padded to several times what they hold takes MANY too and does without the placed units.
   const int warps = gridDim.x * kTmaWarps, mine = blockIdx.x * kTmaWarps + warp;
   const bool few = !MANY && total <= 2 * warps;
   Unit cur = load_unit(few ? mine : next_index());
@@ -685,7 +687,7 @@ __device__ __forceinline__ void store4(T* dst, const float (&v)[4]) {
 }
 
 // One warp per (request, head): merge the request's partials in chunk order.  When a bounded
-// wait of the re-projection kernel ran out (status word 1..7) some partials were never
+// wait of one of the attention kernels ran out (status word 1..7) some partials were never
 // written: the whole output is filled with NaN instead of numbers that look plausible.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -830,6 +832,9 @@ int launch_kv_typed(const WorkspacePtrs& ws, const void* query, const void* key_
       int per_sm = 0;
       APS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTmaWarps * 32, kSmem));
       APS_REQUIRE(per_sm > 0, APS_ERR_CUDA, "the K/V streaming kernel does not fit on this device");
+      // the tables may be six times as wide as two units per warp need before the placed units are given up: padded further,
+      // 24 OPT-13B requests of 60 tokens 12.5 -> 14.4 us, 48 21.6 -> 22.7; without padding a batch at the line streams 0.9 GB,
+      // which the counter evens out, and the test only costs
       if (most > (int64_t)12 * sm_count() * per_sm * kTmaWarps) kernel = kv_attention_tma_kernel<T, D, kStages, true>;
       return launch_chained("kv_attention_tma_kernel", kernel, sm_count() * per_sm, kTmaWarps * 32, kSmem, stream,
                             mk, mv, ws.plan, ws.part_offset, ws.kv_chunks, ws.part_ml, ws.part_acc, (const T*)query,

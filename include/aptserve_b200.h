@@ -198,7 +198,7 @@ int aps_paged_decode_attention(void* out, const void* query, const void* key_cac
 
 /* aps_reshape_and_cache followed by aps_paged_decode_attention over the same caches (a decode batch without hidden-cached
  * requests, aptserve_flash_attn.py:338-345, 449-461), the rows written by the attention's planning launch where everything is
- * in multiples of 16 bytes.  num_slots: entries of slot_mapping, rows of key and value. */
+ * in multiples of 16 bytes.  num_slots: entries of slot_mapping; key and value hold at least as many rows. */
 int aps_plain_decode_step(void* out, const void* query, const void* key, const void* value, void* key_cache,
                           void* value_cache, const int64_t* slot_mapping, int64_t num_slots,
                           const int32_t* block_tables, const int32_t* seq_lens, int batch, int max_blocks_per_seq,
@@ -350,8 +350,8 @@ size_t aps_decode_layer_step_workspace_bytes(int batch, int max_blocks_per_seq, 
 
 /*
  * Reads the status word the attention kernels keep in `workspace` for the last call
- * that used it.  0 = fine.  1..7 = a bounded device-side wait of the re-projection
- * kernel ran out (the kernel returned early; the call's whole output was filled with
+ * that used it.  0 = fine.  1..7 = a bounded device-side wait of one of their
+ * kernels ran out (the kernel returned early; the call's whole output was filled with
  * NaN).  8 = the batch held K/V-cached requests but no K/V cache was passed (their
  * output rows are zero).  Synchronises `stream`: call it where a synchronisation is
  * cheap, e.g. once per engine step next to the sampler's device-to-host copy.
