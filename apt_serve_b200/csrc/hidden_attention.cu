@@ -88,7 +88,7 @@ struct Params {
   float* qscale;         // [request][head] scale * log2(e) / (power of two q was multiplied with)
   float* scores;         // [tile + piece][head][kTile] partial scores over a range of E
   int2* tile_pieces;     // [tile] the first and the last piece with a part of it
-  void* probs;           // [16-token block][term][K half][heads padded][8 tokens]
+  void* probs;           // [16-token block][K half][term][heads padded][8 tokens]; some blocks' first term last (SumColumns)
   float* inv_sum;        // [request][head]
   void* z;               // [term][head][request capacity][E]
   float* out_part;       // [split][hidden request][H * D]
@@ -796,6 +796,43 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   chain_wait();
 }
 
+// ---- columns of the weighted sums ---------------------------------------------------
+// Where an item's accumulators lie in its half of the tensor memory.  The cache blocks take turns among n_hi accumulators for the
+// first terms; the rests have theirs.  STACKED: several terms of a block are columns of one instruction's B operand, so that X is read from
+// shared memory once for them (an M128 K16 instruction takes (4096 + 32 N) / 128 cycles: two for the 48 padded heads of an
+// OPT-13B layer 90, one 56).  A column block then has [first 0 | rests | first 1 | first 2 | first 3]: blocks of turn 0 write
+// the first two, blocks of turn 1 the next two with the weights' terms in the order (rests, first); turns 2 and 3 take an
+// instruction for the first term and one for the rests.  Not stacked: an instruction per term, all rests in one accumulator.
+// Stacked where as many first accumulators fit as without and slices of two column blocks remain (a slice of one reads the
+// weights twice as often): sums in bf16 of 128 OPT-13B requests 216 us not stacked, 249 in stacked slices of one.
+struct SumColumns {
+  bool stacked;
+  uint32_t n_hi, col, set, rest;   // columns from a column block, a first accumulator (not stacked), the first terms to the next / the rests'
+  int rests;                       // accumulators of the rests
+  __host__ __device__ static uint32_t turns(int np, int slice) { return 5 * slice * np <= 256 ? 4 : 3 * slice * np <= 256 ? 2 : 1; }
+  __host__ __device__ static bool fits(int terms, int np, int slice) {
+    return stacked_terms(terms, np) && (terms - 1 + turns(np, slice)) * slice * np <= 256;
+  }
+  __host__ __device__ static bool stack(int terms, int np) { return fits(terms, np, 1) && (fits(terms, np, 2) || 4 * np > 256); }
+  __host__ __device__ SumColumns(int terms, int np, int slice) {
+    n_hi = turns(np, slice);
+    stacked = stack(terms, np) && fits(terms, np, slice);
+    if (stacked) {
+      col = (terms - 1 + n_hi) * np; set = 0; rest = np; rests = terms - 1;
+    } else {
+      col = np; set = slice * np; rests = 2 * slice * np <= 256 ? 1 : 0; rest = rests ? n_hi * set : 0;
+    }
+  }
+  // the k-th accumulator of a column block that has `used` first ones: those, then the rests'
+  template <bool STACKED>
+  __device__ __forceinline__ uint32_t at(int k, int used, int terms, int np) const {
+    if (k >= used) return rest + (k - used) * np;
+    return STACKED ? (k == 0 ? 0u : (uint32_t)((terms - 1 + k) * np)) : k * set;
+  }
+  // The weights of the request's block b have the first term last where b & turn_mask() is 1.
+  __device__ __forceinline__ int turn_mask() const { return stacked ? (int)n_hi - 1 : 0; }
+};
+
 // ---- softmax ------------------------------------------------------------------------
 // One CTA per (request, two heads) at a time, one warp per tile.  A lane takes eight consecutive tokens of the
 // tile for both heads: it adds the tile's partial sums, and after the maxima are known writes the eight weights of each
@@ -809,7 +846,7 @@ constexpr int kSoftmaxWarps = 4;
 constexpr int kHold = 2;
 
 template <typename T, int PER>
-__device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kSoftmaxWarps], float (*s_sum)[kSoftmaxWarps]) {
+__device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kSoftmaxWarps], float (*s_sum)[kSoftmaxWarps], volatile int* turns) {
   constexpr int NT = kTerms<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const GroupPlan* gp = p.plan;
@@ -892,6 +929,9 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
         }
       const int blk = k * kSubs + (lane >> 1);
       if (blk < n_blk) {
+        // a tile begins with a block of turn 0; the mask lies in shared memory for want of registers
+        const bool turned = (lane >> 1 & *turns) == 1;
+        T* at = probs + ((int64_t)((blk0 + blk) * 2 + (lane & 1)) * NT * p.np + h) * 8;   // 32-byte aligned: np and h are even
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
           uint32_t v[2][4] = {};
@@ -899,7 +939,7 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
           for (int i = 0; i < PER; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[i][e] = pack_pair<T>(terms[i][2 * e][t], terms[i][2 * e + 1][t]);
-          T* dst = probs + ((((int64_t)(blk0 + blk) * NT + t) * 2 + (lane & 1)) * p.np + h) * 8;   // 32-byte aligned: np and h are even
+          T* dst = at + (t == 0 ? (turned ? NT - 1 : 0) : turned ? t - 1 : t) * p.np * 8;
           if (two)
             asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]),
                          "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]) : "memory");
@@ -938,10 +978,12 @@ template <typename T>
 __global__ void __launch_bounds__(kSoftmaxWarps * 32, kTerms<T> == 2 ? 6 : 5)
 softmax_kernel(const Params p) {
   __shared__ float s_max[2][kSoftmaxWarps], s_sum[2][kSoftmaxWarps];
+  __shared__ int s_turns;
   chain_wait();
   chain_next();
-  if (p.plan->n * p.heads <= 2 * p.grid_scores) softmax_units<T, 1>(p, s_max, s_sum);
-  else softmax_units<T, 2>(p, s_max, s_sum);
+  if (threadIdx.x == 0) s_turns = SumColumns(kTerms<T>, p.np, p.plan->slice).turn_mask();   // read behind the first barrier of a unit
+  if (p.plan->n * p.heads <= 2 * p.grid_scores) softmax_units<T, 1>(p, s_max, s_sum, &s_turns);
+  else softmax_units<T, 2>(p, s_max, s_sum, &s_turns);
 }
 
 // ---- weighted sums ------------------------------------------------------------------
@@ -955,7 +997,12 @@ softmax_kernel(const Params p) {
 // an MN-major A operand, and the block's weights (one bulk copy, already in the layout of an unswizzled
 // K-major B operand).  The rows of a CTA's first stages are requested while the softmax kernel is still running: what a
 // kernel may read before chain_wait() is what was complete when the one before it called chain_next(), here all up
-// to the scores.  Warps: 0 copies, 1 MMA issue, 2-9 epilogue.
+// to the scores.  Warps: 0 takes the items and copies, 1 MMA issue, 2-9 (2-5) epilogue, the one behind them copies: the two take
+// turns at the stages, since one warp spends as long on a stage's wait and boxes as the stage takes to arrive (128 OPT-13B
+// requests 187 -> 183 us, 24 long ones 69 -> 67.5).  Two producers that take turns need at least as many stages: a stage is then
+// never two rounds behind the one that waits for it.  The columns of the accumulators and how many terms an instruction takes: SumColumns.
+// With both: 128 OPT-13B requests of 740 tokens 187 -> 172 us, 24 of 1800 69 -> 63, 8 of 1500 41 -> 34, 52 OPT-66B tp 8 requests 171 -> 146,
+// 34 OPT-1.3B 31 -> 25, 100 OPT-66B tp 2 280 -> 252, 128 OPT-13B in bf16 216 -> 212.
 // The tensor cores drop what falls below the accumulator's last place at every instruction, so a sum's error grows with
 // the number of instructions that went into one accumulator (terms x cache blocks).  Where few heads leave the
 // tensor memory for it, the rests have accumulators of their own and the cache blocks' first terms take turns among two
@@ -968,7 +1015,7 @@ softmax_kernel(const Params p) {
 // groups on: with one, an item of a short request (300 tokens) takes as long to be split into terms and written as to be read.
 // 64 OPT-13B requests of 340 tokens 77 -> 65 us, 128 of 740 198 -> 191, in bf16 228 -> 217; with fewer groups the second warp
 // costs more than it takes over (52 OPT-66B tp 8 requests, four groups, 170 -> 175; 8 long OPT-13B requests, three, 40 -> 43).
-constexpr int kSumThreads = 320;
+constexpr int kSumThreads = 352;
 // Where no item of the batch can have six, the kernel is launched without the second ones: their registers keep its CTAs from
 // starting beside the softmax's.
 __host__ __device__ inline int sum_epilogue_warps(int slice, int np) { return slice * np >= 96 ? 8 : 4; }
@@ -982,7 +1029,7 @@ __host__ __device__ inline uint32_t sum_stage_bytes(int terms, int np, int slice
   return blocks * slice * 4096 + ((blocks * probs_block_bytes(terms, np) + 1023) & ~1023u);
 }
 
-template <typename T>
+template <typename T, bool STACKED>
 __global__ void __launch_bounds__(kSumThreads, 1)
 sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   constexpr int NT = kTerms<T>;
@@ -999,13 +1046,12 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   if ((int)blockIdx.x >= n_items) { chain_wait(); return; }
   const uint32_t pblk = probs_block_bytes(NT, np), per_stage = sum_stage_blocks(NT, np, slice), x_bytes = per_stage * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
-  // sets of accumulators: n_hi for the first terms, one for the rests (or all terms in one)
-  const uint32_t n_hi = 5 * slice * np <= 256 ? 4 : 3 * slice * np <= 256 ? 2 : 1, rest_set = 2 * slice * np <= 256 ? n_hi : 0;
+  const SumColumns cols(NT, np, slice);
   const int n_epilogue = sum_epilogue_warps(slice, np);   // the others only wait
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], n_epilogue); }
-    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 1 + n_epilogue); }
+    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 2 + n_epilogue); }
     aux.abort_flag = 0;
     mbar_init_fence();
   }
@@ -1024,9 +1070,11 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   int next = blockIdx.x;   // the first item needs no counter
   const uint64_t once = l2_policy_evict_first();
   int ahead = 0;           // stages of the first item whose rows are requested before the wait
-  bool waited = warp != 0;
+  const int copier = warp == 0 ? 0 : warp == 2 + n_epilogue ? 1 : -1;   // the two take turns at the stages
+  uint32_t n_stage = 0;    // of all items so far
+  bool waited = copier < 0;
   if (waited) chain_wait();
-  while (ok && warp < 2 + n_epilogue) {
+  while (ok && warp < 3 + n_epilogue) {
     int item;
     if (warp == 0) {
       item = next;
@@ -1057,15 +1105,16 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
     const int n_blk = (len + 15) >> 4;
     const uint32_t buf = n_local & 1u, use = n_local >> 1;
     ++n_local;
-    if (warp == 0) {
+    if (copier >= 0) {
       const int32_t* bt = p.block_tables + (int64_t)gp->req[slot] * p.max_blocks;
       const char* probs = static_cast<const char*>(p.probs) + (int64_t)gp->blk_off[slot] * pblk;
       int rows = 0;
-      auto request_rows = [&](int b, uint32_t stage) {   // the stage's byte count, then the rows of the blocks from b on
+      auto request_rows = [&](int b, uint32_t stage, bool mine) {   // the stage's byte count, then the rows of the blocks from b on
         if ((b & 31) == 0) {   // first cache rows of the next 32 blocks
           const int tok = (b + lane) * 16;
           rows = b + lane < n_blk ? bt[tok / p.block_size] * p.block_size + tok % p.block_size : 0;
         }
+        if (!mine) return;
         const int nb = min((int)per_stage, n_blk - b);
         const uint32_t bar = full0 + stage * 8, dst = ring + stage * stage_bytes;
         if (lane == 0) mbar_expect_tx_addr(bar, (uint32_t)nb * (n_col * 4096 + pblk));
@@ -1076,27 +1125,30 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       };
       if (!waited) {
         ahead = min(min(stages, 32 / (int)per_stage), (n_blk + (int)per_stage - 1) / (int)per_stage);   // `rows` holds 32 blocks
-        for (int i = 0; i < ahead; ++i) request_rows(i * (int)per_stage, i);
+        for (int i = 0; i < ahead; ++i) request_rows(i * (int)per_stage, i, (i & 1) == copier);
         chain_wait();
         waited = true;
       }
       for (int b = 0; b < n_blk; b += (int)per_stage) {
         const int nb = min((int)per_stage, n_blk - b);
+        const bool mine = (int)(n_stage++ & 1u) == copier;
         if (ahead > 0) {
           --ahead;
         } else {
-          if (!mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
-          request_rows(b, rg.stage);
+          if (mine && !mbar_wait_warp(empty0 + rg.stage * 8, rg.phase ^ 1u, abort_flag, p.status, 1, lane)) { ok = false; break; }
+          request_rows(b, rg.stage, mine);
         }
         const uint32_t bar = full0 + rg.stage * 8, dst = ring + rg.stage * stage_bytes;
-        if (lane == 31) bulk_load(dst + x_bytes, probs + (int64_t)b * pblk, nb * pblk, bar);   // blocks lie one behind the other
+        if (mine && lane == 31) bulk_load(dst + x_bytes, probs + (int64_t)b * pblk, nb * pblk, bar);   // blocks lie one behind the other
         __syncwarp();
         rg.step(stages);
       }
     } else if (warp == 1) {
       if (!mbar_wait_warp(smem_u32(&aux.acc_empty[buf]), (use & 1u) ^ 1u, abort_flag, p.status, 2, lane)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true);
+      const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)np, true), idesc_rests = mma_idesc(kFmt<T>, 128, (uint32_t)((NT - 1) * np), true),
+                     idesc_all = mma_idesc(kFmt<T>, 128, (uint32_t)(STACKED ? NT * np : np), true);
+      const uint32_t mask = cols.n_hi - 1, d0 = tmem + buf * 256;
       for (int b = 0; b < n_blk; b += (int)per_stage) {
         const int nb = min((int)per_stage, n_blk - b);
         if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
@@ -1105,25 +1157,65 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         if (valid < 16) {
           // rows past the sequence length hold whatever the cache block holds; their weights are zero,
           // but zero times NaN is not
-          const uint32_t at = x_at + (nb - 1) * slice * 4096;
-          const int pieces = (16 - valid) * 8;
-          for (int i = lane; i < pieces * 2 * n_col; i += 32) {
-            const int r = valid + (i % pieces) / 8, piece = i % 8, hc = i / pieces;
-            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + hc * 2048 + r * 128 + piece * 16), "r"(0u) : "memory");
-          }
+          const uint32_t at = x_at + (nb - 1) * slice * 4096 + ((lane >> 3) & 1) * 2048 + (lane & 7) * 16;
+          for (int col = 0; col < n_col; ++col)
+            for (int r = valid + (lane >> 4); r < 16; r += 2)
+              asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + col * 4096 + r * 128), "r"(0u) : "memory");
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
         }
         tc_fence_after();
         if (elect_one()) {
-          for (int k = 0; k < nb; ++k) {
-            const uint32_t hi_set = (uint32_t)(b + k) & (n_hi - 1), hi_acc = (uint32_t)(b + k) >= n_hi;
-            const uint32_t a_lo = desc_lo(x_at + k * slice * 4096, 2048), b_lo = desc_lo(p_at + k * pblk, (uint32_t)np * 16);
-            for (int col = 0; col < n_col; ++col)
+          const uint32_t x_lo = desc_lo(x_at, 2048), p_lo = desc_lo(p_at, (uint32_t)(NT * np * 16)), x_step = slice * 256, p_step = pblk >> 4;
+          auto mma = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t what, uint32_t acc) {
+            tc_mma_cta(d, a_lo, desc_hi(1024, true), b_lo, desc_hi(128, false), what, acc);
+          };
+          if constexpr (!STACKED) {
+            for (int k = 0; k < nb; ++k) {
+              const uint32_t turn = (uint32_t)(b + k) & mask, later = (uint32_t)(b + k) > mask;   // later: its first accumulator has been written before
+              for (int col = 0; col < n_col; ++col)
 #pragma unroll
-              for (int i = 0; i < NT; ++i)
-                tc_mma_cta(tmem + buf * 256 + ((i == 0 ? hi_set : rest_set) * slice + col) * np, a_lo + col * 256, desc_hi(1024, true),
-                           b_lo + i * (np * 2), desc_hi(128, false), idesc, i == 0 ? hi_acc : i > 1 || rest_set == 0 || b + k > 0);
+                for (int i = 0; i < NT; ++i)
+                  mma(d0 + (i == 0 ? turn * cols.set : cols.rest) + col * np, x_lo + k * x_step + col * 256, p_lo + k * p_step + i * np, idesc,
+                      i == 0 ? later : i > 1 || cols.rests == 0 || b + k > 0);
+            }
+          } else if (mask == 0) {
+            for (int k = 0; k < nb; ++k)
+#pragma unroll
+              for (int col = 0; col < kMaxSlice; ++col) {
+                if (col >= n_col) break;
+                mma(d0 + col * cols.col, x_lo + k * x_step + col * 256, p_lo + k * p_step, idesc_all, b + k > 0);
+              }
+          } else if ((b & mask) != 0) {   // stages of two blocks, turns 2 and 3
+            for (int k = 0; k < nb; ++k)
+              for (int col = 0; col < n_col; ++col) {
+                mma(d0 + (NT + 1 + k) * np + col * cols.col, x_lo + k * x_step + col * 256, p_lo + k * p_step, idesc, b > 2);
+                mma(d0 + np + col * cols.col, x_lo + k * x_step + col * 256, p_lo + k * p_step + np, idesc_rests, 1u);
+              }
+          } else {
+            // from turn 0 on, in straight line: with a loop that looks at every block's turn the issuing thread was what the kernel waited for
+            const uint32_t d_hi = d0 + (NT - 1) * np, later = b > 0;
+            for (int col = 0; col < n_col; ++col) {
+              const uint32_t at = col * cols.col, x = x_lo + col * 256;
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                if (k >= nb) break;
+                const uint32_t xk = x + k * x_step, pk = p_lo + k * p_step;
+                if (k == 0 || (k == 2 && mask == 1)) {
+                  mma(d0 + at, xk, pk, idesc_all, k == 2 ? 1u : later);
+                } else if (k == 1 || (k == 3 && mask == 1)) {
+                  if (k == 3 || later) {
+                    mma(d0 + np + at, xk, pk, idesc_all, 1u);
+                  } else {
+                    mma(d0 + np + at, xk, pk, idesc_rests, 1u);
+                    mma(d_hi + np + at, xk, pk + (NT - 1) * np, idesc, 0u);
+                  }
+                } else {
+                  mma(d_hi + k * np + at, xk, pk, idesc, later);
+                  mma(d0 + np + at, xk, pk + np, idesc_rests, 1u);
+                }
+              }
+            }
           }
           tc_commit_cta(empty0 + rg.stage * 8);
         }
@@ -1138,28 +1230,36 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       T* z = static_cast<T*>(p.z);
       if (!mbar_wait_warp(smem_u32(&aux.acc_full[buf]), use & 1u, abort_flag, p.status, 4, lane)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t used = min(n_hi, (uint32_t)n_blk);
+      const int used = (int)min(cols.n_hi, (uint32_t)n_blk), n_in = used + cols.rests;
+      // accumulators of a column block: four first terms' and the rests'; that many read together (142 - 144 registers; one after the other,
+      // in 128, short requests' items wait for it: 16 OPT-13B requests of 60 tokens 16.5 -> 19 us)
+      constexpr int kMost = NT + 3, kAtOnce = 6 - NT;
+      uint32_t off[kMost];
+#pragma unroll
+      for (int k = 1; k < kMost; ++k) off[k] = cols.at<STACKED>(k, used, NT, np);
       const int h_steps = np / 16;
       for (int it = turn; it < n_col * h_steps; it += n_epilogue / 4) {
         const int col = it / h_steps, h0 = (it - col * h_steps) * 16;
         const int e = (first + col) * 128 + quarter * 32 + lane;
         uint32_t v[16];
-        const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * np + h0;
+        const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * cols.col + h0;
         tmem_ld16(at, v);
-        uint32_t more[3][16], rest[16];
 #pragma unroll
-        for (uint32_t i = 0; i < 3; ++i)
-          if (i + 1 < used) tmem_ld16(at + (i + 1) * slice * np, more[i]);
-        if (rest_set != 0) tmem_ld16(at + rest_set * slice * np, rest);
-        tmem_ld_wait();
+        for (int k0 = 1; k0 < kMost; k0 += kAtOnce) {
+          if (k0 > 1 && k0 >= n_in) break;
+          uint32_t more[kAtOnce][16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          float x = __uint_as_float(v[j]);
+          for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
+            if (k < n_in) tmem_ld16(at + off[k], more[k - k0]);
+          tmem_ld_wait();
 #pragma unroll
-          for (uint32_t i = 0; i < 3; ++i)
-            if (i + 1 < used) x += __uint_as_float(more[i][j]);
-          if (rest_set != 0) x += __uint_as_float(rest[j]);
-          v[j] = __float_as_uint(x);
+          for (int j = 0; j < 16; ++j) {
+            float x = __uint_as_float(v[j]);
+#pragma unroll
+            for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
+              if (k < n_in) x += __uint_as_float(more[k - k0][j]);
+            v[j] = __float_as_uint(x);
+          }
         }
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
@@ -1345,7 +1445,10 @@ Layout layout_of(int batch, int max_blocks, int block_size, int heads, int head_
   l.splits = splits < 1 ? 1 : splits;
   int ms = 256 / l.np;
   if (ms > kMaxSlice) ms = kMaxSlice;
-  while (ms > 1 && 2 * ms * l.np > 256) --ms;   // room for the rests' accumulators (see sum_kernel)
+  while (ms > 1 && 2 * ms * l.np > 256) --ms;   // room for the rests' accumulators
+  if (SumColumns::stack(nt, l.np))
+    for (int s = 2; s <= ms; ++s)
+      if (!SumColumns::fits(nt, l.np, s)) ms = s - 1;
   while (ms > 1 && 3 * sum_stage_bytes(nt, l.np, ms) > kRingBytes) --ms;   // at least three stages
   l.max_slice = ms;
   const int64_t max_tokens = (int64_t)max_blocks * block_size;
@@ -1429,9 +1532,10 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCa
   if ((st = launch_chained("softmax_kernel", softmax_kernel<T>, units < resident ? units : resident, kSoftmaxWarps * 32, 0,
                            stream, p)) != APS_OK) return st;
   {
-    static bool done[64] = {false};
-    auto k = sum_kernel<T>;
-    if ((st = allow_smem(k, ring, done)) != APS_OK) return st;
+    static bool done[64] = {false}, done_apart[64] = {false};
+    auto k = sum_kernel<T, true>;
+    if (!SumColumns::stack(kTerms<T>, p.np)) k = sum_kernel<T, false>;
+    if ((st = allow_smem(sum_kernel<T, true>, ring, done)) != APS_OK || (st = allow_smem(sum_kernel<T, false>, ring, done_apart)) != APS_OK) return st;
     if ((st = launch_chained("sum_kernel", k, sm_count(), p.sum_threads, ring, stream, m.x_sum, p)) != APS_OK) return st;
   }
   {
@@ -1562,7 +1666,7 @@ int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaS
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_threads = 64 + 32 * sum_epilogue_warps(pa.max_slice, l.np); p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_threads = 96 + 32 * sum_epilogue_warps(pa.max_slice, l.np); p.grid_scores = pa.grid_scores;
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);

@@ -28,6 +28,24 @@ def test_softmax_units(heads, dtype, lens):
     check(workload(heads, 64, 128, dtype, list(lens), [True] * len(lens)), f"{heads} heads, {len(lens)} requests")
 
 
+# weighted sums: terms in one instruction or one for each, one, two and four turns of accumulators, stages of two and four cache blocks,
+# slices of one to four column blocks (many requests), the last one narrower; lengths around a round of turns and a stage
+@pytest.mark.parametrize("dtype", [F, B])
+@pytest.mark.parametrize("heads,d,e,n", [(16, 64, 384, 0), (20, 64, 384, 0), (48, 32, 384, 0), (64, 32, 384, 0), (72, 64, 256, 0), (100, 32, 256, 0),
+                                         (128, 32, 256, 0), (3, 64, 1152, 150), (20, 32, 1152, 150), (40, 32, 1152, 100), (40, 32, 640, 150)])
+def test_columns_of_the_weighted_sums(heads, d, e, n, dtype):
+    lens = [1, 15, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 66, 80, 81, 96, 97, 127, 128, 129, 300]
+    lens = lens + [1 + 37 * i % 90 for i in range(n)]
+    w = workload(heads, d, e, dtype, lens, [True] * len(lens))
+    if n == 0:   # what lies behind the sequences must not be seen
+        rows = O.flat_rows(w.hidden_cache)
+        for r, s in enumerate(lens):
+            if s % 16:
+                last = w.block_tables[r][-1]
+                rows[last * 16 + s % 16: last * 16 + 16] = float("nan")
+    check(w, f"{heads} heads, {len(lens)} requests")
+
+
 # fold: one turn and several turns of 16 requests per epilogue warp, a second chunk of 128; it finds the requests by itself,
 # those past 256 in the plan
 @pytest.mark.parametrize("n,every", [(16, 1), (17, 1), (33, 2), (129, 1), (400, 3), (450, 1), (600, 2)])
