@@ -98,7 +98,7 @@ struct Params {
   int group_first;                           // ordinal of the group's first hidden request
   int n_hidden_cap, splits, grid_scores;
   uint32_t unfold_ring;                      // bytes of the unfold kernel's ring
-  int sum_threads;                           // of the sum kernel
+  int sum_threads, sum_copiers;              // of the sum kernel
   int w_box_rows;                            // rows of a W_v box: 128, fewer when W_v has fewer
   int64_t query_stride;
   float scale_log2;
@@ -295,7 +295,7 @@ step_plan_kernel(const PlanArgs a, const StepWrite w, const int plan_ctas) {
       // 36 / 54 / - / 53.
       int slice = a.max_slice;
       while (slice > 1 && n * ((a.steps + slice - 1) / slice) < a.item_target) --slice;
-      gp->n = n; gp->slice = slice;
+      gp->n = n; gp->slice = slice; gp->turns = (a.turns >> (4 * slice)) & 15;
     }
     // cut the scores work.  No piece is smaller than kMinPiece (more than a full step), so that none is empty
     // and the partial sums of a tile stay few.
@@ -830,7 +830,7 @@ struct SumColumns {
     return STACKED ? (k == 0 ? 0u : (uint32_t)((terms - 1 + k) * np)) : k * set;
   }
   // The weights of the request's block b have the first term last where b & turn_mask() is 1.
-  __device__ __forceinline__ int turn_mask() const { return stacked ? (int)n_hi - 1 : 0; }
+  __host__ __device__ int turn_mask() const { return stacked ? (int)n_hi - 1 : 0; }
 };
 
 // ---- softmax ------------------------------------------------------------------------
@@ -846,7 +846,7 @@ constexpr int kSoftmaxWarps = 4;
 constexpr int kHold = 2;
 
 template <typename T, int PER>
-__device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kSoftmaxWarps], float (*s_sum)[kSoftmaxWarps], volatile int* turns) {
+__device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kSoftmaxWarps], float (*s_sum)[kSoftmaxWarps]) {
   constexpr int NT = kTerms<T>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const GroupPlan* gp = p.plan;
@@ -929,8 +929,10 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
         }
       const int blk = k * kSubs + (lane >> 1);
       if (blk < n_blk) {
-        // a tile begins with a block of turn 0; the mask lies in shared memory for want of registers
-        const bool turned = (lane >> 1 & *turns) == 1;
+        // A tile begins with a block of turn 0.  The mask lies beside what was read of the plan first (in the L1), and is read here for want of registers.
+        int turns;
+        asm volatile("ld.global.ca.s32 %0, [%1];" : "=r"(turns) : "l"(&gp->turns));
+        const bool turned = (lane >> 1 & turns) == 1;
         T* at = probs + ((int64_t)((blk0 + blk) * 2 + (lane & 1)) * NT * p.np + h) * 8;   // 32-byte aligned: np and h are even
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
@@ -978,12 +980,10 @@ template <typename T>
 __global__ void __launch_bounds__(kSoftmaxWarps * 32, kTerms<T> == 2 ? 6 : 5)
 softmax_kernel(const Params p) {
   __shared__ float s_max[2][kSoftmaxWarps], s_sum[2][kSoftmaxWarps];
-  __shared__ int s_turns;
   chain_wait();
   chain_next();
-  if (threadIdx.x == 0) s_turns = SumColumns(kTerms<T>, p.np, p.plan->slice).turn_mask();   // read behind the first barrier of a unit
-  if (p.plan->n * p.heads <= 2 * p.grid_scores) softmax_units<T, 1>(p, s_max, s_sum, &s_turns);
-  else softmax_units<T, 2>(p, s_max, s_sum, &s_turns);
+  if (p.plan->n * p.heads <= 2 * p.grid_scores) softmax_units<T, 1>(p, s_max, s_sum);
+  else softmax_units<T, 2>(p, s_max, s_sum);
 }
 
 // ---- weighted sums ------------------------------------------------------------------
@@ -1016,6 +1016,9 @@ softmax_kernel(const Params p) {
 // 64 OPT-13B requests of 340 tokens 77 -> 65 us, 128 of 740 198 -> 191, in bf16 228 -> 217; with fewer groups the second warp
 // costs more than it takes over (52 OPT-66B tp 8 requests, four groups, 170 -> 175; 8 long OPT-13B requests, three, 40 -> 43).
 constexpr int kSumThreads = 352;
+// Given to the kernel as a value: compiled in, the loops over the stages come out longer and short requests wait for them
+// (32 OPT-66B tp 8 requests of 60 tokens 22.5 -> 26 us).
+constexpr int kSumCopiers = 2;
 // Where no item of the batch can have six, the kernel is launched without the second ones: their registers keep its CTAs from
 // starting beside the softmax's.
 __host__ __device__ inline int sum_epilogue_warps(int slice, int np) { return slice * np >= 96 ? 8 : 4; }
@@ -1048,10 +1051,11 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   const SumColumns cols(NT, np, slice);
   const int n_epilogue = sum_epilogue_warps(slice, np);   // the others only wait
+  const int n_copiers = p.sum_copiers;
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&aux.full[s], 1); mbar_init(&aux.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&aux.acc_full[b], 1); mbar_init(&aux.acc_empty[b], n_epilogue); }
-    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], 2 + n_epilogue); }
+    for (int i = 0; i < kItemSlots; ++i) { mbar_init(&items.full[i], 1); mbar_init(&items.empty[i], n_copiers + n_epilogue); }
     aux.abort_flag = 0;
     mbar_init_fence();
   }
@@ -1070,11 +1074,11 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   int next = blockIdx.x;   // the first item needs no counter
   const uint64_t once = l2_policy_evict_first();
   int ahead = 0;           // stages of the first item whose rows are requested before the wait
-  const int copier = warp == 0 ? 0 : warp == 2 + n_epilogue ? 1 : -1;   // the two take turns at the stages
+  const int copier = warp == 0 ? 0 : n_copiers == 2 && warp == 2 + n_epilogue ? 1 : -1;   // the two take turns at the stages
   uint32_t n_stage = 0;    // of all items so far
   bool waited = copier < 0;
   if (waited) chain_wait();
-  while (ok && warp < 3 + n_epilogue) {
+  while (ok && warp < 1 + n_copiers + n_epilogue) {
     int item;
     if (warp == 0) {
       item = next;
@@ -1125,13 +1129,15 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       };
       if (!waited) {
         ahead = min(min(stages, 32 / (int)per_stage), (n_blk + (int)per_stage - 1) / (int)per_stage);   // `rows` holds 32 blocks
-        for (int i = 0; i < ahead; ++i) request_rows(i * (int)per_stage, i, (i & 1) == copier);
+#pragma unroll 1
+        for (int i = 0; i < ahead; ++i) request_rows(i * (int)per_stage, i, (i & (n_copiers - 1)) == copier);
         chain_wait();
         waited = true;
       }
+#pragma unroll 1
       for (int b = 0; b < n_blk; b += (int)per_stage) {
         const int nb = min((int)per_stage, n_blk - b);
-        const bool mine = (int)(n_stage++ & 1u) == copier;
+        const bool mine = (int)(n_stage++ & (uint32_t)(n_copiers - 1)) == copier;
         if (ahead > 0) {
           --ahead;
         } else {
@@ -1291,7 +1297,9 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
 // D[row of W_v][request] = sum_e W_v[row][e] z[request][head of the row][e]: one CTA per (128 rows of W_v,
 // range of E, 128 / HT requests), HT = 128 / D heads per 128 rows.  Rows of every head are multiplied with
 // every one of the HT heads' z and the epilogue keeps the matching quarter (half): for D = 128 nothing
-// is wasted.  The first term and the rests have accumulators of their own (see sum_kernel).  Partial sums over the
+// is wasted.  The first term and the rests have accumulators of their own (see SumColumns); where few enough requests leave
+// the columns, all terms and heads are columns of one instruction (one OPT-13B request 11.1 -> 10.2 us with the rows below, 16 OPT-125M
+// in bf16 5.2 -> 4.3).  Partial sums over the
 // ranges of E are added by the combine kernel.
 constexpr int kUnfoldThreads = 192;
 
@@ -1312,6 +1320,7 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   if (r0 >= n) { chain_wait(); return; }
   const int m = min(NC, n - r0), boxes = (m + 15) / 16;
   const uint32_t z_head = boxes * 2048;   // bytes of one (term, head) slab
+  const bool stacked = NT * HT * boxes * 16 <= 256;   // their rows lie one behind the other: all as columns of one instruction
   const int head0 = blockIdx.x * HT, n_heads = min(HT, p.heads - head0);
   const int sa = (int)((int64_t)p.slabs * blockIdx.y / gridDim.y), sb = (int)((int64_t)p.slabs * (blockIdx.y + 1) / gridDim.y);
   const uint32_t stage_bytes = unfold_stage_bytes(NT * HT * boxes);
@@ -1345,6 +1354,12 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     // the first stages' rows of W_v are requested while the sum kernel is still running, z once it is complete
     int ahead = min(stages, sb - sa);
     for (int i = 0; i < ahead; ++i) request_w(sa + i, i);
+    // and the other rows of the range as far as L2, where the sum kernel's items leave SMs idle (one OPT-13B request 11.1 -> 10.7 us; with more
+    // items the rows that it still waits for come later: its 576 for 32 OPT-66B tp 8 requests of 60 tokens 22.7 -> 25.9)
+    const int slice = p.plan->slice;
+    if (n * ((p.slabs / 2 + slice - 1) / slice) <= p.grid_scores)
+      for (int s = sa + ahead + lane; s < sb; s += 32) tma_prefetch_2d(&map_w, s * 64, head0 * D);
+    __syncwarp();
     chain_wait();
     for (int s = sa; s < sb; ++s) {
       if (ahead > 0) {
@@ -1363,14 +1378,17 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
       rg.step(stages);
     }
   } else if (warp == 1) {
-    const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)(boxes * 16), false);
+    const uint32_t idesc = mma_idesc(kFmt<T>, 128, (uint32_t)(stacked ? NT * HT * boxes * 16 : boxes * 16), false);
     uint32_t acc = 0;
     for (int s = sa; s < sb; ++s) {
       if (!mbar_wait_warp(full0 + rg.stage * 8, rg.phase, abort_flag, p.status, 3, lane)) { ok = false; break; }
       tc_fence_after();
       if (elect_one()) {
         const uint32_t a_lo = desc_lo(ring + rg.stage * stage_bytes, 16), b_lo = a_lo + (16384 >> 4);
-        for (int hh = 0; hh < n_heads; ++hh) {
+        if (stacked) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) tc_mma_cta(tmem, a_lo + k * 2, desc_hi(1024, true), b_lo + k * 2, desc_hi(1024, true), idesc, k > 0 ? 1u : acc);
+        } else for (int hh = 0; hh < n_heads; ++hh) {
           uint32_t first = acc;
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -1399,11 +1417,16 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int width = p.heads * D;
         float* dst = p.out_part + ((int64_t)blockIdx.y * p.n_hidden_cap + p.group_first + r0) * width + head0 * D + row;
         for (int c = 0; c < m; c += 16) {
-          uint32_t v[16], rest[16];
-          const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + hh * NC + c;
+          uint32_t v[16], rest[16], last[16];
+          const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (stacked ? hh * boxes * 16 : hh * NC) + c;
           tmem_ld16(at, v);
-          tmem_ld16(at + kRestAcc, rest);
+          tmem_ld16(at + (stacked ? HT * boxes * 16 : (int)kRestAcc), rest);
+          if (NT == 3 && stacked) tmem_ld16(at + 2 * HT * boxes * 16, last);
           tmem_ld_wait();
+          if (NT == 3 && stacked) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) rest[j] = __float_as_uint(__uint_as_float(rest[j]) + __uint_as_float(last[j]));
+          }
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             if (c + j < m) dst[(int64_t)(c + j) * width] = fmaf(__uint_as_float(rest[j]), kRestDown<T>, __uint_as_float(v[j]));
@@ -1635,6 +1658,7 @@ int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaS
   pa.max_tokens = s.max_blocks_per_seq * s.block_size; pa.kv_present = have_kv ? 1 : 0; pa.n_groups = l.n_groups;
   pa.steps = e_blocks; pa.grid_scores = sm_count();
   pa.max_slice = l.max_slice < e_blocks ? l.max_slice : e_blocks; pa.item_target = kSumRounds * sm_count();
+  for (int i = 1; i <= kMaxSlice; ++i) pa.turns |= SumColumns(nt, l.np, i).turn_mask() << (4 * i);
   if ((st = launch_step_plan(&pa, nw, cs)) != APS_OK) return st;
 
   Maps m;
@@ -1666,7 +1690,7 @@ int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaS
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_threads = 96 + 32 * sum_epilogue_warps(pa.max_slice, l.np); p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_copiers = kSumCopiers; p.sum_threads = 32 + 32 * (kSumCopiers + sum_epilogue_warps(pa.max_slice, l.np)); p.grid_scores = pa.grid_scores;
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);

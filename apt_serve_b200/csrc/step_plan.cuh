@@ -14,6 +14,7 @@ constexpr int kMaxPieces = kMaxGrid * kMaxLevels;
 struct GroupPlan {
   int n;                      // requests of the group
   int slice;                  // 128-column blocks per item of the sum kernel
+  int turns;                  // which cache blocks' weights have their first term last (SumColumns::turn_mask)
   int levels, per_level;      // pieces of the scores work: levels x per_level
   int next_piece, next_item;  // work counters of the scores and the sum kernel
   int req[kGroup];            // batch row of each request, longest first
@@ -39,6 +40,7 @@ struct PlanArgs {
   int* plan; int* part_offset; int2* kv_chunks; int* hid_slot; int2* hid_list; GroupPlan* groups;
   const int32_t* seq_lens; const int32_t* cache_type;
   int batch, max_tokens, kv_present, n_groups, steps, grid_scores, max_slice, item_target;
+  int turns;   // four bits for each slice
 };
 int launch_step_plan(const PlanArgs* plan, const NewTokenWrite& n, cudaStream_t stream);   // plan may be NULL: the new-token writes alone
 
