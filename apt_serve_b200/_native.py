@@ -38,6 +38,7 @@ PROTOTYPES = {
                                                        c_int64, c_int64, c_int, c_void_p]),
     "aps_hidden_to_cache": (c_int, [c_void_p] * 5 + [c_int64, c_int, c_int64, c_int64, c_int,
                                                      c_void_p]),
+    "aps_gather_hidden_rows": (c_int, [c_void_p] * 5 + [c_int64, c_void_p, c_int64, c_int64, c_int] + [c_int64] * 3 + [c_void_p, c_int, c_void_p]),
     "aps_cache_to_hidden": (c_int, [c_void_p] * 4 + [c_int64, c_int, c_int64, c_int64, c_int,
                                                      c_void_p]),
     "aps_mixed_kv_to_cache": (c_int, [c_void_p] * 10 + [c_int64, c_int64, c_int, c_int, c_int,
@@ -161,6 +162,17 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
 
 def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
+
+
+def only_values(*tensors) -> bool:
+    """Whether a call wants nothing of the tensors but their values: no graph for a backward pass, no tangents, trace, batching
+    or other transform, no fake tensors or modes that watch the operators.  A native call would leave all of these out in
+    silence, the library call is an operator that torch knows."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing()
+                or any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter for t in tensors)
+                or (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
+                or torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch._C._len_torch_dispatch_stack() > 0)
 
 
 class _Nothing:

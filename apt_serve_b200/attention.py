@@ -585,21 +585,13 @@ class FlashAttentionMetadata:
                    use_cuda_graph=False)
 
 
-def _only_values(*tensors) -> bool:
-    """Whether a call wants nothing of the tensors but their values: no graph for a backward pass, no tangents, trace, batching
-    or other transform, no fake tensors or modes that watch the operators.  A native call would leave all of these out in
-    silence, the library call is an operator that torch knows."""
-    return not (torch.compiler.is_compiling() or torch.jit.is_tracing()
-                or any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter for t in tensors)
-                or (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
-                or torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
-                or torch._C._len_torch_dispatch_stack() > 0)
+_only_values = N.only_values
 
 
 def _prefill_supported(q, k, v, bounds, scale) -> bool:
     """Whether ``aps_prefill_attention`` takes the packed prompts: 16-bit, head size 64 or 128, rows of back-to-back heads
     with 16-byte aligned rows, of which nothing but the values is wanted, a scale that is positive in fp32."""
-    if bounds is None or not _only_values(q, k, v, bounds):
+    if bounds is None or not N.only_values(q, k, v, bounds):
         return False
     if q.dim() != 3 or q.dtype not in (torch.float16, torch.bfloat16) or not 2.0 ** -126 <= scale < 2.0 ** 127:
         return False

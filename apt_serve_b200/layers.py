@@ -162,12 +162,9 @@ class OPTAttention(torch.nn.Module):
             mixed_cache_ops.hidden_to_cache(hidden_states, hcache, m.slot_mapping,
                                             m.hidden_cache_use_input, m.hidden_cache_store_tot)
             if m.num_decode_tokens != 0:
-                holder = torch.zeros(m.num_tot_tokens, hidden_states.shape[1],
-                                     device=hidden_states.device, dtype=hidden_states.dtype)
                 q, _ = self.qkv_proj(hidden_states, q_only=True)
-                holder[m.hidden_holder_upd] = hidden_states
-                mixed_cache_ops.cache_to_hidden(holder, hcache, m.slot_mapping,
-                                                m.hidden_cache_use_tot)
+                holder = mixed_cache_ops.gather_hidden_rows(hidden_states, hcache, m.slot_mapping, m.hidden_holder_upd,
+                                                            m.hidden_cache_use_tot, m.num_tot_tokens)
                 kv, _ = self.qkv_proj(holder, kv_only=True)
                 k, v = kv.chunk(chunks=2, dim=-1)
             else:

@@ -62,6 +62,40 @@ def cache_to_hidden(hidden: torch.Tensor, paged_cache: torch.Tensor, slot_mappin
             N.current_stream(dev)))
 
 
+def gather_hidden_rows(hidden_states: torch.Tensor, paged_cache: torch.Tensor, slot_mapping: torch.Tensor,
+                       new_rows: torch.Tensor, cached_rows: torch.Tensor, rows: int) -> torch.Tensor:
+    """The decode batch's gathered input (aptserve_opt.py:112-121): ``rows`` zero rows, ``hidden_states`` written at ``new_rows``, then
+    ``cache_to_hidden`` at ``cached_rows``.  In one pass where the rows are wide and aligned as a layer's are; the three
+    operations one after the other otherwise (other index types, shapes that broadcast, gradients or transforms)."""
+    if _gathers(hidden_states, paged_cache, slot_mapping, new_rows, cached_rows, rows):
+        dev = N.require_cuda(hidden_states, paged_cache, slot_mapping, new_rows, cached_rows)
+        out = torch.empty(rows, hidden_states.shape[1], device=dev, dtype=hidden_states.dtype)
+        sources = torch.empty(rows, device=dev, dtype=torch.int64)
+        with N.on_device(dev):
+            status = N.lib().aps_gather_hidden_rows(
+                out.data_ptr(), hidden_states.data_ptr(), paged_cache.data_ptr(), slot_mapping.data_ptr(), new_rows.data_ptr(),
+                new_rows.shape[0], cached_rows.data_ptr(), cached_rows.shape[0], rows, out.shape[1], out.shape[1],
+                hidden_states.stride(0), paged_cache.stride(2), sources.data_ptr(), N.dtype_enum(hidden_states), N.current_stream(dev))
+        if status != N.APS_ERR_UNSUPPORTED:
+            N.check(status)
+            return out
+    out = torch.zeros(rows, hidden_states.shape[1], device=hidden_states.device, dtype=hidden_states.dtype)
+    out[new_rows] = hidden_states
+    cache_to_hidden(out, paged_cache, slot_mapping, cached_rows)
+    return out
+
+
+def _gathers(hidden, cache, slots, new_rows, cached_rows, rows) -> bool:
+    """Whether the one pass takes these tensors."""
+    return (N.only_values(hidden, cache, slots, new_rows, cached_rows)
+            and hidden.dim() == 2 and hidden.stride(1) == 1 and cache.dim() == 5 and hidden.dtype == cache.dtype
+            and all(t.dim() == 1 and t.dtype == torch.int64 and t.is_contiguous() and t.device == hidden.device
+                    for t in (slots, new_rows, cached_rows))
+            and cache.device == hidden.device and hidden.is_cuda
+            and new_rows.shape[0] == hidden.shape[0] and hidden.stride(0) >= hidden.shape[1]
+            and slots.shape[0] == rows and rows > 0 and hidden.shape[0] > 0 and cached_rows.shape[0] > 0)
+
+
 def mixed_kv_to_cache(key: torch.Tensor, value: torch.Tensor, k_cache: torch.Tensor,
                       v_cache: torch.Tensor, shared_k_cache: torch.Tensor,
                       shared_v_cache: torch.Tensor, slot_mapping: torch.Tensor,

@@ -104,6 +104,21 @@ int aps_cache_to_hidden(void* hidden, const void* paged_cache,
                         int dtype, void* stream);
 
 /*
+ * The gathered input of a decode batch's K/V projection in one pass: what the zero fill (opt.py:112), the indexed write of the step's
+ * rows (opt.py:117-118) and cache_to_hidden (opt.py:120) leave in it one after the other.  For every t in [0, rows):
+ *   out[t, :] = paged_cache[slot_mapping[t] * slot_stride + ...]  if t is among cached_rows and slot_mapping[t] >= 0,
+ *             = hidden[i, :]                                      if t is new_rows[i] (a negative entry counts from the end),
+ *             = 0                                                 otherwise.
+ * Rows and strides in multiples of 16 bytes, rows of at least 512 (APS_ERR_UNSUPPORTED otherwise).
+ * scratch: int64 [rows] of device memory.
+ */
+int aps_gather_hidden_rows(void* out, const void* hidden, const void* paged_cache,
+                           const int64_t* slot_mapping, const int64_t* new_rows, int64_t n_new,
+                           const int64_t* cached_rows, int64_t n_cached, int64_t rows,
+                           int hidden_size, int64_t out_stride, int64_t hidden_stride,
+                           int64_t slot_stride, int64_t* scratch, int dtype, void* stream);
+
+/*
  * Replaces mixed_cache_ops.mixed_kv_to_cache (mc.cu:179-230, kernel mc.cu:56-116;
  * called at fa.py:363-373):
  *   b in [0, n_kv):  tok = kv_cache_use_tot[b], slot = slot_mapping[tok]:
