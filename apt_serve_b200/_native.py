@@ -82,6 +82,7 @@ PROTOTYPES = {
     "aps_decode_metadata_scratch_bytes": (c_size_t, [c_int]),
     "aps_derive_private_tables": (c_int, [c_void_p] * 4 + [c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int,
                                           c_int64, c_int, c_void_p]),
+    "aps_expand_decode_lists": (c_int, [c_void_p] * 6 + [c_int] * 3 + [c_void_p] * 9 + [c_int64, c_int64, c_void_p]),
     "aps_expand_decode_metadata": (c_int, [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 8 +
                                    [c_int64, c_int64, c_void_p, c_void_p, c_size_t, c_void_p]),
 }
@@ -121,6 +122,10 @@ def host_lib():
         handle.aps_measure_decode_batch.argtypes = [ctypes.py_object] * 3 + [c_int64] + [c_void_p] * 3
         handle.aps_pack_decode_batch.restype = c_int
         handle.aps_pack_decode_batch.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 3 + [c_void_p]
+        handle.aps_measure_decode_lists.restype = c_int
+        handle.aps_measure_decode_lists.argtypes = [ctypes.py_object] * 4 + [c_int64] + [c_void_p] * 3
+        handle.aps_pack_decode_lists.restype = c_int
+        handle.aps_pack_decode_lists.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 4 + [c_void_p]
         _host_lib = handle
     return _host_lib
 

@@ -120,6 +120,75 @@ fill_kernel(MetaLayout L, MetaOut O, const int32_t* __restrict__ block_tables,
   }
 }
 
+// The same from tables that nobody has padded, in one launch: a CTA sums up the requests before its own by itself (256 requests: 1 KB a CTA)
+// instead of reading what a layout kernel has left (256 OPT-13B requests, the whole call: 157 us with the two launches and sections padded to
+// 128 bytes, 129 so; 163 with tables padded on the host), and pads the request's tables besides: the private one, the shared one (zero
+// for K/V-cached requests) and the one that the type selects.
+struct MetaLists { const int32_t* own; const int32_t* own_at; const int32_t* shared; const int32_t* shared_at; int32_t* tables; };
+
+__global__ void __launch_bounds__(256)
+expand_lists_kernel(const MetaLists T, MetaOut O, const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ cache_type, int batch,
+                    int max_blocks, int block_size) {
+  __shared__ int s_sum[8][6];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t plane = (int64_t)batch * max_blocks;
+  for (int r = blockIdx.x; r < batch; r += gridDim.x) {
+    // hidden requests and their tokens before r, and in all
+    int v[4] = {0, 0, 0, 0};
+    for (int i = threadIdx.x; i < batch; i += 256) {
+      const int len = cache_type[i] != 0 ? max(1, min(seq_lens[i], max_blocks * block_size)) : 0;
+      if (i < r) { v[0] += len > 0; v[1] += len; }
+      v[2] += len > 0; v[3] += len;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+      if (lane == 0) s_sum[warp][k] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = 0;
+      for (int w = 0; w < 8; ++w) v[k] += s_sum[w][k];
+    }
+    __syncthreads();   // before the next request's
+    const int hid_ord = v[0], kv_ord = r - v[0];
+    const int64_t h0 = v[1], e0 = h0 + kv_ord;
+    const bool hid = cache_type[r] != 0;
+    const int32_t *priv = T.own + T.own_at[r], *shar = T.shared + T.shared_at[r];
+    const int n_priv = min(T.own_at[r + 1] - T.own_at[r], max_blocks), n_shar = min(T.shared_at[r + 1] - T.shared_at[r], max_blocks);
+    int32_t* tables = T.tables + (int64_t)r * max_blocks;
+    for (int b = threadIdx.x; b < max_blocks; b += 256) {
+      const int32_t p = b < n_priv ? priv[b] : 0, s = hid && b < n_shar ? shar[b] : 0;
+      tables[b] = p; tables[plane + b] = s; tables[2 * plane + b] = hid ? s : p;
+    }
+    // the device-side totals must be what the caller sized (and NULL-ed) the outputs for
+    if (v[3] + (int64_t)(batch - v[2]) != O.cap_tot || v[3] != O.cap_hidden || batch - v[2] != O.cap_kv_req || v[2] != O.cap_hid_req) continue;
+    const int len = max(1, min(seq_lens[r], max_blocks * block_size));
+    if (hid) {
+      for (int j = threadIdx.x; j < len; j += 256) {
+        const int b = j / block_size, o = j % block_size;
+        O.slot_mapping[e0 + j] = (int64_t)(b < n_priv ? priv[b] : 0) * block_size + o;
+        O.slot_mapping_shared[h0 + j] = (int64_t)(b < n_shar ? shar[b] : 0) * block_size + o;
+        O.hidden_cache_use_tot[h0 + j] = e0 + j;
+        // every earlier request holds exactly one "current token" entry, and so far none of this one
+        if (j < len - 1) O.hidden_holder_pull[e0 + j - r] = e0 + j;
+      }
+      if (threadIdx.x == 0) {
+        O.hidden_holder_upd[r] = e0 + len - 1;
+        O.hidden_cache_store_tot[hid_ord] = e0 + len - 1;
+        O.hidden_cache_use_input[hid_ord] = r;
+      }
+    } else if (threadIdx.x == 0) {
+      const int j = len - 1, b = j / block_size;
+      O.slot_mapping[e0] = (int64_t)(b < n_priv ? priv[b] : 0) * block_size + j % block_size;
+      O.kv_cache_use_tot[kv_ord] = e0;
+      O.hidden_holder_upd[r] = e0;
+    }
+  }
+}
+
 // Private block tables and the cache-type mask from the reference's decode metadata (what the fused
 // layer-step needs and the reference does not ship): request r is hidden-cached if hidden_rows lists
 // it; its private blocks are then read off its run of slot_mapping, which ends at holder_upd[r], one
@@ -260,4 +329,31 @@ extern "C" int aps_expand_decode_metadata(const int32_t* block_tables, const int
   fill_kernel<<<grid, 256, 0, cs>>>(L, O, block_tables, block_tables_shared, seq_lens, cache_type,
                                     batch, max_blocks_per_seq, block_size);
   return launch_status("fill_kernel");
+}
+
+// One launch; nothing is padded on the host and the tables that the other calls take are left on the device.
+extern "C" int aps_expand_decode_lists(const int32_t* entries, const int32_t* starts, const int32_t* shared_entries,
+                                       const int32_t* shared_starts, const int32_t* seq_lens, const int32_t* cache_type, int batch,
+                                       int max_blocks_per_seq, int block_size, int32_t* tables, int64_t* slot_mapping,
+                                       int64_t* slot_mapping_shared, int64_t* hidden_cache_use_tot, int64_t* kv_cache_use_tot,
+                                       int64_t* hidden_holder_upd, int64_t* hidden_holder_pull, int64_t* hidden_cache_store_tot,
+                                       int64_t* hidden_cache_use_input, int64_t num_tot_tokens, int64_t num_hidden_tokens,
+                                       void* stream) {
+  APS_REQUIRE(batch >= 0 && max_blocks_per_seq > 0 && block_size > 0 && num_tot_tokens >= batch && num_hidden_tokens >= 0 &&
+                  num_hidden_tokens <= num_tot_tokens && num_tot_tokens - num_hidden_tokens <= batch,
+              APS_ERR_SHAPE, "expand_decode_lists: bad sizes (N_tot = %lld, N_h = %lld, batch = %d)", (long long)num_tot_tokens,
+              (long long)num_hidden_tokens, batch);
+  if (batch == 0) return APS_OK;
+  APS_REQUIRE(entries && starts && shared_entries && shared_starts && seq_lens && cache_type && tables && slot_mapping && hidden_holder_upd &&
+                  (num_hidden_tokens == 0 || (slot_mapping_shared && hidden_cache_use_tot && hidden_cache_store_tot && hidden_cache_use_input)) &&
+                  (num_tot_tokens == num_hidden_tokens || kv_cache_use_tot) && (num_tot_tokens == batch || hidden_holder_pull),
+              APS_ERR_NULL_POINTER, "expand_decode_lists: null pointer");
+  const MetaOut O{slot_mapping, slot_mapping_shared, hidden_cache_use_tot, kv_cache_use_tot,
+                  hidden_holder_upd, hidden_holder_pull, hidden_cache_store_tot, hidden_cache_use_input,
+                  num_tot_tokens, num_hidden_tokens, num_tot_tokens - num_hidden_tokens,
+                  batch - (num_tot_tokens - num_hidden_tokens)};
+  const int grid = batch < sm_count() * 8 ? batch : sm_count() * 8;
+  expand_lists_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(MetaLists{entries, starts, shared_entries, shared_starts, tables}, O, seq_lens, cache_type,
+                                                              batch, max_blocks_per_seq, block_size);
+  return launch_status("expand_lists_kernel");
 }

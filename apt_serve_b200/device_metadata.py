@@ -27,11 +27,16 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
                            device) -> DecodeMetadata:
     """Same arguments and result as ``metadata.build_decode_metadata``, with the tensors
     created on ``device`` by the expansion kernels.  Host work is O(number of blocks):
-    padding the two block tables.  Nothing waits for the device: one copy from pinned memory and two launches on
-    the current stream.  The tensors are sections of two allocations (what came from the host, what the kernels wrote)."""
+    reading the two block tables (plain lists natively, unpadded).  Nothing waits for the device: one copy from pinned memory and one
+    launch (two for padded tables) on the current stream.  The tensors are sections of three allocations (what came from the host, the tables, the indices)."""
     dev = torch.device(device)
     b = len(seq_lens)
-    lens, types, (n_h, n_hid_tok, width, least, most) = _measure(seq_lens, use_hidden, block_tables, b)
+    measured = _measure_lists(seq_lens, use_hidden, block_tables, block_tables_4_shared, b)
+    if measured is None:
+        lens, types, counts = _measure(seq_lens, use_hidden, block_tables, b)
+    else:
+        lens, types, counts, entries = measured
+    n_h, n_hid_tok, width, least, most = counts
     if b and least < 1:
         # the kernels count a length below 1 as 1; the host counts must agree with them
         raise ValueError("expand_decode_metadata: every sequence length must be >= 1 "
@@ -43,29 +48,66 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         raise RuntimeError("expand_decode_metadata: not during stream capture (the tables come from host memory)")
     n_kv = b - n_h
     n_tot = n_hid_tok + n_kv
-    # everything the device gets, in one buffer and one copy: the K/V-cached rows, three tables (private, shared, and
-    # the reference's: shared for hidden requests, private otherwise), lengths and types; sections of 128 bytes
-    cuts = _cuts((2 * n_kv, b * width, b * width, b * width, b, b), 32)
-    host = torch.empty(sum(cuts), dtype=torch.int32, pin_memory=dev.type == "cuda")
-    _fill_host(host, cuts, block_tables, block_tables_4_shared, lens, types, width, n_h)
-    rows, priv, shared, ref, d_lens, d_type = host.to(dev, non_blocking=True).split(cuts)[::2]
-    priv, shared, ref = priv.view(b, width), shared.view(b, width), ref.view(b, width)
-    # the eight index tensors and the kernels' scratch, again sections of one buffer
     lib = N.lib()
-    cuts = _cuts((n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h, (lib.aps_decode_metadata_scratch_bytes(b) + 7) // 8), 16)
-    parts = torch.empty(sum(cuts), dtype=torch.int64, device=dev).split(cuts)[::2]
+    index_sizes = (n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h)   # the eight index tensors
+    host = None
+    if measured is not None:
+        # the lists' entries one behind the other; the GPU pads them into the three tables
+        n_own, n_shared = entries
+        at = 2 * (n_kv + b) + 2 * (b + 1)   # the entries, behind the K/V-cached rows, lengths, types and two lists of starts
+        host = torch.empty(at + n_own + n_shared, dtype=torch.int32, pin_memory=dev.type == "cuda")
+        if N.host_lib().aps_pack_decode_lists(block_tables, block_tables_4_shared, lens.ctypes.data, types.ctypes.data, b, n_h, *entries,
+                                              host.data_ptr()) != 0:
+            host = None   # what the general path takes or refuses
+    if host is not None:
+        rows, d_lens, d_type, lists = host.to(dev, non_blocking=True).split((2 * n_kv, b, b, 2 * (b + 1) + n_own + n_shared))
+        kv_rows = rows.view(torch.int64)
+        starts, own = lists.data_ptr(), lists.data_ptr() + 8 * (b + 1)
+        tables = torch.empty(3, b, width, dtype=torch.int32, device=dev)
+        priv, ref = tables[0], tables[2]
+        parts = torch.empty(sum(index_sizes), dtype=torch.int64, device=dev).split(index_sizes)
+        with N.on_device(dev):
+            N.check(lib.aps_expand_decode_lists(
+                own, starts, own + 4 * n_own, starts + 4 * (b + 1), d_lens.data_ptr(), d_type.data_ptr(), b, width, block_size,
+                tables.data_ptr(), *(t.data_ptr() for t in parts), n_tot, n_hid_tok, N.current_stream(dev)))
+    else:
+        # everything the device gets, in one buffer and one copy: the K/V-cached rows, three tables (private, shared, and
+        # the reference's: shared for hidden requests, private otherwise), lengths and types; sections of 128 bytes
+        cuts = _cuts((2 * n_kv, b * width, b * width, b * width, b, b), 32)
+        host = torch.empty(sum(cuts), dtype=torch.int32, pin_memory=dev.type == "cuda")
+        _fill_host(host, cuts, block_tables, block_tables_4_shared, lens, types, width, n_h)
+        rows, priv, shared, ref, d_lens, d_type = host.to(dev, non_blocking=True).split(cuts)[::2]
+        priv, shared, ref = priv.view(b, width), shared.view(b, width), ref.view(b, width)
+        kv_rows = rows.view(torch.int64)
+        cuts = _cuts((*index_sizes, (lib.aps_decode_metadata_scratch_bytes(b) + 7) // 8), 16)   # and the kernels' scratch
+        parts = torch.empty(sum(cuts), dtype=torch.int64, device=dev).split(cuts)[::2]
+        with N.on_device(dev):
+            N.check(lib.aps_expand_decode_metadata(
+                N.ptr(priv), N.ptr(shared), N.ptr(d_lens), N.ptr(d_type), b, width, block_size,
+                *(t.data_ptr() for t in parts[:8]), n_tot, n_hid_tok, None, N.ptr(parts[8]), parts[8].numel() * 8,
+                N.current_stream(dev)))
     names = ("slot_mapping", "slot_mapping_shared", "hidden_cache_use_tot", "kv_cache_use_tot",
              "hidden_holder_upd", "hidden_holder_pull", "hidden_cache_store_tot", "hidden_cache_use_input")
-    with N.on_device(dev):
-        N.check(lib.aps_expand_decode_metadata(
-            N.ptr(priv), N.ptr(shared), N.ptr(d_lens), N.ptr(d_type), b, width, block_size,
-            *(t.data_ptr() for t in parts[:8]), n_tot, n_hid_tok, None, N.ptr(parts[8]), parts[8].numel() * 8,
-            N.current_stream(dev)))
     return DecodeMetadata(
         block_tables=ref, seq_lens_tensor=d_lens, seq_lens=lens.tolist(),
         num_hidden_cache_tokens=n_h, num_tot_tokens=n_tot, num_decode_tokens=b,
         max_decode_seq_len=most, private_block_tables=priv,
-        cache_type=d_type, kv_request_rows=rows.view(torch.int64), **dict(zip(names, parts)))
+        cache_type=d_type, kv_request_rows=kv_rows, **dict(zip(names, parts)))
+
+
+def _measure_lists(seq_lens, use_hidden, tables, shared_tables, b):
+    """Lengths, types and counts as ``_measure`` has them and the entries of the private and the shared tables; None unless
+    everything is plain lists that the host library reads and shared tables fit the private ones' width."""
+    lib = N.host_lib()
+    if lib is None or not b:
+        return None
+    both = np.empty((2, b), dtype=np.int32)
+    counts = np.empty(7, dtype=np.int64)
+    at = both.ctypes.data
+    if lib.aps_measure_decode_lists(seq_lens, use_hidden, tables, shared_tables, b, at, at + 4 * b, counts.ctypes.data) != 0:
+        return None
+    n_h, tokens, width, least, most, own, shared = counts.tolist()
+    return both[0], both[1], (n_h, tokens, max(1, width), least, most), (own, shared)
 
 
 def _cuts(sizes, pitch):

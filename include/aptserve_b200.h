@@ -457,6 +457,20 @@ int aps_expand_decode_metadata(const int32_t* block_tables, const int32_t* block
                                size_t scratch_bytes, void* stream);
 
 /*
+ * The same from tables that nobody has padded, in one launch: request r's private table is entries[starts[r] ... starts[r + 1]), its shared one
+ * shared_entries[shared_starts[r] ... shared_starts[r + 1]) (all int32 device memory, batch + 1 starts; what a table does not have
+ * counts as 0).  tables int32 [3, B, max_blocks] receives the padded private tables, the shared ones (zero for K/V-cached requests) and
+ * the reference's (the one that the request's type selects), also when the counts differ.
+ */
+int aps_expand_decode_lists(const int32_t* entries, const int32_t* starts, const int32_t* shared_entries,
+                            const int32_t* shared_starts, const int32_t* seq_lens, const int32_t* cache_type, int batch,
+                            int max_blocks_per_seq, int block_size, int32_t* tables, int64_t* slot_mapping,
+                            int64_t* slot_mapping_shared, int64_t* hidden_cache_use_tot, int64_t* kv_cache_use_tot,
+                            int64_t* hidden_holder_upd, int64_t* hidden_holder_pull,
+                            int64_t* hidden_cache_store_tot, int64_t* hidden_cache_use_input,
+                            int64_t num_tot_tokens, int64_t num_hidden_tokens, void* stream);
+
+/*
  * The private block tables and the cache-type mask of a decode batch, from the reference's own metadata
  * (model_runner.py:515-564: a hidden-cached request's block_tables row is its SHARED table, its
  * private slots are its run of slot_mapping).  tables: int32 [B, max_blocks_per_seq], contiguous;

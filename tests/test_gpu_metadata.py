@@ -219,3 +219,43 @@ def test_a_step_on_bad_metadata_touches_no_other_request(heads, d, e, dtype, fau
     if good:
         tol = 1e-4 if dtype == torch.float32 else 4e-3
         assert torch.allclose(out[good].float(), want[good].float(), rtol=tol, atol=tol)
+
+
+# tables as lists that the GPU pads and tables padded on the host; rows shorter than their request, empty ones, tuples, a wide table of a
+# K/V-cached request, more requests than a round of the fill kernel's CTAs
+@pytest.mark.parametrize("kind", ["plain", "short rows", "tuples", "one wide", "many"])
+def test_lists_and_padded_tables_agree(kind, monkeypatch):
+    from apt_serve_b200 import device_metadata as DM
+    rng = np.random.default_rng(5)
+    lens = [int(x) for x in rng.integers(1, 600 if kind != "many" else 40, size=1400 if kind == "many" else 23)]
+    hid = [bool(i % 3) for i in range(len(lens))]
+    make = lambda s: [int(x) for x in rng.integers(0, 2 ** 20, size=-(-s // 16))]
+    tables, shared = [make(s) for s in lens], [make(s) if h else [] for s, h in zip(lens, hid)]
+    if kind == "short rows":
+        tables, shared = [t[: len(t) // 2] for t in tables], [t[: len(t) // 3] for t in shared]
+        tables[4] = tables[4] + make(900)
+    elif kind == "tuples":
+        tables, shared = [tuple(t) for t in tables], [tuple(t) for t in shared]
+    elif kind == "one wide":
+        tables[3] = make(5000)
+    assert DM._measure_lists(lens, hid, tables, shared, len(lens)) is not None
+    got = expand_decode_metadata(lens, hid, tables, shared, 16, "cuda")
+    monkeypatch.setattr(DM, "_measure_lists", lambda *a: None)
+    want = expand_decode_metadata(lens, hid, tables, shared, 16, "cuda")
+    for name, value in vars(want).items():
+        other = getattr(got, name)
+        assert torch.equal(value, other) if isinstance(value, torch.Tensor) else value == other, name
+
+
+def test_lists_that_are_not_plain_take_the_general_path():
+    lens, hid = [20, 40, 7], [True, False, True]
+    tables, shared = [[1, 2], [3, 4, 5], [6]], [[7, 8], [], [9]]
+    want = expand_decode_metadata(lens, hid, tables, shared, 16, "cuda")
+    for other in ([np.int64(1), 2], np.array([1, 2], dtype=np.int32)):
+        got = expand_decode_metadata(lens, hid, [other] + tables[1:], shared, 16, "cuda")
+        for name, value in vars(want).items():
+            assert torch.equal(value, getattr(got, name)) if isinstance(value, torch.Tensor) else value == getattr(got, name), name
+    with pytest.raises(ValueError):   # a shared table wider than the widest private one
+        expand_decode_metadata(lens, hid, tables, [[7, 8, 9, 10], [], [9]], 16, "cuda")
+    with pytest.raises((ValueError, OverflowError)):
+        expand_decode_metadata(lens, hid, tables, [[7, 2 ** 31], [], [9]], 16, "cuda")
