@@ -823,11 +823,9 @@ struct SumColumns {
       col = np; set = slice * np; rests = 2 * slice * np <= 256 ? 1 : 0; rest = rests ? n_hi * set : 0;
     }
   }
-  // the k-th accumulator of a column block that has `used` first ones: those, then the rests'
-  template <bool STACKED>
+  // stacked: the k-th accumulator of a column block that has `used` first ones: those, then the rests'
   __device__ __forceinline__ uint32_t at(int k, int used, int terms, int np) const {
-    if (k >= used) return rest + (k - used) * np;
-    return STACKED ? (k == 0 ? 0u : (uint32_t)((terms - 1 + k) * np)) : k * set;
+    return k >= used ? rest + (k - used) * np : k == 0 ? 0u : (uint32_t)((terms - 1 + k) * np);
   }
   // The weights of the request's block b have the first term last where b & turn_mask() is 1.
   __host__ __device__ int turn_mask() const { return stacked ? (int)n_hi - 1 : 0; }
@@ -1238,11 +1236,13 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       tc_fence_after();
       const int used = (int)min(cols.n_hi, (uint32_t)n_blk), n_in = used + cols.rests;
       // accumulators of a column block: four first terms' and the rests'; that many read together (142 - 144 registers; one after the other,
-      // in 128, short requests' items wait for it: 16 OPT-13B requests of 60 tokens 16.5 -> 19 us)
+      // in 128, short requests' items wait for it: 16 OPT-13B requests of 60 tokens 16.5 -> 19 us).  Not stacked, where one set of rests
+      // is all there is, four accumulators at even distances and no table of them: bf16, 91 OPT-13B requests of 71 tokens 71.5 -> 67.8,
+      // 60 of 200 61.4 -> 59, 128 of 400 73.7 -> 71.9
       constexpr int kMost = NT + 3, kAtOnce = 6 - NT;
       uint32_t off[kMost];
 #pragma unroll
-      for (int k = 1; k < kMost; ++k) off[k] = cols.at<STACKED>(k, used, NT, np);
+      for (int k = 1; STACKED && k < kMost; ++k) off[k] = cols.at(k, used, NT, np);
       const int h_steps = np / 16;
       for (int it = turn; it < n_col * h_steps; it += n_epilogue / 4) {
         const int col = it / h_steps, h0 = (it - col * h_steps) * 16;
@@ -1250,20 +1250,38 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         uint32_t v[16];
         const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256 + col * cols.col + h0;
         tmem_ld16(at, v);
+        if constexpr (STACKED) {
 #pragma unroll
-        for (int k0 = 1; k0 < kMost; k0 += kAtOnce) {
-          if (k0 > 1 && k0 >= n_in) break;
-          uint32_t more[kAtOnce][16];
+          for (int k0 = 1; k0 < kMost; k0 += kAtOnce) {
+            if (k0 > 1 && k0 >= n_in) break;
+            uint32_t more[kAtOnce][16];
 #pragma unroll
-          for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
-            if (k < n_in) tmem_ld16(at + off[k], more[k - k0]);
+            for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
+              if (k < n_in) tmem_ld16(at + off[k], more[k - k0]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              float x = __uint_as_float(v[j]);
+#pragma unroll
+              for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
+                if (k < n_in) x += __uint_as_float(more[k - k0][j]);
+              v[j] = __float_as_uint(x);
+            }
+          }
+        } else {
+          uint32_t more[3][16], rest[16];
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            if (i + 1 < used) tmem_ld16(at + (i + 1) * cols.set, more[i]);
+          if (cols.rests != 0) tmem_ld16(at + cols.rest, rest);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             float x = __uint_as_float(v[j]);
 #pragma unroll
-            for (int k = k0; k < k0 + kAtOnce && k < kMost; ++k)
-              if (k < n_in) x += __uint_as_float(more[k - k0][j]);
+            for (int i = 0; i < 3; ++i)
+              if (i + 1 < used) x += __uint_as_float(more[i][j]);
+            if (cols.rests != 0) x += __uint_as_float(rest[j]);
             v[j] = __float_as_uint(x);
           }
         }
