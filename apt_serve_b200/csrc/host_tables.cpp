@@ -42,6 +42,17 @@ bool pack_row(PyObject* row, int64_t width, int32_t* out) {
   return true;
 }
 
+// The entries of a list or tuple.  The integers lie all over the heap: they are asked for ahead of their turn.
+bool read_entries(PyObject* row, int32_t* out) {
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(row);
+  PyObject** items = PySequence_Fast_ITEMS(row);
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    if (i + 12 < n) __builtin_prefetch(items[i + 12]);
+    if (!read_int(items[i], out + i)) return false;
+  }
+  return true;
+}
+
 }  // namespace
 
 // priv, shared, ref: [batch][width].  Row r of priv is tables[r], of shared shared_tables[r] for a hidden-cached request and
@@ -123,71 +134,69 @@ extern "C" int aps_pack_decode_batch(PyObject* tables, PyObject* shared_tables, 
   return 0;
 }
 
-// What aps_pack_decode_lists is sized by, besides aps_measure_decode_batch's counts: counts[5], the entries of the tables, and counts[6],
-// of the hidden-cached requests' shared tables, none of which may be wider than the widest table.
-extern "C" int aps_measure_decode_lists(PyObject* seq_lens, PyObject* use_hidden, PyObject* tables, PyObject* shared_tables, int64_t batch,
-                                        int32_t* lens, int32_t* types, int64_t* counts) {
-  if (aps_measure_decode_batch(seq_lens, use_hidden, tables, batch, lens, types, counts) != 0 || !PyList_CheckExact(shared_tables) ||
-      PyList_GET_SIZE(shared_tables) != batch)
-    return 1;
-  int64_t own = 0, shared = 0;
+// A decode batch without padding, which the GPU adds: one behind the other the K/V-cached rows (int64), lengths, types, where each
+// request's table begins among the entries (batch + 1), the same of the shared tables, the entries, the hidden-cached requests'
+// shared entries.  256 OPT-13B requests (18 000 entries in tables of 128): 76 KB instead of 396 KB written to the staging
+// buffer and copied to the GPU.
+//
+// Sizes and entries are read in one call, during which the interpreter lock is not given away and no Python code runs: what comes
+// back is the lists as they were at one moment, whatever other threads append to them (sized in one call and read in another, a table
+// that had grown in between was written past the end of the buffer).
+// counts = {hidden-cached requests, their tokens, the widest private table, the shortest and the longest length, entries,
+// shared entries}.  None for anything but lists of `batch` plain integers, booleans and lists or tuples of plain integers, and for
+// shared tables wider than the widest private one.
+extern "C" PyObject* aps_read_decode_lists(PyObject* seq_lens, PyObject* use_hidden, PyObject* tables, PyObject* shared_tables,
+                                           int64_t batch, int64_t* counts) {
+  PyObject* const given[4] = {seq_lens, use_hidden, tables, shared_tables};
+  for (PyObject* list : given)
+    if (!PyList_CheckExact(list) || PyList_GET_SIZE(list) != batch) Py_RETURN_NONE;
+  auto row_size = [](PyObject* row) -> int64_t {
+    return PyList_CheckExact(row) || PyTuple_CheckExact(row) ? (int64_t)PySequence_Fast_GET_SIZE(row) : -1;
+  };
+  int64_t n_hidden = 0, width = 0, widest_shared = 0, n_own = 0, n_shared = 0;
   for (int64_t r = 0; r < batch; ++r) {
-    own += PySequence_Fast_GET_SIZE(PyList_GET_ITEM(tables, r));
-    if (types[r] == 0) continue;
-    PyObject* s = PyList_GET_ITEM(shared_tables, r);
-    if (!PyList_CheckExact(s) && !PyTuple_CheckExact(s)) return 1;
-    const int64_t n = PySequence_Fast_GET_SIZE(s);
-    if (n > counts[2]) return 1;
-    shared += n;
+    PyObject* h = PyList_GET_ITEM(use_hidden, r);
+    const bool hidden = h == Py_True;
+    if (!hidden && h != Py_False) Py_RETURN_NONE;
+    const int64_t own = row_size(PyList_GET_ITEM(tables, r)), shared = hidden ? row_size(PyList_GET_ITEM(shared_tables, r)) : 0;
+    if (own < 0 || shared < 0) Py_RETURN_NONE;
+    n_hidden += hidden; n_own += own; n_shared += shared;
+    if (own > width) width = own;
+    if (shared > widest_shared) widest_shared = shared;
   }
-  if (own > INT32_MAX || shared > INT32_MAX) return 1;
-  counts[5] = own; counts[6] = shared;
-  return 0;
-}
-
-namespace {
-
-// The entries of one row.  The integers lie all over the heap: they are asked for ahead of their turn.
-bool pack_entries(PyObject* row, int32_t* out) {
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(row);
-  PyObject** items = PySequence_Fast_ITEMS(row);
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    if (i + 12 < n) __builtin_prefetch(items[i + 12]);
-    if (!read_int(items[i], out + i)) return false;
-  }
-  return true;
-}
-
-}  // namespace
-
-// The same batch without padding, which the GPU adds: one behind the other the K/V-cached rows (int64), lengths, types, where each
-// request's table begins among the entries (batch + 1), the same of the shared tables, the entries, the shared tables' entries.  Returns as aps_pack_block_tables does.  256 OPT-13B requests (18 000 entries in tables of 128): 76 KB instead of 396 KB
-// written to the staging buffer and copied to the GPU.
-extern "C" int aps_pack_decode_lists(PyObject* tables, PyObject* shared_tables, const int32_t* lens, const int32_t* types, int64_t batch,
-                                     int64_t n_hidden, int64_t n_own, int64_t n_shared, int32_t* out) {
-  int64_t* rows = (int64_t*)out;
-  int32_t* d_lens = out + 2 * (batch - n_hidden);
-  int32_t* d_types = d_lens + batch;
-  int32_t* own_at = d_types + batch;
+  if (widest_shared > width || n_own > INT32_MAX || n_shared > INT32_MAX) Py_RETURN_NONE;
+  const int64_t words = 2 * (batch - n_hidden) + 2 * batch + 2 * (batch + 1) + n_own + n_shared;
+  PyObject* result = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)(words * sizeof(int32_t)));
+  if (result == nullptr) return nullptr;
+  // the bytes begin 32 behind an allocation's start: aligned for the rows
+  int64_t* rows = (int64_t*)PyBytes_AS_STRING(result);
+  int32_t* lens = (int32_t*)PyBytes_AS_STRING(result) + 2 * (batch - n_hidden);
+  int32_t* types = lens + batch;
+  int32_t* own_at = types + batch;
   int32_t* shared_at = own_at + batch + 1;
   int32_t* own = shared_at + batch + 1;
   int32_t* shared = own + n_own;
-  int64_t o = 0, s = 0;
+  int64_t tokens = 0, least = INT32_MAX, most = 0, o = 0, s = 0;
   for (int64_t r = 0; r < batch; ++r) {
+    PyObject *t = PyList_GET_ITEM(tables, r), *x = PyList_GET_ITEM(shared_tables, r);
+    types[r] = PyList_GET_ITEM(use_hidden, r) == Py_True ? 1 : 0;
     own_at[r] = (int32_t)o; shared_at[r] = (int32_t)s;
-    PyObject* t = PyList_GET_ITEM(tables, r);
-    if (!pack_entries(t, own + o)) return 1;
+    if (!read_int(PyList_GET_ITEM(seq_lens, r), lens + r) || !read_entries(t, own + o) || (types[r] != 0 && !read_entries(x, shared + s))) {
+      Py_DECREF(result);
+      Py_RETURN_NONE;
+    }
     o += PySequence_Fast_GET_SIZE(t);
     if (types[r] != 0) {
-      PyObject* x = PyList_GET_ITEM(shared_tables, r);
-      if (!pack_entries(x, shared + s)) return 1;
       s += PySequence_Fast_GET_SIZE(x);
+      tokens += lens[r];
     } else {
       *rows++ = r;
     }
+    if (lens[r] < least) least = lens[r];
+    if (lens[r] > most) most = lens[r];
   }
   own_at[batch] = (int32_t)o; shared_at[batch] = (int32_t)s;
-  memcpy(d_lens, lens, (size_t)batch * sizeof(int32_t));
-  memcpy(d_types, types, (size_t)batch * sizeof(int32_t));
-  return o == n_own && s == n_shared ? 0 : 1;
+  const int64_t all[7] = {n_hidden, tokens, width, least, most, n_own, n_shared};
+  memcpy(counts, all, sizeof(all));
+  return result;
 }

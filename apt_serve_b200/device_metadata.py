@@ -12,6 +12,7 @@ to ``metadata.build_decode_metadata``.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import List, Sequence
 
 import numpy as np
@@ -31,11 +32,11 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     launch (two for padded tables) on the current stream.  The tensors are sections of three allocations (what came from the host, the tables, the indices)."""
     dev = torch.device(device)
     b = len(seq_lens)
-    measured = _measure_lists(seq_lens, use_hidden, block_tables, block_tables_4_shared, b)
-    if measured is None:
+    read = _read_lists(seq_lens, use_hidden, block_tables, block_tables_4_shared, b)
+    if read is None:
         lens, types, counts = _measure(seq_lens, use_hidden, block_tables, b)
     else:
-        lens, types, counts, entries = measured
+        lens, counts, (n_own, n_shared), packed = read
     n_h, n_hid_tok, width, least, most = counts
     if b and least < 1:
         # the kernels count a length below 1 as 1; the host counts must agree with them
@@ -50,16 +51,10 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     n_tot = n_hid_tok + n_kv
     lib = N.lib()
     index_sizes = (n_tot, n_hid_tok, n_hid_tok, n_kv, b, n_tot - b, n_h, n_h)   # the eight index tensors
-    host = None
-    if measured is not None:
+    if read is not None:
         # the lists' entries one behind the other; the GPU pads them into the three tables
-        n_own, n_shared = entries
-        at = 2 * (n_kv + b) + 2 * (b + 1)   # the entries, behind the K/V-cached rows, lengths, types and two lists of starts
-        host = torch.empty(at + n_own + n_shared, dtype=torch.int32, pin_memory=dev.type == "cuda")
-        if N.host_lib().aps_pack_decode_lists(block_tables, block_tables_4_shared, lens.ctypes.data, types.ctypes.data, b, n_h, *entries,
-                                              host.data_ptr()) != 0:
-            host = None   # what the general path takes or refuses
-    if host is not None:
+        host = torch.empty(len(packed) // 4, dtype=torch.int32, pin_memory=dev.type == "cuda")
+        ctypes.memmove(host.data_ptr(), packed, len(packed))
         rows, d_lens, d_type, lists = host.to(dev, non_blocking=True).split((2 * n_kv, b, b, 2 * (b + 1) + n_own + n_shared))
         kv_rows = rows.view(torch.int64)
         starts, own = lists.data_ptr(), lists.data_ptr() + 8 * (b + 1)
@@ -95,19 +90,19 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         cache_type=d_type, kv_request_rows=kv_rows, **dict(zip(names, parts)))
 
 
-def _measure_lists(seq_lens, use_hidden, tables, shared_tables, b):
-    """Lengths, types and counts as ``_measure`` has them and the entries of the private and the shared tables; None unless
-    everything is plain lists that the host library reads and shared tables fit the private ones' width."""
+def _read_lists(seq_lens, use_hidden, tables, shared_tables, b):
+    """Lengths and counts as ``_measure`` has them, the entries of the private and the shared tables, and the batch as
+    ``aps_read_decode_lists`` lays it out; None unless everything is plain lists that the host library reads and shared tables fit the
+    private ones' width."""
     lib = N.host_lib()
     if lib is None or not b:
         return None
-    both = np.empty((2, b), dtype=np.int32)
     counts = np.empty(7, dtype=np.int64)
-    at = both.ctypes.data
-    if lib.aps_measure_decode_lists(seq_lens, use_hidden, tables, shared_tables, b, at, at + 4 * b, counts.ctypes.data) != 0:
+    packed = lib.aps_read_decode_lists(seq_lens, use_hidden, tables, shared_tables, b, counts.ctypes.data)
+    if packed is None:
         return None
     n_h, tokens, width, least, most, own, shared = counts.tolist()
-    return both[0], both[1], (n_h, tokens, max(1, width), least, most), (own, shared)
+    return np.frombuffer(packed, np.int32, b, 8 * (b - n_h)), (n_h, tokens, max(1, width), least, most), (own, shared), packed
 
 
 def _cuts(sizes, pitch):
