@@ -123,7 +123,7 @@ def host_lib():
         handle.aps_pack_decode_batch.restype = c_int
         handle.aps_pack_decode_batch.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 3 + [c_void_p]
         handle.aps_read_decode_lists.restype = ctypes.py_object
-        handle.aps_read_decode_lists.argtypes = [ctypes.py_object] * 4 + [c_int64, c_void_p]
+        handle.aps_read_decode_lists.argtypes = [ctypes.py_object] * 4 + [c_int64, c_int64, c_void_p]
         _host_lib = handle
     return _host_lib
 

@@ -143,10 +143,11 @@ extern "C" int aps_pack_decode_batch(PyObject* tables, PyObject* shared_tables, 
 // back is the lists as they were at one moment, whatever other threads append to them (sized in one call and read in another, a table
 // that had grown in between was written past the end of the buffer).
 // counts = {hidden-cached requests, their tokens, the widest private table, the shortest and the longest length, entries,
-// shared entries}.  None for anything but lists of `batch` plain integers, booleans and lists or tuples of plain integers, and for
-// shared tables wider than the widest private one.
+// shared entries, the first request that has more tokens than its private table, or its shared one if it is hidden-cached, has
+// room for, or -1}.  None for anything but lists of `batch` plain integers, booleans and lists or tuples of plain integers, and
+// for shared tables wider than the widest private one.
 extern "C" PyObject* aps_read_decode_lists(PyObject* seq_lens, PyObject* use_hidden, PyObject* tables, PyObject* shared_tables,
-                                           int64_t batch, int64_t* counts) {
+                                           int64_t batch, int64_t block_size, int64_t* counts) {
   PyObject* const given[4] = {seq_lens, use_hidden, tables, shared_tables};
   for (PyObject* list : given)
     if (!PyList_CheckExact(list) || PyList_GET_SIZE(list) != batch) Py_RETURN_NONE;
@@ -176,7 +177,7 @@ extern "C" PyObject* aps_read_decode_lists(PyObject* seq_lens, PyObject* use_hid
   int32_t* shared_at = own_at + batch + 1;
   int32_t* own = shared_at + batch + 1;
   int32_t* shared = own + n_own;
-  int64_t tokens = 0, least = INT32_MAX, most = 0, o = 0, s = 0;
+  int64_t tokens = 0, least = INT32_MAX, most = 0, o = 0, s = 0, too_long = -1;
   for (int64_t r = 0; r < batch; ++r) {
     PyObject *t = PyList_GET_ITEM(tables, r), *x = PyList_GET_ITEM(shared_tables, r);
     types[r] = PyList_GET_ITEM(use_hidden, r) == Py_True ? 1 : 0;
@@ -185,18 +186,22 @@ extern "C" PyObject* aps_read_decode_lists(PyObject* seq_lens, PyObject* use_hid
       Py_DECREF(result);
       Py_RETURN_NONE;
     }
-    o += PySequence_Fast_GET_SIZE(t);
+    int64_t blocks = PySequence_Fast_GET_SIZE(t);
+    o += blocks;
     if (types[r] != 0) {
-      s += PySequence_Fast_GET_SIZE(x);
+      const int64_t n = PySequence_Fast_GET_SIZE(x);
+      s += n;
+      if (n < blocks) blocks = n;
       tokens += lens[r];
     } else {
       *rows++ = r;
     }
+    if (too_long < 0 && lens[r] > blocks * block_size) too_long = r;
     if (lens[r] < least) least = lens[r];
     if (lens[r] > most) most = lens[r];
   }
   own_at[batch] = (int32_t)o; shared_at[batch] = (int32_t)s;
-  const int64_t all[7] = {n_hidden, tokens, width, least, most, n_own, n_shared};
+  const int64_t all[8] = {n_hidden, tokens, width, least, most, n_own, n_shared, too_long};
   memcpy(counts, all, sizeof(all));
   return result;
 }

@@ -29,14 +29,16 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
     """Same arguments and result as ``metadata.build_decode_metadata``, with the tensors
     created on ``device`` by the expansion kernels.  Host work is O(number of blocks):
     reading the two block tables (plain lists natively, unpadded).  Nothing waits for the device: one copy from pinned memory and one
-    launch (two for padded tables) on the current stream.  The tensors are sections of three allocations (what came from the host, the tables, the indices)."""
+    launch (two for padded tables) on the current stream.  The tensors are sections of three allocations (what came from the host, the tables, the indices).
+    A request with more tokens than its private table has room for, or its shared one if it is hidden-cached, is refused
+    (``ValueError``; ``build_decode_metadata`` stops at it with an index error)."""
     dev = torch.device(device)
     b = len(seq_lens)
-    read = _read_lists(seq_lens, use_hidden, block_tables, block_tables_4_shared, b)
+    read = _read_lists(seq_lens, use_hidden, block_tables, block_tables_4_shared, b, block_size)
     if read is None:
         lens, types, counts = _measure(seq_lens, use_hidden, block_tables, b)
     else:
-        lens, counts, (n_own, n_shared), packed = read
+        lens, counts, (n_own, n_shared, too_long), packed = read
     n_h, n_hid_tok, width, least, most = counts
     if b and least < 1:
         # the kernels count a length below 1 as 1; the host counts must agree with them
@@ -44,6 +46,12 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
                          "(it includes the token being decoded)")
     if len(block_tables) != b:
         raise ValueError(f"expand_decode_metadata: {len(block_tables)} block tables for {b} sequences")
+    if read is None:
+        too_long = _first_too_long(lens, types, block_tables, block_tables_4_shared, block_size)
+    if too_long >= 0:
+        # its positions would be those of block 0, which is another request's, or not written at all
+        raise ValueError(f"expand_decode_metadata: request {too_long} has {lens[too_long]} tokens and no table for all of them "
+                         f"(blocks of {block_size})")
     if dev.type == "cuda" and torch.cuda.is_current_stream_capturing():
         # the graph would read the staging buffer again on every replay, long after it has been given back
         raise RuntimeError("expand_decode_metadata: not during stream capture (the tables come from host memory)")
@@ -90,19 +98,28 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
         cache_type=d_type, kv_request_rows=kv_rows, **dict(zip(names, parts)))
 
 
-def _read_lists(seq_lens, use_hidden, tables, shared_tables, b):
-    """Lengths and counts as ``_measure`` has them, the entries of the private and the shared tables, and the batch as
-    ``aps_read_decode_lists`` lays it out; None unless everything is plain lists that the host library reads and shared tables fit the
+def _read_lists(seq_lens, use_hidden, tables, shared_tables, b, block_size):
+    """Lengths and counts as ``_measure`` has them, (the entries of the private and of the shared tables, what
+    ``_first_too_long`` says), and the batch as ``aps_read_decode_lists`` lays it out; None unless everything is plain lists that the host library reads and shared tables fit the
     private ones' width."""
     lib = N.host_lib()
     if lib is None or not b:
         return None
-    counts = np.empty(7, dtype=np.int64)
-    packed = lib.aps_read_decode_lists(seq_lens, use_hidden, tables, shared_tables, b, counts.ctypes.data)
+    counts = np.empty(8, dtype=np.int64)
+    packed = lib.aps_read_decode_lists(seq_lens, use_hidden, tables, shared_tables, b, block_size, counts.ctypes.data)
     if packed is None:
         return None
-    n_h, tokens, width, least, most, own, shared = counts.tolist()
-    return np.frombuffer(packed, np.int32, b, 8 * (b - n_h)), (n_h, tokens, max(1, width), least, most), (own, shared), packed
+    n_h, tokens, width, least, most, *entries = counts.tolist()
+    return np.frombuffer(packed, np.int32, b, 8 * (b - n_h)), (n_h, tokens, max(1, width), least, most), entries, packed
+
+
+def _first_too_long(lens, types, tables, shared_tables, block_size):
+    """The first request with more tokens than its private table, or its shared one if it is hidden-cached, has room for; -1 if none has."""
+    needed = (-(-lens.astype(np.int64) // block_size)).tolist()
+    for r, (n, hidden, own) in enumerate(zip(needed, types.tolist(), tables)):
+        if n > len(own) or (hidden and (r >= len(shared_tables) or n > len(shared_tables[r]))):
+            return r
+    return -1
 
 
 def _cuts(sizes, pitch):

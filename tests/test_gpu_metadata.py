@@ -221,9 +221,9 @@ def test_a_step_on_bad_metadata_touches_no_other_request(heads, d, e, dtype, fau
         assert torch.allclose(out[good].float(), want[good].float(), rtol=tol, atol=tol)
 
 
-# tables as lists that the GPU pads and tables padded on the host; rows shorter than their request, empty ones, tuples, a wide table of a
-# K/V-cached request, more requests than a round of the fill kernel's CTAs
-@pytest.mark.parametrize("kind", ["plain", "short rows", "tuples", "one wide", "many"])
+# tables as lists that the GPU pads and tables padded on the host; rows with spare blocks, tuples, a wide table of a K/V-cached
+# request, more requests than a round of the fill kernel's CTAs
+@pytest.mark.parametrize("kind", ["plain", "spare blocks", "tuples", "one wide", "many"])
 def test_lists_and_padded_tables_agree(kind, monkeypatch):
     from apt_serve_b200 import device_metadata as DM
     rng = np.random.default_rng(5)
@@ -231,8 +231,8 @@ def test_lists_and_padded_tables_agree(kind, monkeypatch):
     hid = [bool(i % 3) for i in range(len(lens))]
     make = lambda s: [int(x) for x in rng.integers(0, 2 ** 20, size=-(-s // 16))]
     tables, shared = [make(s) for s in lens], [make(s) if h else [] for s, h in zip(lens, hid)]
-    if kind == "short rows":
-        tables, shared = [t[: len(t) // 2] for t in tables], [t[: len(t) // 3] for t in shared]
+    if kind == "spare blocks":
+        tables, shared = [t + make(16 * (r % 4)) for r, t in enumerate(tables)], [t + make(16 * (r % 3)) if t else t for r, t in enumerate(shared)]
         tables[4] = tables[4] + make(900)
     elif kind == "tuples":
         tables, shared = [tuple(t) for t in tables], [tuple(t) for t in shared]

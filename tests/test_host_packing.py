@@ -56,12 +56,14 @@ def test_what_numpy_refuses_is_refused(tables, shared):
         DM._fill_host(torch.zeros(sum(cuts), dtype=torch.int32), cuts, tables, shared, lens, types, counts[2], 1)
 
 
-def unpacked(lens, hid, tables, shared):
+def unpacked(lens, hid, tables, shared, changes=False):
     """What the native reading lays out one behind the other, as lists: K/V-cached rows, lengths, types, and the rows of both tables."""
-    read = DM._read_lists(lens, hid, tables, shared, len(lens))
+    read = DM._read_lists(lens, hid, tables, shared, len(lens), 16)
     if read is None:
         return None
-    m_lens, counts, (n_own, n_shared), packed = read
+    m_lens, counts, (n_own, n_shared, too_long), packed = read
+    if not changes:
+        assert too_long == DM._first_too_long(m_lens, np.array(hid), tables, shared, 16)
     b, n_kv = len(m_lens), len(m_lens) - counts[0]
     rows = np.frombuffer(packed, np.int64, n_kv)
     words = np.frombuffer(packed, np.int32)[2 * n_kv:]
@@ -96,7 +98,7 @@ def test_lists_are_read_as_they_are(hid, row):
     ([1, 2], [True, False], [[1], [2]], [None, []]), ([1, True], [True, False], [[1], [2]], [[1], []]),
 ])
 def test_what_is_not_plain_is_left_to_numpy(lens, hid, tables, shared):
-    assert DM._read_lists(lens, hid, tables, shared, 2) is None
+    assert DM._read_lists(lens, hid, tables, shared, 2, 16) is None
 
 
 @needs_host_library
@@ -125,7 +127,7 @@ def test_tables_that_change_while_they_are_read():
     read = 0
     try:
         for _ in range(3000):
-            got = unpacked([5] * b, [r % 2 == 0 for r in range(b)], tables, shared)
+            got = unpacked([5] * b, [r % 2 == 0 for r in range(b)], tables, shared, changes=True)
             if got is None:   # a shared table wider than all private ones
                 continue
             read += 1
@@ -165,3 +167,23 @@ def test_a_table_that_grows_during_the_call_stays_inside_the_buffer(monkeypatch)
     DM.expand_decode_metadata([20, 40], [True, False], tables, shared, 16, "cpu")
     assert (buffers[0][-guard:] == -99).all()
     assert called == [[[1, 2], [3, 4, 5]]]
+
+
+# one token more than there is room for: in the private table of either kind of request, in the shared one, in an empty or missing
+# one; rows that numpy reads as well as plain ones.  Refused before anything is launched or copied.
+@pytest.mark.parametrize("lens,hid,tables,shared,which", [
+    ([100], [True], [[1]], [[2]], 0), ([16, 17], [False, False], [[1], [2]], [[], []], 1),
+    ([16, 33], [False, True], [[1], [2, 3]], [[], [4, 5, 6]], 1), ([33], [True], [[1, 2, 3]], [[4, 5]], 0),
+    ([1, 1], [True, False], [[1], []], [[2], []], 1), ([5, 33, 40], [True, True, False], [[1], [2, 3], [4]], [[1], [2, 3], []], 1),
+    ([1, 1], [False, True], [[1], [2]], [[]], 1),
+])
+@pytest.mark.parametrize("plain", [True, False])
+def test_requests_longer_than_their_tables_are_refused(monkeypatch, lens, hid, tables, shared, which, plain):
+    if not plain:
+        tables = [np.array(t, dtype=np.int32) for t in tables]
+    monkeypatch.setattr(N, "lib", None)
+    with pytest.raises(ValueError, match=f"request {which} has {lens[which]} tokens"):
+        DM.expand_decode_metadata(lens, hid, tables, shared, 16, "cpu")
+    from apt_serve_b200.metadata import build_decode_metadata
+    with pytest.raises(IndexError):
+        build_decode_metadata(lens, hid, tables, shared, 16)
