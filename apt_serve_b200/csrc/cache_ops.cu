@@ -408,27 +408,42 @@ struct CacheToHiddenJobs {
   }
 };
 
-// Rows of the decode batch's gathered input, each written once: which row of the cache or of the step's input it is, or neither, stands
-// in a map that this kernel leaves.
-constexpr int64_t kRowOfNothing = -1;   // below it: -2 - row of the step's input; from 0 on: slot of the cache
-constexpr int kMapThreads = 1024;
+// Rows of the decode batch's gathered input, each written once: where each comes from stands in a map that these two kernels leave.
+// The sources are numbered so that the largest is the one that counts, as the operations come one after the other: nothing, the
+// rows of the step's input, the slots of the cache.  (One CTA that went through the map three times in order took
+// 4.5 us for 2 700 rows, but 0.8 for every 1 024 more: 100 000 rows of 768 in fp16 228 us where the three operations take 169.)
+constexpr int64_t kRowOfNothing = -1;   // from 0 on: row of the step's input; from n_new on: n_new + slot of the cache
+constexpr int kMapThreads = 256;
+inline unsigned map_grid(int64_t n) {
+  const int64_t grid = (n + kMapThreads - 1) / kMapThreads, cap = (int64_t)sm_count() * 8;
+  return (unsigned)(grid < cap ? grid : cap);
+}
+__global__ void __launch_bounds__(kMapThreads)
+row_map_fill_kernel(int64_t* map, int64_t rows) {
+  chain_wait();
+  chain_next();
+  for (int64_t i = (int64_t)blockIdx.x * kMapThreads + threadIdx.x; i < rows; i += (int64_t)gridDim.x * kMapThreads) map[i] = kRowOfNothing;
+}
 __global__ void __launch_bounds__(kMapThreads)
 row_map_kernel(int64_t* map, const int64_t* slot_mapping, const int64_t* new_rows, int64_t n_new, const int64_t* cached_rows, int64_t n_cached,
                int64_t rows) {
   chain_wait();
   chain_next();
-  for (int64_t i = threadIdx.x; i < rows; i += kMapThreads) map[i] = kRowOfNothing;
-  __syncthreads();
-  for (int64_t i = threadIdx.x; i < n_new; i += kMapThreads) {
-    const int64_t t = new_rows[i] < 0 ? new_rows[i] + rows : new_rows[i];
-    if (t >= 0 && t < rows) map[t] = -2 - i;
-  }
-  __syncthreads();   // cached rows after the new ones, as the two operations come
-  for (int64_t i = threadIdx.x; i < n_cached; i += kMapThreads) {
-    const int64_t t = cached_rows[i];
+  for (int64_t i = (int64_t)blockIdx.x * kMapThreads + threadIdx.x; i < n_new + n_cached; i += (int64_t)gridDim.x * kMapThreads) {
+    int64_t t, from;
+    if (i < n_new) {
+      t = new_rows[i] < 0 ? new_rows[i] + rows : new_rows[i];
+      from = i;
+    } else {
+      t = cached_rows[i - n_new];
+    }
     if (t < 0 || t >= rows) continue;
-    const int64_t slot = slot_mapping[t];
-    if (slot >= 0) map[t] = slot;
+    if (i >= n_new) {
+      const int64_t slot = slot_mapping[t];
+      if (slot < 0) continue;
+      from = n_new + slot;
+    }
+    atomicMax(reinterpret_cast<long long*>(map + t), (long long)from);
   }
 }
 
@@ -436,13 +451,13 @@ __device__ uint4 g_zero_piece[kBulkMaxPiece / 16];   // never written
 
 struct GatherJobs {
   char* out; const char* hidden; const char* paged_cache; const int64_t* map;
-  int64_t out_stride_b, hidden_stride_b, slot_stride_b, row_bytes; Pieces pc;
+  int64_t n_new, out_stride_b, hidden_stride_b, slot_stride_b, row_bytes; Pieces pc;
   __device__ BulkJob operator()(int64_t job) const {
     const uint32_t piece = (uint32_t)(job % pc.pieces);
     const int64_t t = job / pc.pieces, from = map[t];
     BulkJob j{nullptr, nullptr, nullptr, 0u};
-    j.src = from >= 0 ? paged_cache + from * slot_stride_b + pc.offset(piece)
-                      : from == kRowOfNothing ? reinterpret_cast<const char*>(g_zero_piece) : hidden + (-2 - from) * hidden_stride_b + pc.offset(piece);
+    j.src = from >= n_new ? paged_cache + (from - n_new) * slot_stride_b + pc.offset(piece)
+                          : from >= 0 ? hidden + from * hidden_stride_b + pc.offset(piece) : reinterpret_cast<const char*>(g_zero_piece);
     j.dst0 = out + t * out_stride_b + pc.offset(piece);
     j.bytes = pc.length(piece, (uint32_t)row_bytes);
     return j;
@@ -740,8 +755,9 @@ extern "C" int aps_cache_to_hidden(void* hidden, const void* paged_cache,
 }
 
 // What a zero fill of the gathered input, an indexed write of the step's rows into it and cache_to_hidden leave (three passes over it, two
-// of them over all or most rows): the rows' sources first, then every row once.  What bounds it is the copy of the rows; 12 OPT-13B requests,
-// 2 700 rows: fill 5.6 us, indexed write 4.2 and gather 8.0, in three launches -> 4.5 + 7.2 in two (the whole layer 225 -> 218 us).
+// of them over all or most rows): the rows' sources first, then every row once.  What bounds it is the copy of the rows.  The three
+// operations -> this, rows not in L2: 300 rows of 768 in fp16 15.4 -> 11.3 us, 9 000 27.6 -> 19.5, 100 000 169 -> 143; of 256 elements
+// 17.4 -> 13.3 for 2 700, 138 -> 120 for 100 000; of 5120 31.7 -> 19.5 for 2 700, 625 -> 357 for 100 000.
 extern "C" int aps_gather_hidden_rows(void* out, const void* hidden, const void* paged_cache, const int64_t* slot_mapping,
                                       const int64_t* new_rows, int64_t n_new, const int64_t* cached_rows, int64_t n_cached, int64_t rows,
                                       int hidden_size, int64_t out_stride, int64_t hidden_stride, int64_t slot_stride, int64_t* scratch,
@@ -760,10 +776,13 @@ extern "C" int aps_gather_hidden_rows(void* out, const void* hidden, const void*
   APS_REQUIRE(bulk_ok(vb, (int64_t)hidden_size * es) && aligned_to(scratch, 8), APS_ERR_UNSUPPORTED,
               "gather_hidden_rows: rows and strides in multiples of 16 bytes, rows of 512 at least");
   cudaStream_t cs = (cudaStream_t)stream;
-  int st = launch_chained("row_map_kernel", row_map_kernel, 1, kMapThreads, 0, cs, scratch, slot_mapping, new_rows, n_new, cached_rows, n_cached, rows);
+  int st = launch_chained("row_map_fill_kernel", row_map_fill_kernel, map_grid(rows), kMapThreads, 0, cs, scratch, rows);
   if (st != APS_OK) return st;
+  if (n_new + n_cached > 0 && (st = launch_chained("row_map_kernel", row_map_kernel, map_grid(n_new + n_cached), kMapThreads, 0, cs, scratch, slot_mapping,
+                                                   new_rows, n_new, cached_rows, n_cached, rows)) != APS_OK)
+    return st;
   const Pieces pc = pieces_for((uint64_t)hidden_size * es);
-  const GatherJobs R{(char*)out, (const char*)hidden, (const char*)paged_cache, scratch, out_stride * es, hidden_stride * es,
+  const GatherJobs R{(char*)out, (const char*)hidden, (const char*)paged_cache, scratch, n_new, out_stride * es, hidden_stride * es,
                      slot_stride * es, (int64_t)hidden_size * es, pc};
   return launch_bulk(R, rows * pc.pieces, pc.piece, cs, "gather_hidden_rows (bulk copy)", true);
 }
