@@ -46,6 +46,8 @@ inline int launch_status(const char* what) {
 
 // cache_type of a request that has no usable tables (derive_tables_kernel): it is neither written nor attended.
 constexpr int32_t kCacheTypeNone = INT32_MIN;
+// Of the cache operations' status: an index outside its tensor.
+constexpr int kStatusBadIndex = 2;
 
 // ---- chained launches ----------------------------------------------------------------
 // The kernels of one call run one after the other on the caller's stream, most of them for 5 - 30 us; a plain

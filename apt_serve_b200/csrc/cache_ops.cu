@@ -213,9 +213,9 @@ static_assert(kBulkLook >= 1 && kBulkLook < kBulkStages, "look-ahead must leave 
 constexpr uint32_t kBulkMaxPiece = APS_BULK_MAX_PIECE;   // rows longer than this are moved in equal pieces
 constexpr long long kBulkWaitBudget = 2000000000LL;  // clock cycles before a wait gives up
 
-// Set when a bulk-copy wait ran out (it never should: a bulk load completes unless its
-// address faults); read back by aps_cache_ops_status.
-__device__ int g_copy_status = 0;
+// [0] is set when a bulk-copy wait ran out (it never should: a bulk load completes unless its
+// address faults), [1] when an index of the gather was outside its tensor; read back by aps_cache_ops_status.
+__device__ int g_copy_status[2] = {0, 0};
 
 struct BulkJob { const char* src; char* dst0; char* dst1; uint32_t bytes; };   // bytes == 0: skip
 
@@ -302,7 +302,7 @@ bulk_copy_kernel(const Resolver R, int64_t n_jobs, uint32_t stage_bytes) {
         for (int spins = 0; !done; ++spins) {
           asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-          if (!done && (spins & 255) == 255 && clock64() - t0 > kBulkWaitBudget) { ok = false; g_copy_status = 1; break; }
+          if (!done && (spins & 255) == 255 && clock64() - t0 > kBulkWaitBudget) { ok = false; g_copy_status[0] = 1; break; }
         }
         if (ok) {
           asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(j.dst0), "r"(src), "r"(j.bytes) : "memory");
@@ -437,7 +437,7 @@ row_map_kernel(int64_t* map, const int64_t* slot_mapping, const int64_t* new_row
     } else {
       t = cached_rows[i - n_new];
     }
-    if (t < 0 || t >= rows) continue;
+    if (t < 0 || t >= rows) { g_copy_status[1] = kStatusBadIndex; continue; }
     if (i >= n_new) {
       const int64_t slot = slot_mapping[t];
       if (slot < 0) continue;
@@ -600,10 +600,13 @@ using namespace aps;
 
 extern "C" int aps_cache_ops_status(int* host_status, void* stream) {
   APS_REQUIRE(host_status != nullptr, APS_ERR_NULL_POINTER, "cache_ops_status: null pointer");
-  void* addr = nullptr;
-  APS_CUDA(cudaGetSymbolAddress(&addr, g_copy_status));
-  APS_CUDA(cudaMemcpyAsync(host_status, addr, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  int* addr = nullptr;
+  int words[2] = {0, 0};
+  APS_CUDA(cudaGetSymbolAddress((void**)&addr, g_copy_status));
+  APS_CUDA(cudaMemcpyAsync(words, addr, sizeof(words), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   APS_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  *host_status = words[0] != 0 ? words[0] : words[1];
+  if (words[0] == 0 && words[1] != 0) APS_CUDA(cudaMemsetAsync(addr + 1, 0, sizeof(int), (cudaStream_t)stream));   // reported once
   if (*host_status != 0) return APS_OK;
   const int st = read_metadata_status(host_status, (cudaStream_t)stream);
   return st != APS_OK || *host_status != 0 ? st : read_prefill_status(host_status, (cudaStream_t)stream);

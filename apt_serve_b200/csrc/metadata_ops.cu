@@ -204,7 +204,6 @@ expand_lists_kernel(const MetaLists T, MetaOut O, const int32_t* __restrict__ se
 // pass for a K/V-cached one), and g_metadata_status is set.
 __device__ int g_metadata_status = 0;
 constexpr int kDeriveThreads = 128;
-constexpr int kStatusBadIndex = 2;   // value of the cache-operation status word
 
 __global__ void __launch_bounds__(kDeriveThreads)
 derive_tables_kernel(int32_t* __restrict__ tables, int32_t* __restrict__ cache_type,

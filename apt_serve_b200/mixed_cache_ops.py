@@ -66,7 +66,9 @@ def gather_hidden_rows(hidden_states: torch.Tensor, paged_cache: torch.Tensor, s
                        new_rows: torch.Tensor, cached_rows: torch.Tensor, rows: int) -> torch.Tensor:
     """The decode batch's gathered input (aptserve_opt.py:112-121): ``rows`` zero rows, ``hidden_states`` written at ``new_rows``, then
     ``cache_to_hidden`` at ``cached_rows``.  In one pass where the rows are wide and aligned as a layer's are; the three
-    operations one after the other otherwise (other index types, shapes that broadcast, gradients or transforms)."""
+    operations one after the other otherwise (other index types, shapes that broadcast, gradients or transforms).  The one
+    pass leaves out indices outside the rows, ``attention.raise_on_device_status`` then raises; the indexed write
+    stops the process's GPU context at them."""
     if _gathers(hidden_states, paged_cache, slot_mapping, new_rows, cached_rows, rows):
         dev = N.require_cuda(hidden_states, paged_cache, slot_mapping, new_rows, cached_rows)
         out = torch.empty(rows, hidden_states.shape[1], device=dev, dtype=hidden_states.dtype)

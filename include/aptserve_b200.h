@@ -107,8 +107,10 @@ int aps_cache_to_hidden(void* hidden, const void* paged_cache,
  * The gathered input of a decode batch's K/V projection in one pass: what the zero fill (opt.py:112), the indexed write of the step's
  * rows (opt.py:117-118) and cache_to_hidden (opt.py:120) leave in it one after the other.  For every t in [0, rows):
  *   out[t, :] = paged_cache[slot_mapping[t] * slot_stride + ...]  if t is among cached_rows and slot_mapping[t] >= 0,
- *             = hidden[i, :]                                      if t is new_rows[i] (a negative entry counts from the end),
+ *             = hidden[i, :]                                      if t is new_rows[i] (a negative entry counts from the end; the
+ *                                                                 last of several),
  *             = 0                                                 otherwise.
+ * Entries of new_rows and cached_rows that name no row of out are left out, and the status that aps_cache_ops_status reads is set.
  * Rows and strides in multiples of 16 bytes, rows of at least 512 (APS_ERR_UNSUPPORTED otherwise).
  * scratch: int64 [rows] of device memory.
  */
@@ -384,8 +386,8 @@ int aps_reprojection_cycles(const void* workspace, unsigned long long* host_cycl
 
 /*
  * Status of the operations without a workspace on the current device: 0, 1 once a bounded wait on a bulk load of a
- * cache operation ran out (the launch then stopped copying), 2 if aps_derive_private_tables has met an index
- * outside its tensor since the last call that returned 2, or 3 if a bounded wait of aps_prefill_attention has run out
+ * cache operation ran out (the launch then stopped copying), 2 if aps_derive_private_tables or aps_gather_hidden_rows has met
+ * an index outside its tensor since a call that returned 2, or 3 if a bounded wait of aps_prefill_attention has run out
  * (up to 128 rows of a head are then NaN) since the last call that returned 3.  Synchronises `stream`.
  */
 int aps_cache_ops_status(int* host_status, void* stream);

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from apt_serve_b200 import attention as A
 from apt_serve_b200 import mixed_cache_ops as M
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,17 @@ def test_gather_keeps_graphs_and_other_indices():
         assert torch.equal(M.gather_hidden_rows(hidden, cache, slots, rows, cached, 8), want)
     leaf = hidden.clone().requires_grad_()
     assert M.gather_hidden_rows(leaf, cache, slots, at.long(), cached, 8).requires_grad
+
+
+@pytest.mark.parametrize("new,cached", [([3, 8], [0, 1]), ([3, -9], [0, 1]), ([3, 7], [0, 8]), ([3, 7], [-1, 0])])
+def test_indices_outside_the_rows_are_left_out_and_reported(new, cached):
+    cache = torch.randn(2, 4, 16, 1, 256, device="cuda", dtype=torch.float16)
+    hidden, slots = torch.randn(2, 256, device="cuda", dtype=torch.float16), torch.arange(8, device="cuda")
+    index = lambda rows: torch.tensor(rows, device="cuda")
+    A.raise_on_device_status()
+    got = M.gather_hidden_rows(hidden, cache, slots, index(new), index(cached), 8)
+    with pytest.raises(RuntimeError, match="outside its tensors"):
+        A.raise_on_device_status()
+    A.raise_on_device_status()   # said once
+    inside = [i for i, t in enumerate(new) if -8 <= t < 8]
+    assert torch.equal(got, three(hidden[inside], cache, slots, index([new[i] for i in inside]), index([t for t in cached if 0 <= t < 8]), 8))
