@@ -222,12 +222,12 @@ def test_a_step_on_bad_metadata_touches_no_other_request(heads, d, e, dtype, fau
 
 
 # tables as lists that the GPU pads and tables padded on the host; rows with spare blocks, tuples, a wide table of a K/V-cached
-# request, more requests than a round of the fill kernel's CTAs
-@pytest.mark.parametrize("kind", ["plain", "spare blocks", "tuples", "one wide", "many"])
+# request, more requests than there are CTAs (two, then four for each)
+@pytest.mark.parametrize("kind", ["plain", "spare blocks", "tuples", "one wide", "many", "very many"])
 def test_lists_and_padded_tables_agree(kind, monkeypatch):
     from apt_serve_b200 import device_metadata as DM
     rng = np.random.default_rng(5)
-    lens = [int(x) for x in rng.integers(1, 600 if kind != "many" else 40, size=1400 if kind == "many" else 23)]
+    lens = [int(x) for x in rng.integers(1, 40 if "many" in kind else 600, size={"many": 1400, "very many": 4001}.get(kind, 23))]
     hid = [bool(i % 3) for i in range(len(lens))]
     make = lambda s: [int(x) for x in rng.integers(0, 2 ** 20, size=-(-s // 16))]
     tables, shared = [make(s) for s in lens], [make(s) if h else [] for s, h in zip(lens, hid)]
