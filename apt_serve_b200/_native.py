@@ -122,6 +122,8 @@ def host_lib():
         handle.aps_measure_decode_batch.argtypes = [ctypes.py_object] * 3 + [c_int64] + [c_void_p] * 3
         handle.aps_pack_decode_batch.restype = c_int
         handle.aps_pack_decode_batch.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 3 + [c_void_p]
+        handle.aps_first_too_long.restype = c_int64
+        handle.aps_first_too_long.argtypes = [ctypes.py_object] * 2 + [c_void_p] * 2 + [c_int64] * 2
         handle.aps_read_decode_lists.restype = ctypes.py_object
         handle.aps_read_decode_lists.argtypes = [ctypes.py_object] * 4 + [c_int64, c_int64, c_void_p]
         _host_lib = handle

@@ -42,6 +42,11 @@ bool pack_row(PyObject* row, int64_t width, int32_t* out) {
   return true;
 }
 
+// Entries of a list or tuple; -1 for anything else.
+inline int64_t row_size(PyObject* row) {
+  return PyList_CheckExact(row) || PyTuple_CheckExact(row) ? (int64_t)PySequence_Fast_GET_SIZE(row) : -1;
+}
+
 // The entries of a list or tuple.  The integers lie all over the heap: they are asked for ahead of their turn.
 bool read_entries(PyObject* row, int32_t* out) {
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(row);
@@ -104,6 +109,22 @@ extern "C" int aps_measure_decode_batch(PyObject* seq_lens, PyObject* use_hidden
   return 0;
 }
 
+// The first request with more tokens than its private table, or its shared one if it is hidden-cached, has room for, -1 if
+// none has, -2 if the tables are not lists of `batch` lists or tuples (shared ones of K/V-cached requests are not looked at).
+// 256 requests: 4 us, one by one in Python 25.
+extern "C" int64_t aps_first_too_long(PyObject* tables, PyObject* shared_tables, const int32_t* lens, const int32_t* types, int64_t batch,
+                                      int64_t block_size) {
+  if (!PyList_CheckExact(tables) || !PyList_CheckExact(shared_tables) || PyList_GET_SIZE(tables) != batch ||
+      PyList_GET_SIZE(shared_tables) != batch)
+    return -2;
+  for (int64_t r = 0; r < batch; ++r) {
+    const int64_t own = row_size(PyList_GET_ITEM(tables, r)), shared = types[r] != 0 ? row_size(PyList_GET_ITEM(shared_tables, r)) : own;
+    if (own < 0 || shared < 0) return -2;
+    if (lens[r] > (own < shared ? own : shared) * block_size) return r;
+  }
+  return -1;
+}
+
 // The buffer's sections, each a multiple of 32 words: the K/V-cached rows (int64), the private, shared and the reference's
 // tables, lengths, types.  Returns as aps_pack_block_tables does.
 extern "C" int aps_pack_decode_batch(PyObject* tables, PyObject* shared_tables, const int32_t* lens, const int32_t* types,
@@ -151,9 +172,6 @@ extern "C" PyObject* aps_read_decode_lists(PyObject* seq_lens, PyObject* use_hid
   PyObject* const given[4] = {seq_lens, use_hidden, tables, shared_tables};
   for (PyObject* list : given)
     if (!PyList_CheckExact(list) || PyList_GET_SIZE(list) != batch) Py_RETURN_NONE;
-  auto row_size = [](PyObject* row) -> int64_t {
-    return PyList_CheckExact(row) || PyTuple_CheckExact(row) ? (int64_t)PySequence_Fast_GET_SIZE(row) : -1;
-  };
   int64_t n_hidden = 0, width = 0, widest_shared = 0, n_own = 0, n_shared = 0;
   for (int64_t r = 0; r < batch; ++r) {
     PyObject* h = PyList_GET_ITEM(use_hidden, r);

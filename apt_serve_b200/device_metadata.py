@@ -100,8 +100,8 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
 
 def _read_lists(seq_lens, use_hidden, tables, shared_tables, b, block_size):
     """Lengths and counts as ``_measure`` has them, (the entries of the private and of the shared tables, what
-    ``_first_too_long`` says), and the batch as ``aps_read_decode_lists`` lays it out; None unless everything is plain lists that the host library reads and shared tables fit the
-    private ones' width."""
+    ``_first_too_long`` says), and the batch as ``aps_read_decode_lists`` lays it out; None unless everything is plain lists that the
+    host library reads and shared tables fit the private ones' width."""
     lib = N.host_lib()
     if lib is None or not b:
         return None
@@ -115,6 +115,11 @@ def _read_lists(seq_lens, use_hidden, tables, shared_tables, b, block_size):
 
 def _first_too_long(lens, types, tables, shared_tables, block_size):
     """The first request with more tokens than its private table, or its shared one if it is hidden-cached, has room for; -1 if none has."""
+    lib, b = N.host_lib(), len(lens)
+    if lib is not None:
+        r = lib.aps_first_too_long(tables, shared_tables, lens.ctypes.data, types.ctypes.data, b, block_size)
+        if r != -2:
+            return r
     needed = (-(-lens.astype(np.int64) // block_size)).tolist()
     for r, (n, hidden, own) in enumerate(zip(needed, types.tolist(), tables)):
         if n > len(own) or (hidden and (r >= len(shared_tables) or n > len(shared_tables[r]))):

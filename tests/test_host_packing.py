@@ -177,10 +177,14 @@ def test_a_table_that_grows_during_the_call_stays_inside_the_buffer(monkeypatch)
     ([1, 1], [True, False], [[1], []], [[2], []], 1), ([5, 33, 40], [True, True, False], [[1], [2, 3], [4]], [[1], [2, 3], []], 1),
     ([1, 1], [False, True], [[1], [2]], [[]], 1),
 ])
-@pytest.mark.parametrize("plain", [True, False])
-def test_requests_longer_than_their_tables_are_refused(monkeypatch, lens, hid, tables, shared, which, plain):
-    if not plain:
+@pytest.mark.parametrize("rows", ["plain", "numpy rows", "numpy lengths", "no library"])
+def test_requests_longer_than_their_tables_are_refused(monkeypatch, lens, hid, tables, shared, which, rows):
+    if rows == "numpy rows":
         tables = [np.array(t, dtype=np.int32) for t in tables]
+    elif rows == "numpy lengths":
+        lens = [np.int64(s) for s in lens]
+    elif rows == "no library":
+        monkeypatch.setattr(N, "host_lib", lambda: None)
     monkeypatch.setattr(N, "lib", None)
     with pytest.raises(ValueError, match=f"request {which} has {lens[which]} tokens"):
         DM.expand_decode_metadata(lens, hid, tables, shared, 16, "cpu")
