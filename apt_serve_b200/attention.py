@@ -585,9 +585,6 @@ class FlashAttentionMetadata:
                    use_cuda_graph=False)
 
 
-_only_values = N.only_values
-
-
 def _prefill_supported(q, k, v, bounds, scale) -> bool:
     """Whether ``aps_prefill_attention`` takes the packed prompts: 16-bit, head size 64 or 128, rows of back-to-back heads
     with 16-byte aligned rows, of which nothing but the values is wanted, a scale that is positive in fp32."""

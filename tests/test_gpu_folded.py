@@ -244,7 +244,7 @@ def test_chained_step_replays_from_a_cuda_graph():
 @pytest.mark.parametrize("dtype", [F, B])
 @pytest.mark.parametrize("n_hidden", [100, 150])
 def test_wide_slices_of_the_weighted_sums(n_hidden, dtype):
-    """Enough requests for slices of three (the last one of two) and of four 128-column blocks."""
+    """Enough requests for slices of three (the last one of two) and of four 128-column blocks in fp16, of two in bf16."""
     rng = np.random.default_rng(n_hidden)
     lens = [int(x) for x in rng.integers(1, 100, size=n_hidden)]
     w = make_decode_workload(LayerShape("t", 5, 128, 1024, dtype), lens, [True] * n_hidden, seed=3, device="cpu")

@@ -101,6 +101,29 @@ def test_counts_that_disagree_with_the_device_side_batch_write_nothing():
         assert seen[0] != n_tot or seen[1] != n_hid
 
 
+@pytest.mark.parametrize("lens,ctype,n_tot,n_hid", [([20, 7, 33], [1, 0, 1], 60, 60), ([20, 0, 33], [1, 1, 1], 53, 53), ([20, 7, 33], [1, 0, 1], 54, 53)])
+def test_lists_whose_counts_disagree_leave_the_indices_alone(lens, ctype, n_tot, n_hid):
+    """The same for the lists that the GPU pads: the index tensors keep their sentinel (unless the counts agree, the last case), the
+    tables are written."""
+    from apt_serve_b200 import _native as N
+    b, bs, width, sent = 3, 16, 4, -7
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    own, shared = [[1, 2], [3], [4, 5, 6]], [[7, 8], [], [9, 10, 11]]
+    starts = lambda rows: i32([0, *np.cumsum([len(t) for t in rows]).tolist()])
+    given = i32(sum(own, [])), starts(own), i32(sum(shared, [])), starts(shared), i32(lens), i32(ctype)
+    tables = torch.full((3, b, width), sent, dtype=torch.int32, device="cuda")
+    n_kv = n_tot - n_hid
+    out = [torch.full((max(n, 1),), sent, dtype=torch.int64, device="cuda") for n in (n_tot, n_hid, n_hid, n_kv, b, n_tot - b, b, b)]
+    N.check(N.lib().aps_expand_decode_lists(*(t.data_ptr() for t in given), b, width, bs, tables.data_ptr(),
+                                            *(None if i == 3 and n_kv == 0 else t.data_ptr() for i, t in enumerate(out)), n_tot, n_hid,
+                                            N.current_stream(tables.device)))
+    agree = n_kv == 1
+    assert all(bool((t == sent).all()) != agree for t in out)
+    pad = lambda t: t + [0] * (width - len(t))
+    used = [s if h else [] for s, h in zip(shared, ctype)]
+    assert tables.tolist() == [[pad(t) for t in own], [pad(t) for t in used], [pad(s if h else t) for t, s, h in zip(own, used, ctype)]]
+
+
 def test_zero_length_is_refused_on_the_host():
     with pytest.raises(ValueError, match=">= 1"):
         expand_decode_metadata([5, 0], [True, False], [[0], [1]], [[2], []], 16, "cuda")

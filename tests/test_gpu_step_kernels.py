@@ -28,21 +28,36 @@ def test_softmax_units(heads, dtype, lens):
     check(workload(heads, 64, 128, dtype, list(lens), [True] * len(lens)), f"{heads} heads, {len(lens)} requests")
 
 
-# weighted sums: terms in one instruction or one for each, one, two and four turns of accumulators, stages of two and four cache blocks,
-# slices of one to four column blocks (many requests), the last one narrower; lengths around a round of turns and a stage
+def slice_of_the_sums(heads, e, dtype, n, sms=148):
+    """Column blocks per item of the weighted sums that the plan gives n hidden-cached requests (csrc/hidden_attention.cu)."""
+    terms, np_, steps = 2 if dtype == F else 3, -(-heads // 16) * 16, -(-e // 128)
+    turns = lambda s: 4 if 5 * s * np_ <= 256 else 2 if 3 * s * np_ <= 256 else 1
+    fits = lambda s: terms * np_ <= 256 and (terms - 1 + turns(s)) * s * np_ <= 256
+    most = next(s for s in (4, 3, 2, 1) if s == 1 or 2 * s * np_ <= 256)
+    if fits(1) and (fits(2) or 4 * np_ > 256):
+        most = next(s for s in range(most, 0, -1) if all(map(fits, range(2, s + 1))))
+    return next(s for s in range(min(most, steps), 0, -1) if s == 1 or n * -(-steps // s) >= 2 * sms)
+
+
+# weighted sums: terms in one instruction or one for each, one, two and four turns of accumulators, stages of two and four cache blocks;
+# lengths around a round of turns and a stage.  slices: column blocks per item in fp16 and in bf16 (one to four, stacked in bf16 at most two),
+# the last one narrower; 3 in fp16 with 16 padded heads has stages of two blocks and four turns
 @pytest.mark.parametrize("dtype", [F, B])
-@pytest.mark.parametrize("heads,d,e,n", [(16, 64, 384, 0), (20, 64, 384, 0), (48, 32, 384, 0), (64, 32, 384, 0), (72, 64, 256, 0), (100, 32, 256, 0),
-                                         (128, 32, 256, 0), (3, 64, 1152, 150), (20, 32, 1152, 150), (40, 32, 1152, 100), (40, 32, 640, 150)])
-def test_columns_of_the_weighted_sums(heads, d, e, n, dtype):
+@pytest.mark.parametrize("heads,d,e,n,slices", [
+    (16, 64, 384, 0, (1, 1)), (20, 64, 384, 0, (1, 1)), (48, 32, 384, 0, (1, 1)), (64, 32, 384, 0, (1, 1)), (72, 64, 256, 0, (1, 1)),
+    (100, 32, 256, 0, (1, 1)), (128, 32, 256, 0, (1, 1)), (3, 64, 1152, 150, (4, 2)), (20, 32, 1152, 150, (4, 2)), (40, 32, 1152, 100, (2, 2)),
+    (40, 32, 640, 150, (2, 2)), (9, 64, 1280, 59, (3, 2)), (20, 32, 1280, 59, (3, 2)),
+])
+def test_columns_of_the_weighted_sums(heads, d, e, n, slices, dtype):
     lens = [1, 15, 16, 17, 31, 32, 33, 48, 49, 63, 64, 65, 66, 80, 81, 96, 97, 127, 128, 129, 300]
     lens = lens + [1 + 37 * i % 90 for i in range(n)]
+    assert slice_of_the_sums(heads, e, dtype, len(lens), torch.cuda.get_device_properties(0).multi_processor_count) == slices[dtype == B]
     w = workload(heads, d, e, dtype, lens, [True] * len(lens))
-    if n == 0:   # what lies behind the sequences must not be seen
-        rows = O.flat_rows(w.hidden_cache)
-        for r, s in enumerate(lens):
-            if s % 16:
-                last = w.block_tables[r][-1]
-                rows[last * 16 + s % 16: last * 16 + 16] = float("nan")
+    rows = O.flat_rows(w.hidden_cache)   # what lies behind the sequences must not be seen
+    for r, s in enumerate(lens):
+        if s % 16:
+            last = w.block_tables[r][-1]
+            rows[last * 16 + s % 16: last * 16 + 16] = float("nan")
     check(w, f"{heads} heads, {len(lens)} requests")
 
 

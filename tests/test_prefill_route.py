@@ -4,15 +4,15 @@ from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.fx.experimental.proxy_tensor import make_fx
 from torch.utils.flop_counter import FlopCounterMode
 
-from apt_serve_b200.attention import _only_values
+from apt_serve_b200._native import only_values
 
 
 def seen(run):
-    """What ``_only_values`` says inside of a transform."""
+    """What ``only_values`` says inside of a transform."""
     answers = []
 
     def f(x):
-        answers.append(_only_values(x))
+        answers.append(only_values(x))
         return x * 2
     run(f)
     assert answers
@@ -21,14 +21,14 @@ def seen(run):
 
 def test_plain_tensors():
     x = torch.ones(3, requires_grad=True)
-    assert _only_values(torch.ones(3), torch.nn.Parameter(torch.ones(3), requires_grad=False))
-    assert not _only_values(torch.ones(3), x)
+    assert only_values(torch.ones(3), torch.nn.Parameter(torch.ones(3), requires_grad=False))
+    assert not only_values(torch.ones(3), x)
     with torch.no_grad():
-        assert _only_values(torch.ones(3), x, torch.nn.Parameter(torch.ones(3)))
+        assert only_values(torch.ones(3), x, torch.nn.Parameter(torch.ones(3)))
     with torch.inference_mode():
-        assert _only_values(torch.ones(3), x)
+        assert only_values(torch.ones(3), x)
     with torch.device("cpu"):   # a mode that only places new tensors
-        assert _only_values(torch.ones(3))
+        assert only_values(torch.ones(3))
 
 
 def test_transforms_and_traces():
@@ -38,12 +38,12 @@ def test_transforms_and_traces():
         assert seen(lambda f: torch.func.jvp(f, (x,), (x,))) == {False}
         assert seen(lambda f: torch.jit.trace(f, (x,), check_trace=False)) == {False}
         assert seen(lambda f: make_fx(f)(x)) == {False}
-        assert not torch.compile(lambda t: t * 2 + (100 if _only_values(t) else 0), backend="eager")(x).gt(50).any()
+        assert not torch.compile(lambda t: t * 2 + (100 if only_values(t) else 0), backend="eager")(x).gt(50).any()
         with FakeTensorMode():
-            assert not _only_values(torch.ones(3))
+            assert not only_values(torch.ones(3))
         with FlopCounterMode(display=False):
-            assert not _only_values(x)
+            assert not only_values(x)
         with torch.autograd.forward_ad.dual_level():
-            assert not _only_values(torch.autograd.forward_ad.make_dual(x, x))
+            assert not only_values(torch.autograd.forward_ad.make_dual(x, x))
     assert seen(lambda f: torch.func.grad(lambda t: f(t).sum())(x)) == {False}
-    assert _only_values(x)
+    assert only_values(x)
