@@ -781,9 +781,10 @@ extern "C" int aps_gather_hidden_rows(void* out, const void* hidden, const void*
   cudaStream_t cs = (cudaStream_t)stream;
   int st = launch_chained("row_map_fill_kernel", row_map_fill_kernel, map_grid(rows), kMapThreads, 0, cs, scratch, rows);
   if (st != APS_OK) return st;
-  if (n_new + n_cached > 0 && (st = launch_chained("row_map_kernel", row_map_kernel, map_grid(n_new + n_cached), kMapThreads, 0, cs, scratch, slot_mapping,
-                                                   new_rows, n_new, cached_rows, n_cached, rows)) != APS_OK)
-    return st;
+  if (n_new + n_cached > 0)
+    st = launch_chained("row_map_kernel", row_map_kernel, map_grid(n_new + n_cached), kMapThreads, 0, cs, scratch, slot_mapping, new_rows,
+                        n_new, cached_rows, n_cached, rows);
+  if (st != APS_OK) return st;
   const Pieces pc = pieces_for((uint64_t)hidden_size * es);
   const GatherJobs R{(char*)out, (const char*)hidden, (const char*)paged_cache, scratch, n_new, out_stride * es, hidden_stride * es,
                      slot_stride * es, (int64_t)hidden_size * es, pc};

@@ -14,8 +14,8 @@
 // What is left is bound by memory: the rows are read twice (scores, weighted sums), W_k once per 128 requests and W_v once
 // per D requests (128, 64 or 32) of a group.
 // Measured on one B200: a step of 256 requests of an OPT-13B layer, half of them hidden-cached (94.7k rows),
-// 0.86 ms against 8.1 - 9.7 ms with the re-projecting kernel; one rank of eight of an OPT-66B layer, 128
-// requests, 0.47 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.20 ms against 2.5.
+// 0.78 - 0.83 ms (the SM clock under the power cap) against 8.1 - 9.7 with the re-projecting kernel; one rank of eight of an
+// OPT-66B layer, 128 requests, 0.41 - 0.43 ms against 1.6 - 2.0; 24 hidden-cached requests of about 1800 tokens 0.18 ms against 2.5.
 //
 //   step_plan_kernel the plan, and the new tokens' cache rows
 //   fold_kernel      qt[r][h] = W_k,h^T q[r][h]                       tcgen05, M = 128 columns of E
@@ -800,7 +800,7 @@ scores_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
 // Where an item's accumulators lie in its half of the tensor memory.  The cache blocks take turns among n_hi accumulators for the
 // first terms; the rests have theirs.  STACKED: several terms of a block are columns of one instruction's B operand, so that X is read from
 // shared memory once for them (an M128 K16 instruction takes (4096 + 32 N) / 128 cycles: two for the 48 padded heads of an
-// OPT-13B layer 90, one 56).  A column block then has [first 0 | rests | first 1 | first 2 | first 3]: blocks of turn 0 write
+// OPT-13B layer 88, one 56).  A column block then has [first 0 | rests | first 1 | first 2 | first 3]: blocks of turn 0 write
 // the first two, blocks of turn 1 the next two with the weights' terms in the order (rests, first); turns 2 and 3 take an
 // instruction for the first term and one for the rests.  Not stacked: an instruction per term, all rests in one accumulator.
 // Stacked where as many first accumulators fit as without and slices of two column blocks remain (a slice of one reads the
@@ -927,7 +927,8 @@ __device__ __forceinline__ void softmax_units(const Params& p, float (*s_max)[kS
         }
       const int blk = k * kSubs + (lane >> 1);
       if (blk < n_blk) {
-        // A tile begins with a block of turn 0.  The mask lies beside what was read of the plan first (in the L1), and is read here for want of registers.
+        // A tile begins with a block of turn 0.  The mask lies beside what was read of the plan first (in the L1), and is read here
+        // for want of registers.
         int turns;
         asm volatile("ld.global.ca.s32 %0, [%1];" : "=r"(turns) : "l"(&gp->turns));
         const bool turned = (lane >> 1 & turns) == 1;
@@ -1045,7 +1046,8 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   const int np = p.np, e_blocks = p.hidden / 128, slice = gp->slice;
   const int n_slices = (e_blocks + slice - 1) / slice, n_items = n * n_slices;
   if ((int)blockIdx.x >= n_items) { chain_wait(); return; }
-  const uint32_t pblk = probs_block_bytes(NT, np), per_stage = sum_stage_blocks(NT, np, slice), x_bytes = per_stage * slice * 4096, stage_bytes = sum_stage_bytes(NT, np, slice);
+  const uint32_t pblk = probs_block_bytes(NT, np), per_stage = sum_stage_blocks(NT, np, slice), x_bytes = per_stage * slice * 4096,
+                 stage_bytes = sum_stage_bytes(NT, np, slice);
   const int stages = min(kMaxStages, (int)(kRingBytes / stage_bytes));
   const SumColumns cols(NT, np, slice);
   const int n_epilogue = sum_epilogue_warps(slice, np);   // the others only wait
@@ -1176,7 +1178,7 @@ sum_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
           };
           if constexpr (!STACKED) {
             for (int k = 0; k < nb; ++k) {
-              const uint32_t turn = (uint32_t)(b + k) & mask, later = (uint32_t)(b + k) > mask;   // later: its first accumulator has been written before
+              const uint32_t turn = (uint32_t)(b + k) & mask, later = (uint32_t)(b + k) > mask;   // later: the turn's accumulator holds a sum
               for (int col = 0; col < n_col; ++col)
 #pragma unroll
                 for (int i = 0; i < NT; ++i)
@@ -1405,7 +1407,8 @@ unfold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const uint32_t a_lo = desc_lo(ring + rg.stage * stage_bytes, 16), b_lo = a_lo + (16384 >> 4);
         if (stacked) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) tc_mma_cta(tmem, a_lo + k * 2, desc_hi(1024, true), b_lo + k * 2, desc_hi(1024, true), idesc, k > 0 ? 1u : acc);
+          for (int k = 0; k < 4; ++k)
+            tc_mma_cta(tmem, a_lo + k * 2, desc_hi(1024, true), b_lo + k * 2, desc_hi(1024, true), idesc, k > 0 ? 1u : acc);
         } else for (int hh = 0; hh < n_heads; ++hh) {
           uint32_t first = acc;
 #pragma unroll
@@ -1576,7 +1579,8 @@ int launch_group(const Maps& m, Params p, int n_cap, int w_tiles, const HybridCa
     static bool done[64] = {false}, done_apart[64] = {false};
     auto k = sum_kernel<T, true>;
     if (!SumColumns::stack(kTerms<T>, p.np)) k = sum_kernel<T, false>;
-    if ((st = allow_smem(sum_kernel<T, true>, ring, done)) != APS_OK || (st = allow_smem(sum_kernel<T, false>, ring, done_apart)) != APS_OK) return st;
+    if ((st = allow_smem(sum_kernel<T, true>, ring, done)) != APS_OK || (st = allow_smem(sum_kernel<T, false>, ring, done_apart)) != APS_OK)
+      return st;
     if ((st = launch_chained("sum_kernel", k, sm_count(), p.sum_threads, ring, stream, m.x_sum, p)) != APS_OK) return st;
   }
   {
@@ -1708,7 +1712,8 @@ int enqueue_folded_attention(const HybridCall& c, const NewTokenWrite& nw, cudaS
   p.status = ws.plan + kPlanStatus;
   p.heads = s.heads; p.np = l.np; p.head_size = s.head_size; p.hidden = c.hidden_size; p.slabs = c.hidden_size / 64;
   p.block_size = s.block_size; p.max_blocks = s.max_blocks_per_seq; p.n_cap = l.n_cap;
-  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.sum_copiers = kSumCopiers; p.sum_threads = 32 + 32 * (kSumCopiers + sum_epilogue_warps(pa.max_slice, l.np)); p.grid_scores = pa.grid_scores;
+  p.n_hidden_cap = l.n_hidden_cap; p.splits = l.splits; p.unfold_ring = l.unfold_ring; p.grid_scores = pa.grid_scores;
+  p.sum_copiers = kSumCopiers; p.sum_threads = 32 + 32 * (kSumCopiers + sum_epilogue_warps(pa.max_slice, l.np));
   p.query_stride = s.query_stride; p.scale_log2 = s.scale * 1.4426950408889634f;
   p.w_box_rows = hd < 128 ? (int)hd : 128;
   const int w_tiles = (int)((hd + 127) / 128);

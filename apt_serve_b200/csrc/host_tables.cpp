@@ -1,10 +1,10 @@
 // Block tables of a decode batch from the engine's Python lists, padded into the int32 arrays that go to the GPU.
 //
 // The reference pads them in its model runner (additional_designs/worker/aptserve_model_runner.py:601-609).
-// Nineteen thousand list elements (256 OPT-13B requests) cost numpy 30 ns each; read through the interpreter's own
+// Eighteen thousand list elements (256 OPT-13B requests) cost numpy 30 ns each; read through the interpreter's own
 // list and integer accessors they cost 3.  With one copy to the device and one allocation for the outputs a
 // call of device_metadata.expand_decode_metadata went from 855 to 218 us, and with lengths, types and counts read here too and
-// the tensors cut out of their buffers by one call from 222 to 160.  A library of its own, because this one needs
+// the tensors cut out of their buffers by one call from 222 to 160; read once and left unpadded it takes 120.  A library of its own, because this one needs
 // the Python process it is loaded into; called with the interpreter lock held (ctypes.PyDLL).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>

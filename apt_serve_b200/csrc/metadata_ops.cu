@@ -6,18 +6,21 @@
 // (:613-648) and everything is shipped to the device (and broadcast to the
 // tensor-parallel workers) every step -- about 2 x 8 bytes per cached hidden token.
 // Here the host ships the two block tables, the sequence lengths and the cache types
-// (a few bytes per 16 tokens) and two small kernels expand them in place:
+// (a few bytes per 16 tokens) and small kernels expand them in place.  Tables that the host has padded:
 //   layout_kernel   one CTA: prefix sums over the requests -> where each request starts
 //                   in the expanded token space, among the hidden tokens, and its ordinal
 //                   among the K/V-cached / hidden-cached requests;
 //   fill_kernel     one CTA per request: writes the request's entries of all eight tensors.
+// Tables as the engine has them, rows of any length one behind the other:
+//   expand_lists_kernel   pads them and does what the two do, in one launch.
 // Integer work only; results are bit-identical to the host construction.
 //
 // The caller sizes the outputs from its own view of the batch (num_tot_tokens,
 // num_hidden_tokens) and may pass NULL for an output that is empty in that view.  The kernels
-// trust neither: layout_kernel recomputes the four totals from the device-side seq_lens and
-// cache_type, and fill_kernel writes nothing at all unless they equal the caller's claim;
-// every store is bounded by its tensor's capacity besides.
+// trust neither: the four totals are recomputed from the device-side seq_lens and
+// cache_type, and unless they equal the caller's claim no entry of the eight tensors is written
+// (expand_lists_kernel pads the tables all the same).  fill_kernel bounds every store by its tensor's capacity besides;
+// in expand_lists_kernel the totals are what bounds them, and where each row of the lists begins is the caller's word.
 
 #include "aps_common.cuh"
 
@@ -351,7 +354,8 @@ extern "C" int aps_expand_decode_lists(const int32_t* entries, const int32_t* st
               (long long)num_hidden_tokens, batch);
   if (batch == 0) return APS_OK;
   APS_REQUIRE(entries && starts && shared_entries && shared_starts && seq_lens && cache_type && tables && slot_mapping && hidden_holder_upd &&
-                  (num_hidden_tokens == 0 || (slot_mapping_shared && hidden_cache_use_tot && hidden_cache_store_tot && hidden_cache_use_input)) &&
+                  (num_hidden_tokens == 0 ||
+                   (slot_mapping_shared && hidden_cache_use_tot && hidden_cache_store_tot && hidden_cache_use_input)) &&
                   (num_tot_tokens == num_hidden_tokens || kv_cache_use_tot) && (num_tot_tokens == batch || hidden_holder_pull),
               APS_ERR_NULL_POINTER, "expand_decode_lists: null pointer");
   const MetaOut O{slot_mapping, slot_mapping_shared, hidden_cache_use_tot, kv_cache_use_tot,
@@ -359,7 +363,7 @@ extern "C" int aps_expand_decode_lists(const int32_t* entries, const int32_t* st
                   num_tot_tokens, num_hidden_tokens, num_tot_tokens - num_hidden_tokens,
                   batch - (num_tot_tokens - num_hidden_tokens)};
   const int grid = batch < sm_count() * 8 ? batch : sm_count() * 8;
-  expand_lists_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(MetaLists{entries, starts, shared_entries, shared_starts, tables}, O, seq_lens, cache_type,
-                                                              batch, max_blocks_per_seq, block_size);
+  const MetaLists T{entries, starts, shared_entries, shared_starts, tables};
+  expand_lists_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(T, O, seq_lens, cache_type, batch, max_blocks_per_seq, block_size);
   return launch_status("expand_lists_kernel");
 }

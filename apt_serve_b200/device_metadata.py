@@ -5,7 +5,8 @@ index lists of a decode batch with a Python loop over every cached position of e
 hidden-cached request and copies them to the GPU each step
 (additional_designs/worker/aptserve_model_runner.py:515-564, 613-648).  Here the host
 only ships the two block tables, the sequence lengths and the cache types;
-``aps_expand_decode_metadata`` writes the eight tensors on the device, bit-identical
+``aps_expand_decode_lists`` (plain lists) or ``aps_expand_decode_metadata`` (tables padded on
+the host, from rows of any other kind) writes the eight tensors on the device, bit-identical
 to ``metadata.build_decode_metadata``.
 
 ``python -m apt_serve_b200.device_metadata`` times both constructions on configuration 2.
@@ -28,8 +29,9 @@ def expand_decode_metadata(seq_lens: Sequence[int], use_hidden: Sequence[bool],
                            device) -> DecodeMetadata:
     """Same arguments and result as ``metadata.build_decode_metadata``, with the tensors
     created on ``device`` by the expansion kernels.  Host work is O(number of blocks):
-    reading the two block tables (plain lists natively, unpadded).  Nothing waits for the device: one copy from pinned memory and one
-    launch (two for padded tables) on the current stream.  The tensors are sections of three allocations (what came from the host, the tables, the indices).
+    reading the two block tables (plain lists natively and unpadded, at one moment).  Nothing waits for the device: one
+    copy from pinned memory and one launch (two for padded tables) on the current stream.  The tensors are sections of three
+    allocations (what came from the host, the tables, the indices).
     A request with more tokens than its private table has room for, or its shared one if it is hidden-cached, is refused
     (``ValueError``; ``build_decode_metadata`` stops at it with an index error)."""
     dev = torch.device(device)
@@ -134,7 +136,8 @@ def _cuts(sizes, pitch):
 
 def _measure(seq_lens, use_hidden, tables, b):
     """Lengths and types as int32 arrays, and (hidden-cached requests, their tokens, the widest table or 1, the shortest length,
-    the longest): natively for plain lists where the host library has been built."""
+    the longest): natively for plain lists where the host library has been built (lists that come here are those whose shared
+    tables ``_read_lists`` does not take)."""
     lib = N.host_lib()
     if lib is not None and b:
         both = np.empty((2, b), dtype=np.int32)
@@ -152,7 +155,8 @@ def _measure(seq_lens, use_hidden, tables, b):
 
 
 def _fill_host(host, cuts, tables, shared_tables, lens, types, width, n_hidden):
-    """The sections of the buffer that goes to the device."""
+    """The sections of the buffer that goes to the device: natively where the rows are plain, whatever the lengths came as (256 requests
+    46 us, otherwise 76)."""
     lib, b = N.host_lib(), len(lens)
     if lib is not None and lib.aps_pack_decode_batch(tables, shared_tables, lens.ctypes.data, types.ctypes.data, b, width,
                                                      n_hidden, host.data_ptr()) == 0:

@@ -15,11 +15,11 @@ def three(hidden, cache, slots, new_rows, cached, rows):
     return out
 
 
-# rows of one piece and of two (more than 16 KB), too short for the one pass, not aligned; more rows than a CTA and than all CTAs of the map's kernels have threads;
-# rows that nothing is written to, rows of both kinds, slots of -1, indices from the end
+# rows of one piece and of two (more than 16 KB), too short for the one pass, not aligned; more rows than a CTA and than all CTAs of the
+# map's kernels have threads; rows that nothing is written to, rows of both kinds, slots of -1, indices from the end
 @pytest.mark.parametrize("e,dtype,rows,n_new,one_pass", [
-    (256, torch.float16, 3, 1, True), (5120, torch.float16, 700, 12, True), (9216, torch.bfloat16, 65, 5, True), (768, torch.float32, 2500, 40, True),
-    (256, torch.bfloat16, 310000, 700, True),
+    (256, torch.float16, 3, 1, True), (5120, torch.float16, 700, 12, True), (9216, torch.bfloat16, 65, 5, True),
+    (768, torch.float32, 2500, 40, True), (256, torch.bfloat16, 310000, 700, True),
     (128, torch.float16, 90, 7, False), (260, torch.float16, 90, 7, False),
 ])
 @pytest.mark.parametrize("strided", [False, True])

@@ -255,7 +255,8 @@ def test_lists_and_padded_tables_agree(kind, monkeypatch):
     make = lambda s: [int(x) for x in rng.integers(0, 2 ** 20, size=-(-s // 16))]
     tables, shared = [make(s) for s in lens], [make(s) if h else [] for s, h in zip(lens, hid)]
     if kind == "spare blocks":
-        tables, shared = [t + make(16 * (r % 4)) for r, t in enumerate(tables)], [t + make(16 * (r % 3)) if t else t for r, t in enumerate(shared)]
+        tables = [t + make(16 * (r % 4)) for r, t in enumerate(tables)]
+        shared = [t + make(16 * (r % 3)) if t else t for r, t in enumerate(shared)]
         tables[4] = tables[4] + make(900)
     elif kind == "tuples":
         tables, shared = [tuple(t) for t in tables], [tuple(t) for t in shared]
